@@ -125,6 +125,25 @@ __device__ __forceinline__ bool mbarrier_wait_warp(uint64_t *barrier, uint32_t p
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// The same on a shared-window address, for a converged warp that stays converged: every lane polls (one instruction
+// for the warp), nothing but the vote between the polls.
+__device__ __forceinline__ bool mbarrier_wait_uniform(uint32_t barrier, uint32_t parity, uint32_t *status, uint32_t code, uint32_t backoff_ns = 0) {
+    uint64_t start = 0;
+    for (uint32_t spin = 0;; ++spin) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
+                     : "=r"(done) : "r"(barrier), "r"(parity) : "memory");
+        if (__all_sync(0xffffffffu, done != 0)) return true;
+        if (backoff_ns != 0) __nanosleep(backoff_ns);
+        if (spin < WAIT_FAST_SPINS) continue;
+        if (start == 0) start = global_timer_ns();
+        const bool over = global_timer_ns() - start > WAIT_LIMIT_NS || *reinterpret_cast<volatile uint32_t *>(status) != 0;
+        if (__any_sync(0xffffffffu, over)) break;
+    }
+    if ((threadIdx.x & 31) == 0) atomicCAS(status, 0u, code);
+    return false;
+}
+
 // ---- TMA ---------------------------------------------------------------------------------
 
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
