@@ -125,15 +125,20 @@ __device__ __forceinline__ bool mbarrier_wait_warp(uint64_t *barrier, uint32_t p
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
-// The same on a shared-window address, for a converged warp that stays converged: every lane polls (one instruction
-// for the warp), nothing but the vote between the polls.
-__device__ __forceinline__ bool mbarrier_wait_uniform(uint32_t barrier, uint32_t parity, uint32_t *status, uint32_t code, uint32_t backoff_ns = 0) {
+// Waits of a converged warp that stays converged, on shared-window addresses: every lane polls (one instruction for the
+// warp), nothing but the vote between the polls. The second form waits for two barriers, whose polls overlap.
+__device__ __forceinline__ uint32_t mbarrier_poll_u32(uint32_t barrier, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
+                 : "=r"(done) : "r"(barrier), "r"(parity) : "memory");
+    return done;
+}
+__device__ __forceinline__ bool mbarrier_wait_uniform2(uint32_t barrier_a, uint32_t parity_a, uint32_t barrier_b, uint32_t parity_b,
+                                                       uint32_t *status, uint32_t code, uint32_t backoff_ns = 0) {
     uint64_t start = 0;
     for (uint32_t spin = 0;; ++spin) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
-                     : "=r"(done) : "r"(barrier), "r"(parity) : "memory");
-        if (__all_sync(0xffffffffu, done != 0)) return true;
+        const uint32_t a = mbarrier_poll_u32(barrier_a, parity_a), b = barrier_b != barrier_a ? mbarrier_poll_u32(barrier_b, parity_b) : 1u;
+        if (__all_sync(0xffffffffu, (a & b) != 0)) return true;
         if (backoff_ns != 0) __nanosleep(backoff_ns);
         if (spin < WAIT_FAST_SPINS) continue;
         if (start == 0) start = global_timer_ns();
@@ -143,6 +148,38 @@ __device__ __forceinline__ bool mbarrier_wait_uniform(uint32_t barrier, uint32_t
     if ((threadIdx.x & 31) == 0) atomicCAS(status, 0u, code);
     return false;
 }
+__device__ __forceinline__ bool mbarrier_wait_uniform(uint32_t barrier, uint32_t parity, uint32_t *status, uint32_t code, uint32_t backoff_ns = 0) {
+    return mbarrier_wait_uniform2(barrier, parity, barrier, parity, status, code, backoff_ns);
+}
+__device__ __forceinline__ void mbarrier_arrive_u32(uint32_t barrier) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(barrier) : "memory");
+}
+__device__ __forceinline__ void mbarrier_arrive_expect_tx_u32(uint32_t barrier, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(barrier), "r"(bytes) : "memory");
+}
+
+// Programmatic dependent launch: a kernel launched with that attribute may start while the one before it in the stream
+// drains. Nothing that an earlier kernel wrote, reads or will write may be touched before grid_wait() returns (it waits
+// for that kernel's end and its writes); grid_release() lets the next kernel of the stream start its own prologue.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Every kernel that is launched that way calls grid_wait() in all its threads before its first access to global memory,
+// so that the chain of waits reaches back over any number of such launches.
+template <typename... Parameters, typename... Arguments>
+inline cudaError_t launch_overlapped(void (*kernel)(Parameters...), unsigned grid, int threads, int smem_bytes, cudaStream_t stream,
+                                     const Arguments &...arguments) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem_bytes;
+    config.stream = stream;
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Parameters>(arguments)...);
+}
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- TMA ---------------------------------------------------------------------------------
 
@@ -158,6 +195,14 @@ __device__ __forceinline__ void tma_load_2d(void *smem, const CUtensorMap *map, 
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_u32(smem)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(barrier)), "r"(x), "r"(y)
+        : "memory");
+}
+
+// The same by shared-window addresses.
+__device__ __forceinline__ void tma_load_2d_u32(uint32_t smem, const CUtensorMap *map, uint32_t barrier, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(barrier), "r"(x), "r"(y)
         : "memory");
 }
 
@@ -197,6 +242,10 @@ __device__ __forceinline__ void tcgen05_commit(uint64_t *barrier) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      smem_u32(barrier))
                  : "memory");
+}
+
+__device__ __forceinline__ void tcgen05_commit_u32(uint32_t barrier) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barrier) : "memory");
 }
 
 // Shared-memory operand descriptor for a K-major tile in the 128-byte-swizzled canonical
@@ -384,6 +433,13 @@ __device__ __forceinline__ void tma_load_2d_pair(void *smem, const CUtensorMap *
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_u32(smem)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(barrier) & PAIR_LEADER_MASK), "r"(x), "r"(y)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_2d_pair_u32(uint32_t smem, const CUtensorMap *map, uint32_t barrier, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(barrier & PAIR_LEADER_MASK), "r"(x), "r"(y)
         : "memory");
 }
 

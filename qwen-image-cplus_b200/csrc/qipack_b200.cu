@@ -14,6 +14,7 @@
 #include "w4a16_gemv.cuh"
 #include "w4a16_gemv_stream.cuh"
 #include "w4a16_pair_gemm.cuh"
+#include "w4a16_swap_gemm.cuh"
 #include "w4a4_gemm.cuh"
 #include "w4a4_wide_gemm.cuh"
 #include "w4a4_pair_gemm.cuh"
@@ -116,9 +117,9 @@ int launch_w4a16(const void *x_half, const void *codes, const void *scales, cons
     if (const cudaError_t error = configure_once(kernel, T::SMEM_BYTES, configured[device])) return static_cast<int>(error);
     const int tiles = ((shape.m + T::BM - 1) / T::BM) * ((shape.n + BN - 1) / BN);
     const int grid = tiles < sm_count(device) ? tiles : sm_count(device);
-    kernel<<<grid, w4a16::THREADS, T::SMEM_BYTES, stream>>>(map_x, map_codes, static_cast<const __half *>(scales),
-                                                            static_cast<const __half *>(minimums), bias, y, shape);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(kernel, grid, w4a16::THREADS, T::SMEM_BYTES, stream, map_x, map_codes,
+                                      static_cast<const __half *>(scales), static_cast<const __half *>(minimums),
+                                      bias, y, shape));
 }
 
 template <int STAGES>
@@ -131,7 +132,7 @@ int launch_w4a16_pair(const void *x_half, const void *codes, const void *scales,
                   static_cast<uint64_t>(shape.k) * 2, 64, wp::BM, CU_TENSOR_MAP_SWIZZLE_128B))
         return INVALID;
     if (!make_map(&map_codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes, shape.k / 2, shape.n,
-                  static_cast<uint64_t>(shape.k) / 2, 32, wp::BN / 2, CU_TENSOR_MAP_SWIZZLE_NONE))
+                  static_cast<uint64_t>(shape.k) / 2, 128, wp::BN / 2, CU_TENSOR_MAP_SWIZZLE_128B))
         return INVALID;
     auto kernel = wp::gemm_kernel<STAGES>;
     static std::atomic<bool> configured[MAX_DEVICES];
@@ -139,9 +140,122 @@ int launch_w4a16_pair(const void *x_half, const void *codes, const void *scales,
     const int tiles = ((shape.m + 2 * wp::BM - 1) / (2 * wp::BM)) * ((shape.n + wp::BN - 1) / wp::BN);
     const int pairs = sm_count(device) / 2;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);  // the kernel carries __cluster_dims__(2, 1, 1)
-    kernel<<<grid, wp::THREADS, T::SMEM_BYTES, stream>>>(map_x, map_codes, static_cast<const __half *>(scales),
-                                                         static_cast<const __half *>(minimums), bias, y, shape);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(kernel, grid, wp::THREADS, T::SMEM_BYTES, stream, map_x, map_codes,
+                                      static_cast<const __half *>(scales), static_cast<const __half *>(minimums),
+                                      bias, y, shape));
+}
+
+// ---- the exchanged-operand kernel (w4a16_swap_gemm.cuh): its plan for a shape ----------------------------------------
+
+struct SwapSmem {
+    int stages, code_stages, bytes;
+};
+SwapSmem swap_smem(int columns) {
+    namespace ws = w4a16_swap;
+    // At least two chunks of codes; more of them, before more of the activations, as long as four stages of those fit.
+    const int room = 232448 - ws::BARRIER_BYTES - 1024;
+    int code_stages = (room - 4 * ws::stage_bytes(columns)) / ws::CODE_BYTES;
+    code_stages = code_stages < 2 ? 2 : code_stages > ws::MAX_CODE_STAGES ? ws::MAX_CODE_STAGES : code_stages;
+    int stages = (room - code_stages * ws::CODE_BYTES) / ws::stage_bytes(columns);
+    if (stages > ws::MAX_STAGES) stages = ws::MAX_STAGES;
+    // One CTA per SM, always: it takes all of TMEM, and a second would wait for it while its cluster waits for the second.
+    int bytes = ws::smem_bytes(columns, stages, code_stages);
+    if (bytes < 116 * 1024) bytes = 116 * 1024;
+    return {stages, code_stages, bytes};
+}
+
+template <bool PAIRED>
+cudaError_t configure_swap(int device) {
+    static std::atomic<bool> configured[MAX_DEVICES];
+    return configure_once(w4a16_swap::gemm_kernel<PAIRED>, 232448, configured[device]);
+}
+
+void swap_config(cudaLaunchConfig_t &config, cudaLaunchAttribute (&attributes)[2], int ctas, int split, int smem_bytes, cudaStream_t stream) {
+    config = {};
+    config.gridDim = dim3(ctas);
+    config.blockDim = dim3(w4a16_swap::THREADS);
+    config.dynamicSmemBytes = smem_bytes;
+    config.stream = stream;
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = split, attributes[1].val.clusterDim.y = 1, attributes[1].val.clusterDim.z = 1;
+    config.attrs = attributes;
+    config.numAttrs = 2;
+}
+
+// Clusters of `split` CTAs that run at the same time: fewer than SMs / split, because a cluster lies within one GPC. Asked
+// of the driver once per size.
+int resident_clusters(int device, int split) {
+    namespace ws = w4a16_swap;
+    if (split == 1) return sm_count(device);
+    static std::atomic<int> cached[MAX_DEVICES][ws::MAX_SPLIT + 1];
+    int count = cached[device][split].load(std::memory_order_relaxed);
+    if (count == 0) {
+        cudaLaunchConfig_t config;
+        cudaLaunchAttribute attributes[2];
+        swap_config(config, attributes, split, split, 116 * 1024, nullptr);
+        config.attrs = attributes + 1, config.numAttrs = 1;
+        if (configure_swap<true>(device) != cudaSuccess || cudaOccupancyMaxActiveClusters(&count, ws::gemm_kernel<true>, &config) != cudaSuccess || count <= 0) {
+            (void)cudaGetLastError();
+            count = sm_count(device) / (2 * split) > 0 ? sm_count(device) / (2 * split) : 1;
+        }
+        cached[device][split].store(count, std::memory_order_relaxed);
+    }
+    return count;
+}
+
+struct SwapPlan {
+    int columns, split;
+    double us;  // estimated
+};
+
+// Microseconds as measured on B200 with the weights in L2 or streaming from HBM (77 x {12288, 9216} x 3072, 16 x 18432 x
+// 3072, {77, 256} x 3072 x 12288, {256, 1024} rows): a step of 128 inputs costs a CTA 0.25 (its unpack warps) or 0.003
+// per column (its tensor cores and their operand), a tile 4 + 0.006 per column for its start, its first loads and
+// its results, and sharing a tile over a cluster another 0.8 + 0.016 per column.
+SwapPlan plan_w4a16_swap(int m, int n, int k, int device) {
+    namespace ws = w4a16_swap;
+    const int tiles_n = (n + ws::BN - 1) / ws::BN, steps = (k + ws::BK - 1) / ws::BK;
+    SwapPlan best = {0, 0, 1e30};
+    for (int tiles_m = (m + ws::MAX_COLUMNS - 1) / ws::MAX_COLUMNS, most = tiles_m + 8; tiles_m < most; ++tiles_m) {
+        const int columns = ((m + tiles_m - 1) / tiles_m + 15) / 16 * 16;
+        if (tiles_m > 1 && columns < 64) break;
+        const double step = columns * 0.003 > 0.25 ? columns * 0.003 : 0.25;
+        for (int split = 1; split <= ws::MAX_SPLIT && split <= steps; ++split) {
+            const long long tiles = static_cast<long long>(tiles_n) * ((m + columns - 1) / columns);
+            const int resident = resident_clusters(device, split);
+            const long long waves = (tiles + resident - 1) / resident;
+            if (split > 1 && waves > 1) break;
+            const double us = waves * (4.0 + columns * 0.006 + (steps + split - 1) / split * step + (split > 1 ? 0.8 + 0.016 * columns : 0.0));
+            if (us < best.us) best = {columns, split, us};
+        }
+    }
+    return best;
+}
+
+int launch_w4a16_swap(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
+                      void *y, const GemmShape &shape, int columns, int split, cudaStream_t stream, int device) {
+    namespace ws = w4a16_swap;
+    CUtensorMap map_x, map_codes;
+    if (!make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x_half, shape.k, shape.m,
+                  static_cast<uint64_t>(shape.k) * 2, 64, columns, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    if (!make_map(&map_codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes, shape.k / 2, shape.n,
+                  static_cast<uint64_t>(shape.k) / 2, 128, ws::BN, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    const bool paired = ((reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(minimums)) & 3) == 0 && shape.k % 128 == 0;
+    if (const cudaError_t error = paired ? configure_swap<true>(device) : configure_swap<false>(device)) return static_cast<int>(error);
+    const SwapSmem smem = swap_smem(columns);
+    const ws::Plan plan = {columns, split, smem.stages, smem.code_stages};
+    const long long ctas = static_cast<long long>((shape.m + columns - 1) / columns) * ((shape.n + ws::BN - 1) / ws::BN) * split;
+    if (ctas > 0x7fffffffLL) return INVALID;
+    cudaLaunchConfig_t config;
+    cudaLaunchAttribute attributes[2];
+    swap_config(config, attributes, static_cast<int>(ctas), split, smem.bytes, stream);
+    auto kernel = paired ? ws::gemm_kernel<true> : ws::gemm_kernel<false>;
+    return static_cast<int>(cudaLaunchKernelEx(&config, kernel, map_x, map_codes, static_cast<const __half *>(scales),
+                                               static_cast<const __half *>(minimums), bias, y, shape, plan));
 }
 
 template <int BN, int STAGES>
@@ -161,9 +275,9 @@ int launch_w4a4(const void *a_codes, const void *a_scales, const void *w_codes, 
         return static_cast<int>(error);
     const int tiles = ((shape.m + T::BM - 1) / T::BM) * ((shape.n + BN - 1) / BN);
     const int grid = tiles < sm_count(device) ? tiles : sm_count(device);
-    kernel<<<grid, w4a4::THREADS, T::SMEM_BYTES, stream>>>(map_a, map_w, static_cast<const __half *>(a_scales),
-                                                           static_cast<const __half *>(w_scales), bias, y, dots, shape);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(kernel, grid, w4a4::THREADS, T::SMEM_BYTES, stream, map_a, map_w,
+                                      static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
+                                      bias, y, dots, shape));
 }
 
 template <int STAGES>
@@ -183,9 +297,9 @@ int launch_w4a4_wide(const void *a_bytes, const void *a_scales, const void *w_by
         return static_cast<int>(error);
     const int tiles = ((shape.m + w4a4_wide::BM - 1) / w4a4_wide::BM) * ((shape.n + w4a4_wide::BN - 1) / w4a4_wide::BN);
     const int grid = tiles < sm_count(device) ? tiles : sm_count(device);
-    kernel<<<grid, w4a4_wide::THREADS, T::SMEM_BYTES, stream>>>(map_a, map_w, static_cast<const __half *>(a_scales),
-                                                                static_cast<const __half *>(w_scales), bias, y, dots, shape);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(kernel, grid, w4a4_wide::THREADS, T::SMEM_BYTES, stream, map_a, map_w,
+                                      static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
+                                      bias, y, dots, shape));
 }
 
 int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
@@ -210,10 +324,9 @@ int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_by
     const int tiles = ((shape.m + 2 * wp::BM - 1) / (2 * wp::BM)) * ((shape.n + wp::BN - 1) / wp::BN);
     const int pairs = sm_count(device) / 2;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);  // the kernel carries __cluster_dims__(2, 1, 1)
-    kernel<<<grid, wp::THREADS, wp::SMEM_BYTES, stream>>>(map_a, map_w, static_cast<const __half *>(a_scales),
-                                                          static_cast<const __half *>(w_scales), bias, y, dots, shape,
-                                                          outputs);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(kernel, grid, wp::THREADS, wp::SMEM_BYTES, stream, map_a, map_w,
+                                      static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
+                                      bias, y, dots, shape, outputs));
 }
 
 bool output_ok(const void *y, int y_dtype, long long ldy, int n) {
@@ -262,11 +375,21 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
         if (stages >= 1) {
             const int smem_bytes = stages * w4a16::stream_stage_bytes(k) + w4a16::stream_x_bytes(m, k) + 128;
             const int tiles = n / w4a16::STREAM_ROWS, resident = 2 * sm_count(device);
-            w4a16::gemv_stream_kernel<<<tiles < resident ? tiles : resident, w4a16::STREAM_THREADS, smem_bytes, stream>>>(
-                static_cast<const __half *>(x_half), static_cast<const uint8_t *>(codes), static_cast<const __half *>(scales),
-                static_cast<const __half *>(minimums), bias, y, m, n, k, ldy, y_dtype == QI_DTYPE_F16, stages);
-            return static_cast<int>(cudaGetLastError());
+            return static_cast<int>(launch_overlapped(w4a16::gemv_stream_kernel, tiles < resident ? tiles : resident,
+                                      w4a16::STREAM_THREADS, smem_bytes, stream, static_cast<const __half *>(x_half),
+                                      static_cast<const uint8_t *>(codes), static_cast<const __half *>(scales),
+                                      static_cast<const __half *>(minimums), bias, y, m, n, k, ldy,
+                                      y_dtype == QI_DTYPE_F16, stages));
         }
+    }
+    // Longer rows: the exchanged-operand GEMM kernel, whose clusters split K, where its alignments hold (5 x 4096 x 12288:
+    // 12.2 us against 17.2 by the kernel below).
+    if (n % 32 == 0 && output_ok(y, y_dtype, ldy, n)) {
+        const int device = current_device();
+        if (device < 0) return INVALID;
+        const SwapPlan plan = plan_w4a16_swap(m, n, k, device);
+        const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
+        return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, plan.columns, plan.split, stream, device);
     }
     const int quads = (k / 64 + 3) / 4;
     int k_splits = 1;
@@ -274,10 +397,10 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
         if (quads % candidate == 0) { k_splits = candidate; break; }
     const int row_tiles = w4a16::GEMV_WARPS / k_splits;
     const int blocks = (n / 16 + row_tiles - 1) / row_tiles;
-    w4a16::gemv_kernel<<<blocks, w4a16::GEMV_THREADS, 0, stream>>>(
-        static_cast<const __half *>(x_half), static_cast<const uint8_t *>(codes), static_cast<const __half *>(scales),
-        static_cast<const __half *>(minimums), bias, y, m, n, k, ldy, y_dtype == QI_DTYPE_F16, k_splits);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(w4a16::gemv_kernel, blocks, w4a16::GEMV_THREADS, 0, stream,
+                                      static_cast<const __half *>(x_half), static_cast<const uint8_t *>(codes),
+                                      static_cast<const __half *>(scales), static_cast<const __half *>(minimums),
+                                      bias, y, m, n, k, ldy, y_dtype == QI_DTYPE_F16, k_splits));
 }
 
 // Several matrices of one shape against the same activations: launches of up to STREAM_GROUP matrices each.
@@ -329,26 +452,21 @@ int w4a16_gemm(const void *x_half, const void *codes, const void *scales, const 
     if (device < 0) return INVALID;
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
     if (tile == 0) {
-        // Measured on B200 (4096 x {3072, 9216, 12288} x {3072, 12288}, 1024 and 256 rows): per tile the
-        // 256x256 tile on one CTA is about 4 % faster than the same tile on a CTA pair, but a pair wave is
-        // 74 tiles instead of 148, which wastes less of the last wave; below two single-CTA waves the pair
-        // (half the unpacking per CTA, overlapped epilogue) wins outright; 128x128 wins when even pairs
-        // would leave most of the machine idle.
-        const int sms = sm_count(device);
+        // The exchanged-operand kernel's estimate against the pair kernel's: per wave of pairs 0.46 us for 64 inputs of a
+        // 256 x 256 tile (4096 x {3072, 9216} x 3072, 4096 x 3072 x 12288: 22 and 89 us a wave), and 5 us once.
+        const SwapPlan swap = plan_w4a16_swap(m, n, k, device);
         const long long tiles_256 = static_cast<long long>((m + 255) / 256) * ((n + 255) / 256);
-        const long long pairs = sms / 2;
-        const double single_waves = static_cast<double>((tiles_256 + sms - 1) / sms) / 1.04;
-        const double pair_waves = static_cast<double>((tiles_256 + pairs - 1) / pairs) / 2.0;
-        if (tiles_256 >= 2LL * sms) tile = single_waves <= pair_waves ? 4 : 5;
-        else if (tiles_256 * 4 >= sms) tile = 5;
-        else tile = 1;
+        const long long pairs = sm_count(device) / 2;
+        const double pair_us = 5.0 + static_cast<double>((tiles_256 + pairs - 1) / pairs) * (k / 64) * 0.46;
+        if (swap.us < pair_us) return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, swap.columns, swap.split, stream, device);
+        tile = 5;
     }
     switch (tile) {
         case 1: return launch_w4a16<1, 128, 6>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
         case 2: return launch_w4a16<2, 128, 4>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
         case 3: return launch_w4a16<1, 256, 4>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
         case 4: return launch_w4a16<2, 256, 3>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
-        case 5: return launch_w4a16_pair<6>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
+        case 5: return launch_w4a16_pair<5>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
         default: return INVALID;
     }
 }
@@ -498,9 +616,8 @@ int qi_w4a4_widen_codes_ex(const void *codes, void *bytes, long long rows, int k
     const long long chunks = rows * (k / 32);
     const long long blocks = (chunks + 255) / 256;
     if (blocks > 0x7fffffffLL) return INVALID;
-    w4a4_wide::widen_codes_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t *>(codes), static_cast<uint8_t *>(bytes), chunks);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(w4a4_wide::widen_codes_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
+                                              static_cast<const uint8_t *>(codes), static_cast<uint8_t *>(bytes), chunks));
 }
 
 int qi_w4a4_gemm_wide_ex(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,

@@ -119,6 +119,8 @@ __global__ void __launch_bounds__(QUANT_THREADS)
 quantize_activations_kernel(const Source source, uint8_t *__restrict__ codes, __half *__restrict__ scales,
                             uint8_t *__restrict__ bytes, long long chunks) {
     __shared__ __align__(16) float transpose[(QUANT_THREADS / 32) * 2 * REGION];
+    grid_wait();
+    grid_release();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int half_warp = lane >> 4, l = lane & 15;
     float *region = transpose + (warp * 2 + half_warp) * REGION;
@@ -296,6 +298,8 @@ __global__ void __launch_bounds__(QUANT_THREADS)
 quantize_pairs_kernel(const T *__restrict__ x, uint8_t *__restrict__ codes, __half *__restrict__ scales,
                       uint8_t *__restrict__ bytes, long long chunks) {
     __shared__ __align__(16) uint64_t transpose[(QUANT_THREADS / 32) * 2 * PAIR_REGION];
+    grid_wait();
+    grid_release();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int half_warp = lane >> 4, l = lane & 15;
     uint64_t *region = transpose + (warp * 2 + half_warp) * PAIR_REGION;
@@ -420,6 +424,8 @@ quantize_pairs_kernel(const T *__restrict__ x, uint8_t *__restrict__ codes, __ha
 
 __global__ void f32_to_f16_kernel(const float *__restrict__ source, __half *__restrict__ out,
                                   unsigned long long count) {
+    grid_wait();
+    grid_release();
     // eight values per thread when both pointers allow 16-byte accesses, scalar tail otherwise
     const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
     const unsigned long long thread = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -461,27 +467,25 @@ inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, voi
         const int variant = (bytes != nullptr ? 2 : 0) | (codes != nullptr ? 1 : 0);  // 1: codes, 2: bytes, 3: both
         if (x_is_half) {
             const __half *xs = static_cast<const __half *>(x);
-            if (variant == 1) quantize_pairs_kernel<__half, true, false><<<pairs_grid, QUANT_THREADS, 0, stream>>>(xs, c, s, b, chunks);
-            else if (variant == 2) quantize_pairs_kernel<__half, false, true><<<pairs_grid, QUANT_THREADS, 0, stream>>>(xs, c, s, b, chunks);
-            else quantize_pairs_kernel<__half, true, true><<<pairs_grid, QUANT_THREADS, 0, stream>>>(xs, c, s, b, chunks);
+            if (variant == 1) return launch_overlapped(quantize_pairs_kernel<__half, true, false>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
+            else if (variant == 2) return launch_overlapped(quantize_pairs_kernel<__half, false, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
+            else return launch_overlapped(quantize_pairs_kernel<__half, true, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
         } else {
             const float *xs = static_cast<const float *>(x);
-            if (variant == 1) quantize_pairs_kernel<float, true, false><<<pairs_grid, QUANT_THREADS, 0, stream>>>(xs, c, s, b, chunks);
-            else if (variant == 2) quantize_pairs_kernel<float, false, true><<<pairs_grid, QUANT_THREADS, 0, stream>>>(xs, c, s, b, chunks);
-            else quantize_pairs_kernel<float, true, true><<<pairs_grid, QUANT_THREADS, 0, stream>>>(xs, c, s, b, chunks);
+            if (variant == 1) return launch_overlapped(quantize_pairs_kernel<float, true, false>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
+            else if (variant == 2) return launch_overlapped(quantize_pairs_kernel<float, false, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
+            else return launch_overlapped(quantize_pairs_kernel<float, true, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
         }
-        return cudaGetLastError();
     }
     const PlainSource<__half> from_half = {static_cast<const __half *>(x)};
     const PlainSource<float> from_float = {static_cast<const float *>(x)};
     if (bytes != nullptr) {
-        if (x_is_half) quantize_activations_kernel<PlainSource<__half>, true><<<grid, QUANT_THREADS, 0, stream>>>(from_half, c, s, b, chunks);
-        else quantize_activations_kernel<PlainSource<float>, true><<<grid, QUANT_THREADS, 0, stream>>>(from_float, c, s, b, chunks);
+        if (x_is_half) return launch_overlapped(quantize_activations_kernel<PlainSource<__half>, true>, grid, QUANT_THREADS, 0, stream, from_half, c, s, b, chunks);
+        else return launch_overlapped(quantize_activations_kernel<PlainSource<float>, true>, grid, QUANT_THREADS, 0, stream, from_float, c, s, b, chunks);
     } else {
-        if (x_is_half) quantize_activations_kernel<PlainSource<__half>, false><<<grid, QUANT_THREADS, 0, stream>>>(from_half, c, s, b, chunks);
-        else quantize_activations_kernel<PlainSource<float>, false><<<grid, QUANT_THREADS, 0, stream>>>(from_float, c, s, b, chunks);
+        if (x_is_half) return launch_overlapped(quantize_activations_kernel<PlainSource<__half>, false>, grid, QUANT_THREADS, 0, stream, from_half, c, s, b, chunks);
+        else return launch_overlapped(quantize_activations_kernel<PlainSource<float>, false>, grid, QUANT_THREADS, 0, stream, from_float, c, s, b, chunks);
     }
-    return cudaGetLastError();
 }
 
 // producer: 1 = SwiGLU of (first, second), 2 = GELU-tanh of first
@@ -498,13 +502,12 @@ inline cudaError_t launch_fused_quantize(int producer, const float *first, const
     const SwigluSource swiglu = {first, second};
     const GeluSource gelu = {first};
     if (producer == 1) {
-        if (bytes != nullptr) quantize_activations_kernel<SwigluSource, true><<<grid, QUANT_THREADS, 0, stream>>>(swiglu, c, s, b, chunks);
-        else quantize_activations_kernel<SwigluSource, false><<<grid, QUANT_THREADS, 0, stream>>>(swiglu, c, s, b, chunks);
+        if (bytes != nullptr) return launch_overlapped(quantize_activations_kernel<SwigluSource, true>, grid, QUANT_THREADS, 0, stream, swiglu, c, s, b, chunks);
+        else return launch_overlapped(quantize_activations_kernel<SwigluSource, false>, grid, QUANT_THREADS, 0, stream, swiglu, c, s, b, chunks);
     } else {
-        if (bytes != nullptr) quantize_activations_kernel<GeluSource, true><<<grid, QUANT_THREADS, 0, stream>>>(gelu, c, s, b, chunks);
-        else quantize_activations_kernel<GeluSource, false><<<grid, QUANT_THREADS, 0, stream>>>(gelu, c, s, b, chunks);
+        if (bytes != nullptr) return launch_overlapped(quantize_activations_kernel<GeluSource, true>, grid, QUANT_THREADS, 0, stream, gelu, c, s, b, chunks);
+        else return launch_overlapped(quantize_activations_kernel<GeluSource, false>, grid, QUANT_THREADS, 0, stream, gelu, c, s, b, chunks);
     }
-    return cudaGetLastError();
 }
 
 inline cudaError_t launch_f32_to_f16(const float *source, void *out, unsigned long long count, cudaStream_t stream) {
@@ -512,8 +515,7 @@ inline cudaError_t launch_f32_to_f16(const float *source, void *out, unsigned lo
     unsigned long long blocks = (count / 8 + 255) / 256;
     if (blocks < 1) blocks = 1;
     if (blocks > 148ull * 16) blocks = 148ull * 16;
-    f32_to_f16_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(source, static_cast<__half *>(out), count);
-    return cudaGetLastError();
+    return launch_overlapped(f32_to_f16_kernel, static_cast<unsigned>(blocks), 256, 0, stream, source, static_cast<__half *>(out), count);
 }
 
 }  // namespace qi

@@ -57,22 +57,21 @@ struct Tile {
     static_assert((3 * STAGES + 2 * ACC_STAGES) * 8 + 8 <= BARRIER_BYTES, "barrier block");
 };
 
-// 32 packed nibbles (16 bytes) -> 32 fp16 values in input order.
+// WORDS x 8 packed nibbles -> WORDS x 8 fp16 values in input order.
 // Byte b of a word holds codes 2b (low nibble) and 2b + 1. The fast path puts each code into mantissa bits 4..7 of
 // an fp16 with a zero exponent field, i.e. the subnormal code * 2^-20, and lets ONE fused multiply-add per pair do
 // the rest: fma(code * 2^-20, scale * 2^20, minimum) = fp16(code * scale + minimum), the product exact and the
 // sum rounded once like the reference's (gemm.cu:223-230). It needs scale * 2^20 to be an fp16 number: |scale| < 1/16.
 // Any other scale (a NaN included) takes the path that first makes each code an fp16 integer.
-__device__ __forceinline__ void unpack32(const uint4 packed, const __half2 scale2, const __half2 minimum2,
-                                         uint4 (&out)[4]) {
-    const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
-    uint32_t values[16];
+template <int WORDS>
+__device__ __forceinline__ void unpack_words(const uint32_t (&words)[WORDS], const __half2 scale2, const __half2 minimum2,
+                                             uint32_t (&values)[4 * WORDS]) {
     const __half sixteenth = __ushort_as_half(0x2C00), two_to_10 = __ushort_as_half(0x6400);
     if (__hlt(__habs(__low2half(scale2)), sixteenth)) {
         const __half2 up = __half2half2(two_to_10);
         const __half2 scale_up = __hmul2(__hmul2(scale2, up), up);
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
+        for (int w = 0; w < WORDS; ++w) {
             const uint32_t low_nibbles_up = words[w] << 4;
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
@@ -85,7 +84,7 @@ __device__ __forceinline__ void unpack32(const uint4 packed, const __half2 scale
     } else {
         const __half2 offsets = __halves2half2(__ushort_as_half(0x6400), __ushort_as_half(0x5400));  // (1024, 64)
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
+        for (int w = 0; w < WORDS; ++w) {
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 const uint32_t spread = __byte_perm(words[w], 0u, 0x4040u + 0x0101u * b);  // [byte b, 0, byte b, 0]
@@ -96,8 +95,24 @@ __device__ __forceinline__ void unpack32(const uint4 packed, const __half2 scale
             }
         }
     }
+}
+
+__device__ __forceinline__ void unpack32(const uint4 packed, const __half2 scale2, const __half2 minimum2,
+                                         uint4 (&out)[4]) {
+    const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
+    uint32_t values[16];
+    unpack_words<4>(words, scale2, minimum2, values);
 #pragma unroll
     for (int j = 0; j < 4; ++j) out[j] = make_uint4(values[4 * j], values[4 * j + 1], values[4 * j + 2], values[4 * j + 3]);
+}
+
+// A whole group of one row.
+__device__ __forceinline__ void unpack64(const uint4 (&packed)[2], const __half2 scale2, const __half2 minimum2, uint4 (&out)[8]) {
+    const uint32_t words[8] = {packed[0].x, packed[0].y, packed[0].z, packed[0].w, packed[1].x, packed[1].y, packed[1].z, packed[1].w};
+    uint32_t values[32];
+    unpack_words<8>(words, scale2, minimum2, values);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[j] = make_uint4(values[4 * j], values[4 * j + 1], values[4 * j + 2], values[4 * j + 3]);
 }
 
 template <int NUM_M, int BN, int STAGES>
@@ -141,6 +156,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    grid_wait();
+    grid_release();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == PRODUCER_WARP) {

@@ -52,6 +52,8 @@ gemv_kernel(const __half *__restrict__ x, const uint8_t *__restrict__ codes, con
     const int groups = k / 64, quads = (groups + 3) / 4;
     const bool rows_inside = n0 < n;  // n is a multiple of 16
 
+    grid_wait();
+    grid_release();
     float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (rows_inside) {
         const size_t row_a = static_cast<size_t>(n0 + r), row_b = row_a + 8;

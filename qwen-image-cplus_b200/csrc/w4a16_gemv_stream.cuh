@@ -99,6 +99,8 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         for (int s = 0; s < stages; ++s) mbarrier_init(&full[s], 1);
         fence_barrier_init();
     }
+    grid_wait();
+    grid_release();
     // the activations, once per CTA, every eight inputs in the order (0,4,1,5,2,6,3,7) the unpacked pairs have
     uint4 *x_pairs = reinterpret_cast<uint4 *>(smem + static_cast<size_t>(stages) * stage_bytes);  // [m][k / 8]
     for (int item = threadIdx.x; item < m * (k / 8); item += STREAM_THREADS) {

@@ -27,17 +27,20 @@ constexpr int UNPACK_GROUPS = 2;  // groups of eight unpack warps that take the 
 constexpr int THREADS = 256 + UNPACK_GROUPS * 256;
 constexpr int BK = 64;
 constexpr int BM = 128, BN = 256;  // per CTA rows; pair tile is 256 x 256, each CTA unpacks 128 weight rows
-constexpr int PRODUCER_WARP = 0, MMA_WARP = 1, MMA_WARPS = 1, EPILOGUE_WARP0 = 4, UNPACK_WARP0 = 8, UNPACK_WARPS = 8;  // per group
+constexpr int PRODUCER_WARP = 0, MMA_WARP = 1, CODE_WARP = 2, EPILOGUE_WARP0 = 4, UNPACK_WARP0 = 8, UNPACK_WARPS = 8;  // per group
 constexpr int ACC_STAGES = 2;
-constexpr int A_BYTES = BM * 128, B_BYTES = (BN / 2) * 128, C_BYTES = (BN / 2) * 32;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES + C_BYTES;
+constexpr int CODE_BLOCKS = 4, CODE_STAGES = 3;  // K blocks of codes fetched together (128 bytes of a row); chunks in flight
+constexpr int A_BYTES = BM * 128, B_BYTES = (BN / 2) * 128, C_BYTES = (BN / 2) * CODE_BLOCKS * 32;
+constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr uint32_t AHEAD_BACKOFF_NS = 100;  // pause between the polls of the roles that run ahead
 constexpr int BARRIER_BYTES = 512;
 
 template <int STAGES>
 struct Tile {
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BARRIER_BYTES + 1024;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CODE_STAGES * C_BYTES + BARRIER_BYTES + 1024;
     static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA");
-    static_assert((4 * STAGES + 2 * ACC_STAGES + MMA_WARPS) * 8 + 8 <= BARRIER_BYTES, "barrier block");
+    static_assert(STAGES >= CODE_BLOCKS, "a chunk's K blocks wrap around the stages at most once");
+    static_assert((3 * STAGES + 2 * CODE_STAGES + 2 * ACC_STAGES) * 8 + 8 <= BARRIER_BYTES, "barrier block");
 };
 
 template <int STAGES>
@@ -50,8 +53,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     uint8_t *smem_a = smem;
     uint8_t *smem_b = smem_a + STAGES * A_BYTES;
     uint8_t *smem_c = smem_b + STAGES * B_BYTES;
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem_c + STAGES * C_BYTES);  // own code tile
-    uint64_t *a_full = full + STAGES;                                          // the leader's: both CTAs' x tiles
+    uint64_t *code_full = reinterpret_cast<uint64_t *>(smem_c + CODE_STAGES * C_BYTES);  // own codes
+    uint64_t *code_empty = code_full + CODE_STAGES;
+    uint64_t *a_full = code_empty + CODE_STAGES;                                // the leader's: both CTAs' x tiles
     uint64_t *ready = a_full + STAGES;                                         // the leader's: both CTAs' unpack warps
     uint64_t *empty = ready + STAGES;
     uint64_t *tmem_full = empty + STAGES;
@@ -66,10 +70,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            mbarrier_init(&full[s], 1);
             mbarrier_init(&a_full[s], 1);
             mbarrier_init(&ready[s], 2 * UNPACK_WARPS);
             mbarrier_init(&empty[s], 1);
+        }
+        for (int s = 0; s < CODE_STAGES; ++s) {
+            mbarrier_init(&code_full[s], 1);
+            mbarrier_init(&code_empty[s], UNPACK_GROUPS * UNPACK_WARPS);
         }
         for (int a = 0; a < ACC_STAGES; ++a) {
             mbarrier_init(&tmem_full[a], 1);
@@ -85,29 +92,48 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     __syncthreads();
     cluster_sync();  // both CTAs' barriers exist before anything arrives on them from the other side
     tcgen05_fence_after();
+    grid_wait();
+    grid_release();
     const uint32_t leader_ready = map_to_cta(smem_u32(ready), 0), leader_tmem_empty = map_to_cta(smem_u32(tmem_empty), 0);
     const uint32_t tmem_base = *tmem_slot;
 
+    // The single-threaded roles run as converged warps with one elected lane: their addresses and descriptors live in
+    // uniform registers; a diverged thread takes several times as long for the same few instructions.
     if (warp == PRODUCER_WARP) {
-        if (lane == 0) {
-            prefetch_tensormap(&map_x);
-            prefetch_tensormap(&map_codes);
-            uint32_t iteration = 0;
-            bool alive = true;
-            for (int tile = pair; tile < tiles && alive; tile += pairs) {
-                const int m0 = (tile % tiles_m) * (2 * BM) + cta * BM, n0 = (tile / tiles_m) * BN + cta * (BN / 2);
-                for (int kb = 0; kb < k_blocks; ++kb, ++iteration) {
-                    const int s = iteration % STAGES;
-                    const uint32_t phase = (iteration / STAGES) & 1;
-                    if (!mbarrier_wait(&empty[s], phase ^ 1, &g_status, STATUS_WAIT_EMPTY | 0x7000 | s)) { alive = false; break; }
-                    if (cta == 0) mbarrier_arrive_expect_tx(&a_full[s], 2 * A_BYTES);  // both CTAs' x tiles
-                    mbarrier_arrive_expect_tx(&full[s], C_BYTES);
-                    tma_load_2d_pair(smem_a + s * A_BYTES, &map_x, &a_full[s], kb * BK, m0);
-                    tma_load_2d(smem_c + s * C_BYTES, &map_codes, &full[s], kb * (BK / 2), n0);
+        if (elect_one()) prefetch_tensormap(&map_x);
+        const uint32_t a_full_u = smem_u32(a_full), empty_u = smem_u32(empty), a_u = smem_u32(smem_a);
+        uint32_t s = 0, phase = 1;
+        bool alive = true;
+        for (int tile = pair; tile < tiles && alive; tile += pairs) {
+            const int m0 = (tile % tiles_m) * (2 * BM) + cta * BM;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!mbarrier_wait_uniform(empty_u + s * 8, phase, &g_status, STATUS_WAIT_EMPTY | 0x7000 | s, AHEAD_BACKOFF_NS)) { alive = false; break; }
+                if (elect_one()) {
+                    if (cta == 0) mbarrier_arrive_expect_tx_u32(a_full_u + s * 8, 2 * A_BYTES);  // both CTAs' x tiles
+                    tma_load_2d_pair_u32(a_u + s * A_BYTES, &map_x, a_full_u + s * 8, kb * BK, m0);
                 }
+                __syncwarp();
+                if (++s == STAGES) s = 0, phase ^= 1;
             }
         }
-    } else if (warp >= MMA_WARP && warp < MMA_WARP + MMA_WARPS) {
+    } else if (warp == CODE_WARP) {
+        if (elect_one()) prefetch_tensormap(&map_codes);
+        const uint32_t full_u = smem_u32(code_full), empty_u = smem_u32(code_empty), c_u = smem_u32(smem_c);
+        uint32_t s = 0, phase = 1;
+        bool alive = true;
+        for (int tile = pair; tile < tiles && alive; tile += pairs) {
+            const int n0 = (tile / tiles_m) * BN + cta * (BN / 2);
+            for (int kb = 0; kb < k_blocks; kb += CODE_BLOCKS) {
+                if (!mbarrier_wait_uniform(empty_u + s * 8, phase, &g_status, STATUS_WAIT_EMPTY | 0x7300 | s, AHEAD_BACKOFF_NS)) { alive = false; break; }
+                if (elect_one()) {
+                    mbarrier_arrive_expect_tx_u32(full_u + s * 8, C_BYTES);
+                    tma_load_2d_u32(c_u + s * C_BYTES, &map_codes, full_u + s * 8, kb * (BK / 2), n0);
+                }
+                __syncwarp();
+                if (++s == CODE_STAGES) s = 0, phase ^= 1;
+            }
+        }
+    } else if (warp == MMA_WARP) {
         if (cta == 0) {
             constexpr uint32_t idesc = umma_idesc_f16_f32(2 * BM, BN);
             const uint64_t a_first = umma_desc_k_sw128(smem_u32(smem_a)), b_first = umma_desc_k_sw128(smem_u32(smem_b));
@@ -118,8 +144,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
                 if (!mbarrier_wait_uniform(tmem_empty_u + acc * 8, acc_phase, &g_status, STATUS_WAIT_TMEM_EMPTY | 0x7000 | acc)) break;
                 const uint32_t tmem_acc = tmem_base + acc * BN;
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbarrier_wait_uniform(a_full_u + s * 8, phase, &g_status, STATUS_WAIT_FULL | 0x7000 | s) ||
-                        !mbarrier_wait_uniform(ready_u + s * 8, phase, &g_status, STATUS_WAIT_READY | 0x7000 | s)) { alive = false; break; }
+                    if (!mbarrier_wait_uniform2(a_full_u + s * 8, phase, ready_u + s * 8, phase, &g_status, STATUS_WAIT_READY | 0x7000 | s)) { alive = false; break; }
                     tcgen05_fence_after();
                     if (elect_one()) {
                         const uint64_t a_desc = a_first + s * (A_BYTES >> 4), b_desc = b_first + s * (B_BYTES >> 4);
@@ -141,37 +166,49 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         const int unpacker = threadIdx.x - UNPACK_WARP0 * 32;
         const int d = unpacker & 255, group = unpacker >> 8;
         const int half_row = d & 1, local_row = d >> 1;
-        uint32_t iteration = group;
-        int kb = group, tile = pair;
-        int row_global = (tile / tiles_m) * BN + cta * (BN / 2) + local_row;
-        while (true) {
-            if (kb >= k_blocks) {
-                do {
-                    kb -= k_blocks;
-                    tile += pairs;
-                } while (kb >= k_blocks);
-                row_global = (tile / tiles_m) * BN + cta * (BN / 2) + local_row;
-            }
-            if (tile >= tiles) break;
+        const uint32_t code_full_u = smem_u32(code_full), empty_u = smem_u32(empty);
+        uint32_t base = 0, base_phase = 1, chunk = 0, chunk_phase = 0;  // stage of the chunk's first K block; the chunk
+        bool alive = true;
+        for (int tile = pair; tile < tiles && alive; tile += pairs) {
+            const int row_global = (tile / tiles_m) * BN + cta * (BN / 2) + local_row;
             const bool inside = row_global < shape.n;
-            const __half scale = inside ? __ldg(scales + static_cast<size_t>(row_global) * groups + kb) : __ushort_as_half(0);
-            const __half minimum = inside ? __ldg(minimums + static_cast<size_t>(row_global) * groups + kb) : __ushort_as_half(0);
-            const int s = iteration % STAGES;
-            const uint32_t phase = (iteration / STAGES) & 1;
-            if (!mbarrier_wait_warp(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0x7100 | s, lane)) break;
-            const uint8_t *codes_tile = smem_c + s * C_BYTES;
-            uint8_t *b_tile = smem_b + s * B_BYTES;
-            const uint4 packed = *reinterpret_cast<const uint4 *>(codes_tile + local_row * 32 + half_row * 16);
-            uint4 out[4];
-            unpack32(packed, __half2half2(scale), __half2half2(minimum), out);
+            const __half *row_scales = scales + static_cast<size_t>(inside ? row_global : 0) * groups;
+            const __half *row_minimums = minimums + static_cast<size_t>(inside ? row_global : 0) * groups;
+            const __half nothing = __ushort_as_half(0);
+#pragma unroll 1
+            for (int first = 0; first < k_blocks && alive; first += CODE_BLOCKS) {
+                __half scale[CODE_BLOCKS / UNPACK_GROUPS], minimum[CODE_BLOCKS / UNPACK_GROUPS];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<uint4 *>(b_tile + local_row * 128 + (((half_row * 4 + j) ^ (local_row & 7)) << 4)) = out[j];
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbarrier_arrive_cluster(leader_ready + s * 8);
-            iteration += UNPACK_GROUPS;
-            kb += UNPACK_GROUPS;
+                for (int t = 0; t < CODE_BLOCKS / UNPACK_GROUPS; ++t) {
+                    const int kb = first + group + t * UNPACK_GROUPS;
+                    scale[t] = inside && kb < k_blocks ? __ldg(row_scales + kb) : nothing, minimum[t] = inside && kb < k_blocks ? __ldg(row_minimums + kb) : nothing;
+                }
+                if (!mbarrier_wait_uniform(code_full_u + chunk * 8, chunk_phase, &g_status, STATUS_WAIT_FULL | 0x7100 | chunk)) { alive = false; break; }
+                const uint8_t *codes = smem_c + chunk * C_BYTES + local_row * 128;  // 16-byte pieces swizzled by the row
+#pragma unroll
+                for (int t = 0; t < CODE_BLOCKS / UNPACK_GROUPS; ++t) {
+                    const int offset = group + t * UNPACK_GROUPS;
+                    if (first + offset >= k_blocks) break;
+                    const uint4 packed = *reinterpret_cast<const uint4 *>(codes + (((2 * offset + half_row) ^ (local_row & 7)) << 4));
+                    uint32_t s = base + offset, phase = base_phase;
+                    if (s >= STAGES) s -= STAGES, phase ^= 1;
+                    uint4 out[4];
+                    unpack32(packed, __half2half2(scale[t]), __half2half2(minimum[t]), out);
+                    // the tensor cores are done with what the stage held before
+                    if (!mbarrier_wait_uniform(empty_u + s * 8, phase, &g_status, STATUS_WAIT_EMPTY | 0x7100 | s)) { alive = false; break; }
+                    uint8_t *b_row = smem_b + s * B_BYTES + local_row * 128;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4 *>(b_row + (((half_row * 4 + j) ^ (local_row & 7)) << 4)) = out[j];
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbarrier_arrive_cluster(leader_ready + s * 8);
+                }
+                __syncwarp();
+                if (lane == 0) mbarrier_arrive(&code_empty[chunk]);
+                if (++chunk == CODE_STAGES) chunk = 0, chunk_phase ^= 1;
+                base += k_blocks - first < CODE_BLOCKS ? k_blocks - first : CODE_BLOCKS;
+                if (base >= STAGES) base -= STAGES, base_phase ^= 1;
+            }
         }
     } else if (warp >= EPILOGUE_WARP0 && warp < EPILOGUE_WARP0 + 4) {
         const int quadrant = warp & 3;  // TMEM lanes 32*quadrant .. +31 belong to this warp

@@ -112,6 +112,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    grid_wait();
+    grid_release();
     const uint32_t tmem_base = *tmem_slot;
 
     // Warpgroup 0 = control, 1 = widen, 2-3 = fold. The fold warps hold the fp32 accumulators

@@ -538,6 +538,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     __syncthreads();
     cluster_sync();  // both CTAs' barriers exist before anything arrives on them from the other side
     tcgen05_fence_after();
+    grid_wait();
+    grid_release();
     const uint32_t tmem_base = *tmem_slot;
     const View view = {tile_a, tile_b, sw_tile, sa_tile, ring, full, scale_ready, empty, dot_full, dot_empty,
                        tmem_base, cta, pair, pairs, tiles, tiles_m, k_stages, groups};

@@ -61,6 +61,8 @@ struct Tile {
 
 // Packed nibbles -> one E4M3 byte per code, same element order. One thread per 16 input bytes.
 __global__ void widen_codes_kernel(const uint8_t *__restrict__ codes, uint8_t *__restrict__ bytes, long long chunks) {
+    grid_wait();
+    grid_release();
     const long long chunk = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (chunk >= chunks) return;
     const uint4 packed = __ldg(reinterpret_cast<const uint4 *>(codes) + chunk);
@@ -130,6 +132,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    grid_wait();
+    grid_release();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp < FOLD_WARP0) {

@@ -209,6 +209,24 @@ def test_w4a16_gemm_ex_bias_fp16_and_leading_dimension(qi):
     assert qt.max_relative_error(y16.cpu().numpy().astype(np.float32), expected) <= OUTPUT_TOLERANCE
 
 
+@pytest.mark.parametrize("m,n,k", [(9, 32, 64), (16, 160, 192), (17, 4096, 64), (77, 288, 1216), (100, 1024, 3072), (255, 416, 448),
+                                   (257, 96, 1024), (130, 3072, 128), (1, 256, 12288), (8, 480, 4160), (520, 64, 640)])
+def test_w4a16_exchanged_operands_at_the_edges_of_their_tiles(qi, m, n, k):
+    # rows and columns that end inside a tile, an odd number of groups, K split over a cluster and not; few enough rows
+    # (or long enough ones) that the kernel with the weights as first operand takes the shape
+    rng = np.random.default_rng(4000 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x16, bias = qt.make_activations(rng, m, k), qt.make_bias(rng, n)
+    expected = qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        wide = torch.full((m + 1, n + 32), -7.0, dtype=dtype, device="cuda")
+        assert qi.w4a16_gemm_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), wide, code, n + 32, m, n, k) == 0
+        check_status(qi)
+        got = wide.float().cpu().numpy()
+        assert np.all(got[m:] == -7.0) and np.all(got[:, n:] == -7.0)  # nothing outside the matrix
+        assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
+
+
 def test_w4a16_gemm_rejects_what_the_reference_rejects(qi):  # gemm.cu:264
     t = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
     assert qi.w4a16_gemm(t, t, t, t, t, 100, 128, 64) == qi.CUDA_ERROR_INVALID_VALUE
