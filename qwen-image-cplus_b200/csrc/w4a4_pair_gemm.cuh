@@ -25,9 +25,14 @@
 //     some 440 cycles, however deep the pipeline, but not those of other threads. So each team has
 //     two issuing threads (in different warps) that take turns group by group.
 //   * A fold warp copies its 32 x 32 dots of a group with one tcgen05.ld.32x32b.x32 (about 360
-//     B/clk/SM with eight warps; the 16x256b fragment shape reaches 230), computes half of the
-//     group's scale products while the copy is in flight, hands the buffer back and then does
-//     the rest of the arithmetic from registers.
+//     B/clk/SM with eight warps; the 16x256b fragment shape reaches 230), hands the buffer back and
+//     does the arithmetic from registers, as (dot * sa) * sw + acc: dot * sa and sa * sw are both exact
+//     (at most 23 bits), so the bits are the same, and a product just made is a cheaper operand of the
+//     fused multiply-add than three registers that were read long ago (4.1 against 4.5 to 5 cycles
+//     per pair and scheduler for the two instructions).
+//   * The MMA-issuing warps stay converged and elect one lane per slab: descriptors live in uniform
+//     registers, and four MMAs with their commit leave in 150 cycles instead of 400. Both together:
+//     280 -> 262 us at 4096 x 9216 x 3072, 53.1 -> 50.0 at 1024 x 4096 x 4096.
 //   * A wait on a barrier whose phase is complete must cost one try_wait. A polling loop with a
 //     lane-0 / shuffle wrapper around it cost 230 cycles, a try_wait with a vote about 100.
 //   * Integer division costs a warp over a hundred cycles: the per-stage roles walk the
@@ -41,7 +46,7 @@
 // Per CTA (rank 0 = leader issues the MMAs for both), 24 warps:
 //   warp 0      one thread: TMA for own A rows and own B rows
 //   warps 1, 2  stage the scales (sw: the tile's 128 columns; sa: this CTA's 128 rows; four groups per stage)
-//   warps 4-7   leader only, one thread each: tcgen05.mma.cta_group::2 kind::f8f6f4 (two K = 32 steps
+//   warps 4-7   leader only, one elected lane each: tcgen05.mma.cta_group::2 kind::f8f6f4 (two K = 32 steps
 //               per group, two groups per buffer) and the commit that arrives on both CTAs' barriers
 //   warps 8-23  fold this CTA's 128 rows x 128 columns, 32 rows x 32 columns per warp
 //   (warp 3 only gives up its registers: setmaxnreg works on groups of four warps)
@@ -107,6 +112,11 @@ __device__ __forceinline__ void tmem_load_wait_32(uint32_t (&r)[32]) {
         :: "memory");
 }
 
+__device__ __forceinline__ void tcgen05_commit_pair_u32(uint32_t barrier) {
+    const uint16_t both = 3;
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(barrier), "h"(both) : "memory");
+}
+
 constexpr int TEAMS = 2;       // independent fold pipelines, each with its own half of the columns
 constexpr int THREADS = 768;
 constexpr int BM = 128;        // rows per CTA; the pair covers 256
@@ -140,9 +150,9 @@ constexpr uint32_t AHEAD_BACKOFF_NS = 256;
 // warps that are behind included (measured: 588 -> 660 TOP/s on the block when the waiting is done by one
 // lane per warp with a pause between polls; a try_wait with a suspend-time hint instead was slower, 572).
 constexpr uint32_t FOLD_BACKOFF_NS = 200, MMA_BACKOFF_NS = 64;
-// Columns whose scale products sa * sw a fold thread computes while its copy of the dots out of TMEM is still in
-// flight (measured on 4096 x 9216 x 3072: 0 -> 295 us, 16 -> 293 .. 288, more than 16 no better: registers).
-constexpr int HOIST = 16;
+// Columns whose weight scales a fold thread fetches while its copy of the dots out of TMEM is still in flight (100 launches
+// in a row of 4096 x 9216 x 3072: 0 -> 269 us, 8 -> 262, 16 -> 268, 24 -> 267: registers).
+constexpr int HOIST = 8;
 constexpr int SCALE_AHEAD = 3, SCALE_RING = 4;  // stages of scales in flight; ring slots
 
 constexpr int A_HALF_BYTES = BM * 128, B_HALF_BYTES = (BN / 2) * 128;  // one 128-byte-wide slab of a stage
@@ -286,7 +296,7 @@ __device__ __forceinline__ void scale_role(const View &v, const __half *__restri
     cp_async_wait<0>();
 }
 
-// Warps 4-7 of the leader, one thread each. Thread `mine` serves team (mine % TEAMS) and multiplies the
+// Warps 4-7 of the leader. Warp `mine` serves team (mine % TEAMS) and multiplies the
 // slabs (128 bytes of K = two groups) whose running number is (mine / TEAMS) modulo TURNS into that team's TMEM
 // buffers: N = 64 columns per MMA, the slab's first group into the buffer's first 64 columns, the second into the
 // other 64. A slab's number fixes everything else: its pipeline stage (two slabs per stage) and its buffer.
@@ -295,24 +305,27 @@ __device__ __forceinline__ void mma_role(const View &v, uint32_t mine) {
     const int my_tiles = v.pair < v.tiles ? (v.tiles - 1 - v.pair) / v.pairs + 1 : 0;
     const uint32_t total_slabs = static_cast<uint32_t>(my_tiles) * v.groups / 2;  // a slab: 128 bytes of K = two groups
     const uint32_t team = mine % TEAMS, turn = mine / TEAMS;
-    uint64_t *dot_full = v.dot_full + team * BUFFERS, *dot_empty = v.dot_empty + team * BUFFERS;
+    static_assert(TURNS == BUFFERS && K_HALVES == TURNS, "a warp keeps to one buffer and to one half of every stage");
+    const uint32_t full = smem_u32(v.full), dot_full = smem_u32(v.dot_full + team * BUFFERS + turn), dot_empty = smem_u32(v.dot_empty + team * BUFFERS + turn);
+    const uint64_t a_first = umma_desc_k_sw128(smem_u32(v.tile_a) + turn * A_HALF_BYTES);
+    const uint64_t b_first = umma_desc_k_sw128(smem_u32(v.tile_b) + turn * B_HALF_BYTES + team * (B_BOX_ROWS * 128));
+    const uint32_t accumulator = v.tmem_base + (team * BUFFERS + turn) * BUFFER_COLUMNS;
+    uint32_t s = 0, phase = 0, buffer_phase = 1;
     for (uint32_t slab = turn; slab < total_slabs; slab += TURNS) {
-        const uint32_t iteration = slab / K_HALVES, half = slab % K_HALVES;
-        const uint32_t s = iteration % STAGES, phase = (iteration / STAGES) & 1;
-        const uint32_t buffer = slab % BUFFERS, buffer_phase = (slab / BUFFERS) & 1;
-        if (!mbarrier_wait(&v.full[s], phase, &g_status, STATUS_WAIT_FULL | 0x5000 | s, MMA_BACKOFF_NS)) break;
-        if (!mbarrier_wait(&dot_empty[buffer], buffer_phase ^ 1, &g_status, STATUS_WAIT_TMEM_EMPTY | 0x5000 | buffer, MMA_BACKOFF_NS)) break;
+        if (!mbarrier_wait_uniform2(full + s * 8, phase, dot_empty, buffer_phase, &g_status, STATUS_WAIT_TMEM_EMPTY | 0x5000 | s, MMA_BACKOFF_NS)) break;
         tcgen05_fence_after();
-        const uint32_t a_address = smem_u32(v.tile_a + s * A_BYTES + half * A_HALF_BYTES);
-        const uint32_t b_address = smem_u32(v.tile_b + s * B_BYTES + half * B_HALF_BYTES + team * (B_BOX_ROWS * 128));
-        const uint32_t accumulator = v.tmem_base + (team * BUFFERS + buffer) * BUFFER_COLUMNS;
+        if (elect_one()) {
+            const uint64_t a_desc = a_first + s * (A_BYTES >> 4), b_desc = b_first + s * (B_BYTES >> 4);
 #pragma unroll
-        for (int gl = 0; gl < 2; ++gl)
+            for (int gl = 0; gl < 2; ++gl)
 #pragma unroll
-            for (int kk = 0; kk < 2; ++kk)
-                umma_f8_pair(accumulator + gl * TEAM_COLUMNS, umma_desc_k_sw128(a_address + gl * 64 + kk * 32),
-                             umma_desc_k_sw128(b_address + gl * 64 + kk * 32), idesc, kk);
-        tcgen05_commit_pair(&dot_full[buffer]);
+                for (int kk = 0; kk < 2; ++kk)
+                    umma_f8_pair(accumulator + gl * TEAM_COLUMNS, a_desc + gl * 4 + kk * 2, b_desc + gl * 4 + kk * 2, idesc, kk);
+            tcgen05_commit_pair_u32(dot_full);
+        }
+        __syncwarp();
+        buffer_phase ^= 1;
+        if (++s == STAGES) s = 0, phase ^= 1;
     }
 }
 
@@ -367,17 +380,17 @@ __device__ __forceinline__ void fold_role(const View &v, const float *__restrict
                     tcgen05_fence_after();
                 }
                 tmem_load_32x32(tmem_lane + buffer * BUFFER_COLUMNS + (gl & 1) * TEAM_COLUMNS, dots);
-                // while the copy is in flight: the scale products of the first HOIST columns
+                // while the copy is in flight: the weight scales of the first HOIST columns
                 const float scale = lds_f32(sa_base + s * SA_BYTES + gl * 4);
                 const uint64_t sa2 = pack_f32x2(scale, scale);
                 const uint32_t sw_group = sw_stage + gl * BN * 4;
                 uint64_t p[HOIST / 2];
-#pragma unroll
                 ulonglong2 sw4;
+#pragma unroll
                 for (int q = 0; q < HOIST / 4; ++q) {
                     sw4 = lds_pairs(sw_group + 16 * q);
-                    p[2 * q] = mul_f32x2(sa2, sw4.x);
-                    p[2 * q + 1] = mul_f32x2(sa2, sw4.y);
+                    p[2 * q] = sw4.x;
+                    p[2 * q + 1] = sw4.y;
                 }
                 tmem_load_wait_32(dots);
                 if ((gl & 1) == 1) {  // both groups of the slab are in registers or folded: hand the buffer back
@@ -394,14 +407,14 @@ __device__ __forceinline__ void fold_role(const View &v, const float *__restrict
                 }
 #pragma unroll
                 for (int q = 0; q < HOIST / 4; ++q) {
-                    acc[2 * q] = fma_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), p[2 * q], acc[2 * q]);
-                    acc[2 * q + 1] = fma_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), p[2 * q + 1], acc[2 * q + 1]);
+                    acc[2 * q] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), sa2), p[2 * q], acc[2 * q]);
+                    acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), p[2 * q + 1], acc[2 * q + 1]);
                 }
 #pragma unroll
                 for (int q = HOIST / 4; q < COLUMNS / 4; ++q) {
                     sw4 = lds_pairs(sw_group + 16 * q);  // four columns, as two pairs
-                    acc[2 * q] = fma_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), mul_f32x2(sa2, sw4.x), acc[2 * q]);
-                    acc[2 * q + 1] = fma_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), mul_f32x2(sa2, sw4.y), acc[2 * q + 1]);
+                    acc[2 * q] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), sa2), sw4.x, acc[2 * q]);
+                    acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), sw4.y, acc[2 * q + 1]);
                 }
                         }
             __syncwarp();
@@ -509,7 +522,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     uint64_t *dot_empty = dot_full + TEAMS * BUFFERS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(dot_empty + TEAMS * BUFFERS);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t cta = cluster_ctarank();  // 0 = leader
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int tiles_m = (shape.m + 2 * BM - 1) / (2 * BM), tiles_n = (shape.n + BN - 1) / BN;
@@ -539,7 +552,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     cluster_sync();  // both CTAs' barriers exist before anything arrives on them from the other side
     tcgen05_fence_after();
     grid_wait();
-    grid_release();
+
     const uint32_t tmem_base = *tmem_slot;
     const View view = {tile_a, tile_b, sw_tile, sa_tile, ring, full, scale_ready, empty, dot_full, dot_empty,
                        tmem_base, cta, pair, pairs, tiles, tiles_m, k_stages, groups};
@@ -552,7 +565,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             scale_role<false>(view, w_scales, shape.n, lane);
         } else if (warp == SA_WARP) {
             scale_role<true>(view, a_scales, shape.m, lane);
-        } else if (lane == 0 && cta == 0 && warp >= MMA_WARP0 && warp < MMA_WARP0 + MMA_WARPS) {
+        } else if (cta == 0 && warp >= MMA_WARP0 && warp < MMA_WARP0 + MMA_WARPS) {
             mma_role(view, static_cast<uint32_t>(warp - MMA_WARP0));
         }
     } else {
