@@ -302,6 +302,23 @@ int launch_w4a4_wide(const void *a_bytes, const void *a_scales, const void *w_by
                                       bias, y, dots, shape));
 }
 
+// How the pair kernel's tiles cover the output (see w4a4_pair::Tiling): the last, partial wave is cut into the narrowest
+// tiles that still fit one wave.
+w4a4_pair::Tiling w4a4_tiling(int m, int n, int pairs, bool may_narrow) {
+    namespace wp = w4a4_pair;
+    const int tiles_m = (m + 2 * wp::BM - 1) / (2 * wp::BM), tiles_n = (n + wp::BN - 1) / wp::BN, tiles = tiles_m * tiles_n;
+    const int wide = tiles / pairs * pairs;
+    if (may_narrow && wide < tiles) {
+        const int tail_n = wide / tiles_m * wp::BN, tail_m0 = wide % tiles_m;
+        for (int width = 64; width < wp::BN; width += 32) {
+            const int later = n > tail_n + wp::BN ? (n - tail_n - wp::BN + width - 1) / width : 0, sooner = (n - tail_n + width - 1) / width;
+            const int narrow = tail_m0 * later + (tiles_m - tail_m0) * sooner;
+            if (narrow <= pairs) return {wide + narrow, wide, width, tail_m0, tail_n, later, sooner};
+        }
+    }
+    return {tiles, tiles, wp::BN, 0, 0, 0, 0};
+}
+
 int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
                      const float *bias, void *y, int32_t *dots, const GemmShape &shape, cudaStream_t stream, int device,
                      const w4a4_pair::PeerOutputs *peers = nullptr) {
@@ -321,12 +338,12 @@ int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_by
     if (const cudaError_t error = configure_once(kernel, wp::SMEM_BYTES, configured[device][variant]))
         return static_cast<int>(error);
     const wp::PeerOutputs outputs = peers != nullptr ? *peers : wp::PeerOutputs{};
-    const int tiles = ((shape.m + 2 * wp::BM - 1) / (2 * wp::BM)) * ((shape.n + wp::BN - 1) / wp::BN);
     const int pairs = sm_count(device) / 2;
-    const int grid = 2 * (tiles < pairs ? tiles : pairs);  // the kernel carries __cluster_dims__(2, 1, 1)
+    const wp::Tiling tiling = w4a4_tiling(shape.m, shape.n, pairs, variant == 0);
+    const int grid = 2 * (tiling.tiles < pairs ? tiling.tiles : pairs);  // the kernel carries __cluster_dims__(2, 1, 1)
     return static_cast<int>(launch_overlapped(kernel, grid, wp::THREADS, wp::SMEM_BYTES, stream, map_a, map_w,
-                                      static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
-                                      bias, y, dots, shape, outputs));
+                                              static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
+                                              bias, y, dots, shape, outputs, tiling));
 }
 
 bool output_ok(const void *y, int y_dtype, long long ldy, int n) {

@@ -151,8 +151,8 @@ constexpr uint32_t AHEAD_BACKOFF_NS = 256;
 // lane per warp with a pause between polls; a try_wait with a suspend-time hint instead was slower, 572).
 constexpr uint32_t FOLD_BACKOFF_NS = 200, MMA_BACKOFF_NS = 64;
 // Columns whose weight scales a fold thread fetches while its copy of the dots out of TMEM is still in flight (100 launches
-// in a row of 4096 x 9216 x 3072: 0 -> 269 us, 8 -> 262, 16 -> 268, 24 -> 267: registers).
-constexpr int HOIST = 8;
+// in a row of 4096 x 9216 x 3072: 0 -> 265 us, 4 -> 258, 8 -> 272, 16 -> 280, 24 -> 295: registers).
+constexpr int HOIST = 4;
 constexpr int SCALE_AHEAD = 3, SCALE_RING = 4;  // stages of scales in flight; ring slots
 
 constexpr int A_HALF_BYTES = BM * 128, B_HALF_BYTES = (BN / 2) * 128;  // one 128-byte-wide slab of a stage
@@ -178,6 +178,19 @@ struct PeerOutputs {
     int count, first;
 };
 
+// The order of the tiles. Tiles of 256 x 128 walk down the rows first. `wide` of them, a multiple of the pairs that run
+// at once, come first; what would be a last, partly idle wave of them is cut again, into tiles of `width` columns, as many
+// as there are pairs or fewer: 1024 x 4096 outputs are 128 tiles, two waves of 74 pairs, or one wave and 74 tiles of 96
+// columns (K = 4096: 49.9 -> 47.5 us); 4096 x 3072 are 384, five waves and 14, or 28 of 64 (K = 12288: 385 -> 360 us). tail_m0 rows of tiles start their narrow tiles one wide tile later than the others.
+struct Tiling {
+    int tiles, wide, width;
+    int tail_m0, tail_n;       // first column (of the rows of tiles from tail_m0 on) that is left to narrow tiles
+    int tail_later, tail_sooner;  // narrow tiles per row of tiles, for the first tail_m0 rows and for the others
+};
+struct TilePlace {
+    int m_index, n0, width;
+};
+
 // Everything a role needs to find its way around the CTA's shared memory and the problem.
 struct View {
     uint8_t *tile_a, *tile_b;
@@ -186,25 +199,31 @@ struct View {
     uint2 *ring;
     uint64_t *full, *scale_ready, *empty, *dot_full, *dot_empty;
     uint32_t tmem_base, cta;
-    int pair, pairs, tiles, tiles_m, k_stages, groups;
+    int pair, pairs, tiles_m, k_stages, groups;
+    Tiling tiling;
+    __device__ __forceinline__ TilePlace place(int tile) const {
+        if (tile < tiling.wide) return {tile % tiles_m, tile / tiles_m * BN, BN};
+        int narrow = tile - tiling.wide;
+        const int later = tiling.tail_m0 * tiling.tail_later;
+        if (narrow < later) return {narrow % tiling.tail_m0, tiling.tail_n + BN + narrow / tiling.tail_m0 * tiling.width, tiling.width};
+        narrow -= later;
+        const int rows = tiles_m - tiling.tail_m0;
+        return {tiling.tail_m0 + narrow % rows, tiling.tail_n + narrow / rows * tiling.width, tiling.width};
+    }
 };
 
-// A walk over this pair's (tile, stage) sequence without divisions in the loop: integer division
-// costs a warp more than a hundred cycles, and a role that pays several per stage becomes the
-// pace-setter of the whole kernel.
+// A walk over this pair's (tile, stage) sequence. Integer division costs a warp more than a hundred cycles: it happens
+// once per tile, not per stage.
 struct StageWalk {
-    int tile, ks, m_index, n_index;
-    __device__ __forceinline__ StageWalk(const View &v) : tile(v.pair), ks(0), m_index(v.pair % v.tiles_m), n_index(v.pair / v.tiles_m) {}
-    __device__ __forceinline__ bool done(const View &v) const { return tile >= v.tiles; }
+    int tile, ks;
+    TilePlace at;
+    __device__ __forceinline__ StageWalk(const View &v) : tile(v.pair), ks(0), at(v.place(v.pair)) {}
+    __device__ __forceinline__ bool done(const View &v) const { return tile >= v.tiling.tiles; }
     __device__ __forceinline__ void next(const View &v) {
         if (++ks == v.k_stages) {
             ks = 0;
             tile += v.pairs;
-            m_index += v.pairs;  // pairs may exceed tiles_m: reduce by repeated subtraction of the few wraps
-            while (m_index >= v.tiles_m) {
-                m_index -= v.tiles_m;
-                ++n_index;
-            }
+            at = v.place(tile);
         }
     }
 };
@@ -218,8 +237,10 @@ __device__ __forceinline__ void producer_role(const View &v, const CUtensorMap *
     uint32_t s = 0, phase = 0;
     for (StageWalk walk(v); !walk.done(v); walk.next(v)) {
         if (!mbarrier_wait(&v.empty[s], phase ^ 1, &g_status, STATUS_WAIT_EMPTY | 0x5000 | s, AHEAD_BACKOFF_NS)) break;
-        const int m0 = walk.m_index * 2 * BM + static_cast<int>(v.cta) * BM;
-        const int n0 = walk.n_index * BN + static_cast<int>(v.cta) * B_BOX_ROWS;
+        // A tile's columns belong half to one team and half to the other; of a team's columns this CTA holds the first or
+        // the second half (of a narrow tile it loads some rows that nothing reads).
+        const int m0 = walk.at.m_index * 2 * BM + static_cast<int>(v.cta) * BM;
+        const int n0 = walk.at.n0 + static_cast<int>(v.cta) * (walk.at.width / (2 * TEAMS));
         // the leader expects the bytes of both CTAs' loads on its barrier
         if (v.cta == 0) mbarrier_arrive_expect_tx(&v.full[s], 2 * (A_BYTES + B_BYTES));
 #pragma unroll
@@ -229,7 +250,7 @@ __device__ __forceinline__ void producer_role(const View &v, const CUtensorMap *
 #pragma unroll
             for (int team = 0; team < TEAMS; ++team)  // this CTA's half of each team's columns
                 tma_load_2d_pair(v.tile_b + s * B_BYTES + half * B_HALF_BYTES + team * (B_BOX_ROWS * 128), map_w, &v.full[s], k0,
-                                 n0 + team * TEAM_COLUMNS);
+                                 n0 + team * (walk.at.width / TEAMS));
         }
         if (++s == STAGES) s = 0, phase ^= 1;
     }
@@ -246,7 +267,7 @@ __device__ __forceinline__ void scale_role(const View &v, const __half *__restri
     uint32_t ahead_slot = 0;
     auto fetch = [&]() {
         if (!ahead.done(v)) {
-            const int first = ROWS ? ahead.m_index * 2 * BM + static_cast<int>(v.cta) * BM : ahead.n_index * BN;
+            const int first = ROWS ? ahead.at.m_index * 2 * BM + static_cast<int>(v.cta) * BM : ahead.at.n0;
             uint2 *slot = v.ring + ahead_slot * (BN + BM) + RING_OFFSET + lane;
             const __half *source = values + static_cast<size_t>(first + lane) * v.groups + STAGE_GROUPS * ahead.ks;
 #pragma unroll
@@ -301,9 +322,6 @@ __device__ __forceinline__ void scale_role(const View &v, const __half *__restri
 // buffers: N = 64 columns per MMA, the slab's first group into the buffer's first 64 columns, the second into the
 // other 64. A slab's number fixes everything else: its pipeline stage (two slabs per stage) and its buffer.
 __device__ __forceinline__ void mma_role(const View &v, uint32_t mine) {
-    constexpr uint32_t idesc = umma_idesc_e4m3_f32(2 * BM, TEAM_COLUMNS);
-    const int my_tiles = v.pair < v.tiles ? (v.tiles - 1 - v.pair) / v.pairs + 1 : 0;
-    const uint32_t total_slabs = static_cast<uint32_t>(my_tiles) * v.groups / 2;  // a slab: 128 bytes of K = two groups
     const uint32_t team = mine % TEAMS, turn = mine / TEAMS;
     static_assert(TURNS == BUFFERS && K_HALVES == TURNS, "a warp keeps to one buffer and to one half of every stage");
     const uint32_t full = smem_u32(v.full), dot_full = smem_u32(v.dot_full + team * BUFFERS + turn), dot_empty = smem_u32(v.dot_empty + team * BUFFERS + turn);
@@ -311,7 +329,8 @@ __device__ __forceinline__ void mma_role(const View &v, uint32_t mine) {
     const uint64_t b_first = umma_desc_k_sw128(smem_u32(v.tile_b) + turn * B_HALF_BYTES + team * (B_BOX_ROWS * 128));
     const uint32_t accumulator = v.tmem_base + (team * BUFFERS + turn) * BUFFER_COLUMNS;
     uint32_t s = 0, phase = 0, buffer_phase = 1;
-    for (uint32_t slab = turn; slab < total_slabs; slab += TURNS) {
+    for (StageWalk walk(v); !walk.done(v); walk.next(v)) {
+        const uint32_t idesc = umma_idesc_e4m3_f32(2 * BM, 0) | (static_cast<uint32_t>(walk.at.width / TEAMS >> 3) << 17);
         if (!mbarrier_wait_uniform2(full + s * 8, phase, dot_empty, buffer_phase, &g_status, STATUS_WAIT_TMEM_EMPTY | 0x5000 | s, MMA_BACKOFF_NS)) break;
         tcgen05_fence_after();
         if (elect_one()) {
@@ -332,12 +351,165 @@ __device__ __forceinline__ void mma_role(const View &v, uint32_t mine) {
 // Warps 8-23: a warp folds 32 rows x 32 columns of this CTA's half of the tile; a thread owns one
 // row (its TMEM lane) and 32 accumulators.
 // Per slab a warp looks at the barrier once; per group it starts the copy of its 32 x 32 dots into registers (one
-// tcgen05.ld.32x32b.x32, the shape with the highest TMEM read rate), computes the scale products
+// tcgen05.ld.32x32b.x32, the shape with the highest TMEM read rate), fetches the weight scales
 // of its first HOIST columns meanwhile and does the arithmetic once the copy has landed; the buffer goes back
 // when the copy of the slab's second group has landed. The other three warps of its scheduler fill the waits.
 // All lanes need the same weight scales: one 16-byte broadcast load per four columns.
 // The arithmetic is the packed fp32 pair form of  acc = fma(dot, sa * sw, acc): each half is
 // IEEE-rounded exactly like the scalar instruction, so the result has the reference's bits.
+struct FoldState {
+    uint32_t dot_full, leader_dot_empty, sa_base, scale_ready, empty;
+    uint32_t s, phase, group_count;
+    bool failed;
+};
+
+// One tile: WIDTH columns per warp, 32 of a wide tile, 24 or 16 of a narrow one. False when a wait ran out of time.
+// A look at a barrier is one try_wait by every lane; a lane that finds the phase incomplete polls on its own, with
+// pauses (the fold warps are the pace-setters: that path is for the first groups and for errors). A wait that ran
+// out of time sets `failed` in its lane; the warp looks at the flags once per stage.
+template <int WIDTH, bool DUMP_DOTS, bool SCATTER>
+__device__ __forceinline__ bool fold_tile(FoldState &f, int row, int n0, uint32_t tmem_lane, uint32_t sw_base, int k_stages, int groups,
+                                          const float *__restrict__ bias, void *__restrict__ y, const PeerOutputs &peers,
+                                          int32_t *__restrict__ dots_out, const GemmShape &shape, int lane) {
+    uint32_t dots[COLUMNS];  // dots[j] = dot of this thread's row and column j of the warp's
+    uint64_t acc[WIDTH / 2];  // acc[j] = columns 2 j, 2 j + 1
+#pragma unroll
+    for (int j = 0; j < WIDTH / 2; ++j) acc[j] = 0;
+    for (int ks = 0; ks < k_stages; ++ks) {
+        if (__any_sync(0xffffffffu, f.failed)) return false;
+        f.failed = false;
+        if (!try_wait_u32(f.scale_ready + f.s * 8, f.phase)) f.failed = !wait_slow_u32(f.scale_ready + f.s * 8, f.phase, STATUS_WAIT_READY | 0x5000 | f.s, FOLD_BACKOFF_NS);
+        __syncwarp();
+        const uint32_t sw_stage = sw_base + f.s * SW_BYTES;
+#pragma unroll
+        for (int gl = 0; gl < STAGE_GROUPS; ++gl, ++f.group_count) {
+            const uint32_t slab = f.group_count >> 1, buffer = slab % BUFFERS, slab_parity = (slab / BUFFERS) & 1;
+            if ((gl & 1) == 0) {
+                if (!try_wait_u32(f.dot_full + buffer * 8, slab_parity))
+                    f.failed |= !wait_slow_u32(f.dot_full + buffer * 8, slab_parity, STATUS_WAIT_TMEM_FULL | 0x5000 | buffer, FOLD_BACKOFF_NS);
+                __syncwarp();
+                tcgen05_fence_after();
+            }
+            tmem_load_32x32(tmem_lane + buffer * BUFFER_COLUMNS + (gl & 1) * TEAM_COLUMNS, dots);
+            // while the copy is in flight: the weight scales of the first HOIST columns
+            const float scale = lds_f32(f.sa_base + f.s * SA_BYTES + gl * 4);
+            const uint64_t sa2 = pack_f32x2(scale, scale);
+            const uint32_t sw_group = sw_stage + gl * BN * 4;
+            uint64_t p[HOIST / 2];
+            ulonglong2 sw4;
+#pragma unroll
+            for (int q = 0; q < HOIST / 4; ++q) {
+                sw4 = lds_pairs(sw_group + 16 * q);
+                p[2 * q] = sw4.x;
+                p[2 * q + 1] = sw4.y;
+            }
+            tmem_load_wait_32(dots);
+            if ((gl & 1) == 1) {  // both groups of the slab are in registers or folded: hand the buffer back
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbarrier_arrive_cluster(f.leader_dot_empty + buffer * 8);
+            }
+            if (DUMP_DOTS && row < shape.m) {
+#pragma unroll
+                for (int j = 0; j < WIDTH; ++j)
+                    if (n0 + j < shape.n)
+                        dots_out[(static_cast<size_t>(row) * shape.n + n0 + j) * groups + ks * STAGE_GROUPS + gl] =
+                            static_cast<int32_t>(__uint_as_float(dots[j]));
+            }
+#pragma unroll
+            for (int q = 0; q < HOIST / 4; ++q) {
+                acc[2 * q] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), sa2), p[2 * q], acc[2 * q]);
+                acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), p[2 * q + 1], acc[2 * q + 1]);
+            }
+#pragma unroll
+            for (int q = HOIST / 4; q < WIDTH / 4; ++q) {
+                sw4 = lds_pairs(sw_group + 16 * q);  // four columns, as two pairs
+                acc[2 * q] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), sa2), sw4.x, acc[2 * q]);
+                acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), sw4.y, acc[2 * q + 1]);
+            }
+        }
+        __syncwarp();
+        if (lane == 0) arrive_u32(f.empty + f.s * 8);  // done with this stage'f.s scales; its codes were consumed before the dots arrived
+        if (++f.s == STAGES) f.s = 0, f.phase ^= 1;
+    }
+    if (row >= shape.m) return true;
+    // y: this thread's row, WIDTH adjacent columns
+    float out[WIDTH];
+#pragma unroll
+    for (int j = 0; j < WIDTH / 2; ++j) unpack_f32x2(acc[j], out[2 * j], out[2 * j + 1]);
+    if (bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < WIDTH; ++j)
+            if (n0 + j < shape.n) out[j] += __ldg(bias + n0 + j);
+    }
+    const size_t element = static_cast<size_t>(row) * shape.ldy + n0;
+    if constexpr (SCATTER) {
+        // The launcher admits only outputs that take whole 32-byte sectors (32-byte aligned copies,
+        // n a multiple of 32, ldy a multiple of a sector): a warp's 32 columns lie wholly inside the
+        // matrix or wholly outside it (n not a multiple of the tile's 128 columns).
+        if (n0 >= shape.n) return true;
+        if (shape.y_is_half) {
+            uint32_t packed[WIDTH / 2];
+#pragma unroll
+            for (int j = 0; j < WIDTH / 2; ++j) {
+                const __half2 h = __floats2half2_rn(out[2 * j], out[2 * j + 1]);
+                packed[j] = *reinterpret_cast<const uint32_t *>(&h);
+            }
+            int index = peers.first;
+            for (int copy = 0; copy < peers.count; ++copy) {
+                __half *target = static_cast<__half *>(peers.y[index]) + element;
+#pragma unroll
+                for (int j = 0; j < WIDTH / 16; ++j)
+                    st_global_v8(target + 16 * j, *reinterpret_cast<const uint32_t(*)[8]>(&packed[8 * j]));
+                if (++index == peers.count) index = 0;
+            }
+        } else {
+            int index = peers.first;
+            for (int copy = 0; copy < peers.count; ++copy) {
+                float *target = static_cast<float *>(peers.y[index]) + element;
+#pragma unroll
+                for (int j = 0; j < WIDTH / 8; ++j)
+                    st_global_v8(target + 8 * j, *reinterpret_cast<const uint32_t(*)[8]>(&out[8 * j]));
+                if (++index == peers.count) index = 0;
+            }
+        }
+        return true;
+    }
+    // whole 32-byte sectors when the row segment is aligned for them, else 16 bytes at a time (n is a multiple of 32)
+    const bool sectors = WIDTH == 32 && (reinterpret_cast<uintptr_t>(y) & 31) == 0 && shape.ldy % (shape.y_is_half ? 16 : 8) == 0;
+#pragma unroll
+    for (int j = 0; j < WIDTH; j += 16) {
+        if (n0 + j >= shape.n) break;
+        const bool whole = WIDTH - j >= 16 && n0 + j + 16 <= shape.n;
+        if (shape.y_is_half) {
+            uint32_t packed[8];
+#pragma unroll
+            for (int i = 0; i < 8 && j + 2 * i < WIDTH; ++i) {
+                const __half2 h = __floats2half2_rn(out[j + 2 * i], out[j + 2 * i + 1]);
+                packed[i] = *reinterpret_cast<const uint32_t *>(&h);
+            }
+            __half *target = static_cast<__half *>(y) + element + j;
+            if (sectors) {
+                st_global_v8(target, packed);
+            } else {
+                *reinterpret_cast<uint4 *>(target) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                if (whole) *reinterpret_cast<uint4 *>(target + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+            }
+        } else {
+            float *target = static_cast<float *>(y) + element + j;
+            if (sectors) {
+                st_global_v8(target, reinterpret_cast<const uint32_t(&)[8]>(out[j]));
+                st_global_v8(target + 8, reinterpret_cast<const uint32_t(&)[8]>(out[j + 8]));
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16 && j + i < WIDTH; i += 4)
+                    if (i < 8 || whole) *reinterpret_cast<float4 *>(target + i) = make_float4(out[j + i], out[j + i + 1], out[j + i + 2], out[j + i + 3]);
+            }
+        }
+    }
+    return true;
+}
+
 template <bool DUMP_DOTS, bool SCATTER>
 __device__ __forceinline__ void fold_role(const View &v, const float *__restrict__ bias, void *__restrict__ y,
                                           const PeerOutputs &peers,
@@ -345,158 +517,24 @@ __device__ __forceinline__ void fold_role(const View &v, const float *__restrict
     static_assert(COLUMNS == 32, "one tcgen05.ld.32x32b.x32 per warp and group");
     // The hardware ties a warp to the TMEM lanes 32 * (warp % 4); four consecutive warps make one column slice.
     const int quadrant = warp & 3, slice = (warp - FOLD_WARP0) >> 2, team = slice / (TEAM_COLUMNS / COLUMNS);
-    const uint32_t dot_full = smem_u32(v.dot_full + team * BUFFERS);
-    const uint32_t leader_dot_empty = map_to_cta(smem_u32(v.dot_empty + team * BUFFERS), 0);
-    const uint32_t tmem_lane = v.tmem_base + team * BUFFERS * BUFFER_COLUMNS + (slice % (TEAM_COLUMNS / COLUMNS)) * COLUMNS +
-                               (static_cast<uint32_t>(quadrant * 32) << 16);
-    const uint32_t sw_base = smem_u32(v.sw_tile) + slice * COLUMNS * 4;
-    const uint32_t sa_base = smem_u32(v.sa_tile) + (quadrant * 32 + lane) * 16;
-    const uint32_t scale_ready = smem_u32(v.scale_ready), empty = smem_u32(v.empty);
-    uint32_t dots[COLUMNS];  // dots[j] = dot of this thread's row and column j of the warp's 32
-    // A look at a barrier is one try_wait by every lane; a lane that finds the phase incomplete polls on its own, with
-    // pauses (the fold warps are the pace-setters: that path is for the first groups and for errors). A wait that ran
-    // out of time sets `failed` in its lane; the warp looks at the flags once per stage.
-    bool alive = true, failed = false;
-    uint32_t s = 0, phase = 0, group_count = 0;
-    for (int tile = v.pair; tile < v.tiles && alive; tile += v.pairs) {
-        const int row = (tile % v.tiles_m) * 2 * BM + static_cast<int>(v.cta) * BM + quadrant * 32 + lane;
-        const int n0 = (tile / v.tiles_m) * BN + slice * COLUMNS;
-        uint64_t acc[COLUMNS / 2];  // acc[j] = columns 2 j, 2 j + 1
-#pragma unroll
-        for (int j = 0; j < COLUMNS / 2; ++j) acc[j] = 0;
-        for (int ks = 0; ks < v.k_stages && alive; ++ks) {
-            if (__any_sync(0xffffffffu, failed)) { alive = false; break; }
-            failed = false;
-            if (!try_wait_u32(scale_ready + s * 8, phase)) failed = !wait_slow_u32(scale_ready + s * 8, phase, STATUS_WAIT_READY | 0x5000 | s, FOLD_BACKOFF_NS);
-            __syncwarp();
-            const uint32_t sw_stage = sw_base + s * SW_BYTES;
-#pragma unroll
-            for (int gl = 0; gl < STAGE_GROUPS; ++gl, ++group_count) {
-                const uint32_t slab = group_count >> 1, buffer = slab % BUFFERS, slab_parity = (slab / BUFFERS) & 1;
-                if ((gl & 1) == 0) {
-                    if (!try_wait_u32(dot_full + buffer * 8, slab_parity))
-                        failed |= !wait_slow_u32(dot_full + buffer * 8, slab_parity, STATUS_WAIT_TMEM_FULL | 0x5000 | buffer, FOLD_BACKOFF_NS);
-                    __syncwarp();
-                    tcgen05_fence_after();
-                }
-                tmem_load_32x32(tmem_lane + buffer * BUFFER_COLUMNS + (gl & 1) * TEAM_COLUMNS, dots);
-                // while the copy is in flight: the weight scales of the first HOIST columns
-                const float scale = lds_f32(sa_base + s * SA_BYTES + gl * 4);
-                const uint64_t sa2 = pack_f32x2(scale, scale);
-                const uint32_t sw_group = sw_stage + gl * BN * 4;
-                uint64_t p[HOIST / 2];
-                ulonglong2 sw4;
-#pragma unroll
-                for (int q = 0; q < HOIST / 4; ++q) {
-                    sw4 = lds_pairs(sw_group + 16 * q);
-                    p[2 * q] = sw4.x;
-                    p[2 * q + 1] = sw4.y;
-                }
-                tmem_load_wait_32(dots);
-                if ((gl & 1) == 1) {  // both groups of the slab are in registers or folded: hand the buffer back
-                    tcgen05_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbarrier_arrive_cluster(leader_dot_empty + buffer * 8);
-                }
-                if (DUMP_DOTS && row < shape.m) {
-#pragma unroll
-                    for (int j = 0; j < COLUMNS; ++j)
-                        if (n0 + j < shape.n)
-                            dots_out[(static_cast<size_t>(row) * shape.n + n0 + j) * v.groups + ks * STAGE_GROUPS + gl] =
-                                static_cast<int32_t>(__uint_as_float(dots[j]));
-                }
-#pragma unroll
-                for (int q = 0; q < HOIST / 4; ++q) {
-                    acc[2 * q] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), sa2), p[2 * q], acc[2 * q]);
-                    acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), p[2 * q + 1], acc[2 * q + 1]);
-                }
-#pragma unroll
-                for (int q = HOIST / 4; q < COLUMNS / 4; ++q) {
-                    sw4 = lds_pairs(sw_group + 16 * q);  // four columns, as two pairs
-                    acc[2 * q] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), sa2), sw4.x, acc[2 * q]);
-                    acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), sw4.y, acc[2 * q + 1]);
-                }
-                        }
-            __syncwarp();
-            if (lane == 0) arrive_u32(empty + s * 8);  // done with this stage's scales; its codes were consumed before the dots arrived
-            if (++s == STAGES) s = 0, phase ^= 1;
-        }
+    FoldState f = {smem_u32(v.dot_full + team * BUFFERS), map_to_cta(smem_u32(v.dot_empty + team * BUFFERS), 0),
+                   smem_u32(v.sa_tile) + (quadrant * 32 + lane) * 16, smem_u32(v.scale_ready), smem_u32(v.empty), 0, 0, 0, false};
+    const uint32_t tmem_lane = v.tmem_base + team * BUFFERS * BUFFER_COLUMNS + (static_cast<uint32_t>(quadrant * 32) << 16);
+    const uint32_t sw_tile = smem_u32(v.sw_tile);
+    for (int tile = v.pair; tile < v.tiling.tiles; tile += v.pairs) {
+        const TilePlace at = v.place(tile);
+        const int row = at.m_index * 2 * BM + static_cast<int>(v.cta) * BM + quadrant * 32 + lane;
+        const int columns = at.width / (TEAMS * TEAM_COLUMNS / COLUMNS);  // of this warp
+        const int in_team = slice % (TEAM_COLUMNS / COLUMNS) * columns, in_tile = slice * columns;
+        bool alive;
+        if (at.width == BN)
+            alive = fold_tile<32, DUMP_DOTS, SCATTER>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane);
+        else if (DUMP_DOTS || SCATTER) alive = false;  // the launcher cuts no narrow tiles for these
+        else if (at.width == 96)
+            alive = fold_tile<24, false, false>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane);
+        else
+            alive = fold_tile<16, false, false>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane);
         if (!alive) break;
-        if (row >= shape.m) continue;
-        // y: this thread's row, 32 adjacent columns
-        float out[COLUMNS];
-#pragma unroll
-        for (int j = 0; j < COLUMNS / 2; ++j) unpack_f32x2(acc[j], out[2 * j], out[2 * j + 1]);
-        if (bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < COLUMNS; ++j)
-                if (n0 + j < shape.n) out[j] += __ldg(bias + n0 + j);
-        }
-        const size_t element = static_cast<size_t>(row) * shape.ldy + n0;
-        if constexpr (SCATTER) {
-            // The launcher admits only outputs that take whole 32-byte sectors (32-byte aligned copies,
-            // n a multiple of 32, ldy a multiple of a sector): a warp's 32 columns lie wholly inside the
-            // matrix or wholly outside it (n not a multiple of the tile's 128 columns).
-            if (n0 >= shape.n) continue;
-            if (shape.y_is_half) {
-                uint32_t packed[COLUMNS / 2];
-#pragma unroll
-                for (int j = 0; j < COLUMNS / 2; ++j) {
-                    const __half2 h = __floats2half2_rn(out[2 * j], out[2 * j + 1]);
-                    packed[j] = *reinterpret_cast<const uint32_t *>(&h);
-                }
-                int index = peers.first;
-                for (int copy = 0; copy < peers.count; ++copy) {
-                    __half *target = static_cast<__half *>(peers.y[index]) + element;
-#pragma unroll
-                    for (int j = 0; j < COLUMNS / 16; ++j)
-                        st_global_v8(target + 16 * j, *reinterpret_cast<const uint32_t(*)[8]>(&packed[8 * j]));
-                    if (++index == peers.count) index = 0;
-                }
-            } else {
-                int index = peers.first;
-                for (int copy = 0; copy < peers.count; ++copy) {
-                    float *target = static_cast<float *>(peers.y[index]) + element;
-#pragma unroll
-                    for (int j = 0; j < COLUMNS / 8; ++j)
-                        st_global_v8(target + 8 * j, *reinterpret_cast<const uint32_t(*)[8]>(&out[8 * j]));
-                    if (++index == peers.count) index = 0;
-                }
-            }
-            continue;
-        }
-        // whole 32-byte sectors when the row segment is aligned for them, else element by element
-        const bool sectors = n0 + COLUMNS <= shape.n &&
-                             (reinterpret_cast<uintptr_t>(y) & 31) == 0 && shape.ldy % (shape.y_is_half ? 16 : 8) == 0;
-        if (shape.y_is_half) {
-            uint32_t packed[COLUMNS / 2];
-#pragma unroll
-            for (int j = 0; j < COLUMNS / 2; ++j) {
-                const __half2 h = __floats2half2_rn(out[2 * j], out[2 * j + 1]);
-                packed[j] = *reinterpret_cast<const uint32_t *>(&h);
-            }
-            __half *target = static_cast<__half *>(y) + element;
-            if (sectors) {
-#pragma unroll
-                for (int j = 0; j < COLUMNS / 16; ++j)
-                    st_global_v8(target + 16 * j, *reinterpret_cast<const uint32_t(*)[8]>(&packed[8 * j]));
-            } else {
-#pragma unroll
-                for (int j = 0; j < COLUMNS; ++j)
-                    if (n0 + j < shape.n) target[j] = __float2half_rn(out[j]);
-            }
-        } else {
-            float *target = static_cast<float *>(y) + element;
-            if (sectors) {
-#pragma unroll
-                for (int j = 0; j < COLUMNS / 8; ++j)
-                    st_global_v8(target + 8 * j, *reinterpret_cast<const uint32_t(*)[8]>(&out[8 * j]));
-            } else {
-#pragma unroll
-                for (int j = 0; j < COLUMNS; ++j)
-                    if (n0 + j < shape.n) target[j] = out[j];
-            }
-        }
     }
     tmem_load_wait();  // nothing of this warp may still be in flight at teardown
 }
@@ -506,7 +544,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
             const __half *__restrict__ a_scales, const __half *__restrict__ w_scales,
             const float *__restrict__ bias, void *__restrict__ y, int32_t *__restrict__ dots_out,
-            const GemmShape shape, const __grid_constant__ PeerOutputs peers) {
+            const GemmShape shape, const __grid_constant__ PeerOutputs peers, const __grid_constant__ Tiling tiling) {
     extern __shared__ uint8_t smem_raw[];
     // the same offsets in both CTAs: the dynamic shared window starts at the same address in each
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -525,8 +563,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t cta = cluster_ctarank();  // 0 = leader
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const int tiles_m = (shape.m + 2 * BM - 1) / (2 * BM), tiles_n = (shape.n + BN - 1) / BN;
-    const int tiles = tiles_m * tiles_n, k_stages = shape.k / STAGE_K, groups = shape.k / 64;
+    const int tiles_m = (shape.m + 2 * BM - 1) / (2 * BM), k_stages = shape.k / STAGE_K, groups = shape.k / 64;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -555,7 +592,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 
     const uint32_t tmem_base = *tmem_slot;
     const View view = {tile_a, tile_b, sw_tile, sa_tile, ring, full, scale_ready, empty, dot_full, dot_empty,
-                       tmem_base, cta, pair, pairs, tiles, tiles_m, k_stages, groups};
+                       tmem_base, cta, pair, pairs, tiles_m, k_stages, groups, tiling};
 
     if (warp < FOLD_WARP0) {
         setmaxnreg_dec<CONTROL_REGISTERS>();

@@ -579,6 +579,27 @@ def test_w4a4_wide_gemm_equals_packed_kernel_on_many_tiles(qi, wide_kernel, m, n
         assert torch.equal(y, expected)
 
 
+@pytest.mark.parametrize("m,n,k", [(1024, 4096, 256), (4096, 3072, 256), (300, 3072, 512), (1500, 2112, 256), (256, 32, 256), (2048, 9600, 256)])
+def test_w4a4_wide_gemm_last_wave_in_narrow_tiles(qi, m, n, k):
+    # numbers of 256 x 128 tiles that leave part of a last wave to narrower tiles (74 pairs of CTAs), against the int8
+    # kernel; float16 into a slice of a wider matrix with a bias, and float32
+    rng = np.random.default_rng(m + n + k)
+    a_codes, a_scales = qt.random_w4a4_pack(rng, m, k, 0.02, 0.2)
+    w_codes, w_scales = qt.random_w4a4_pack(rng, n, k, 0.002, 0.01)
+    a, sa, w, sw = up(a_codes), up(a_scales.view(np.float16)), up(w_codes), up(w_scales.view(np.float16))
+    bias = up(qt.make_bias(rng, n))
+    a_wide = torch.empty(m, k, dtype=torch.uint8, device="cuda")
+    w_wide = torch.empty(n, k, dtype=torch.uint8, device="cuda")
+    assert qi.w4a4_widen_codes_ex(a, a_wide, m, k) == 0 and qi.w4a4_widen_codes_ex(w, w_wide, n, k) == 0
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        ldy = n + 8
+        got, expected = (torch.full((m, ldy), -7.0, dtype=dtype, device="cuda") for _ in range(2))
+        assert qi.w4a4_gemm_wide_ex(a_wide, sa, w_wide, sw, bias, got, code, ldy, m, n, k) == 0
+        assert qi.w4a4_gemm_path_ex(a, sa, w, sw, bias, expected, code, ldy, m, n, k, qi.W4A4_PATH_INT8) == 0
+        check_status(qi)
+        assert torch.equal(got, expected)
+
+
 def test_w4a4_wide_gemm_extreme_dots(qi, wide_kernel):
     # all codes +-7: every group dot is +-3136, the largest the format allows; fp32 accumulation must stay exact
     m, n, k = 128, 128, 512
