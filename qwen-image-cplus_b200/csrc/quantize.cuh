@@ -20,12 +20,11 @@
 // rounding; a lane whose quotient lies within 2^-16 of a rounding tie redoes it with the
 // IEEE division the reference uses, so the codes are identical.
 //
-// Two forms. The older one (one chunk per half-warp, scalar arithmetic) issues 34 instructions per value and
-// is bound by that, at 0.37-0.42 of the HBM rate. The paired form gives a half-warp TWO chunks and keeps value
-// i of both in one 64-bit register, so that the butterflies, the rounding and its check are packed fp32 pair
-// instructions (add / sub / fma .f32x2: the same IEEE results, half the issue slots), moves the pairs through
-// the transposes with 8- and 16-byte accesses, checks for rounding ties once per thread instead of once per
-// value, and emits only the code formats asked for. It is used whenever there are at least two chunks.
+// A half-warp takes TWO chunks and keeps value i of both in one 64-bit register, so that the butterflies, the rounding
+// and its check are packed fp32 pair instructions (add / sub / fma .f32x2: the same IEEE results, half the issue
+// slots), moves the pairs through the transposes with 8- and 16-byte accesses, checks for rounding ties once per
+// thread instead of once per value, and emits only the code formats asked for. One chunk per half-warp and scalar
+// arithmetic took 34 instructions per value instead of 19 and was bound by that.
 #pragma once
 #include <cuda_fp8.h>
 
@@ -36,171 +35,8 @@ namespace qi {
 namespace {
 
 constexpr int QUANT_THREADS = 256;
-constexpr int PITCH = 20;                  // floats per transposed row: 128-bit reads stay conflict-free
-constexpr int REGION = 16 * PITCH + 16;    // second half-warp lands 16 banks away from the first
 constexpr float MAGIC = 12582912.0f;       // 1.5 * 2^23: adding it rounds to an integer, ties to even
-constexpr int MAGIC_BITS = 0x4B400000;
 constexpr float SCALE_FLOOR = 5.9604645e-08f;  // 2^-24, gemm.cu:45
-
-__device__ __forceinline__ void load16(const float *source, float (&v)[16]) {
-    const float4 *p = reinterpret_cast<const float4 *>(source);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float4 q = __ldg(p + i);
-        v[4 * i] = q.x, v[4 * i + 1] = q.y, v[4 * i + 2] = q.z, v[4 * i + 3] = q.w;
-    }
-}
-
-__device__ __forceinline__ void load16(const __half *source, float (&v)[16]) {
-    const uint4 *p = reinterpret_cast<const uint4 *>(source);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const uint4 q = __ldg(p + i);
-        const uint32_t words[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 pair = __half22float2(*reinterpret_cast<const __half2 *>(&words[j]));
-            v[8 * i + 2 * j] = pair.x, v[8 * i + 2 * j + 1] = pair.y;
-        }
-    }
-}
-
-// gemm.cu:33-36 without the halving.
-__device__ __forceinline__ void butterfly(float &a, float &b, float &c, float &d) {
-    const float sum = a + b, difference = a - b, reversed = b - a;  // b - a == (-a) + b exactly
-    const float o0 = (sum + c) - d;
-    const float o1 = (sum - c) + d;
-    const float o2 = (difference + c) + d;
-    const float o3 = (reversed + c) + d;
-    a = o0, b = o1, c = o2, d = o3;
-}
-
-// Strides 1 and 4 of a 16-value array (also strides 16 and 64 after the transpose).
-__device__ __forceinline__ void two_passes(float (&v)[16]) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) butterfly(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-#pragma unroll
-    for (int o = 0; o < 4; ++o) butterfly(v[o], v[o + 4], v[o + 8], v[o + 12]);
-}
-
-// What the quantiser reads. Plain: the activations themselves. The other two compute the activation on the
-// fly from what its producer would have read, with the producer's own expression, so that the [m, k] float32
-// matrix between the two kernels of the reference is never written or read:
-//   SwiGLU (qwen_image_cuda/cuda/ops.cu:133-138):    g / (1 + expf(-g)) * up
-//   GELU-tanh (qwen_image_cuda/cuda/ops.cu:155-160): 0.5 v (1 + tanhf(0.7978845608028654 (v + 0.044715 v v v)))
-template <typename T>
-struct PlainSource {
-    const T *x;
-    __device__ __forceinline__ void load(long long offset, float (&v)[16]) const { load16(x + offset, v); }
-};
-struct SwigluSource {
-    const float *gate, *up;
-    __device__ __forceinline__ void load(long long offset, float (&v)[16]) const {
-        float u[16];
-        load16(gate + offset, v);
-        load16(up + offset, u);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = v[i] / (1.0f + expf(-v[i])) * u[i];
-    }
-};
-struct GeluSource {
-    const float *x;
-    __device__ __forceinline__ void load(long long offset, float (&v)[16]) const {
-        load16(x + offset, v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + tanhf(0.7978845608028654f * (v[i] + 0.044715f * v[i] * v[i] * v[i])));
-    }
-};
-
-// WIDE: also (or only, when codes is null) write every code as one FP8 E4M3 byte, [m, k], the
-// operand layout of w4a4_wide_gemm.cuh.
-template <typename Source, bool WIDE>
-__global__ void __launch_bounds__(QUANT_THREADS)
-quantize_activations_kernel(const Source source, uint8_t *__restrict__ codes, __half *__restrict__ scales,
-                            uint8_t *__restrict__ bytes, long long chunks) {
-    __shared__ __align__(16) float transpose[(QUANT_THREADS / 32) * 2 * REGION];
-    grid_wait();
-    grid_release();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int half_warp = lane >> 4, l = lane & 15;
-    float *region = transpose + (warp * 2 + half_warp) * REGION;
-    const long long chunk = (static_cast<long long>(blockIdx.x) * (QUANT_THREADS / 32) + warp) * 2 + half_warp;
-    const bool active = chunk < chunks;
-
-    float v[16];
-    if (active) {
-        source.load(chunk * 256 + l * 16, v);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.0f;
-    }
-    two_passes(v);  // strides 1, 4
-
-    // contiguous -> strided: lane l ends up with elements 16 * r + l, r = 0..15
-#pragma unroll
-    for (int c = 0; c < 16; ++c) region[c * PITCH + l] = v[c];
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float4 q = *reinterpret_cast<const float4 *>(region + l * PITCH + 4 * j);
-        v[4 * j] = q.x, v[4 * j + 1] = q.y, v[4 * j + 2] = q.z, v[4 * j + 3] = q.w;
-    }
-    two_passes(v);  // strides 16, 64
-
-    // strided -> contiguous (each lane rewrites only the row it has just read)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<float4 *>(region + l * PITCH + 4 * j) =
-            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    __syncwarp();
-#pragma unroll
-    for (int c = 0; c < 16; ++c) v[c] = region[c * PITCH + l];
-
-    // v holds 16 * (rotated value); four lanes share one 64-group (gemm.cu:40-51)
-    float peak16 = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) peak16 = fmaxf(peak16, fabsf(v[i]));
-    peak16 = fmaxf(peak16, __shfl_xor_sync(0xffffffffu, peak16, 1));
-    peak16 = fmaxf(peak16, __shfl_xor_sync(0xffffffffu, peak16, 2));
-    const float peak = peak16 * 0.0625f;
-    const __half scale_half = __float2half_rn(fmaxf(peak / 7.0f, SCALE_FLOOR));
-    const float scale16 = __half2float(scale_half) * 16.0f;  // v / scale == (16 v) / (16 scale)
-    const float reciprocal = 1.0f / scale16;
-
-    uint32_t packed[2] = {0u, 0u};
-    uint32_t wide[4] = {0u, 0u, 0u, 0u};
-    float previous = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float rounded = fmaf(v[i], reciprocal, MAGIC);
-        const float integer = rounded - MAGIC;
-        const float residual = fmaf(v[i], reciprocal, -integer);
-        int bits = __float_as_int(rounded);
-        if (!(fabsf(residual) < 0.5f - 1.52587890625e-05f)) {
-            // near a tie (or not finite): the reference's own expression
-            const float exact = fminf(fmaxf(rintf(v[i] / scale16), -7.0f), 7.0f);
-            bits = MAGIC_BITS + static_cast<int>(exact);
-        }
-        bits = min(max(bits, MAGIC_BITS - 7), MAGIC_BITS + 7);
-        packed[i >> 3] |= static_cast<uint32_t>(bits & 0xF) << (4 * (i & 7));
-        if (WIDE) {
-            const float code = __int_as_float(bits) - MAGIC;  // exact
-            if (i & 1) {
-                const uint32_t pair = __nv_cvt_float2_to_fp8x2(make_float2(previous, code), __NV_SATFINITE, __NV_E4M3);
-                wide[i >> 2] |= pair << (8 * (i & 2));
-            }
-            previous = code;
-        }
-    }
-    if (active) {
-        if (!WIDE || codes != nullptr)
-            *reinterpret_cast<uint2 *>(codes + chunk * 128 + l * 8) = make_uint2(packed[0], packed[1]);
-        if (WIDE) *reinterpret_cast<uint4 *>(bytes + chunk * 256 + l * 16) = make_uint4(wide[0], wide[1], wide[2], wide[3]);
-        if ((l & 3) == 0) scales[chunk * 4 + (l >> 2)] = scale_half;
-    }
-}
-
-// ---- the paired form -------------------------------------------------------------------------------------
 
 constexpr int PAIR_PITCH = 18;                      // 64-bit elements per transposed row: 16-byte reads stay conflict-free
 constexpr int PAIR_REGION = 16 * PAIR_PITCH + 8;    // the second half-warp lands 16 banks away from the first
@@ -289,27 +125,52 @@ struct Raw16<float> {
     }
 };
 
+// What the quantiser reads. Plain: the activations themselves. The other two compute the activation on the
+// fly from what its producer would have read, with the producer's own expression, so that the [m, k] float32
+// matrix between the two kernels of the reference is never written or read:
+//   SwiGLU (qwen_image_cuda/cuda/ops.cu:133-138):    g / (1 + expf(-g)) * up
+//   GELU-tanh (qwen_image_cuda/cuda/ops.cu:155-160): 0.5 v (1 + tanhf(0.7978845608028654 (v + 0.044715 v v v)))
+// A source's Raw is what it loads for one lane's 16 values, in flight while the lane works on earlier ones.
+template <typename T>
+struct PlainSource {
+    const T *x;
+    struct Raw : Raw16<T> {
+        __device__ __forceinline__ void load(const PlainSource &source, long long offset, bool active) { Raw16<T>::load(source.x + offset, active); }
+    };
+};
+struct GeluSource {
+    const float *x;
+    struct Raw : Raw16<float> {
+        __device__ __forceinline__ void load(const GeluSource &source, long long offset, bool active) { Raw16<float>::load(source.x + offset, active); }
+        __device__ __forceinline__ void convert(float (&v)[16]) const {
+            Raw16<float>::convert(v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + tanhf(0.7978845608028654f * (v[i] + 0.044715f * v[i] * v[i] * v[i])));
+        }
+    };
+};
+
 // CODES: write nibble-packed codes [m, k/2]; WIDE: write one FP8 E4M3 byte per code [m, k]. At least one of them.
 // A half-warp walks over pairs of chunks with the stride of the grid; the loads of its next pair are in flight
 // while it works on the current one (the kernel holds 16 warps per SM: without that, too few bytes are under way
 // to keep HBM busy).
-template <typename T, bool CODES, bool WIDE>
-__global__ void __launch_bounds__(QUANT_THREADS)
-quantize_pairs_kernel(const T *__restrict__ x, uint8_t *__restrict__ codes, __half *__restrict__ scales,
+template <typename Source, bool CODES, bool WIDE>
+__global__ void __launch_bounds__(QUANT_THREADS, 2)
+quantize_pairs_kernel(const Source source, uint8_t *__restrict__ codes, __half *__restrict__ scales,
                       uint8_t *__restrict__ bytes, long long chunks) {
     __shared__ __align__(16) uint64_t transpose[(QUANT_THREADS / 32) * 2 * PAIR_REGION];
     grid_wait();
     grid_release();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int half_warp = lane >> 4, l = lane & 15;
     uint64_t *region = transpose + (warp * 2 + half_warp) * PAIR_REGION;
-    const long long pairs = (chunks + 1) / 2, stride = static_cast<long long>(gridDim.x) * (QUANT_THREADS / 16);
-    long long pair = (static_cast<long long>(blockIdx.x) * (QUANT_THREADS / 32) + warp) * 2 + half_warp;
-    Raw16<T> next_a, next_b;
-    next_a.load(x + (2 * pair) * 256 + l * 16, 2 * pair < chunks);
-    next_b.load(x + (2 * pair + 1) * 256 + l * 16, 2 * pair + 1 < chunks);
+    const long long pairs = (chunks + 1) / 2, stride = static_cast<long long>(gridDim.x) * warps * 2;
+    long long pair = (static_cast<long long>(blockIdx.x) * warps + warp) * 2 + half_warp;
+    typename Source::Raw next_a, next_b;
+    next_a.load(source, (2 * pair) * 256 + l * 16, 2 * pair < chunks);
+    next_b.load(source, (2 * pair + 1) * 256 + l * 16, 2 * pair + 1 < chunks);
     // every half-warp of a warp runs the same number of rounds (the shuffles and __syncwarp below are warp-wide)
-    const long long first_of_warp = (static_cast<long long>(blockIdx.x) * (QUANT_THREADS / 32) + warp) * 2;
+    const long long first_of_warp = (static_cast<long long>(blockIdx.x) * warps + warp) * 2;
     for (long long base = first_of_warp; base < pairs; base += stride, pair += stride) {
     const long long chunk_a = 2 * pair, chunk_b = chunk_a + 1;
     const bool active_a = chunk_a < chunks, active_b = chunk_b < chunks;
@@ -320,8 +181,8 @@ quantize_pairs_kernel(const T *__restrict__ x, uint8_t *__restrict__ codes, __ha
         next_a.convert(a);
         next_b.convert(b);
         const long long after = pair + stride;
-        next_a.load(x + (2 * after) * 256 + l * 16, 2 * after < chunks);
-        next_b.load(x + (2 * after + 1) * 256 + l * 16, 2 * after + 1 < chunks);
+        next_a.load(source, (2 * after) * 256 + l * 16, 2 * after < chunks);
+        next_b.load(source, (2 * after + 1) * 256 + l * 16, 2 * after + 1 < chunks);
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = pack_f32x2(a[i], b[i]);
     }
@@ -422,6 +283,139 @@ quantize_pairs_kernel(const T *__restrict__ x, uint8_t *__restrict__ codes, __ha
     }
 }
 
+// ---- SwiGLU: one chunk per half-warp ------------------------------------------------------------------------------------
+// The two loads and the division of silu(gate) * up want warps rather than registers: with 40 registers a thread this
+// form takes 28.8 us at 1024 x 12288, the paired one 42.8 (32.1 without loads ahead).
+
+constexpr int PITCH = 20;                  // floats per transposed row: 128-bit reads stay conflict-free
+constexpr int REGION = 16 * PITCH + 16;    // second half-warp lands 16 banks away from the first
+constexpr int MAGIC_BITS = 0x4B400000;
+
+__device__ __forceinline__ void load16(const float *source, float (&v)[16]) {
+    const float4 *p = reinterpret_cast<const float4 *>(source);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 q = __ldg(p + i);
+        v[4 * i] = q.x, v[4 * i + 1] = q.y, v[4 * i + 2] = q.z, v[4 * i + 3] = q.w;
+    }
+}
+
+// gemm.cu:33-36 without the halving.
+__device__ __forceinline__ void butterfly(float &a, float &b, float &c, float &d) {
+    const float sum = a + b, difference = a - b, reversed = b - a;  // b - a == (-a) + b exactly
+    const float o0 = (sum + c) - d;
+    const float o1 = (sum - c) + d;
+    const float o2 = (difference + c) + d;
+    const float o3 = (reversed + c) + d;
+    a = o0, b = o1, c = o2, d = o3;
+}
+
+// Strides 1 and 4 of a 16-value array (also strides 16 and 64 after the transpose).
+__device__ __forceinline__ void two_passes(float (&v)[16]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) butterfly(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+#pragma unroll
+    for (int o = 0; o < 4; ++o) butterfly(v[o], v[o + 4], v[o + 8], v[o + 12]);
+}
+
+struct SwigluSource {
+    const float *gate, *up;
+    __device__ __forceinline__ void load(long long offset, float (&v)[16]) const {
+        float u[16];
+        load16(gate + offset, v);
+        load16(up + offset, u);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = v[i] / (1.0f + expf(-v[i])) * u[i];
+    }
+};
+// WIDE: also (or only, when codes is null) write every code as one FP8 E4M3 byte, [m, k], the
+// operand layout of w4a4_wide_gemm.cuh.
+template <bool WIDE>
+__global__ void __launch_bounds__(QUANT_THREADS)
+quantize_swiglu_kernel(const SwigluSource source, uint8_t *__restrict__ codes, __half *__restrict__ scales,
+                            uint8_t *__restrict__ bytes, long long chunks) {
+    __shared__ __align__(16) float transpose[(QUANT_THREADS / 32) * 2 * REGION];
+    grid_wait();
+    grid_release();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int half_warp = lane >> 4, l = lane & 15;
+    float *region = transpose + (warp * 2 + half_warp) * REGION;
+    const long long chunk = (static_cast<long long>(blockIdx.x) * (QUANT_THREADS / 32) + warp) * 2 + half_warp;
+    const bool active = chunk < chunks;
+
+    float v[16];
+    if (active) {
+        source.load(chunk * 256 + l * 16, v);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+    }
+    two_passes(v);  // strides 1, 4
+
+    // contiguous -> strided: lane l ends up with elements 16 * r + l, r = 0..15
+#pragma unroll
+    for (int c = 0; c < 16; ++c) region[c * PITCH + l] = v[c];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 q = *reinterpret_cast<const float4 *>(region + l * PITCH + 4 * j);
+        v[4 * j] = q.x, v[4 * j + 1] = q.y, v[4 * j + 2] = q.z, v[4 * j + 3] = q.w;
+    }
+    two_passes(v);  // strides 16, 64
+
+    // strided -> contiguous (each lane rewrites only the row it has just read)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4 *>(region + l * PITCH + 4 * j) =
+            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 16; ++c) v[c] = region[c * PITCH + l];
+
+    // v holds 16 * (rotated value); four lanes share one 64-group (gemm.cu:40-51)
+    float peak16 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) peak16 = fmaxf(peak16, fabsf(v[i]));
+    peak16 = fmaxf(peak16, __shfl_xor_sync(0xffffffffu, peak16, 1));
+    peak16 = fmaxf(peak16, __shfl_xor_sync(0xffffffffu, peak16, 2));
+    const float peak = peak16 * 0.0625f;
+    const __half scale_half = __float2half_rn(fmaxf(peak / 7.0f, SCALE_FLOOR));
+    const float scale16 = __half2float(scale_half) * 16.0f;  // v / scale == (16 v) / (16 scale)
+    const float reciprocal = 1.0f / scale16;
+
+    uint32_t packed[2] = {0u, 0u};
+    uint32_t wide[4] = {0u, 0u, 0u, 0u};
+    float previous = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float rounded = fmaf(v[i], reciprocal, MAGIC);
+        const float integer = rounded - MAGIC;
+        const float residual = fmaf(v[i], reciprocal, -integer);
+        int bits = __float_as_int(rounded);
+        if (!(fabsf(residual) < 0.5f - 1.52587890625e-05f)) {
+            // near a tie (or not finite): the reference's own expression
+            const float exact = fminf(fmaxf(rintf(v[i] / scale16), -7.0f), 7.0f);
+            bits = MAGIC_BITS + static_cast<int>(exact);
+        }
+        bits = min(max(bits, MAGIC_BITS - 7), MAGIC_BITS + 7);
+        packed[i >> 3] |= static_cast<uint32_t>(bits & 0xF) << (4 * (i & 7));
+        if (WIDE) {
+            const float code = __int_as_float(bits) - MAGIC;  // exact
+            if (i & 1) {
+                const uint32_t pair = __nv_cvt_float2_to_fp8x2(make_float2(previous, code), __NV_SATFINITE, __NV_E4M3);
+                wide[i >> 2] |= pair << (8 * (i & 2));
+            }
+            previous = code;
+        }
+    }
+    if (active) {
+        if (!WIDE || codes != nullptr)
+            *reinterpret_cast<uint2 *>(codes + chunk * 128 + l * 8) = make_uint2(packed[0], packed[1]);
+        if (WIDE) *reinterpret_cast<uint4 *>(bytes + chunk * 256 + l * 16) = make_uint4(wide[0], wide[1], wide[2], wide[3]);
+        if ((l & 3) == 0) scales[chunk * 4 + (l >> 2)] = scale_half;
+    }
+}
+
 __global__ void f32_to_f16_kernel(const float *__restrict__ source, __half *__restrict__ out,
                                   unsigned long long count) {
     grid_wait();
@@ -447,67 +441,43 @@ __global__ void f32_to_f16_kernel(const float *__restrict__ source, __half *__re
 
 }  // namespace
 
-inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, void *codes, void *scales, void *bytes,
-                                               int m, int k, cudaStream_t stream) {
-    const long long chunks = static_cast<long long>(m) * (k / 256);
+template <typename Source>
+inline cudaError_t launch_quantize_pairs(const Source &source, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream) {
+    const long long chunks = static_cast<long long>(m) * (k / 256), pairs = (chunks + 1) / 2;
     if (chunks == 0) return cudaSuccess;
-    const int chunks_per_block = QUANT_THREADS / 16;
-    const long long blocks = (chunks + chunks_per_block - 1) / chunks_per_block;
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    int device = 0, sms = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // Two CTAs of 256 threads stay resident per SM and walk over the pairs of chunks, a half-warp at a time. Fewer pairs than
+    // that are spread over more and smaller CTAs: 77 x 3072 are 462 pairs, 29 CTAs of 256 threads or 116 of 64.
+    const int threads = pairs >= static_cast<long long>(sms) * (QUANT_THREADS / 16) ? QUANT_THREADS : 64;
+    long long blocks = (pairs + threads / 16 - 1) / (threads / 16);
+    const long long resident = static_cast<long long>(sms) * (threads == QUANT_THREADS ? 2 : 4);
+    if (blocks > resident) blocks = resident;
     const unsigned grid = static_cast<unsigned>(blocks);
     uint8_t *c = static_cast<uint8_t *>(codes), *b = static_cast<uint8_t *>(bytes);
     __half *s = static_cast<__half *>(scales);
-    if (chunks >= 2) {
-        // a half-warp takes two chunks
-        long long pair_blocks = (chunks + 2 * chunks_per_block - 1) / (2 * chunks_per_block);
-        int device = 0, sms = 148;
-        if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (pair_blocks > 2LL * sms) pair_blocks = 2LL * sms;  // two CTAs per SM stay resident and walk over the rest
-        const unsigned pairs_grid = static_cast<unsigned>(pair_blocks);
-        const int variant = (bytes != nullptr ? 2 : 0) | (codes != nullptr ? 1 : 0);  // 1: codes, 2: bytes, 3: both
-        if (x_is_half) {
-            const __half *xs = static_cast<const __half *>(x);
-            if (variant == 1) return launch_overlapped(quantize_pairs_kernel<__half, true, false>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
-            else if (variant == 2) return launch_overlapped(quantize_pairs_kernel<__half, false, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
-            else return launch_overlapped(quantize_pairs_kernel<__half, true, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
-        } else {
-            const float *xs = static_cast<const float *>(x);
-            if (variant == 1) return launch_overlapped(quantize_pairs_kernel<float, true, false>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
-            else if (variant == 2) return launch_overlapped(quantize_pairs_kernel<float, false, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
-            else return launch_overlapped(quantize_pairs_kernel<float, true, true>, pairs_grid, QUANT_THREADS, 0, stream, xs, c, s, b, chunks);
-        }
-    }
-    const PlainSource<__half> from_half = {static_cast<const __half *>(x)};
-    const PlainSource<float> from_float = {static_cast<const float *>(x)};
-    if (bytes != nullptr) {
-        if (x_is_half) return launch_overlapped(quantize_activations_kernel<PlainSource<__half>, true>, grid, QUANT_THREADS, 0, stream, from_half, c, s, b, chunks);
-        else return launch_overlapped(quantize_activations_kernel<PlainSource<float>, true>, grid, QUANT_THREADS, 0, stream, from_float, c, s, b, chunks);
-    } else {
-        if (x_is_half) return launch_overlapped(quantize_activations_kernel<PlainSource<__half>, false>, grid, QUANT_THREADS, 0, stream, from_half, c, s, b, chunks);
-        else return launch_overlapped(quantize_activations_kernel<PlainSource<float>, false>, grid, QUANT_THREADS, 0, stream, from_float, c, s, b, chunks);
-    }
+    if (c != nullptr && b != nullptr) return launch_overlapped(quantize_pairs_kernel<Source, true, true>, grid, threads, 0, stream, source, c, s, b, chunks);
+    if (b != nullptr) return launch_overlapped(quantize_pairs_kernel<Source, false, true>, grid, threads, 0, stream, source, c, s, b, chunks);
+    return launch_overlapped(quantize_pairs_kernel<Source, true, false>, grid, threads, 0, stream, source, c, s, b, chunks);
+}
+
+inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, void *codes, void *scales, void *bytes,
+                                               int m, int k, cudaStream_t stream) {
+    if (x_is_half) return launch_quantize_pairs(PlainSource<__half>{static_cast<const __half *>(x)}, codes, scales, bytes, m, k, stream);
+    return launch_quantize_pairs(PlainSource<float>{static_cast<const float *>(x)}, codes, scales, bytes, m, k, stream);
 }
 
 // producer: 1 = SwiGLU of (first, second), 2 = GELU-tanh of first
 inline cudaError_t launch_fused_quantize(int producer, const float *first, const float *second, void *codes, void *scales,
                                          void *bytes, int m, int k, cudaStream_t stream) {
-    const long long chunks = static_cast<long long>(m) * (k / 256);
-    if (chunks == 0) return cudaSuccess;
-    const int chunks_per_block = QUANT_THREADS / 16;
-    const long long blocks = (chunks + chunks_per_block - 1) / chunks_per_block;
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    const unsigned grid = static_cast<unsigned>(blocks);
-    uint8_t *c = static_cast<uint8_t *>(codes), *b = static_cast<uint8_t *>(bytes);
-    __half *s = static_cast<__half *>(scales);
-    const SwigluSource swiglu = {first, second};
-    const GeluSource gelu = {first};
     if (producer == 1) {
-        if (bytes != nullptr) return launch_overlapped(quantize_activations_kernel<SwigluSource, true>, grid, QUANT_THREADS, 0, stream, swiglu, c, s, b, chunks);
-        else return launch_overlapped(quantize_activations_kernel<SwigluSource, false>, grid, QUANT_THREADS, 0, stream, swiglu, c, s, b, chunks);
-    } else {
-        if (bytes != nullptr) return launch_overlapped(quantize_activations_kernel<GeluSource, true>, grid, QUANT_THREADS, 0, stream, gelu, c, s, b, chunks);
-        else return launch_overlapped(quantize_activations_kernel<GeluSource, false>, grid, QUANT_THREADS, 0, stream, gelu, c, s, b, chunks);
+        const long long chunks = static_cast<long long>(m) * (k / 256), blocks = (chunks + QUANT_THREADS / 16 - 1) / (QUANT_THREADS / 16);
+        if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+        return launch_overlapped(bytes != nullptr ? quantize_swiglu_kernel<true> : quantize_swiglu_kernel<false>, static_cast<unsigned>(blocks), QUANT_THREADS, 0,
+                                 stream, SwigluSource{first, second}, static_cast<uint8_t *>(codes), static_cast<__half *>(scales),
+                                 static_cast<uint8_t *>(bytes), chunks);
     }
+    return launch_quantize_pairs(GeluSource{first}, codes, scales, bytes, m, k, stream);
 }
 
 inline cudaError_t launch_f32_to_f16(const float *source, void *out, unsigned long long count, cudaStream_t stream) {
