@@ -18,6 +18,7 @@
 #include "w4a4_gemm.cuh"
 #include "w4a4_wide_gemm.cuh"
 #include "w4a4_pair_gemm.cuh"
+#include "w4a4_narrow_gemm.cuh"
 #include "probe.cuh"
 
 namespace qi {
@@ -346,6 +347,47 @@ int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_by
                                               bias, y, dots, shape, outputs, tiling));
 }
 
+template <int BN>
+int launch_w4a4_narrow(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
+                       void *y, const GemmShape &shape, cudaStream_t stream, int device) {
+    namespace wn = w4a4_narrow;
+    using T = wn::Tile<BN>;
+    // rows that do not exist are not loaded: what the tensor cores make of the rest of the tile nobody reads
+    const int box_rows = shape.m >= wn::BM ? wn::BM : (shape.m + 15) / 16 * 16;
+    CUtensorMap map_a, map_w;
+    if (!make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_bytes, shape.k, shape.m, static_cast<uint64_t>(shape.k),
+                  128, box_rows, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    if (!make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w_bytes, shape.k, shape.n, static_cast<uint64_t>(shape.k),
+                  128, BN, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    static std::atomic<bool> configured[MAX_DEVICES];
+    if (const cudaError_t error = configure_once(wn::gemm_kernel<BN>, T::SMEM_BYTES, configured[device])) return static_cast<int>(error);
+    const int tiles = ((shape.m + wn::BM - 1) / wn::BM) * ((shape.n + BN - 1) / BN);
+    const int grid = tiles < sm_count(device) ? tiles : sm_count(device);
+    return static_cast<int>(launch_overlapped(wn::gemm_kernel<BN>, grid, wn::THREADS, T::SMEM_BYTES, stream, map_a, map_w,
+                                              static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
+                                              bias, y, shape, box_rows));
+}
+
+// Byte operands with k a multiple of 256 and 8-byte aligned scales: CTA pairs, or single CTAs with 64 or 32 columns where
+// those are estimated to be faster. Microseconds per group and wave as measured on B200 ({77, 128, 256, 512} rows,
+// outputs 3072 to 12288, K 3072 to 12288): 0.185 and 0.12 for the narrow tiles, 0.35 for a wave of wide pairs, 0.37 and
+// 0.29 for a last wave of 96 or 64 columns.
+int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
+                      void *y, const GemmShape &shape, cudaStream_t stream, int device) {
+    namespace wn = w4a4_narrow;
+    const int sms = sm_count(device), pairs = sms / 2;
+    const w4a4_pair::Tiling tiling = w4a4_tiling(shape.m, shape.n, pairs, true);
+    const double pair_us = (tiling.wide + pairs - 1) / pairs * 0.35 + (tiling.tiles > tiling.wide ? (tiling.width == 64 ? 0.29 : 0.37) : 0.0);
+    const long long tiles_m = (shape.m + wn::BM - 1) / wn::BM;
+    const double us_64 = static_cast<double>((tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms) * 0.185;
+    const double us_32 = static_cast<double>((tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms) * 0.12;
+    if (us_64 <= us_32 && us_64 < pair_us) return launch_w4a4_narrow<64>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    if (us_32 < pair_us) return launch_w4a4_narrow<32>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    return launch_w4a4_pair(a_bytes, a_scales, w_bytes, w_scales, bias, y, nullptr, shape, stream, device);
+}
+
 bool output_ok(const void *y, int y_dtype, long long ldy, int n) {
     if (y == nullptr || !aligned16(y) || ldy < n) return false;
     if (y_dtype == QI_DTYPE_F32) return ldy % 4 == 0;
@@ -505,6 +547,7 @@ int w4a4_gemm_wide(const void *a_bytes, const void *a_scales, const void *w_byte
     const bool scales_aligned8 = ((reinterpret_cast<uintptr_t>(a_scales) | reinterpret_cast<uintptr_t>(w_scales)) & 7) == 0;
     if (single_cta || k % w4a4_pair::STAGE_K != 0 || !scales_aligned8)
         return launch_w4a4_wide<6>(a_bytes, a_scales, w_bytes, w_scales, bias, y, dots, shape, stream, device);
+    if (dots == nullptr) return launch_w4a4_bytes(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
     return launch_w4a4_pair(a_bytes, a_scales, w_bytes, w_scales, bias, y, dots, shape, stream, device);
 }
 
@@ -566,7 +609,7 @@ int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, co
             int status = qi_w4a4_widen_codes_ex(a_codes, scratch, m, k, stream);
             if (status == 0) status = qi_w4a4_widen_codes_ex(w_codes, scratch + a_bytes, n, k, stream);
             if (status == 0)
-                status = launch_w4a4_pair(scratch, a_scales, scratch + a_bytes, w_scales, bias, y, nullptr, shape, stream, device);
+                status = launch_w4a4_bytes(scratch, a_scales, scratch + a_bytes, w_scales, bias, y, shape, stream, device);
             const cudaError_t freed = cudaFreeAsync(scratch, stream);
             return status != 0 ? status : static_cast<int>(freed);
         }
@@ -751,7 +794,7 @@ int qi_w4a4_gemm_noalloc_ex(const void *a_codes, const void *a_scales, const voi
     if (status == 0) status = qi_w4a4_widen_codes_ex(w_codes, scratch + a_bytes, n, k, stream);
     if (status != 0) return status;
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
-    return launch_w4a4_pair(scratch, a_scales, scratch + a_bytes, w_scales, bias, y, nullptr, shape, on, device);
+    return launch_w4a4_bytes(scratch, a_scales, scratch + a_bytes, w_scales, bias, y, shape, on, device);
 }
 
 int qi_w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, const void *w_scales, float *y,

@@ -579,10 +579,11 @@ def test_w4a4_wide_gemm_equals_packed_kernel_on_many_tiles(qi, wide_kernel, m, n
         assert torch.equal(y, expected)
 
 
-@pytest.mark.parametrize("m,n,k", [(1024, 4096, 256), (4096, 3072, 256), (300, 3072, 512), (1500, 2112, 256), (256, 32, 256), (2048, 9600, 256)])
-def test_w4a4_wide_gemm_last_wave_in_narrow_tiles(qi, m, n, k):
-    # numbers of 256 x 128 tiles that leave part of a last wave to narrower tiles (74 pairs of CTAs), against the int8
-    # kernel; float16 into a slice of a wider matrix with a bias, and float32
+@pytest.mark.parametrize("m,n,k", [(1024, 4096, 256), (4096, 3072, 256), (300, 3072, 512), (1500, 2112, 256), (256, 32, 256), (2048, 9600, 256),
+                                   (1, 32, 256), (16, 96, 512), (17, 9216, 256), (77, 3104, 1280), (129, 2048, 768), (300, 480, 2304)])
+def test_w4a4_wide_gemm_in_narrow_tiles(qi, m, n, k):
+    # numbers of 256 x 128 tiles that leave part of a last wave to narrower tiles (74 pairs of CTAs), and few rows, which
+    # take tiles of 64 or 32 columns on single CTAs, against the int8 kernel; float16 into a slice of a wider matrix with a bias, and float32
     rng = np.random.default_rng(m + n + k)
     a_codes, a_scales = qt.random_w4a4_pack(rng, m, k, 0.02, 0.2)
     w_codes, w_scales = qt.random_w4a4_pack(rng, n, k, 0.002, 0.01)
