@@ -424,8 +424,8 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
     if (k <= w4a16::STREAM_MAX_K && aligned16(scales) && aligned16(minimums)) {
         const int device = current_device();
         if (device < 0) return INVALID;
-        // two CTAs per SM: as many stages (at most three) as fit 110 KB beside the activations
-        constexpr int CTA_BYTES = 110 * 1024;
+        // one CTA per SM: as many stages (at most eight) as fit beside the activations and the partial sums
+        constexpr int CTA_BYTES = 207 * 1024;
         int stages = (CTA_BYTES - 128 - w4a16::stream_x_bytes(m, k)) / w4a16::stream_stage_bytes(k);
         stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
         static std::atomic<bool> configured[MAX_DEVICES];
@@ -433,7 +433,7 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
             return static_cast<int>(error);
         if (stages >= 1) {
             const int smem_bytes = stages * w4a16::stream_stage_bytes(k) + w4a16::stream_x_bytes(m, k) + 128;
-            const int tiles = n / w4a16::STREAM_ROWS, resident = 2 * sm_count(device);
+            const int tiles = n / w4a16::STREAM_ROWS, resident = sm_count(device);
             return static_cast<int>(launch_overlapped(w4a16::gemv_stream_kernel, tiles < resident ? tiles : resident,
                                       w4a16::STREAM_THREADS, smem_bytes, stream, static_cast<const __half *>(x_half),
                                       static_cast<const uint8_t *>(codes), static_cast<const __half *>(scales),
@@ -475,7 +475,7 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
     }
     const int device = current_device();
     if (device < 0) return INVALID;
-    constexpr int CTA_BYTES = 110 * 1024;  // two CTAs per SM, as for the single matrix
+    constexpr int CTA_BYTES = 207 * 1024;  // one CTA per SM, as for the single matrix
     int stages = (CTA_BYTES - 128 - w4a16::stream_x_bytes(m, k)) / w4a16::stream_stage_bytes(k);
     stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
     if (stages < 1) return INVALID;
@@ -483,7 +483,7 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
     if (const cudaError_t error = configure_once(w4a16::gemv_stream_grouped_kernel, CTA_BYTES, configured[device]))
         return static_cast<int>(error);
     const int smem_bytes = stages * w4a16::stream_stage_bytes(k) + w4a16::stream_x_bytes(m, k) + 128;
-    const int resident = 2 * sm_count(device);
+    const int resident = sm_count(device);
     for (int first = 0; first < count; first += w4a16::STREAM_GROUP) {
         const int now = count - first < w4a16::STREAM_GROUP ? count - first : w4a16::STREAM_GROUP;
         w4a16::StreamItems group;

@@ -27,7 +27,8 @@
 namespace qi {
 namespace w4a16 {
 
-constexpr int STREAM_THREADS = 256, STREAM_WARPS = STREAM_THREADS / 32, STREAM_MAX_STAGES = 3, STREAM_ROWS = 16;
+constexpr int STREAM_THREADS = 512, STREAM_MAX_STAGES = 8, STREAM_ROWS = 16;
+constexpr int STREAM_TEAMS = 4, STREAM_TEAM_WARPS = STREAM_THREADS / 32 / STREAM_TEAMS;
 constexpr int STREAM_MAX_K = 4096;  // 16 rows of codes, scales and minimums: 36 KB per stage
 
 __host__ __device__ constexpr int stream_stage_bytes(int k) { return STREAM_ROWS * (k / 2) + 2 * STREAM_ROWS * (k / 64) * 2; }
@@ -87,8 +88,10 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     __shared__ uint64_t full[STREAM_MAX_STAGES];
-    __shared__ float partial[STREAM_WARPS][16][8];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ volatile int fetched[STREAM_MAX_STAGES];  // the tile that was last sent for into each stage
+    __shared__ float partials[STREAM_TEAMS][2][STREAM_TEAM_WARPS][16][8];
+    const int team = threadIdx.x / (STREAM_TEAM_WARPS * 32), warp = threadIdx.x / 32 % STREAM_TEAM_WARPS, lane = threadIdx.x & 31;
+    const int team_thread = threadIdx.x % (STREAM_TEAM_WARPS * 32);
     const int r = lane >> 2, q = lane & 3;
     const int groups = k / 64, steps = (groups + 1) / 2;  // a step: two groups, a quarter of the lanes on each half group
     const int code_bytes = STREAM_ROWS * (k / 2), scale_bytes = STREAM_ROWS * groups * 2;
@@ -96,7 +99,10 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     const int tiles_each = n / STREAM_ROWS, tiles = GROUPED ? tiles_each * count : tiles_each;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) mbarrier_init(&full[s], 1);
+        for (int s = 0; s < stages; ++s) {
+            mbarrier_init(&full[s], 1);
+            fetched[s] = -1;
+        }
         fence_barrier_init();
     }
     grid_wait();
@@ -109,8 +115,9 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
                                    __byte_perm(v.y, v.w, 0x7632));
     }
     __syncthreads();
-    auto fetch = [&](int tile, int s) {  // thread 0 only
+    auto fetch = [&](int tile, int s) {  // one thread
         uint8_t *stage = smem + static_cast<size_t>(s) * stage_bytes;
+        const int of_launch = tile;
         const uint8_t *from_codes = codes;
         const __half *from_scales = scales, *from_minimums = minimums;
         if (GROUPED) {
@@ -123,6 +130,8 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         bulk_load(stage, from_codes + row0 * (k / 2), code_bytes, &full[s]);
         bulk_load(stage + code_bytes, from_scales + row0 * groups, scale_bytes, &full[s]);
         bulk_load(stage + code_bytes + scale_bytes, from_minimums + row0 * groups, scale_bytes, &full[s]);
+        __threadfence_block();
+        fetched[s] = of_launch;
     };
     if (threadIdx.x == 0) {
         int tile = blockIdx.x;
@@ -132,15 +141,27 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     const __half nothing = __ushort_as_half(0), quarter = __float2half(0.25f), two_to_9 = __ushort_as_half(0x6000);
     const bool has_x = r < m;
-    uint32_t s = 0, phase = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const bool arrived = mbarrier_wait(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
+    // Team t takes the CTA's tiles t, t + 4, ...; tile i of the CTA lies in stage i modulo the number of stages.
+    uint32_t s = team, phase = 0;
+    while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
+    int parity = 0;
+    for (int tile = blockIdx.x + team * gridDim.x; tile < tiles; tile += STREAM_TEAMS * gridDim.x, parity ^= 1) {
+        float (&partial)[STREAM_TEAM_WARPS][16][8] = partials[team][parity];
+        // The stage's last user may have been another team. Only once this tile has been sent for is the phase before complete,
+        // and the parity of this one's unambiguous.
+        bool arrived = fetched[s] == tile;
+        for (uint32_t spin = 0; !arrived && spin < (1u << 24); ++spin) {
+            __nanosleep(32);
+            arrived = fetched[s] == tile;
+        }
+        if (!arrived) atomicCAS(&g_status, 0u, STATUS_WAIT_EMPTY | 0xB000 | s);
+        arrived = arrived && mbarrier_wait(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
         const uint8_t *stage = smem + static_cast<size_t>(s) * stage_bytes;
         const __half *stage_scales = reinterpret_cast<const __half *>(stage + code_bytes);
         const __half *stage_minimums = reinterpret_cast<const __half *>(stage + code_bytes + scale_bytes);
         float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (arrived) {
-            for (int step = warp; step < steps; step += STREAM_WARPS) {
+            for (int step = warp; step < steps; step += STREAM_TEAM_WARPS) {
                 const int g = 2 * step + (q >> 1), half_group = q & 1;
                 const bool valid = g < groups;  // every lane runs the same mma.sync; a lane past a ragged end feeds zeros
                 const int column = g * 32 + half_group * 16;  // byte offset of this lane's 32 codes in a row
@@ -188,13 +209,15 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         // c[0], c[1]: weight row r, activation rows 2q, 2q+1; c[2], c[3]: weight row r + 8
         partial[warp][r][2 * q] = c[0], partial[warp][r][2 * q + 1] = c[1];
         partial[warp][r + 8][2 * q] = c[2], partial[warp][r + 8][2 * q + 1] = c[3];
-        __syncthreads();  // every warp is done with the stage, and the partial sums are complete
-        if (threadIdx.x == 0) {
+        // The team is done with the stage, and the partial sums are complete. The sums alternate between two places: those of
+        // this tile are read below and written again two tiles on, with the next tile's barrier in between.
+        named_barrier_sync(1 + team, STREAM_TEAM_WARPS * 32);
+        if (team_thread == 0) {
             const int next = tile + stages * gridDim.x;
             if (next < tiles) fetch(next, s);
         }
-        if (threadIdx.x < 16 * 8) {  // fixed-order sum over the K slices: thread -> (weight row, activation row)
-            const int row = threadIdx.x >> 3, b = threadIdx.x & 7;
+        {  // fixed-order sum over the K slices: thread -> (weight row, activation row)
+            const int row = team_thread >> 3, b = team_thread & 7;
             const float *to_bias = bias;
             void *to_y = y;
             int local_tile = tile;
@@ -207,25 +230,25 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
             if (b < m) {
                 float total = 0.0f;
 #pragma unroll
-                for (int slice = 0; slice < STREAM_WARPS; ++slice) total += partial[slice][row][b];
+                for (int slice = 0; slice < STREAM_TEAM_WARPS; ++slice) total += partial[slice][row][b];
                 if (to_bias != nullptr) total += __ldg(to_bias + out_row);
                 if (y_is_half) static_cast<__half *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = __float2half_rn(total);
                 else static_cast<float *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = total;
             }
         }
-        __syncthreads();  // the partial sums have been read before the next tile overwrites them
-        if (++s == static_cast<uint32_t>(stages)) s = 0, phase ^= 1;
+        s += STREAM_TEAMS;
+        while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
     }
 }
 
-__global__ void __launch_bounds__(STREAM_THREADS, 2)
+__global__ void __launch_bounds__(STREAM_THREADS, 1)
 gemv_stream_kernel(const __half *__restrict__ x, const uint8_t *__restrict__ codes, const __half *__restrict__ scales,
                    const __half *__restrict__ minimums, const float *__restrict__ bias, void *__restrict__ y,
                    int m, int n, int k, long long ldy, int y_is_half, int stages) {
     gemv_stream_body<false>(x, codes, scales, minimums, bias, y, m, n, k, ldy, y_is_half, stages, nullptr, 1);
 }
 
-__global__ void __launch_bounds__(STREAM_THREADS, 2)
+__global__ void __launch_bounds__(STREAM_THREADS, 1)
 gemv_stream_grouped_kernel(const __half *__restrict__ x, const __grid_constant__ StreamItems group, int count,
                            int m, int n, int k, long long ldy, int y_is_half, int stages) {
     gemv_stream_body<true>(x, nullptr, nullptr, nullptr, nullptr, nullptr, m, n, k, ldy, y_is_half, stages, &group, count);
