@@ -425,7 +425,7 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
         const int device = current_device();
         if (device < 0) return INVALID;
         // one CTA per SM: as many stages (at most eight) as fit beside the activations and the partial sums
-        constexpr int CTA_BYTES = 207 * 1024;
+        constexpr int CTA_BYTES = 200 * 1024;
         int stages = (CTA_BYTES - 128 - w4a16::stream_x_bytes(m, k)) / w4a16::stream_stage_bytes(k);
         stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
         static std::atomic<bool> configured[MAX_DEVICES];
@@ -475,7 +475,7 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
     }
     const int device = current_device();
     if (device < 0) return INVALID;
-    constexpr int CTA_BYTES = 207 * 1024;  // one CTA per SM, as for the single matrix
+    constexpr int CTA_BYTES = 200 * 1024;  // one CTA per SM, as for the single matrix
     int stages = (CTA_BYTES - 128 - w4a16::stream_x_bytes(m, k)) / w4a16::stream_stage_bytes(k);
     stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
     if (stages < 1) return INVALID;
