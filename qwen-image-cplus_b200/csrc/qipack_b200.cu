@@ -15,6 +15,7 @@
 #include "w4a16_gemv_stream.cuh"
 #include "w4a16_pair_gemm.cuh"
 #include "w4a16_swap_gemm.cuh"
+#include "w4a16_pair_swap_gemm.cuh"
 #include "w4a4_gemm.cuh"
 #include "w4a4_wide_gemm.cuh"
 #include "w4a4_pair_gemm.cuh"
@@ -146,6 +147,15 @@ int launch_w4a16_pair(const void *x_half, const void *codes, const void *scales,
                                       bias, y, shape));
 }
 
+// Tiles walk down the rows first, so every pass over them reads all activations again, from L2 as long as they stay there.
+// Where they are larger than half of it, tiles walk through blocks of rows of which 24 MB are activations: the number of
+// tiles of such a block (16384 x 9216 x 3072: 1057 -> 757 us).
+int rows_in_l2(int tiles_m, long long tile_bytes) {
+    if (tiles_m * tile_bytes <= (64LL << 20)) return tiles_m;
+    const long long fit = (24LL << 20) / tile_bytes;
+    return fit < 8 ? (tiles_m < 8 ? tiles_m : 8) : fit < tiles_m ? static_cast<int>(fit) : tiles_m;
+}
+
 // ---- the exchanged-operand kernel (w4a16_swap_gemm.cuh): its plan for a shape ----------------------------------------
 
 struct SwapSmem {
@@ -257,6 +267,44 @@ int launch_w4a16_swap(const void *x_half, const void *codes, const void *scales,
     auto kernel = paired ? ws::gemm_kernel<true> : ws::gemm_kernel<false>;
     return static_cast<int>(cudaLaunchKernelEx(&config, kernel, map_x, map_codes, static_cast<const __half *>(scales),
                                                static_cast<const __half *>(minimums), bias, y, shape, plan));
+}
+
+// The widest tile is not always the best: 4096 x 3072 outputs are 192 tiles of 256 x 256, three waves of 74 pairs, or 288 of
+// 256 x 176, four waves (73.4 against 68.4 us at K = 3072). Microseconds: per column 0.0031 a step of 128 inputs and 0.0137 a
+// tile (4096 x {3072, 9216, 12288} x 3072, 4096 x 3072 x 12288, 1024 x 4096 x 4096), and 3 once.
+SwapPlan plan_w4a16_pair_swap(int m, int n, int k, int device) {
+    namespace wp = w4a16_pair_swap;
+    const int pairs = sm_count(device) / 2, steps = (k + 255) / 256 * 2;
+    const long long tiles_n = (n + 2 * wp::BN - 1) / (2 * wp::BN);
+    SwapPlan best = {0, 2, 1e30};
+    for (int columns = wp::MAX_COLUMNS; columns >= 128; columns -= 16) {
+        const long long waves = (tiles_n * ((m + columns - 1) / columns) + pairs - 1) / pairs;
+        const double us = 3.0 + waves * columns * (steps * 0.0031 + 0.0137);
+        if (us < best.us) best = {columns, 2, us};
+    }
+    return best;
+}
+
+int launch_w4a16_pair_swap(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
+                           void *y, const GemmShape &shape, int columns, cudaStream_t stream, int device) {
+    namespace wp = w4a16_pair_swap;
+    CUtensorMap map_x, map_codes;
+    if (!make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x_half, shape.k, shape.m,
+                  static_cast<uint64_t>(shape.k) * 2, 64, columns / 2, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    if (!make_map(&map_codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes, shape.k / 2, shape.n,
+                  static_cast<uint64_t>(shape.k) / 2, 128, wp::BN, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    const bool paired = ((reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(minimums)) & 3) == 0 && shape.k % 128 == 0;
+    auto kernel = paired ? wp::gemm_kernel<true> : wp::gemm_kernel<false>;
+    static std::atomic<bool> configured[MAX_DEVICES][2];
+    if (const cudaError_t error = configure_once(kernel, wp::SMEM_BYTES, configured[device][paired])) return static_cast<int>(error);
+    const int tiles = ((shape.m + columns - 1) / columns) * ((shape.n + 2 * wp::BN - 1) / (2 * wp::BN));
+    const int pairs = sm_count(device) / 2;
+    const int grid = 2 * (tiles < pairs ? tiles : pairs);  // the kernel carries __cluster_dims__(2, 1, 1)
+    return static_cast<int>(launch_overlapped(kernel, grid, wp::THREADS, wp::SMEM_BYTES, stream, map_x, map_codes,
+                                              static_cast<const __half *>(scales), static_cast<const __half *>(minimums),
+                                              bias, y, shape, columns, rows_in_l2((shape.m + columns - 1) / columns, 2LL * columns * shape.k)));
 }
 
 template <int BN, int STAGES>
@@ -372,7 +420,7 @@ int launch_w4a4_narrow(const void *a_bytes, const void *a_scales, const void *w_
 
 // Byte operands with k a multiple of 256 and 8-byte aligned scales: CTA pairs, or single CTAs with 64 or 32 columns where
 // those are estimated to be faster. Microseconds per group and wave as measured on B200 ({77, 128, 256, 512} rows,
-// outputs 3072 to 12288, K 3072 to 12288): 0.185 and 0.12 for the narrow tiles, 0.35 for a wave of wide pairs, 0.37 and
+// outputs 3072 to 12288, K 3072 to 12288): 0.185 and 0.12 for the narrow tiles (0.21 and 0.135 in several waves), 0.35 for a wave of wide pairs, 0.37 and
 // 0.29 for a last wave of 96 or 64 columns.
 int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
                       void *y, const GemmShape &shape, cudaStream_t stream, int device) {
@@ -381,8 +429,8 @@ int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_b
     const w4a4_pair::Tiling tiling = w4a4_tiling(shape.m, shape.n, pairs, true);
     const double pair_us = (tiling.wide + pairs - 1) / pairs * 0.35 + (tiling.tiles > tiling.wide ? (tiling.width == 64 ? 0.29 : 0.37) : 0.0);
     const long long tiles_m = (shape.m + wn::BM - 1) / wn::BM;
-    const double us_64 = static_cast<double>((tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms) * 0.185;
-    const double us_32 = static_cast<double>((tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms) * 0.12;
+    const long long waves_64 = (tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms, waves_32 = (tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms;
+    const double us_64 = waves_64 * (waves_64 == 1 ? 0.185 : 0.21), us_32 = waves_32 * (waves_32 == 1 ? 0.12 : 0.135);
     if (us_64 <= us_32 && us_64 < pair_us) return launch_w4a4_narrow<64>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
     if (us_32 < pair_us) return launch_w4a4_narrow<32>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
     return launch_w4a4_pair(a_bytes, a_scales, w_bytes, w_scales, bias, y, nullptr, shape, stream, device);
@@ -510,15 +558,15 @@ int w4a16_gemm(const void *x_half, const void *codes, const void *scales, const 
     const int device = current_device();
     if (device < 0) return INVALID;
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
+#ifdef SWEEP
+    if (tile >= 10000) return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, tile % 10000, tile / 10000, stream, device);
+    if (tile >= 1000) return launch_w4a16_pair_swap(x_half, codes, scales, minimums, bias, y, shape, tile - 1000, stream, device);
+#endif
     if (tile == 0) {
-        // The exchanged-operand kernel's estimate against the pair kernel's: per wave of pairs 0.46 us for 64 inputs of a
-        // 256 x 256 tile (4096 x {3072, 9216} x 3072, 4096 x 3072 x 12288: 22 and 89 us a wave), and 5 us once.
-        const SwapPlan swap = plan_w4a16_swap(m, n, k, device);
-        const long long tiles_256 = static_cast<long long>((m + 255) / 256) * ((n + 255) / 256);
-        const long long pairs = sm_count(device) / 2;
-        const double pair_us = 5.0 + static_cast<double>((tiles_256 + pairs - 1) / pairs) * (k / 64) * 0.46;
-        if (swap.us < pair_us) return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, swap.columns, swap.split, stream, device);
-        tile = 5;
+        // The exchanged-operand kernels: single CTAs and clusters, or persistent pairs, whichever is estimated to be faster.
+        const SwapPlan swap = plan_w4a16_swap(m, n, k, device), pair = plan_w4a16_pair_swap(m, n, k, device);
+        if (swap.us < pair.us) return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, swap.columns, swap.split, stream, device);
+        return launch_w4a16_pair_swap(x_half, codes, scales, minimums, bias, y, shape, pair.columns, stream, device);
     }
     switch (tile) {
         case 1: return launch_w4a16<1, 128, 6>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
@@ -830,7 +878,9 @@ int qi_w4a16_gemm_ex(const void *x_half, const void *codes, const void *scales, 
 int qi_w4a16_gemm_tile_ex(const void *x_half, const void *codes, const void *scales, const void *minimums,
                           const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, int tile,
                           void *stream) {
+#ifndef SWEEP
     if (tile < 0 || tile > 5) return INVALID;
+#endif
     return w4a16_gemm(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, tile, static_cast<cudaStream_t>(stream));
 }
 

@@ -227,6 +227,26 @@ def test_w4a16_exchanged_operands_at_the_edges_of_their_tiles(qi, m, n, k):
         assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
 
 
+@pytest.mark.parametrize("m,n,k", [(2048, 2048, 128), (4000, 1504, 192), (3000, 2336, 1216), (9000, 288, 320)])
+def test_w4a16_exchanged_operands_on_pairs_over_several_tiles(qi, m, n, k):
+    # more 256-row tiles than pairs of CTAs, ragged on both sides, an odd number of groups, steps past the end of K;
+    # against the unpacked weights in float32 on the device, every output
+    rng = np.random.default_rng(5000 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x, bias = up(qt.make_activations(rng, m, k)), up(qt.make_bias(rng, n))
+    c, s, z = up(codes), up(scales.view(np.float16)), up(minimums.view(np.float16))
+    weights = torch.empty(n, k, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_dequantize_ex(c, s, z, weights, n, k) == 0
+    expected = (x.double() @ weights.double().T + bias.double()).cpu().numpy()
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        wide = torch.full((m + 1, n + 32), -7.0, dtype=dtype, device="cuda")
+        assert qi.w4a16_gemm_ex(x, c, s, z, bias, wide, code, n + 32, m, n, k) == 0
+        check_status(qi)
+        got = wide.float().cpu().numpy()
+        assert np.all(got[m:] == -7.0) and np.all(got[:, n:] == -7.0)  # nothing outside the matrix
+        assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
+
+
 def test_w4a16_gemm_rejects_what_the_reference_rejects(qi):  # gemm.cu:264
     t = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
     assert qi.w4a16_gemm(t, t, t, t, t, 100, 128, 64) == qi.CUDA_ERROR_INVALID_VALUE
