@@ -558,10 +558,6 @@ int w4a16_gemm(const void *x_half, const void *codes, const void *scales, const 
     const int device = current_device();
     if (device < 0) return INVALID;
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
-#ifdef SWEEP
-    if (tile >= 10000) return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, tile % 10000, tile / 10000, stream, device);
-    if (tile >= 1000) return launch_w4a16_pair_swap(x_half, codes, scales, minimums, bias, y, shape, tile - 1000, stream, device);
-#endif
     if (tile == 0) {
         // The exchanged-operand kernels: single CTAs and clusters, or persistent pairs, whichever is estimated to be faster.
         const SwapPlan swap = plan_w4a16_swap(m, n, k, device), pair = plan_w4a16_pair_swap(m, n, k, device);
@@ -633,6 +629,17 @@ cudaMemPool_t scratch_pool(int device) {
     }
     return pool;
 }
+// One launch widens both operands: the second would add ~2 us to calls of 10.
+int launch_widen_codes(const void *a_codes, void *a_bytes, long long a_rows, const void *w_codes, void *w_bytes, long long w_rows,
+                       int k, cudaStream_t stream) {
+    constexpr long long PER_BLOCK = w4a4_wide::WIDEN_THREADS * w4a4_wide::WIDEN_PIECES;
+    const w4a4_wide::Widening a = {static_cast<const uint8_t *>(a_codes), static_cast<uint8_t *>(a_bytes), a_rows * (k / 16)};
+    const w4a4_wide::Widening w = {static_cast<const uint8_t *>(w_codes), static_cast<uint8_t *>(w_bytes), w_rows * (k / 16)};
+    const long long a_blocks = (a.pieces + PER_BLOCK - 1) / PER_BLOCK, w_blocks = (w.pieces + PER_BLOCK - 1) / PER_BLOCK;
+    if (a_blocks + w_blocks > 0x7fffffffLL) return INVALID;
+    return static_cast<int>(launch_overlapped(w4a4_wide::widen_codes_kernel, static_cast<unsigned>(a_blocks + w_blocks),
+                                              w4a4_wide::WIDEN_THREADS, 0, stream, a, w, static_cast<int>(a_blocks)));
+}
 int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, const void *w_scales, const float *bias,
               void *y, int y_dtype, long long ldy, int32_t *dots, int m, int n, int k, int path, cudaStream_t stream) {
     if (m <= 0 || n <= 0 || k <= 0 || n % 32 != 0 || k % 128 != 0 || path < 0 || path >= W4A4_PATHS) return INVALID;
@@ -646,7 +653,12 @@ int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, co
     const bool scales_aligned8 = ((reinterpret_cast<uintptr_t>(a_scales) | reinterpret_cast<uintptr_t>(w_scales)) & 7) == 0;
     const bool pair_takes_it = dots == nullptr && k % w4a4_pair::STAGE_K == 0 && scales_aligned8;
     if (path == 2 && !pair_takes_it) return INVALID;
-    if (path == 2 || (path == 0 && pair_takes_it && m >= 256 && n >= 256)) {
+    // Widening first (two launches, ~9 us at the least) against the int8 kernel, whose time is k's: 0.01 us per element
+    // and tile, 9 us at k = 768 whatever m and n. Measured, int8 and widened: 1 x 128 x 3072 29.9 and 9.1 us, 77 x 9216 x
+    // 3072 32.8 and 17.2, 4096 x 32 x 3072 30.8 and 11.4, 1 x 18432 x 3072 31.5 and 28.2, 1 x 32 x 256 5.9 and 9.4,
+    // 255 x 4096 x 256 9.0 and 9.3; with more tiles than SMs the widened form leads at any k.
+    const bool widened_is_faster = k >= 768 || (m >= 256 && n >= 256);
+    if (path == 2 || (path == 0 && pair_takes_it && widened_is_faster)) {
         const size_t a_bytes = (static_cast<size_t>(m) * k + 255) & ~static_cast<size_t>(255);
         const size_t w_bytes = static_cast<size_t>(n) * k;
         uint8_t *scratch = nullptr;
@@ -654,8 +666,7 @@ int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, co
         const cudaError_t allocated = pool == nullptr ? cudaErrorMemoryAllocation
                                                       : cudaMallocFromPoolAsync(reinterpret_cast<void **>(&scratch), a_bytes + w_bytes, pool, stream);
         if (allocated == cudaSuccess) {
-            int status = qi_w4a4_widen_codes_ex(a_codes, scratch, m, k, stream);
-            if (status == 0) status = qi_w4a4_widen_codes_ex(w_codes, scratch + a_bytes, n, k, stream);
+            int status = launch_widen_codes(a_codes, scratch, m, w_codes, scratch + a_bytes, n, k, stream);
             if (status == 0)
                 status = launch_w4a4_bytes(scratch, a_scales, scratch + a_bytes, w_scales, bias, y, shape, stream, device);
             const cudaError_t freed = cudaFreeAsync(scratch, stream);
@@ -721,11 +732,7 @@ int qi_w4a4_widen_codes_ex(const void *codes, void *bytes, long long rows, int k
     if (rows < 0 || k <= 0 || k % 32 != 0) return INVALID;
     if (rows == 0) return 0;
     if (!codes || !bytes || !aligned16(codes) || !aligned16(bytes)) return INVALID;
-    const long long chunks = rows * (k / 32);
-    const long long blocks = (chunks + 255) / 256;
-    if (blocks > 0x7fffffffLL) return INVALID;
-    return static_cast<int>(launch_overlapped(w4a4_wide::widen_codes_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
-                                              static_cast<const uint8_t *>(codes), static_cast<uint8_t *>(bytes), chunks));
+    return launch_widen_codes(codes, bytes, rows, nullptr, nullptr, 0, k, static_cast<cudaStream_t>(stream));
 }
 
 int qi_w4a4_gemm_wide_ex(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
@@ -838,8 +845,7 @@ int qi_w4a4_gemm_noalloc_ex(const void *a_codes, const void *a_scales, const voi
         address[device].store(scratch, std::memory_order_release);
     }
     const cudaStream_t on = static_cast<cudaStream_t>(stream);
-    int status = qi_w4a4_widen_codes_ex(a_codes, scratch, m, k, stream);
-    if (status == 0) status = qi_w4a4_widen_codes_ex(w_codes, scratch + a_bytes, n, k, stream);
+    const int status = launch_widen_codes(a_codes, scratch, m, w_codes, scratch + a_bytes, n, k, on);
     if (status != 0) return status;
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
     return launch_w4a4_bytes(scratch, a_scales, scratch + a_bytes, w_scales, bias, y, shape, on, device);
@@ -878,9 +884,7 @@ int qi_w4a16_gemm_ex(const void *x_half, const void *codes, const void *scales, 
 int qi_w4a16_gemm_tile_ex(const void *x_half, const void *codes, const void *scales, const void *minimums,
                           const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, int tile,
                           void *stream) {
-#ifndef SWEEP
     if (tile < 0 || tile > 5) return INVALID;
-#endif
     return w4a16_gemm(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, tile, static_cast<cudaStream_t>(stream));
 }
 

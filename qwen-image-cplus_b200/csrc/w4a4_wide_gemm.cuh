@@ -59,34 +59,54 @@ struct Tile {
     static_assert((3 * STAGES + 2 * BUFFERS) * 8 + 8 <= BARRIER_BYTES, "barrier block");
 };
 
-// Packed nibbles -> one E4M3 byte per code, same element order. One thread per 16 input bytes.
-__global__ void widen_codes_kernel(const uint8_t *__restrict__ codes, uint8_t *__restrict__ bytes, long long chunks) {
+// Four signed nibbles in the low half of `codes` -> four E4M3 bytes, same order. A byte permute whose selector is the
+// nibble itself reads a table of eight by the low three bits and gives the table byte's sign (0 here) where the fourth
+// bit is set, so the magnitudes of 0..7 and of -8..-1 come from one permute each and the sign bits from a third.
+__device__ __forceinline__ uint32_t signed_permute(uint32_t low, uint32_t high, uint32_t selector) {
+    uint32_t out;  // __byte_perm does not promise the sign form
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(out) : "r"(low), "r"(high), "r"(selector));
+    return out;
+}
+__device__ __forceinline__ uint32_t e4m3_of_nibbles(uint32_t codes, uint32_t signs) {
+    const uint32_t up = signed_permute(0x44403800u, 0x4E4C4A48u, codes);              // 0, 1, 2, 3 | 4, 5, 6, 7
+    const uint32_t down = signed_permute(0x4A4C4E50u, 0x38404448u, codes ^ 0x8888u);  // 8, 7, 6, 5 | 4, 3, 2, 1
+    return up | down | (signs & 0x80808080u);
+}
+
+constexpr int WIDEN_THREADS = 256, WIDEN_PIECES = 4;
+
+// Packed nibbles -> one E4M3 byte per code, same element order, for one or two matrices in one launch. Bound by memory
+// (half a byte in, one byte out per code): a thread takes WIDEN_PIECES pieces of 8 bytes, all loaded before the first is
+// used, and a warp stores 512 consecutive bytes at a time.
+struct Widening {
+    const uint8_t *codes;
+    uint8_t *bytes;
+    long long pieces;  // of 8 bytes of codes
+};
+__global__ void __launch_bounds__(WIDEN_THREADS) widen_codes_kernel(const Widening first, const Widening second, int first_blocks) {
     grid_wait();
     grid_release();
-    const long long chunk = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (chunk >= chunks) return;
-    const uint4 packed = __ldg(reinterpret_cast<const uint4 *>(codes) + chunk);
-    const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
-    uint32_t out[8];
+    const bool is_first = static_cast<int>(blockIdx.x) < first_blocks;
+    const Widening work = is_first ? first : second;
+    const long long block = is_first ? blockIdx.x : blockIdx.x - first_blocks;
+    const long long start = block * (WIDEN_THREADS * WIDEN_PIECES) + threadIdx.x;
+    uint2 packed[WIDEN_PIECES];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int i = 0; i < WIDEN_PIECES; ++i)
+        if (start + i * WIDEN_THREADS < work.pieces) packed[i] = __ldg(reinterpret_cast<const uint2 *>(work.codes) + start + i * WIDEN_THREADS);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t four = 0;
+    for (int i = 0; i < WIDEN_PIECES; ++i) {
+        if (start + i * WIDEN_THREADS >= work.pieces) break;
+        const uint32_t words[2] = {packed[i].x, packed[i].y};
+        uint32_t out[4];
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const int nibble = h * 4 + p * 2;
-                const float lo = static_cast<float>((static_cast<int32_t>(words[w] << (28 - 4 * nibble))) >> 28);
-                const float hi = static_cast<float>((static_cast<int32_t>(words[w] << (24 - 4 * nibble))) >> 28);
-                const uint32_t pair = __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
-                four |= pair << (16 * p);
-            }
-            out[2 * w + h] = four;
+        for (int w = 0; w < 2; ++w) {
+            const uint32_t even = words[w] << 4;  // the even nibbles' signs to their bytes' top bits
+            out[2 * w] = e4m3_of_nibbles(words[w], __byte_perm(even, words[w], 0x5140));
+            out[2 * w + 1] = e4m3_of_nibbles(words[w] >> 16, __byte_perm(even, words[w], 0x7362));
         }
+        reinterpret_cast<uint4 *>(work.bytes)[start + i * WIDEN_THREADS] = make_uint4(out[0], out[1], out[2], out[3]);
     }
-    uint4 *destination = reinterpret_cast<uint4 *>(bytes) + 2 * chunk;
-    destination[0] = make_uint4(out[0], out[1], out[2], out[3]);
-    destination[1] = make_uint4(out[4], out[5], out[6], out[7]);
 }
 
 template <int STAGES, bool DUMP_DOTS>

@@ -504,6 +504,27 @@ def test_widen_codes_matches_e4m3_table(qi):
     assert np.array_equal(out.cpu().numpy(), e4m3_of_codes(codes))
 
 
+@pytest.mark.parametrize("rows,k", [(1, 32), (33, 992), (16, 1024), (3, 5472)])  # around 16384 codes a block
+def test_widen_codes_at_the_edges_of_its_blocks(qi, rows, k):
+    codes = np.random.default_rng(92 + rows).integers(0, 256, size=(rows, k // 2), dtype=np.uint8)
+    out = torch.full((rows * k + 64,), 0xAB, dtype=torch.uint8, device="cuda")
+    assert qi.w4a4_widen_codes_ex(up(codes), out, rows, k) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(out[:rows * k].cpu().numpy().reshape(rows, k), e4m3_of_codes(codes))
+    assert bool((out[rows * k:] == 0xAB).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 32, 512), (1, 32, 768), (5, 96, 1024), (300, 32, 768), (17, 288, 4096)])
+def test_w4a4_packed_few_rows_or_outputs_by_shape(qi, m, n, k):
+    rng = np.random.default_rng(94 + m + n + k)
+    w_codes, w_scales = qt.pack_w4a4(qt.make_weights(rng, n, k))
+    a_codes, a_scales = qo.quantize_activations(qt.make_activations(rng, m, k))
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a4_gemm_ex(up(a_codes), up(a_scales), up(w_codes), up(w_scales), None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f16"])
 def test_quantize_wide_writes_the_same_codes_as_bytes(qi, dtype):
     rng = np.random.default_rng(93)
