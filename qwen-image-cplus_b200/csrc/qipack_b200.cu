@@ -542,9 +542,9 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
         }
         for (int i = now; i < w4a16::STREAM_GROUP; ++i) group.item[i] = {nullptr, nullptr, nullptr, nullptr, nullptr};
         const long long tiles = static_cast<long long>(now) * (n / w4a16::STREAM_ROWS);
-        w4a16::gemv_stream_grouped_kernel<<<tiles < resident ? static_cast<int>(tiles) : resident, w4a16::STREAM_THREADS, smem_bytes, stream>>>(
-            static_cast<const __half *>(x_half), group, now, m, n, k, ldy, y_dtype == QI_DTYPE_F16, stages);
-        const cudaError_t launched = cudaGetLastError();
+        const cudaError_t launched = launch_overlapped(w4a16::gemv_stream_grouped_kernel, tiles < resident ? static_cast<int>(tiles) : resident,
+                                                       w4a16::STREAM_THREADS, smem_bytes, stream, static_cast<const __half *>(x_half), group,
+                                                       now, m, n, k, ldy, y_dtype == QI_DTYPE_F16, stages);
         if (launched != cudaSuccess) return static_cast<int>(launched);
     }
     return 0;

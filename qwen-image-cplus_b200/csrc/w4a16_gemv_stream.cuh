@@ -13,14 +13,15 @@
 // per tile, 18432 x 3072 went from 14.7 to 11.9 us alone and from 9.1 to 7.5 us in groups of 60 (512 threads: 12.2 and
 // 7.9; 1024: 11.6 and 8.0).
 //
-// Unpacking is what the SMs spend their time on (measured on 18432 x 3072: copies alone 6 us, unpacking alone
-// 10 us, the tensor-core step nothing), so it is cut to three instructions per two weights. A nibble moved to
-// bits 6..9 of a 16-bit lane is the fp16 denormal code * 2^-18; one half2 fused multiply-add with the scale
-// times 2^18 and the minimum gives fp16(code * scale + minimum) with a single rounding, which is what the
-// reference's __float2half(fmaf(code, scale, minimum)) gives whenever |w| <= 1 (gemm.cu:229-230; see
-// w4a16_gemm.cuh). A word of eight nibbles yields the pairs (0,4), (1,5), (2,6), (3,7) by one shift and one
-// mask each; the activations are stored once per CTA in shared memory in that order. A scale of 1/4 or more,
-// whose 2^18-fold is no fp16 number, sends the warp's step down a slower path with the same pairing.
+// Unpacking is what the SMs spend their time on (18432 x 3072 in groups of 60: the copies alone 4.6 us a matrix; before,
+// 62 % of the integer pipe and 205 instructions per 2048 weights, 7.5 us; now 167 and 6.3 us; alone 11.9 -> 10.8), so it is
+// cut to ten instructions per eight weights. A nibble moved to bits 2..5 or 6..9 of a 16-bit lane is the fp16 denormal
+// code * 2^-22 or code * 2^-18, so one shift serves two nibbles; one half2 fused multiply-add with the scale times 2^22 or
+// 2^18 and the minimum gives fp16(code * scale + minimum) with a single rounding, which is what the reference's
+// __float2half(fmaf(code, scale, minimum)) gives whenever |w| <= 1 (gemm.cu:229-230; see w4a16_gemm.cuh). A word of eight
+// nibbles yields the pairs (0,4), (1,5), (2,6), (3,7); the activations are stored once per CTA in shared memory in that
+// order. A scale of 1/64 or more, whose 2^22-fold is no fp16 number, sends the warp's step down a path in which the smaller
+// multiple alone is used (below 1/4), or down the slowest, with each code made an fp16 integer first.
 #pragma once
 #include "ptx.cuh"
 #include "w4a16_gemv.cuh"
@@ -33,7 +34,10 @@ constexpr int STREAM_TEAMS = 4, STREAM_TEAM_WARPS = STREAM_THREADS / 32 / STREAM
 constexpr int STREAM_MAX_K = 4096;  // 16 rows of codes, scales and minimums: 36 KB per stage
 
 __host__ __device__ constexpr int stream_stage_bytes(int k) { return STREAM_ROWS * (k / 2) + 2 * STREAM_ROWS * (k / 64) * 2; }
-__host__ __device__ constexpr int stream_x_bytes(int m, int k) { return m * k * 2; }
+// a row of activations: a step's 16 pieces of 16 bytes, the four lanes' first pieces, their second, ...; 64 bytes more
+// set the next row on the other banks
+__host__ __device__ constexpr int stream_x_pieces(int k) { return (k + 127) / 128 * 16 + 4; }
+__host__ __device__ constexpr int stream_x_bytes(int m, int k) { return m * stream_x_pieces(k) * 16; }
 
 // global -> shared, any multiple of 16 bytes, both addresses 16-byte aligned; completion on an mbarrier of this CTA
 __device__ __forceinline__ void bulk_load(void *smem, const void *global, uint32_t bytes, uint64_t *barrier) {
@@ -42,14 +46,18 @@ __device__ __forceinline__ void bulk_load(void *smem, const void *global, uint32
                  : "memory");
 }
 
-// Eight nibbles of one row -> four half2 of dequantised weights, pairs (0,4), (1,5), (2,6), (3,7).
-// scale_up = scale * 2^18 in both lanes.
-__device__ __forceinline__ void unpack_word(uint32_t word, __half2 scale_up, __half2 minimum2, uint32_t (&out)[4]) {
-    uint32_t moved[4] = {(word << 6) & 0x03C003C0u, (word << 2) & 0x03C003C0u, (word >> 2) & 0x03C003C0u,
-                         (word >> 6) & 0x03C003C0u};
+// Eight nibbles of one row -> four half2 of dequantised weights, pairs (0,4), (1,5), (2,6), (3,7). A nibble at bits 2..5 of
+// a 16-bit lane is code * 2^-22 and takes the scale times 2^22, at bits 6..9 it is code * 2^-18 and takes it times 2^18.
+// LARGE: the scale times 2^18 only, the nibbles at bits 2..5 times 16 first (exact).
+template <bool LARGE>
+__device__ __forceinline__ void unpack_word(uint32_t word, __half2 scale_22, __half2 scale_18, __half2 minimum2, uint32_t (&out)[4]) {
+    const uint32_t up = word << 2, down = word >> 6;
+    const uint32_t moved[4] = {up & 0x003C003Cu, up & 0x03C003C0u, down & 0x003C003Cu, down & 0x03C003C0u};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const __half2 weight = __hfma2(*reinterpret_cast<__half2 *>(&moved[j]), scale_up, minimum2);
+        __half2 code = *reinterpret_cast<const __half2 *>(&moved[j]);
+        if (LARGE && j % 2 == 0) code = __hmul2(code, scale_22);  // sixteen
+        const __half2 weight = __hfma2(code, !LARGE && j % 2 == 0 ? scale_22 : scale_18, minimum2);
         out[j] = *reinterpret_cast<const uint32_t *>(&weight);
     }
 }
@@ -90,7 +98,7 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     __shared__ uint64_t full[STREAM_MAX_STAGES];
     __shared__ volatile int fetched[STREAM_MAX_STAGES];  // the tile that was last sent for into each stage
-    __shared__ float partials[STREAM_TEAMS][2][STREAM_TEAM_WARPS][16][8];
+    __shared__ alignas(8) float partials[STREAM_TEAMS][2][STREAM_TEAM_WARPS][16][8];
     const int team = threadIdx.x / (STREAM_TEAM_WARPS * 32), warp = threadIdx.x / 32 % STREAM_TEAM_WARPS, lane = threadIdx.x & 31;
     const int team_thread = threadIdx.x % (STREAM_TEAM_WARPS * 32);
     const int r = lane >> 2, q = lane & 3;
@@ -109,11 +117,14 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     grid_wait();
     grid_release();
     // the activations, once per CTA, every eight inputs in the order (0,4,1,5,2,6,3,7) the unpacked pairs have
-    uint4 *x_pairs = reinterpret_cast<uint4 *>(smem + static_cast<size_t>(stages) * stage_bytes);  // [m][k / 8]
-    for (int item = threadIdx.x; item < m * (k / 8); item += STREAM_THREADS) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(x) + item);
-        x_pairs[item] = make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410),
-                                   __byte_perm(v.y, v.w, 0x7632));
+    uint4 *x_pairs = reinterpret_cast<uint4 *>(smem + static_cast<size_t>(stages) * stage_bytes);
+    const int x_row = stream_x_pieces(k);
+    for (int item = threadIdx.x; item < m * steps * 16; item += STREAM_THREADS) {
+        const int row = item / (steps * 16), piece = item % (steps * 16);  // input / 8; a ragged last step is filled with zeros
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (piece < k / 8) v = __ldg(reinterpret_cast<const uint4 *>(x) + static_cast<size_t>(row) * (k / 8) + piece);
+        x_pairs[row * x_row + piece / 16 * 16 + piece % 4 * 4 + piece / 4 % 4] =
+            make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
     }
     __syncthreads();
     auto fetch = [&](int tile, int s) {  // one thread
@@ -139,9 +150,11 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         for (int s = 0; s < stages && tile < tiles; ++s, tile += gridDim.x) fetch(tile, s);
     }
 
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    const __half nothing = __ushort_as_half(0), quarter = __float2half(0.25f), two_to_9 = __ushort_as_half(0x6000);
-    const bool has_x = r < m;
+    const __half nothing = __ushort_as_half(0);
+    const __half2 sixty_fourth = __float2half2_rn(1.0f / 64.0f), quarter = __float2half2_rn(0.25f), two_to_9 = __float2half2_rn(512.0f), sixteen = __float2half2_rn(16.0f);
+    // Activation row lane / 4 is the B operand's column of that number, and a column only ever meets its own results: a
+    // lane past the last row feeds row 0 again, and what comes of it is not stored.
+    const uint4 *my_x = x_pairs + (r < m ? r : 0) * x_row + q;
     // Team t takes the CTA's tiles t, t + 4, ...; tile i of the CTA lies in stage i modulo the number of stages.
     uint32_t s = team, phase = 0;
     while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
@@ -163,53 +176,58 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (arrived) {
             for (int step = warp; step < steps; step += STREAM_TEAM_WARPS) {
-                const int g = 2 * step + (q >> 1), half_group = q & 1;
-                const bool valid = g < groups;  // every lane runs the same mma.sync; a lane past a ragged end feeds zeros
-                const int column = g * 32 + half_group * 16;  // byte offset of this lane's 32 codes in a row
-                const uint4 code_a = valid ? *reinterpret_cast<const uint4 *>(stage + r * (k / 2) + column) : zero;
-                const uint4 code_b = valid ? *reinterpret_cast<const uint4 *>(stage + (r + 8) * (k / 2) + column) : zero;
-                const __half scale_a = valid ? stage_scales[r * groups + g] : nothing;
-                const __half scale_b = valid ? stage_scales[(r + 8) * groups + g] : nothing;
-                const __half2 ma = __half2half2(valid ? stage_minimums[r * groups + g] : nothing);
-                const __half2 mb = __half2half2(valid ? stage_minimums[(r + 8) * groups + g] : nothing);
+                const int g = 2 * step + (q >> 1);  // this lane's group; q & 1 is the half of it
+                const uint8_t *my_codes = stage + r * (k / 2) + step * 64 + q * 16;
+                const uint4 code_a = *reinterpret_cast<const uint4 *>(my_codes);
+                const uint4 code_b = *reinterpret_cast<const uint4 *>(my_codes + 8 * (k / 2));
+                __half scale_a = stage_scales[r * groups + g], scale_b = stage_scales[(r + 8) * groups + g];
+                __half minimum_a = stage_minimums[r * groups + g], minimum_b = stage_minimums[(r + 8) * groups + g];
+                if (2 * step + 1 >= groups && q >= 2) {  // past a ragged end: what was read lies in the CTA's shared memory; zeros
+                    scale_a = scale_b = minimum_a = minimum_b = nothing;
+                }
                 const uint32_t wa[4] = {code_a.x, code_a.y, code_a.z, code_a.w};
                 const uint32_t wb[4] = {code_b.x, code_b.y, code_b.z, code_b.w};
-                // activation row (lane / 4) supplies the B operand for the same 32 inputs
-                const uint4 *px = x_pairs + static_cast<size_t>(r) * (k / 8) + g * 8 + half_group * 4;
-                const bool has_operand = has_x && valid;
-                // scale * 2^18 stays an fp16 number below 1/4 (a NaN fails the test and takes the other path too)
-                const bool small = __hlt(__habs(scale_a), quarter) && __hlt(__habs(scale_b), quarter);
-                if (__all_sync(0xffffffffu, small)) {
-                    const __half2 sa = __half2half2(__hmul(__hmul(scale_a, two_to_9), two_to_9));
-                    const __half2 sb = __half2half2(__hmul(__hmul(scale_b, two_to_9), two_to_9));
+                const __half2 ma = __half2half2(minimum_a), mb = __half2half2(minimum_b);
+                const uint4 *px = my_x + step * 16;
+                auto multiply = [&](auto unpack) {
 #pragma unroll
                     for (int w = 0; w < 4; ++w) {  // 8 inputs of each row per word, two MMA steps
-                        const uint4 xv = has_operand ? px[w] : zero;
+                        const uint4 xv = px[4 * w];
                         uint32_t pa[4], pb[4];
-                        unpack_word(wa[w], sa, ma, pa);
-                        unpack_word(wb[w], sb, mb, pb);
+                        unpack(wa[w], wb[w], pa, pb);
                         const uint32_t first[4] = {pa[0], pb[0], pa[1], pb[1]}, second[4] = {pa[2], pb[2], pa[3], pb[3]};
                         mma_m16n8k16(c, first, xv.x, xv.y);
                         mma_m16n8k16(c, second, xv.z, xv.w);
                     }
+                };
+                // scale * 2^22 is an fp16 number below 1/64, scale * 2^18 below 1/4 (a NaN fails both tests)
+                const __half2 magnitudes = __habs2(__halves2half2(scale_a, scale_b));
+                if (__all_sync(0xffffffffu, __hblt2(magnitudes, sixty_fourth))) {
+                    const __half2 sa = __hmul2(__hmul2(__half2half2(scale_a), two_to_9), two_to_9), sa_22 = __hmul2(sa, sixteen);
+                    const __half2 sb = __hmul2(__hmul2(__half2half2(scale_b), two_to_9), two_to_9), sb_22 = __hmul2(sb, sixteen);
+                    multiply([&](uint32_t a, uint32_t b, uint32_t(&pa)[4], uint32_t(&pb)[4]) {
+                        unpack_word<false>(a, sa_22, sa, ma, pa);
+                        unpack_word<false>(b, sb_22, sb, mb, pb);
+                    });
+                } else if (__all_sync(0xffffffffu, __hblt2(magnitudes, quarter))) {
+                    const __half2 sa = __hmul2(__hmul2(__half2half2(scale_a), two_to_9), two_to_9);
+                    const __half2 sb = __hmul2(__hmul2(__half2half2(scale_b), two_to_9), two_to_9);
+                    multiply([&](uint32_t a, uint32_t b, uint32_t(&pa)[4], uint32_t(&pb)[4]) {
+                        unpack_word<true>(a, sixteen, sa, ma, pa);
+                        unpack_word<true>(b, sixteen, sb, mb, pb);
+                    });
                 } else {
                     const __half2 sa = __half2half2(scale_a), sb = __half2half2(scale_b);
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const uint4 xv = has_operand ? px[w] : zero;
-                        uint32_t pa[4], pb[4];
-                        unpack_word_any_scale(wa[w], sa, ma, pa);
-                        unpack_word_any_scale(wb[w], sb, mb, pb);
-                        const uint32_t first[4] = {pa[0], pb[0], pa[1], pb[1]}, second[4] = {pa[2], pb[2], pa[3], pb[3]};
-                        mma_m16n8k16(c, first, xv.x, xv.y);
-                        mma_m16n8k16(c, second, xv.z, xv.w);
-                    }
+                    multiply([&](uint32_t a, uint32_t b, uint32_t(&pa)[4], uint32_t(&pb)[4]) {
+                        unpack_word_any_scale(a, sa, ma, pa);
+                        unpack_word_any_scale(b, sb, mb, pb);
+                    });
                 }
             }
         }
         // c[0], c[1]: weight row r, activation rows 2q, 2q+1; c[2], c[3]: weight row r + 8
-        partial[warp][r][2 * q] = c[0], partial[warp][r][2 * q + 1] = c[1];
-        partial[warp][r + 8][2 * q] = c[2], partial[warp][r + 8][2 * q + 1] = c[3];
+        *reinterpret_cast<float2 *>(&partial[warp][r][2 * q]) = make_float2(c[0], c[1]);
+        *reinterpret_cast<float2 *>(&partial[warp][r + 8][2 * q]) = make_float2(c[2], c[3]);
         // The team is done with the stage, and the partial sums are complete. The sums alternate between two places: those of
         // this tile are read below and written again two tiles on, with the next tile's barrier in between.
         named_barrier_sync(1 + team, STREAM_TEAM_WARPS * 32);
@@ -217,8 +235,9 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
             const int next = tile + stages * gridDim.x;
             if (next < tiles) fetch(next, s);
         }
-        {  // fixed-order sum over the K slices: thread -> (weight row, activation row)
-            const int row = team_thread >> 3, b = team_thread & 7;
+        // fixed-order sum over the K slices: thread -> (activation row, weight row), so that few rows keep few warps
+        const int b = team_thread >> 4, row = team_thread & 15;
+        if (b < m) {
             const float *to_bias = bias;
             void *to_y = y;
             int local_tile = tile;
@@ -228,14 +247,12 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
                 local_tile = tile % tiles_each;
             }
             const int out_row = local_tile * STREAM_ROWS + row;
-            if (b < m && row < STREAM_ROWS) {
-                float total = 0.0f;
+            float total = 0.0f;
 #pragma unroll
-                for (int slice = 0; slice < STREAM_TEAM_WARPS; ++slice) total += partial[slice][row][b];
-                if (to_bias != nullptr) total += __ldg(to_bias + out_row);
-                if (y_is_half) static_cast<__half *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = __float2half_rn(total);
-                else static_cast<float *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = total;
-            }
+            for (int slice = 0; slice < STREAM_TEAM_WARPS; ++slice) total += partial[slice][row][b];
+            if (to_bias != nullptr) total += __ldg(to_bias + out_row);
+            if (y_is_half) static_cast<__half *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = __float2half_rn(total);
+            else static_cast<float *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = total;
         }
         s += STREAM_TEAMS;
         while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;

@@ -297,6 +297,23 @@ def test_w4a16_gemv_scales_of_every_size(qi, m):
     assert qt.max_relative_error(y.cpu().numpy(), expected) <= OUTPUT_TOLERANCE
 
 
+@pytest.mark.parametrize("low,high", [(2.0 ** -9, 1 / 64 - 2.0 ** -16), (1 / 64, 1 / 4 - 2.0 ** -12), (1 / 4, 1.0)])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 64), (8, 48, 4096), (5, 2384, 1216)])
+def test_w4a16_gemv_scales_of_one_range(qi, m, n, k, low, high):
+    # all scales of a matrix in one of the three ranges that the unpack tells apart, both ends of each included
+    rng = np.random.default_rng(3150 + m + n + k)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    scales = rng.uniform(low, high, size=(n, k // 64)).astype(np.float16)
+    scales[0, 0], scales[-1, -1] = np.float16(low), np.float16(-high)
+    minimums = (-7.5 * scales.astype(np.float32)).astype(np.float16)
+    x16 = qt.make_activations(rng, m, k)
+    expected = qo.w4a16_gemm(x16, codes, scales.view(np.uint16), minimums.view(np.uint16))
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(up(x16), up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert qt.max_relative_error(y.cpu().numpy(), expected) <= OUTPUT_TOLERANCE
+
+
 @pytest.mark.parametrize("m,count,n,k", [(1, 3, 1024, 1216), (1, 70, 256, 512), (2, 5, 18432, 3072)])
 def test_w4a16_gemv_grouped_matches_oracle_and_the_single_launches(qi, m, count, n, k):
     """Several matrices of one shape against the same activations in one launch (two for more than 64 matrices): every
