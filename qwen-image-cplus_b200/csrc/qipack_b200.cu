@@ -395,27 +395,28 @@ int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_by
                                               bias, y, dots, shape, outputs, tiling));
 }
 
-template <int BN>
+template <int BN, bool EXCHANGED>
 int launch_w4a4_narrow(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
                        void *y, const GemmShape &shape, cudaStream_t stream, int device) {
     namespace wn = w4a4_narrow;
     using T = wn::Tile<BN>;
+    const int rows = EXCHANGED ? shape.n : shape.m, columns = EXCHANGED ? shape.m : shape.n;
     // rows that do not exist are not loaded: what the tensor cores make of the rest of the tile nobody reads
-    const int box_rows = shape.m >= wn::BM ? wn::BM : (shape.m + 15) / 16 * 16;
-    CUtensorMap map_a, map_w;
-    if (!make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_bytes, shape.k, shape.m, static_cast<uint64_t>(shape.k),
+    const int box_rows = rows >= wn::BM ? wn::BM : (rows + 15) / 16 * 16;
+    CUtensorMap map_rows, map_columns;
+    if (!make_map(&map_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, EXCHANGED ? w_bytes : a_bytes, shape.k, rows, static_cast<uint64_t>(shape.k),
                   128, box_rows, CU_TENSOR_MAP_SWIZZLE_128B))
         return INVALID;
-    if (!make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w_bytes, shape.k, shape.n, static_cast<uint64_t>(shape.k),
+    if (!make_map(&map_columns, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, EXCHANGED ? a_bytes : w_bytes, shape.k, columns, static_cast<uint64_t>(shape.k),
                   128, BN, CU_TENSOR_MAP_SWIZZLE_128B))
         return INVALID;
     static std::atomic<bool> configured[MAX_DEVICES];
-    if (const cudaError_t error = configure_once(wn::gemm_kernel<BN>, T::SMEM_BYTES, configured[device])) return static_cast<int>(error);
-    const int tiles = ((shape.m + wn::BM - 1) / wn::BM) * ((shape.n + BN - 1) / BN);
+    if (const cudaError_t error = configure_once(wn::gemm_kernel<BN, EXCHANGED>, T::SMEM_BYTES, configured[device])) return static_cast<int>(error);
+    const int tiles = ((rows + wn::BM - 1) / wn::BM) * ((columns + BN - 1) / BN);
     const int grid = tiles < sm_count(device) ? tiles : sm_count(device);
-    return static_cast<int>(launch_overlapped(wn::gemm_kernel<BN>, grid, wn::THREADS, T::SMEM_BYTES, stream, map_a, map_w,
-                                              static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
-                                              bias, y, shape, box_rows));
+    return static_cast<int>(launch_overlapped(wn::gemm_kernel<BN, EXCHANGED>, grid, wn::THREADS, T::SMEM_BYTES, stream, map_rows, map_columns,
+                                              static_cast<const __half *>(EXCHANGED ? w_scales : a_scales),
+                                              static_cast<const __half *>(EXCHANGED ? a_scales : w_scales), bias, y, shape, box_rows));
 }
 
 // Byte operands with k a multiple of 256 and 8-byte aligned scales: CTA pairs, or single CTAs with 64 or 32 columns where
@@ -431,8 +432,24 @@ int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_b
     const long long tiles_m = (shape.m + wn::BM - 1) / wn::BM;
     const long long waves_64 = (tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms, waves_32 = (tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms;
     const double us_64 = waves_64 * (waves_64 == 1 ? 0.185 : 0.21), us_32 = waves_32 * (waves_32 == 1 ? 0.12 : 0.135);
-    if (us_64 <= us_32 && us_64 < pair_us) return launch_w4a4_narrow<64>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    if (us_32 < pair_us) return launch_w4a4_narrow<32>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    // Weights as the 128 rows of a tile, activation rows as its columns, where that folds less for rows that do not exist:
+    // 0.115, 0.135 and 0.16 for 16, 32 and 48 columns, 15 % more in several waves (16 x 9216 x 3072 11.3 -> 8.7 us, 77 x
+    // 9216 x 3072 11.7 -> 10.4, 77 x 12288 x 3072 18.3 -> 15.4, 256 x 3072 x 3072 11.8 -> 10.0, 16 x 15776 x 768 8.3 -> 6.3).
+    const double others_us = us_64 < us_32 ? (us_64 < pair_us ? us_64 : pair_us) : (us_32 < pair_us ? us_32 : pair_us);
+    const long long tiles_n = (shape.n + wn::BM - 1) / wn::BM;
+    const auto exchanged_us = [&](int columns, double us) {
+        const long long waves = (tiles_n * ((shape.m + columns - 1) / columns) + sms - 1) / sms;
+        return waves == 1 ? us : waves * us * 1.15;
+    };
+    const double us_16_rows = exchanged_us(16, 0.115), us_32_rows = exchanged_us(32, 0.135), us_48_rows = exchanged_us(48, 0.16);
+    if (us_16_rows <= us_32_rows && us_16_rows <= us_48_rows && us_16_rows < others_us)
+        return launch_w4a4_narrow<16, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    if (us_32_rows <= us_48_rows && us_32_rows < others_us)
+        return launch_w4a4_narrow<32, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    if (us_48_rows < others_us)
+        return launch_w4a4_narrow<48, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    if (us_64 <= us_32 && us_64 < pair_us) return launch_w4a4_narrow<64, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    if (us_32 < pair_us) return launch_w4a4_narrow<32, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
     return launch_w4a4_pair(a_bytes, a_scales, w_bytes, w_scales, bias, y, nullptr, shape, stream, device);
 }
 

@@ -542,6 +542,24 @@ def test_w4a4_packed_few_rows_or_outputs_by_shape(qi, m, n, k):
     assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 32, 256), (16, 4000, 512), (17, 3072, 1024), (33, 9216, 256), (77, 9216, 512), (96, 9248, 256), (130, 3072, 512), (77, 12288, 256), (256, 3072, 768)])
+def test_w4a4_wide_few_rows_as_columns(qi, m, n, k):
+    rng = np.random.default_rng(95 + m + n + k)
+    w_codes, w_scales = qt.random_w4a4_pack(rng, n, k, 1e-3, 6e-3)
+    a_codes, a_scales = qt.random_w4a4_pack(rng, m, k, 0.05, 0.6)
+    bias = qt.make_bias(rng, n)
+    expected = qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales, bias=bias)
+    args = (up(e4m3_of_codes(a_codes)), up(a_scales), up(e4m3_of_codes(w_codes)), up(w_scales), up(bias))
+    y = torch.full((m + 1, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a4_gemm_wide_ex(*args, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert np.array_equal(y[:m].cpu().numpy(), expected) and bool(torch.isnan(y[m]).all())
+    y16 = torch.zeros(m, n, dtype=torch.float16, device="cuda")
+    assert qi.w4a4_gemm_wide_ex(*args, y16, qi.DTYPE_F16, n, m, n, k) == 0
+    check_status(qi)
+    assert np.array_equal(y16.cpu().numpy(), expected.astype(np.float16))
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f16"])
 def test_quantize_wide_writes_the_same_codes_as_bytes(qi, dtype):
     rng = np.random.default_rng(93)
