@@ -433,7 +433,7 @@ int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_b
     const long long waves_64 = (tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms, waves_32 = (tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms;
     const double us_64 = waves_64 * (waves_64 == 1 ? 0.185 : 0.21), us_32 = waves_32 * (waves_32 == 1 ? 0.12 : 0.135);
     // Weights as the 128 rows of a tile, activation rows as its columns, where that folds less for rows that do not exist:
-    // 0.115, 0.135 and 0.16 for 16, 32 and 48 columns, 15 % more in several waves (16 x 9216 x 3072 11.3 -> 8.7 us, 77 x
+    // 0.12, 0.135 (one block of rows: 0.105) and 0.16 for 16, 32 and 48 columns, 15 % more in several waves (16 x 9216 x 3072 11.3 -> 8.7 us, 77 x
     // 9216 x 3072 11.7 -> 10.4, 77 x 12288 x 3072 18.3 -> 15.4, 256 x 3072 x 3072 11.8 -> 10.0, 16 x 15776 x 768 8.3 -> 6.3).
     const double others_us = us_64 < us_32 ? (us_64 < pair_us ? us_64 : pair_us) : (us_32 < pair_us ? us_32 : pair_us);
     const long long tiles_n = (shape.n + wn::BM - 1) / wn::BM;
@@ -441,7 +441,7 @@ int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_b
         const long long waves = (tiles_n * ((shape.m + columns - 1) / columns) + sms - 1) / sms;
         return waves == 1 ? us : waves * us * 1.15;
     };
-    const double us_16_rows = exchanged_us(16, 0.115), us_32_rows = exchanged_us(32, 0.135), us_48_rows = exchanged_us(48, 0.16);
+    const double us_16_rows = exchanged_us(16, 0.12), us_32_rows = exchanged_us(32, shape.m <= 32 ? 0.105 : 0.135), us_48_rows = exchanged_us(48, 0.16);
     if (us_16_rows <= us_32_rows && us_16_rows <= us_48_rows && us_16_rows < others_us)
         return launch_w4a4_narrow<16, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
     if (us_32_rows <= us_48_rows && us_32_rows < others_us)
