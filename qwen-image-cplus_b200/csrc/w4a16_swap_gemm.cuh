@@ -15,7 +15,8 @@
 //   warps 4-19  four groups of four, steps in turn: a thread unpacks 128 codes of one weight row and stores them into its
 //               TMEM lane (tcgen05.st), where the tensor core reads them as its first operand: the unpacked weights
 //               never pass through shared memory
-//   warp 1      tcgen05.mma kind::f16 with A in TMEM (M = 128, N = columns, K = 16) x 8
+//   warps 1, 3  tcgen05.mma kind::f16 with A in TMEM (M = 128, N = columns, K = 16) x 8; up to 128 columns the two take
+//               the steps in turn, each into an accumulator of its own, above that warp 1 issues all
 // then all warps: accumulator -> shared memory, sum over the cluster, bias, store (rows of y contiguous per warp).
 #pragma once
 #include "ptx.cuh"
@@ -26,20 +27,23 @@ namespace w4a16_swap {
 
 constexpr int BK = 128, BN = 128;         // inputs per step: two quantisation groups; weight rows of a tile
 constexpr int MAX_COLUMNS = 256, MAX_STAGES = 8, MAX_SPLIT = 8;
+static_assert(MAX_STAGES % 2 == 0, "the longest ring");
 constexpr int PRODUCER_WARP = 0, MMA_WARP = 1, CODE_WARP = 2, SECOND_MMA_WARP = 3, UNPACK_WARP0 = 4;
-constexpr int ISSUERS = 2;
 constexpr int UNPACK_GROUPS = 4, UNPACK_WARPS = 4 * UNPACK_GROUPS;  // a group: one warp per 32 TMEM lanes; groups take the steps in turn
 constexpr int THREADS = 128 + 32 * UNPACK_WARPS;
 constexpr int A_SLOTS = 4, A_COLUMNS = BK / 2;  // TMEM columns of one unpacked step: two fp16 each
 constexpr int TMEM_COLUMNS = 512;
 static_assert(MAX_COLUMNS + A_SLOTS * A_COLUMNS <= TMEM_COLUMNS, "accumulator and unpacked steps");
 static_assert(A_SLOTS % UNPACK_GROUPS == 0, "a group keeps to its own slots");
+constexpr int TWO_ISSUERS_COLUMNS = 128;  // widest tile of which two accumulators fit
+static_assert(2 * TWO_ISSUERS_COLUMNS + A_SLOTS * A_COLUMNS <= TMEM_COLUMNS, "two accumulators and unpacked steps");
+__host__ __device__ constexpr int issuers_of(int columns) { return columns <= TWO_ISSUERS_COLUMNS ? 2 : 1; }
 constexpr int CODE_STEPS = 2, MAX_CODE_STAGES = 6;  // steps of codes fetched together: 128 bytes of a row; chunks in flight
 constexpr int CODE_BYTES = BN * CODE_STEPS * (BK / 2);
 constexpr int CODE_READERS = CODE_STEPS * 4;    // warps that read a chunk: one group per step
 static_assert(UNPACK_GROUPS % CODE_STEPS == 0, "a group's next step is in a chunk a whole number of chunks on");
 constexpr int BARRIER_BYTES = 512;
-static_assert((2 * MAX_STAGES + 2 * MAX_CODE_STAGES + 2 * A_SLOTS + ISSUERS + 1) * 8 + 4 <= BARRIER_BYTES, "barrier block");
+static_assert((2 * MAX_STAGES + 2 * MAX_CODE_STAGES + A_SLOTS + 1) * 8 + 4 <= BARRIER_BYTES, "barrier block");
 constexpr uint32_t AHEAD_BACKOFF_NS = 100, UNPACK_BACKOFF_NS = 20;  // pauses between polls: a polling warp takes issue slots
 
 struct Plan {
@@ -122,35 +126,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     const int columns = plan.columns, share = (plan.columns + plan.split - 1) / plan.split, stages = plan.stages, code_stages = plan.code_stages, split = plan.split, half_bytes = columns * 128, x_bytes = 2 * half_bytes;
     uint8_t *smem_x = smem, *smem_c = smem + stages * x_bytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + tile_bytes(columns, stages, code_stages));
-    uint64_t *empty = full + MAX_STAGES;
-    uint64_t *code_full = empty + MAX_STAGES;
+    uint64_t *step_done = full + MAX_STAGES;  // a ring: one commit says that a step's stage and its slot are free
+    uint64_t *code_full = step_done + MAX_STAGES;
     uint64_t *code_empty = code_full + MAX_CODE_STAGES;
     uint64_t *a_ready = code_empty + MAX_CODE_STAGES;
-    uint64_t *a_empty = a_ready + A_SLOTS;
-    uint64_t *token = a_empty + A_SLOTS;  // passes the turn between the two issuing warps
-    uint64_t *done = token + ISSUERS;
+    uint64_t *done = a_ready + A_SLOTS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = static_cast<int>(blockIdx.x) % split, tile = static_cast<int>(blockIdx.x) / split;
     const int tiles_n = (shape.n + BN - 1) / BN, groups = shape.k / 64, k_steps = (groups + 1) / 2;
     const int n0 = (tile % tiles_n) * BN, m0 = (tile / tiles_n) * columns;
+    // The ring is at least as long as the stages of activations and the slots of unpacked weights, and even, so that a barrier
+    // belongs to one issuer: it then completes for a later step only after both that wait on it have passed the earlier one.
+    // (With five barriers the other issuer's next step could complete a slot's barrier before the slot's own step was unpacked.)
+    const int issuers = issuers_of(columns), ring = ((stages >= A_SLOTS ? stages : A_SLOTS) + 1) / 2 * 2;
     const int first = k_steps * rank / split, steps = k_steps * (rank + 1) / split - first;  // this CTA's share of K
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) {
-            mbarrier_init(&full[s], 1);
-            mbarrier_init(&empty[s], 1);
-        }
+        for (int s = 0; s < stages; ++s) mbarrier_init(&full[s], 1);
+        for (int s = 0; s < ring; ++s) mbarrier_init(&step_done[s], 1);
         for (int s = 0; s < code_stages; ++s) {
             mbarrier_init(&code_full[s], 1);
             mbarrier_init(&code_empty[s], CODE_READERS);
         }
-        for (int s = 0; s < A_SLOTS; ++s) {
-            mbarrier_init(&a_ready[s], 4);
-            mbarrier_init(&a_empty[s], 1);
-        }
-        for (int i = 0; i < ISSUERS; ++i) mbarrier_init(&token[i], 1);
-        mbarrier_init(done, steps > 1 ? ISSUERS : 1);
+        for (int s = 0; s < A_SLOTS; ++s) mbarrier_init(&a_ready[s], 4);
+        mbarrier_init(done, steps < issuers ? steps : issuers);
         fence_barrier_init();
     }
     __syncthreads();
@@ -161,17 +161,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     // uniform registers; a diverged thread takes several times as long for the same few instructions.
     if (warp == PRODUCER_WARP) {
         if (elect_one()) prefetch_tensormap(&map_x);
-        const uint32_t full_u = smem_u32(full), empty_u = smem_u32(empty), x_u = smem_u32(smem_x);
-        uint32_t s = 0, phase = 1;
+        const uint32_t full_u = smem_u32(full), done_u = smem_u32(step_done), x_u = smem_u32(smem_x);
+        uint32_t s = 0;
+        int before = -1, before_phase = 0;  // the step that had the stage before
         for (int step = 0; step < steps; ++step) {
-            if (!mbarrier_wait_uniform(empty_u + s * 8, phase, &g_status, STATUS_WAIT_EMPTY | 0x8000 | s, AHEAD_BACKOFF_NS)) break;
+            if (step >= stages) {
+                if (++before == ring) before = 0, before_phase ^= 1;
+                if (!mbarrier_wait_uniform(done_u + before * 8, before_phase, &g_status, STATUS_WAIT_EMPTY | 0x8000 | s, AHEAD_BACKOFF_NS)) break;
+            }
             if (elect_one()) {
                 mbarrier_arrive_expect_tx_u32(full_u + s * 8, x_bytes);
                 tma_load_2d_u32(x_u + s * x_bytes, &map_x, full_u + s * 8, (first + step) * BK, m0);
                 tma_load_2d_u32(x_u + s * x_bytes + half_bytes, &map_x, full_u + s * 8, (first + step) * BK + 64, m0);
             }
             __syncwarp();
-            if (++s == static_cast<uint32_t>(stages)) s = 0, phase ^= 1;
+            if (++s == static_cast<uint32_t>(stages)) s = 0;
         }
     } else if (warp == CODE_WARP) {
         if (elect_one()) prefetch_tensormap(&map_codes);
@@ -195,36 +199,32 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         }
         named_barrier_sync(1, 32 * (2 + UNPACK_WARPS));
         tcgen05_fence_after();
-        const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + (TMEM_COLUMNS - A_SLOTS * A_COLUMNS);
-        // A step's waits, eight MMAs and commits take a warp some 600 cycles, the tensor cores four per column: two warps
-        // take the steps in turn. A token keeps the MMAs in the order of K, so that every bit of y is fixed.
+        // A step's waits, eight MMAs and commit take a warp some 600 cycles, the tensor cores four per column: up to 128
+        // columns two warps take the steps in turn, each into an accumulator of its own. Only the MMAs of ONE thread are sure
+        // to reach an accumulator in the order they were issued in; two warps on one accumulator, with a token that passed
+        // the turn, gave sums in another order from run to run. One warp for all: 77 x 12288 x 3072 12.4 -> 13.8 us.
         const uint32_t mine = warp == MMA_WARP ? 0 : 1;
+        const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + (TMEM_COLUMNS - A_SLOTS * A_COLUMNS), accumulator = tmem_base + mine * TWO_ISSUERS_COLUMNS;
         const uint32_t idesc = umma_idesc_f16_f32(BN, 0) | (static_cast<uint32_t>(columns >> 3) << 17);
-        const uint32_t full_u = smem_u32(full), empty_u = smem_u32(empty), a_ready_u = smem_u32(a_ready), a_empty_u = smem_u32(a_empty),
-                       done_u = smem_u32(done), token_u = smem_u32(token);
+        const uint32_t full_u = smem_u32(full), step_done_u = smem_u32(step_done), a_ready_u = smem_u32(a_ready), done_u = smem_u32(done);
         const uint64_t b_first = umma_desc_k_sw128(smem_u32(smem_x));
-        uint32_t s = mine, phase = 0;  // at least three stages
-        for (uint32_t step = mine; step < static_cast<uint32_t>(steps); step += ISSUERS) {
-            const uint32_t slot = step % A_SLOTS, slot_phase = (step / A_SLOTS) & 1, turn = (step / ISSUERS) & 1;
+        uint32_t s = mine, phase = 0, slot = mine, slot_phase = 0, at = mine;
+        for (int step = mine < static_cast<uint32_t>(issuers) ? static_cast<int>(mine) : steps; step < steps; step += issuers) {
             if (!mbarrier_wait_uniform2(full_u + s * 8, phase, a_ready_u + slot * 8, slot_phase, &g_status, STATUS_WAIT_READY | 0x8000 | s)) break;
-            // the first step needs no token: the parity before a barrier's first phase counts as complete
-            if (!mbarrier_wait_uniform(token_u + mine * 8, mine == 0 ? turn ^ 1 : turn, &g_status, STATUS_WAIT_READY | 0x8400 | mine)) break;
             tcgen05_fence_after();
             if (elect_one()) {
                 const uint64_t b_desc = b_first + s * (x_bytes >> 4);
                 const uint32_t a = tmem_a + slot * A_COLUMNS;
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; ++kk)
-                    umma_f16_a_tmem(tmem_base, a + kk * 8, b_desc + (kk >> 2) * (half_bytes >> 4) + (kk & 3) * 2, idesc, (step | kk) != 0 ? 1u : 0u);
-                tcgen05_fence_before();
-                mbarrier_arrive_u32(token_u + (mine ^ 1) * 8);
-                tcgen05_commit_u32(empty_u + s * 8);  // the stage, and the slot where there are enough stages
-                if (stages < A_SLOTS) tcgen05_commit_u32(a_empty_u + slot * 8);
-                if (step + ISSUERS >= static_cast<uint32_t>(steps)) tcgen05_commit_u32(done_u);  // each issuer's last
+                    umma_f16_a_tmem(accumulator, a + kk * 8, b_desc + (kk >> 2) * (half_bytes >> 4) + (kk & 3) * 2, idesc, (step >= issuers || kk != 0) ? 1u : 0u);
+                tcgen05_commit_u32(step + issuers >= steps ? done_u : step_done_u + at * 8);  // nobody waits for an issuer's last step
             }
             __syncwarp();
-            s += ISSUERS;
+            s += issuers, slot += issuers, at += issuers;
             if (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
+            if (slot >= A_SLOTS) slot -= A_SLOTS, slot_phase ^= 1;
+            if (at >= static_cast<uint32_t>(ring)) at -= ring;
         }
     } else if (warp >= UNPACK_WARP0) {
         const int quadrant = warp & 3, group = (warp - UNPACK_WARP0) >> 2;
@@ -239,10 +239,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         uint32_t scale_next = local < steps ? load_scale_pair<PAIRED>(row_scales, 2 * (first + local), groups, inside) : 0u;
         uint32_t minimum_next = local < steps ? load_scale_pair<PAIRED>(row_minimums, 2 * (first + local), groups, inside) : 0u;
         uint32_t s = group / CODE_STEPS, phase = 0;  // the chunk of this group's step
-        // A slot is free when the MMAs of the step four before are done. That step's stage of activations says so too, unless
-        // there are fewer than four of them: then the stage may be done with a later step already, and a phase too far on.
-        const int ring = stages >= A_SLOTS ? stages : A_SLOTS;
-        const uint32_t free_u = stages >= A_SLOTS ? smem_u32(empty) : smem_u32(a_empty);
+        // A slot is free when the MMAs of the step four before are done.
+        const uint32_t free_u = smem_u32(step_done);
         int before = group - A_SLOTS, before_phase = 0;
         named_barrier_sync(1, 32 * (2 + UNPACK_WARPS));
         tcgen05_fence_after();
@@ -271,13 +269,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             s += UNPACK_GROUPS / CODE_STEPS;
             if (s >= static_cast<uint32_t>(code_stages)) s -= code_stages, phase ^= 1;
         }
-        // Every MMA is done, so nothing reads or writes the stages any more.
+        // Every MMA is done, so nothing of this CTA reads or writes the stages any more.
         alive = mbarrier_wait_uniform(smem_u32(done), 0, &g_status, STATUS_WAIT_TMEM_FULL | 0x8000) && alive;
         tcgen05_fence_after();
     }
-    if (split > 1) cluster_sync();  // in no CTA of the cluster
+    if (split > 1) cluster_sync();  // every CTA of the cluster is done with its stages
     if (warp >= UNPACK_WARP0) {
-        // The accumulator (lane = weight row, column = activation row) goes to the CTA that sums that activation row, in
+        // The accumulator, or the sum of the two (lane = weight row, column = activation row) goes to the CTA that sums that activation row, in
         // shared memory as [source CTA][row of the share][weight row]: pushed, because a load from another CTA's shared
         // memory is a round trip of a thousand cycles and a store is not.
         const int quadrant = warp & 3, group = (warp - UNPACK_WARP0) >> 2;
@@ -287,7 +285,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             uint32_t r[16];
             tmem_load_32x16(tmem_lane + c, r);
             int owner = c / share, row = c - owner * share;
-            tmem_load_wait();
+            if (issuers == 2 && steps > 1) {
+                uint32_t second[16];
+                tmem_load_32x16(tmem_lane + TWO_ISSUERS_COLUMNS + c, second);
+                tmem_load_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(second[j]));
+            } else {
+                tmem_load_wait();
+            }
             if (split == 1) {
                 float *partial = reinterpret_cast<float *>(smem) + c * BN + quadrant * 32 + lane;
 #pragma unroll

@@ -247,6 +247,25 @@ def test_w4a16_exchanged_operands_on_pairs_over_several_tiles(qi, m, n, k):
         assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
 
 
+@pytest.mark.parametrize("m,n,k", [(9, 96, 3072), (77, 12288, 3072), (96, 1024, 6144), (100, 3072, 3072), (200, 9216, 3072), (256, 3072, 12288),
+                                   (384, 1024, 6144), (512, 1536, 12288), (1024, 384, 3072), (1500, 1152, 3072), (300, 1024, 192)])
+def test_w4a16_same_bits_on_every_call(qi, m, n, k):
+    # one accumulator and two, from eight stages of activations down to three, K split over a cluster and not: the order of
+    # the sums is fixed, whatever else runs at the time; and each result is the product of the unpacked weights
+    rng = np.random.default_rng(5500 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x, c, s, z = up(qt.make_activations(rng, m, k)), up(codes), up(scales.view(np.float16)), up(minimums.view(np.float16))
+    weights = torch.empty(n, k, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_dequantize_ex(c, s, z, weights, n, k) == 0
+    results = [torch.full((m, n), float("nan"), device="cuda") for _ in range(8)]
+    for y in results:
+        assert qi.w4a16_gemm_ex(x, c, s, z, None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert all(torch.equal(results[0], y) for y in results[1:])
+    exact = x.double() @ weights.double().T
+    assert float((results[0] - exact).norm() / exact.norm()) <= 1e-4  # 12288 float32 additions: 12288 ** 0.5 * 2 ** -23 = 1.3e-5
+
+
 def test_w4a16_gemm_rejects_what_the_reference_rejects(qi):  # gemm.cu:264
     t = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
     assert qi.w4a16_gemm(t, t, t, t, t, 100, 128, 64) == qi.CUDA_ERROR_INVALID_VALUE
