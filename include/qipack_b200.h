@@ -341,7 +341,9 @@ int qi_shard_all_gather(void *context, const void *y_local, void *y_slabs, int o
                         void *stream);
 
 /* qi_linear on this rank's shard (local_record->n = N/R rows) into y_local [rows, N/R], then the
- * all-gather into y_slabs (skipped when y_slabs is NULL or there is one rank). */
+ * all-gather into y_slabs (skipped when y_slabs is NULL or there is one rank). Every rank's local_record is taken for
+ * 1/R of the matrix: the gathered y is bit for bit what qi_linear gives for the whole record on one GPU. (A caller that
+ * runs qi_linear or qi_w4a16_gemm_ex on slices by itself gets the order of float32 sums that suits the slice.) */
 int qi_shard_linear(void *context, const qi_packed_linear *local_record, const qi_linear_work *work,
                     const void *input, int input_dtype, void *y_local, void *y_slabs, int output_dtype, int rows,
                     int reuse_input, void *stream);

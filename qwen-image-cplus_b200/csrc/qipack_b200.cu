@@ -225,19 +225,21 @@ struct SwapPlan {
 // 3072, {77, 256} x 3072 x 12288, {256, 1024} rows): a step of 128 inputs costs a CTA 0.25 (its unpack warps) or 0.003
 // per column (its tensor cores and their operand), a tile 4 + 0.006 per column for its start, its first loads and
 // its results, and sharing a tile over a cluster another 0.8 + 0.016 per column.
-SwapPlan plan_w4a16_swap(int m, int n, int k, int device) {
+// `like`: only plans that add up K in that plan's order.
+SwapPlan plan_w4a16_swap(int m, int n, int k, int device, const SwapPlan *like = nullptr) {
     namespace ws = w4a16_swap;
     const int tiles_n = (n + ws::BN - 1) / ws::BN, steps = (k + ws::BK - 1) / ws::BK;
     SwapPlan best = {0, 0, 1e30};
     for (int tiles_m = (m + ws::MAX_COLUMNS - 1) / ws::MAX_COLUMNS, most = tiles_m + 8; tiles_m < most; ++tiles_m) {
         const int columns = ((m + tiles_m - 1) / tiles_m + 15) / 16 * 16;
         if (tiles_m > 1 && columns < 64) break;
+        if (like != nullptr && ws::issuers_of(columns) != ws::issuers_of(like->columns)) continue;
         const double step = columns * 0.003 > 0.25 ? columns * 0.003 : 0.25;
         for (int split = 1; split <= ws::MAX_SPLIT && split <= steps; ++split) {
             const long long tiles = static_cast<long long>(tiles_n) * ((m + columns - 1) / columns);
             const int resident = resident_clusters(device, split);
             const long long waves = (tiles + resident - 1) / resident;
-            if (split > 1 && waves > 1) break;
+            if (like != nullptr ? split != like->split : split > 1 && waves > 1) continue;
             const double us = waves * (4.0 + columns * 0.006 + (steps + split - 1) / split * step + (split > 1 ? 0.8 + 0.016 * columns : 0.0));
             if (us < best.us) best = {columns, split, us};
         }
@@ -283,6 +285,28 @@ SwapPlan plan_w4a16_pair_swap(int m, int n, int k, int device) {
         if (us < best.us) best = {columns, 2, us};
     }
     return best;
+}
+
+// The kernel for a shape, or for a slice of `n` of a matrix's `whole_n` weight rows. A column-sharded linear promises the bits
+// of the unsharded one, and those depend on the order in which K is added up: on the number of CTAs that share it and of
+// accumulators. So a slice takes the order that the whole matrix would take, and what is fastest for the slice among the
+// kernels and tiles that have it. What that costs against a free choice: nothing at 4096 rows of 9216 x 3072, 8.6 against
+// 7.4 us for an eighth of it at 77 rows, 19.1 against 10.3 for an eighth of 3072 x 12288 at 256.
+struct W4A16Choice {
+    bool pairs;  // of CTAs (w4a16_pair_swap_gemm.cuh)
+    SwapPlan plan;
+};
+W4A16Choice choose_w4a16(int m, int n, int k, int whole_n, int device) {
+    if (whole_n != n) {
+        const W4A16Choice whole = choose_w4a16(m, whole_n, k, whole_n, device);
+        const bool in_order = whole.pairs || (whole.plan.split == 1 && w4a16_swap::issuers_of(whole.plan.columns) == 1);  // one accumulator, all of K
+        const SwapPlan pair = plan_w4a16_pair_swap(m, n, k, device);
+        SwapPlan in_order_plan = {w4a16_swap::MAX_COLUMNS, 1, 0.0};
+        const SwapPlan swap = plan_w4a16_swap(m, n, k, device, in_order ? &in_order_plan : &whole.plan);
+        return in_order && pair.us <= swap.us ? W4A16Choice{true, pair} : W4A16Choice{false, swap};
+    }
+    const SwapPlan swap = plan_w4a16_swap(m, n, k, device), pair = plan_w4a16_pair_swap(m, n, k, device);
+    return swap.us < pair.us ? W4A16Choice{false, swap} : W4A16Choice{true, pair};
 }
 
 int launch_w4a16_pair_swap(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
@@ -480,7 +504,7 @@ __global__ void dequantize_kernel(const uint8_t *__restrict__ codes, const __hal
 }
 
 int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
-               void *y, int y_dtype, long long ldy, int m, int n, int k, cudaStream_t stream) {
+               void *y, int y_dtype, long long ldy, int m, int n, int k, int whole_n, cudaStream_t stream) {
     if (m < 1 || m > 8 || n <= 0 || k <= 0 || n % 16 != 0 || k % 64 != 0) return INVALID;
     if (!x_half || !codes || !scales || !minimums || !y) return INVALID;
     if (!aligned16(x_half) || !aligned16(codes) || (k % 8) != 0) return INVALID;
@@ -511,7 +535,8 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
     if (n % 32 == 0 && output_ok(y, y_dtype, ldy, n)) {
         const int device = current_device();
         if (device < 0) return INVALID;
-        const SwapPlan plan = plan_w4a16_swap(m, n, k, device);
+        const SwapPlan whole = plan_w4a16_swap(m, whole_n, k, device);  // see choose_w4a16
+        const SwapPlan plan = whole_n == n ? whole : plan_w4a16_swap(m, n, k, device, &whole);
         const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
         return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, plan.columns, plan.split, stream, device);
     }
@@ -568,7 +593,7 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
 }
 
 int w4a16_gemm(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
-               void *y, int y_dtype, long long ldy, int m, int n, int k, int tile, cudaStream_t stream) {
+               void *y, int y_dtype, long long ldy, int m, int n, int k, int whole_n, int tile, cudaStream_t stream) {
     if (m <= 0 || n <= 0 || k <= 0 || n % 32 != 0 || k % 64 != 0) return INVALID;
     if (!x_half || !codes || !scales || !minimums) return INVALID;
     if (!aligned16(x_half) || !aligned16(codes) || !output_ok(y, y_dtype, ldy, n)) return INVALID;
@@ -577,9 +602,9 @@ int w4a16_gemm(const void *x_half, const void *codes, const void *scales, const 
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
     if (tile == 0) {
         // The exchanged-operand kernels: single CTAs and clusters, or persistent pairs, whichever is estimated to be faster.
-        const SwapPlan swap = plan_w4a16_swap(m, n, k, device), pair = plan_w4a16_pair_swap(m, n, k, device);
-        if (swap.us < pair.us) return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, swap.columns, swap.split, stream, device);
-        return launch_w4a16_pair_swap(x_half, codes, scales, minimums, bias, y, shape, pair.columns, stream, device);
+        const W4A16Choice choice = choose_w4a16(m, n, k, whole_n, device);
+        if (choice.pairs) return launch_w4a16_pair_swap(x_half, codes, scales, minimums, bias, y, shape, choice.plan.columns, stream, device);
+        return launch_w4a16_swap(x_half, codes, scales, minimums, bias, y, shape, choice.plan.columns, choice.plan.split, stream, device);
     }
     switch (tile) {
         case 1: return launch_w4a16<1, 128, 6>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
@@ -589,6 +614,12 @@ int w4a16_gemm(const void *x_half, const void *codes, const void *scales, const 
         case 5: return launch_w4a16_pair<5>(x_half, codes, scales, minimums, bias, y, shape, stream, device);
         default: return INVALID;
     }
+}
+
+int w4a16_linear(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias, void *y, int y_dtype,
+          long long ldy, int m, int n, int k, int whole_n, cudaStream_t stream) {
+    if (m >= 1 && m <= 8 && n % 16 == 0) return w4a16_gemv(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, whole_n, stream);
+    return w4a16_gemm(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, whole_n, 0, stream);
 }
 
 // single_cta: always the one-CTA kernel (128 x 128 tiles); otherwise CTA pairs where the shape and pointers allow.
@@ -883,7 +914,7 @@ int qi_w4a4_group_dots_ex(const void *a_codes, const void *a_scales, const void 
 
 int qi_w4a16_gemv_ex(const void *x_half, const void *codes, const void *scales, const void *minimums,
                      const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, void *stream) {
-    return w4a16_gemv(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, static_cast<cudaStream_t>(stream));
+    return w4a16_gemv(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, n, static_cast<cudaStream_t>(stream));
 }
 
 int qi_w4a16_gemv_grouped_ex(const void *x_half, const qi_gemv_item *items, int count, int y_dtype, long long ldy, int m,
@@ -893,22 +924,20 @@ int qi_w4a16_gemv_grouped_ex(const void *x_half, const qi_gemv_item *items, int 
 
 int qi_w4a16_gemm_ex(const void *x_half, const void *codes, const void *scales, const void *minimums,
                      const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, void *stream) {
-    if (m >= 1 && m <= 8 && n % 16 == 0)
-        return w4a16_gemv(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, static_cast<cudaStream_t>(stream));
-    return w4a16_gemm(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, 0, static_cast<cudaStream_t>(stream));
+    return w4a16_linear(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, n, static_cast<cudaStream_t>(stream));
 }
 
 int qi_w4a16_gemm_tile_ex(const void *x_half, const void *codes, const void *scales, const void *minimums,
                           const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, int tile,
                           void *stream) {
     if (tile < 0 || tile > 5) return INVALID;
-    return w4a16_gemm(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, tile, static_cast<cudaStream_t>(stream));
+    return w4a16_gemm(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, n, tile, static_cast<cudaStream_t>(stream));
 }
 
 int qi_w4a16_gemm(const void *x_half, const void *codes, const void *scales, const void *minimums, float *y, int m,
                   int n, int k) {
     if (m % 128 != 0 || n % 128 != 0 || k % 64 != 0) return INVALID;  // gemm.cu:264
-    return w4a16_gemm(x_half, codes, scales, minimums, nullptr, y, QI_DTYPE_F32, n, m, n, k, 0, nullptr);
+    return w4a16_gemm(x_half, codes, scales, minimums, nullptr, y, QI_DTYPE_F32, n, m, n, k, n, 0, nullptr);
 }
 
 int qi_f32_to_f16(const float *source, void *out, unsigned long long count) {
@@ -936,8 +965,9 @@ int qi_w4a16_dequantize_ex(const void *codes, const void *scales, const void *mi
     return static_cast<int>(cudaGetLastError());
 }
 
-int qi_linear(const qi_packed_linear *record, const qi_linear_work *work, const void *input, int input_dtype,
-              void *output, int output_dtype, long long ld_output, int rows, int reuse_input, void *stream) {
+// The dispatcher for a record that holds record->n of a matrix's whole_n weight rows.
+static int linear_slice(const qi_packed_linear *record, int whole_n, const qi_linear_work *work, const void *input, int input_dtype,
+                        void *output, int output_dtype, long long ld_output, int rows, int reuse_input, void *stream) {
     if (!record || !work || !input || !output || rows <= 0) return INVALID;
     if (record->group_size != 64) return INVALID;
     if (input_dtype != QI_DTYPE_F32 && input_dtype != QI_DTYPE_F16) return INVALID;
@@ -974,10 +1004,15 @@ int qi_linear(const qi_packed_linear *record, const qi_linear_work *work, const 
             }
             x_half = work->halves;
         }
-        return qi_w4a16_gemm_ex(x_half, record->weights, record->scales, record->zeros, record->bias, output,
-                                output_dtype, ld_output, rows, n, k, stream);
+        return w4a16_linear(x_half, record->weights, record->scales, record->zeros, record->bias, output, output_dtype, ld_output, rows, n, k,
+                     whole_n, static_cast<cudaStream_t>(stream));
     }
     return INVALID;
+}
+
+int qi_linear(const qi_packed_linear *record, const qi_linear_work *work, const void *input, int input_dtype,
+              void *output, int output_dtype, long long ld_output, int rows, int reuse_input, void *stream) {
+    return record == nullptr ? INVALID : linear_slice(record, record->n, work, input, input_dtype, output, output_dtype, ld_output, rows, reuse_input, stream);
 }
 
 int qi_kernel_status(unsigned int *status) {

@@ -373,8 +373,10 @@ int qi_shard_linear(void *context, const qi_packed_linear *local_record, const q
     Context *c = checked(context);
     if (c == nullptr || local_record == nullptr) return static_cast<int>(cudaErrorInvalidValue);
     if (local_record->n % 128 != 0) return static_cast<int>(cudaErrorInvalidValue);
-    const int status = qi_linear(local_record, work, input, input_dtype, y_local, output_dtype, local_record->n, rows,
-                                 reuse_input, stream);
+    // whole_n chooses the order in which a scheme 5 linear adds up K, so that the gathered slices are the unsharded bits
+    const long long whole_n = static_cast<long long>(local_record->n) * c->ranks;
+    const int status = linear_slice(local_record, whole_n <= 0x7fffffffLL ? static_cast<int>(whole_n) : local_record->n, work, input, input_dtype, y_local, output_dtype,
+                                    local_record->n, rows, reuse_input, stream);
     if (status != 0 || y_slabs == nullptr || c->ranks == 1) return status;
     return qi_shard_all_gather(context, y_local, y_slabs, output_dtype, rows, local_record->n, stream);
 }

@@ -1,8 +1,10 @@
 """Column-sharded packed linears on 2 GPUs through the C ABI (NCCL all-gather over NVLink, and the W4A4
 GEMM that stores its slice into every rank's output itself).
-Skipped on a box with fewer than two GPUs."""
+The tests of two ranks are skipped on a box with fewer than two GPUs."""
 import os
 import socket
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -160,6 +162,62 @@ def _worker(rank, ranks, port, result_path):
         with open(result_path, "w") as handle:
             handle.write("ok" if ok else "mismatch")
     dist.destroy_process_group()
+
+
+NCCL_STAND_IN = """
+#include <string.h>
+typedef struct { char internal[128]; } Id;
+int ncclGetUniqueId(Id *id) { memset(id, 0, sizeof(*id)); return 0; }
+int ncclCommInitRank(void **comm, int ranks, Id id, int rank) { (void)ranks, (void)id, (void)rank; *comm = (void *)1; return 0; }
+int ncclCommDestroy(void *comm) { (void)comm; return 0; }
+int ncclAllGather(const void *from, void *to, size_t count, int type, void *comm, void *stream) { (void)from, (void)to, (void)count, (void)type, (void)comm, (void)stream; return 1; }
+"""
+
+SLICES = """
+import itertools, sys
+import torch
+import __graft_entry__ as entry
+qi = entry.load_package()
+random = torch.Generator(device="cuda")
+random.manual_seed(31)
+different = []
+for m, (n, k) in itertools.product((1, 5, 40, 256, 1024, 4096), ((9216, 3072), (3072, 12288), (2048, 192), (3072, 576))):
+    codes = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=random)
+    scales = (torch.rand(n, k // 64, device="cuda", generator=random) * 0.006 + 0.001).half()
+    minimums = (-7.5 * scales.float()).half()
+    x = torch.randn(m, k, device="cuda", generator=random).half()
+    work = qi.LinearWork(None, None, None)
+    whole = torch.empty(m, n, device="cuda")
+    assert qi.linear(qi.PackedLinear(qi.SCHEME_W4A16, n, k, codes, scales, minimums), work, x, whole, m, input_dtype=qi.DTYPE_F16) == 0
+    for ranks in (2, 4, 8):
+        for rank in range(ranks):
+            context = qi.ShardContext(rank, ranks, bytes(128))
+            first, count = qi.shard_plan(n, ranks, rank)
+            rows = slice(first, first + count)
+            record = qi.PackedLinear(qi.SCHEME_W4A16, count, k, codes[rows].contiguous(), scales[rows].contiguous(), minimums[rows].contiguous())
+            mine = torch.empty(m, count, device="cuda")
+            assert context.linear(record, work, x, mine, None, m, input_dtype=qi.DTYPE_F16) == 0
+            torch.cuda.synchronize()
+            assert qi.kernel_status() == 0 and context.destroy() == 0
+            if not torch.equal(mine, whole[:, rows]):
+                different.append((m, n, k, ranks, rank))
+sys.exit(f"slices that are not the whole's bits: {different}" if different else 0)
+"""
+
+
+def test_every_rank_computes_the_bits_of_the_unsharded_w4a16_linear(tmp_path):
+    """Each rank's part of the column-sharded linear, one rank after the other on one GPU and without the gather (a stand-in
+    for NCCL makes the contexts), against the same columns of the unsharded one."""
+    if not torch.cuda.is_available():
+        pytest.fail("the gpu tests need a CUDA device")
+    source, library, script = tmp_path / "nccl.c", tmp_path / "libnccl_stand_in.so", tmp_path / "slices.py"
+    source.write_text(NCCL_STAND_IN)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(library), str(source)], check=True)
+    script.write_text(SLICES)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    environment = dict(os.environ, QI_NCCL_LIBRARY=str(library), PYTHONPATH=root)
+    done = subprocess.run([sys.executable, str(script)], cwd=root, env=environment, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
 
 
 def test_two_ranks_all_gather_the_unsharded_result(tmp_path):
