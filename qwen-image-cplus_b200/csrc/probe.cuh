@@ -62,16 +62,22 @@ __global__ void __launch_bounds__(THREADS, 1) mma_rate_kernel(int batches) {
     }
 }
 
-// A wait that nothing ends: one thread waits on an mbarrier nobody arrives on until `limit_ns` have passed, then
-// does what every wait of this library does when it runs out of time: records the code and returns. Lets a test
-// see the status path (code set, read clears it, the next launch is healthy) without anything going wrong.
+// A wait that nothing ends: a warp waits on an mbarrier nobody arrives on until `limit_ns` have passed, then does what
+// every wait of this library does when it runs out of time: records the code and returns. Every other lane finds its own
+// barrier complete at once (the phase before a new barrier's first counts as complete), so that the lanes disagree for as
+// long as the wait lasts: they have to give up together, and the shuffle that follows needs them all. Lets a test see the
+// status path (code set, read clears it, the next launch is healthy) without anything going wrong.
 __global__ void __launch_bounds__(32, 1) wait_timeout_kernel(unsigned long long limit_ns) {
     __shared__ uint64_t never;
     if (threadIdx.x == 0) {
         mbarrier_init(&never, 1);
         fence_barrier_init();
-        mbarrier_wait_spin(&never, 0, &g_status, STATUS_WAIT_FULL | 0xA000, 0, limit_ns);
     }
+    __syncwarp();
+    const uint32_t barrier = smem_u32(&never), parity = threadIdx.x & 1;
+    const bool waited = wait_uniform([&]() { return mbarrier_poll_u32(barrier, parity) != 0; }, &g_status, STATUS_WAIT_FULL | 0xA000, 0, limit_ns);
+    const bool neighbour = __shfl_xor_sync(0xffffffffu, waited ? 1 : 0, 1) != 0;
+    if (waited || neighbour) atomicExch(&g_status, STATUS_BAD_ARGUMENT | 0xA000);
 }
 
 }  // namespace probe

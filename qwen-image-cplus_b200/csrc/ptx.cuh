@@ -125,8 +125,24 @@ __device__ __forceinline__ bool mbarrier_wait_warp(uint64_t *barrier, uint32_t p
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
-// Waits of a converged warp that stays converged, on shared-window addresses: every lane polls (one instruction for the
-// warp), nothing but the vote between the polls. The second form waits for two barriers, whose polls overlap.
+// Waits of a converged warp that stays converged: every lane asks, nothing but the vote between the questions, and the
+// answer is the vote's, the same in every lane. What follows may then use the whole warp (a vote, a shuffle, tcgen05.ld,
+// mma.sync), which a wait that each lane gives up on by itself must not: lanes that left would be waited for without end.
+template <typename Ready>
+__device__ __forceinline__ bool wait_uniform(Ready ready, uint32_t *status, uint32_t code, uint32_t backoff_ns = 0, uint64_t limit_ns = WAIT_LIMIT_NS) {
+    uint64_t start = 0;
+    for (uint32_t spin = 0;; ++spin) {
+        if (__all_sync(0xffffffffu, ready())) return true;
+        if (backoff_ns != 0) __nanosleep(backoff_ns);
+        if (spin < WAIT_FAST_SPINS) continue;
+        if (start == 0) start = global_timer_ns();
+        const bool over = global_timer_ns() - start > limit_ns || *reinterpret_cast<volatile uint32_t *>(status) != 0;
+        if (__any_sync(0xffffffffu, over)) break;
+    }
+    if ((threadIdx.x & 31) == 0) atomicCAS(status, 0u, code);
+    return false;
+}
+// On barriers, by shared-window addresses. The first form waits for two, whose polls overlap.
 __device__ __forceinline__ uint32_t mbarrier_poll_u32(uint32_t barrier, uint32_t parity) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
@@ -135,18 +151,10 @@ __device__ __forceinline__ uint32_t mbarrier_poll_u32(uint32_t barrier, uint32_t
 }
 __device__ __forceinline__ bool mbarrier_wait_uniform2(uint32_t barrier_a, uint32_t parity_a, uint32_t barrier_b, uint32_t parity_b,
                                                        uint32_t *status, uint32_t code, uint32_t backoff_ns = 0) {
-    uint64_t start = 0;
-    for (uint32_t spin = 0;; ++spin) {
+    return wait_uniform([&]() {
         const uint32_t a = mbarrier_poll_u32(barrier_a, parity_a), b = barrier_b != barrier_a ? mbarrier_poll_u32(barrier_b, parity_b) : 1u;
-        if (__all_sync(0xffffffffu, (a & b) != 0)) return true;
-        if (backoff_ns != 0) __nanosleep(backoff_ns);
-        if (spin < WAIT_FAST_SPINS) continue;
-        if (start == 0) start = global_timer_ns();
-        const bool over = global_timer_ns() - start > WAIT_LIMIT_NS || *reinterpret_cast<volatile uint32_t *>(status) != 0;
-        if (__any_sync(0xffffffffu, over)) break;
-    }
-    if ((threadIdx.x & 31) == 0) atomicCAS(status, 0u, code);
-    return false;
+        return (a & b) != 0;
+    }, status, code, backoff_ns);
 }
 __device__ __forceinline__ bool mbarrier_wait_uniform(uint32_t barrier, uint32_t parity, uint32_t *status, uint32_t code, uint32_t backoff_ns = 0) {
     return mbarrier_wait_uniform2(barrier, parity, barrier, parity, status, code, backoff_ns);

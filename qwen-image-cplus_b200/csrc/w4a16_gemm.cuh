@@ -238,7 +238,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
                         minimum_next[p] = __ldg(minimums + static_cast<size_t>(row) * groups + kb + 1);
                     }
                 }
-                if (!mbarrier_wait(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0x100 | s)) { alive = false; break; }
+                if (!mbarrier_wait_warp(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0x100 | s, lane)) { alive = false; break; }
                 const uint8_t *codes_tile = smem_c + s * T::C_BYTES;
                 uint8_t *b_tile = smem_b + s * T::B_BYTES;
 #pragma unroll
@@ -262,7 +262,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++tile_count) {
             const int m0 = (tile % tiles_m) * T::BM, n0 = (tile / tiles_m) * BN;
             const uint32_t acc = tile_count % T::ACC_STAGES, acc_phase = (tile_count / T::ACC_STAGES) & 1;
-            if (!mbarrier_wait(&tmem_full[acc], acc_phase, &g_status, STATUS_WAIT_TMEM_FULL | acc)) break;
+            if (!mbarrier_wait_warp(&tmem_full[acc], acc_phase, &g_status, STATUS_WAIT_TMEM_FULL | acc, lane)) break;
             tcgen05_fence_after();
 #pragma unroll
             for (int mi = 0; mi < NUM_M; ++mi) {

@@ -159,17 +159,13 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     uint32_t s = team, phase = 0;
     while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
     int parity = 0;
+    bool gave_up = false;
     for (int tile = blockIdx.x + team * gridDim.x; tile < tiles; tile += STREAM_TEAMS * gridDim.x, parity ^= 1) {
         float (&partial)[STREAM_TEAM_WARPS][16][8] = partials[team][parity];
         // The stage's last user may have been another team. Only once this tile has been sent for is the phase before complete,
         // and the parity of this one's unambiguous.
-        bool arrived = fetched[s] == tile;
-        for (uint32_t spin = 0; !arrived && spin < (1u << 24); ++spin) {
-            __nanosleep(32);
-            arrived = fetched[s] == tile;
-        }
-        if (!arrived) atomicCAS(&g_status, 0u, STATUS_WAIT_EMPTY | 0xB000 | s);
-        arrived = arrived && mbarrier_wait(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
+        const bool arrived = wait_uniform([&]() { return fetched[s] == tile; }, &g_status, STATUS_WAIT_EMPTY | 0xB000 | s, 32) &&
+                             mbarrier_wait_uniform(smem_u32(&full[s]), phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
         const uint8_t *stage = smem + static_cast<size_t>(s) * stage_bytes;
         const __half *stage_scales = reinterpret_cast<const __half *>(stage + code_bytes);
         const __half *stage_minimums = reinterpret_cast<const __half *>(stage + code_bytes + scale_bytes);
@@ -231,7 +227,8 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         // The team is done with the stage, and the partial sums are complete. The sums alternate between two places: those of
         // this tile are read below and written again two tiles on, with the next tile's barrier in between.
         named_barrier_sync(1 + team, STREAM_TEAM_WARPS * 32);
-        if (team_thread == 0) {
+        gave_up |= !arrived;
+        if (team_thread == 0 && arrived) {
             const int next = tile + stages * gridDim.x;
             if (next < tiles) fetch(next, s);
         }
@@ -256,6 +253,11 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         }
         s += STREAM_TEAMS;
         while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
+    }
+    // Every copy has a team that waits for it. Where a wait gave up, let the copies already issued land. (Asking the status
+    // word instead is a round trip to L2 at the end of every CTA: 4080 x 4096 5.6 -> 5.9 us.)
+    if (gave_up) {
+        for (int i = 0; i < 64; ++i) __nanosleep(2000);
     }
 }
 

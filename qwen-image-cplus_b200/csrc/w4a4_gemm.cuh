@@ -186,7 +186,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         pair = __ldg(reinterpret_cast<const __half2 *>(w_scales + static_cast<size_t>(col) * groups + 2 * ks));
                     sw_pair[p][0] = __low2float(pair), sw_pair[p][1] = __high2float(pair);
                 }
-                if (!mbarrier_wait(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0x1000 | s)) { alive = false; break; }
+                if (!mbarrier_wait_warp(&full[s], phase, &g_status, STATUS_WAIT_FULL | 0x1000 | s, lane)) { alive = false; break; }
                 float *sw_stage = sw_tile + s * 2 * BN;
 #pragma unroll
                 for (int p = 0; p < BN / 128; ++p) {
@@ -239,14 +239,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 const int s = iteration % STAGES;
                 const uint32_t phase = (iteration / STAGES) & 1;
                 const __half2 sa_pair = __ldg(reinterpret_cast<const __half2 *>(sa_row + 2 * ks));
-                if (!mbarrier_wait(&ready[s], phase, &g_status, STATUS_WAIT_READY | 0x2000 | s)) { alive = false; break; }
+                if (!mbarrier_wait_warp(&ready[s], phase, &g_status, STATUS_WAIT_READY | 0x2000 | s, lane)) { alive = false; break; }
                 const float *sw_stage = sw_tile + s * 2 * BN + column_half * COLUMNS;
 #pragma unroll
                 for (int gl = 0; gl < 2; ++gl, ++group_count) {
                     const uint32_t buffer = group_count & 1, buffer_phase = (group_count >> 1) & 1;
                     // 2^-8 undoes the 16 x 16 of the widened operands; exact
                     const float sa = (gl == 0 ? __low2float(sa_pair) : __high2float(sa_pair)) * 0.00390625f;
-                    if (!mbarrier_wait(&dot_full[buffer], buffer_phase, &g_status, STATUS_WAIT_TMEM_FULL | 0x1000 | buffer)) { alive = false; break; }
+                    if (!mbarrier_wait_warp(&dot_full[buffer], buffer_phase, &g_status, STATUS_WAIT_TMEM_FULL | 0x1000 | buffer, lane)) { alive = false; break; }
                     tcgen05_fence_after();
                     const uint32_t tmem_row = tmem_base + buffer * BN + column_half * COLUMNS + (static_cast<uint32_t>(quadrant * 32) << 16);
                     const float *sw_group = sw_stage + gl * BN;

@@ -741,8 +741,9 @@ def test_linear_takes_the_wide_path_when_given_wide_operands(qi):
 
 def test_a_wait_that_runs_out_reports_its_code_and_leaves_the_device_healthy(qi):
     # every device-side wait of the library is bounded; this makes one run out on purpose (a barrier nothing
-    # arrives on, limit 1 ms) and follows the error path a caller would see: code set, cleared by reading it,
-    # and the next launches unaffected
+    # arrives on, limit 1 ms, in a warp of which every other lane waits for nothing: the lanes have to give up
+    # together, another code says they did not) and follows the error path a caller would see: code set, cleared
+    # by reading it, and the next launches unaffected
     assert qi.kernel_status() == 0
     assert qi.probe_wait_timeout(1_000_000) == 0
     torch.cuda.synchronize()
