@@ -60,6 +60,33 @@ __device__ __forceinline__ void tmem_wait_16(uint32_t (&r)[16]) {
                    "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
 }
 
+// The order of the tiles: blocks of group_m rows of tiles; within a block the rows come first. The unpack warps, which run
+// ahead, ask past the last tile too: there is no row of tiles left to divide by then, and the place is beyond the matrix.
+struct TilePlace {
+    int m_index, n_index;
+};
+__host__ __device__ constexpr TilePlace tile_place(int tile, int tiles_m, int tiles_n, int group_m) {
+    if (tile >= tiles_m * tiles_n) return {0, tiles_n};
+    const int of_block = group_m * tiles_n, block = tile / of_block, first = block * group_m;
+    const int within = tile - block * of_block, rows = tiles_m - first < group_m ? tiles_m - first : group_m;
+    return {first + within % rows, within / rows};
+}
+// Every tile once, nothing inside the matrix past the last; a division by zero would not compile.
+constexpr bool covers(int tiles_m, int tiles_n, int group_m, int past) {
+    bool seen[64] = {};
+    for (int tile = 0; tile < tiles_m * tiles_n + past; ++tile) {
+        const TilePlace at = tile_place(tile, tiles_m, tiles_n, group_m);
+        if (tile >= tiles_m * tiles_n) {
+            if (at.n_index < tiles_n) return false;
+            continue;
+        }
+        if (at.m_index < 0 || at.m_index >= tiles_m || at.n_index < 0 || at.n_index >= tiles_n || seen[at.m_index * tiles_n + at.n_index]) return false;
+        seen[at.m_index * tiles_n + at.n_index] = true;
+    }
+    return true;
+}
+static_assert(covers(1, 1, 1, 300) && covers(7, 5, 7, 80) && covers(8, 8, 8, 80) && covers(13, 4, 8, 80) && covers(17, 3, 8, 80) && covers(16, 4, 8, 80), "the walk over the tiles");
+
 // `columns`: activation rows of a tile, a multiple of 16. PAIRED: see load_scale_pair.
 template <bool PAIRED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
@@ -83,11 +110,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     const int cta = static_cast<int>(cluster_ctarank());  // 0 = leader
     const int pair = static_cast<int>(blockIdx.x >> 1), pairs = static_cast<int>(gridDim.x >> 1);
     const int tiles_m = (shape.m + columns - 1) / columns, tiles_n = (shape.n + 2 * BN - 1) / (2 * BN), tiles = tiles_m * tiles_n;
-    // Blocks of group_m rows of tiles; within a block the rows come first.
     auto place = [&](int tile, int &m_index, int &n_index) {
-        const int of_block = group_m * tiles_n, block = tile / of_block, first = block * group_m;
-        const int within = tile - block * of_block, rows = tiles_m - first < group_m ? tiles_m - first : group_m;
-        m_index = first + within % rows, n_index = within / rows;
+        const TilePlace at = tile_place(tile, tiles_m, tiles_n, group_m);
+        m_index = at.m_index, n_index = at.n_index;
     };
     const int groups = shape.k / 64, steps = (groups + 3) / 4 * 2;  // an even number: a step past the end is all zeros
     const int half_bytes = columns / 2 * 128;                       // 64 inputs of this CTA's activation rows
@@ -199,7 +224,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             int m_index, n_index;
             place(tile, m_index, n_index);
             const int row = n_index * (2 * BN) + cta * BN + local_row;
-            inside = row < shape.n && tile < tiles;
+            inside = row < shape.n;  // past the last tile no row is
             row_scales = scales + static_cast<size_t>(inside ? row : 0) * groups;
             row_minimums = minimums + static_cast<size_t>(inside ? row : 0) * groups;
         };
