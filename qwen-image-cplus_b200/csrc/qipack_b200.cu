@@ -688,6 +688,15 @@ int launch_widen_codes(const void *a_codes, void *a_bytes, long long a_rows, con
     return static_cast<int>(launch_overlapped(w4a4_wide::widen_codes_kernel, static_cast<unsigned>(a_blocks + w_blocks),
                                               w4a4_wide::WIDEN_THREADS, 0, stream, a, w, static_cast<int>(a_blocks)));
 }
+bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        (void)cudaGetLastError();  // the legacy stream during another's capture: the launch will say so
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, const void *w_scales, const float *bias,
               void *y, int y_dtype, long long ldy, int32_t *dots, int m, int n, int k, int path, cudaStream_t stream) {
     if (m <= 0 || n <= 0 || k <= 0 || n % 32 != 0 || k % 128 != 0 || path < 0 || path >= W4A4_PATHS) return INVALID;
@@ -705,8 +714,10 @@ int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, co
     // and tile, 9 us at k = 768 whatever m and n. Measured, int8 and widened: 1 x 128 x 3072 29.9 and 9.1 us, 77 x 9216 x
     // 3072 32.8 and 17.2, 4096 x 32 x 3072 30.8 and 11.4, 1 x 18432 x 3072 31.5 and 28.2, 1 x 32 x 256 5.9 and 9.4,
     // 255 x 4096 x 256 9.0 and 9.3; with more tiles than SMs the widened form leads at any k.
-    const bool widened_is_faster = k >= 768 || (m >= 256 && n >= 256);
-    if (path == 2 || (path == 0 && pair_takes_it && widened_is_faster)) {
+    // Not under stream capture where the int8 kernel will do: scratch makes a graph with allocation nodes, of which CUDA allows
+    // one instance and no clone or child, and a caller that captures a prompt's calls may want several.
+    const bool large = m >= 256 && n >= 256;
+    if (path == 2 || (path == 0 && pair_takes_it && (large || (k >= 768 && !capturing(stream))))) {
         const size_t a_bytes = (static_cast<size_t>(m) * k + 255) & ~static_cast<size_t>(255);
         const size_t w_bytes = static_cast<size_t>(n) * k;
         uint8_t *scratch = nullptr;

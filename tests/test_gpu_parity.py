@@ -561,6 +561,37 @@ def test_w4a4_packed_few_rows_or_outputs_by_shape(qi, m, n, k):
     assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 32, 768), (77, 96, 1024)])
+def test_w4a4_packed_few_rows_captured(qi, m, n, k):
+    # a captured call of few rows is one kernel without scratch: its graph can be instantiated more than once
+    rng = np.random.default_rng(96 + m + n + k)
+    w_codes, w_scales = qt.random_w4a4_pack(rng, n, k, 1e-3, 6e-3)
+    a_codes, a_scales = qt.random_w4a4_pack(rng, m, k, 0.05, 0.6)
+    args = (up(a_codes), up(a_scales), up(w_codes), up(w_scales), None)
+    y = torch.full((m, n), float("nan"), device="cuda")
+    assert qi.w4a4_gemm_ex(*args, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    stream, runtime = torch.cuda.Stream(), ctypes.CDLL("libcudart.so.12")
+    on, graph, first, second = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
+    captured = torch.full((m, n), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    assert runtime.cudaStreamBeginCapture(on, 0) == 0
+    status = qi.w4a4_gemm_ex(*args, captured, qi.DTYPE_F32, n, m, n, k, stream.cuda_stream)
+    assert runtime.cudaStreamEndCapture(on, ctypes.byref(graph)) == 0 and status == 0
+    instances = [runtime.cudaGraphInstantiate(ctypes.byref(instance), graph, ctypes.c_ulonglong(0)) for instance in (first, second)]
+    runtime.cudaGetLastError()
+    assert instances == [0, 0]
+    for instance in (first, second):
+        captured.fill_(float("nan"))
+        torch.cuda.synchronize()
+        assert runtime.cudaGraphLaunch(instance, on) == 0
+        check_status(qi)
+        assert torch.equal(captured, y)
+        assert runtime.cudaGraphExecDestroy(instance) == 0
+    assert runtime.cudaGraphDestroy(graph) == 0
+    assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 32, 256), (16, 4000, 512), (17, 3072, 1024), (33, 9216, 256), (77, 9216, 512), (96, 9248, 256), (130, 3072, 512), (77, 12288, 256), (256, 3072, 768)])
 def test_w4a4_wide_few_rows_as_columns(qi, m, n, k):
     rng = np.random.default_rng(95 + m + n + k)
