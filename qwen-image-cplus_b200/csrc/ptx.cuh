@@ -170,6 +170,11 @@ __device__ __forceinline__ void mbarrier_arrive_expect_tx_u32(uint32_t barrier, 
 // drains. Nothing that an earlier kernel wrote, reads or will write may be touched before grid_wait() returns (it waits
 // for that kernel's end and its writes); grid_release() lets the next kernel of the stream start its own prologue.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What a launch returned, taken out of the runtime's last error too: the next call's cudaGetLastError() is about that call.
+inline cudaError_t launched(cudaError_t result) {
+    const cudaError_t last = cudaGetLastError();
+    return result != cudaSuccess ? result : last;
+}
 // Every kernel that is launched that way calls grid_wait() in all its threads before its first access to global memory,
 // so that the chain of waits reaches back over any number of such launches.
 template <typename... Parameters, typename... Arguments>
@@ -185,7 +190,7 @@ inline cudaError_t launch_overlapped(void (*kernel)(Parameters...), unsigned gri
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, static_cast<Parameters>(arguments)...);
+    return launched(cudaLaunchKernelEx(&config, kernel, static_cast<Parameters>(arguments)...));
 }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -267,8 +267,8 @@ int launch_w4a16_swap(const void *x_half, const void *codes, const void *scales,
     cudaLaunchAttribute attributes[2];
     swap_config(config, attributes, static_cast<int>(ctas), split, smem.bytes, stream);
     auto kernel = paired ? ws::gemm_kernel<true> : ws::gemm_kernel<false>;
-    return static_cast<int>(cudaLaunchKernelEx(&config, kernel, map_x, map_codes, static_cast<const __half *>(scales),
-                                               static_cast<const __half *>(minimums), bias, y, shape, plan));
+    return static_cast<int>(launched(cudaLaunchKernelEx(&config, kernel, map_x, map_codes, static_cast<const __half *>(scales),
+                                                        static_cast<const __half *>(minimums), bias, y, shape, plan)));
 }
 
 // The widest tile is not always the best: 4096 x 3072 outputs are 192 tiles of 256 x 256, three waves of 74 pairs, or 288 of

@@ -561,6 +561,24 @@ def test_w4a4_packed_few_rows_or_outputs_by_shape(qi, m, n, k):
     assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
 
 
+def test_a_refused_launch_is_reported_once(qi):
+    # the legacy stream takes no launch while another stream that waits for it is captured: the call says so, and the next
+    # call's status is its own
+    runtime, on, graph = ctypes.CDLL("libcudart.so.12"), ctypes.c_void_p(), ctypes.c_void_p()
+    x, out = torch.ones(1024, device="cuda"), torch.zeros(4096, dtype=torch.float16, device="cuda")
+    codes, halves = torch.zeros(64 * 32, dtype=torch.uint8, device="cuda"), torch.zeros(64, dtype=torch.float16, device="cuda")
+    assert qi.f32_to_f16(x, out, 1024) == 0
+    check_status(qi)
+    assert runtime.cudaStreamCreateWithFlags(ctypes.byref(on), 0) == 0 and runtime.cudaStreamBeginCapture(on, 0) == 0
+    refused = qi.f32_to_f16(x, out, 1024)
+    ended = runtime.cudaStreamEndCapture(on, ctypes.byref(graph))
+    runtime.cudaGetLastError()
+    following = qi.w4a16_dequantize_ex(codes, halves, halves, out, 64, 64)
+    assert runtime.cudaStreamDestroy(on) == 0
+    assert (refused, ended, following) == (906, 901, 0)  # implicit use of the legacy stream, capture invalidated, success
+    check_status(qi)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 32, 768), (77, 96, 1024)])
 def test_w4a4_packed_few_rows_captured(qi, m, n, k):
     # a captured call of few rows is one kernel without scratch: its graph can be instantiated more than once
