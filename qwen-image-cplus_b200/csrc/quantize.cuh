@@ -138,6 +138,7 @@ struct PlainSource {
         __device__ __forceinline__ void load(const PlainSource &source, long long offset, bool active) { Raw16<T>::load(source.x + offset, active); }
     };
 };
+__device__ __forceinline__ float gelu_tanh(float v) { return 0.5f * v * (1.0f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v))); }
 struct GeluSource {
     const float *x;
     struct Raw : Raw16<float> {
@@ -145,7 +146,7 @@ struct GeluSource {
         __device__ __forceinline__ void convert(float (&v)[16]) const {
             Raw16<float>::convert(v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.5f * v[i] * (1.0f + tanhf(0.7978845608028654f * (v[i] + 0.044715f * v[i] * v[i] * v[i])));
+            for (int i = 0; i < 16; ++i) v[i] = gelu_tanh(v[i]);
         }
     };
 };
@@ -238,8 +239,9 @@ quantize_pairs_kernel(const Source source, uint8_t *__restrict__ codes, __half *
         unpack_f32x2(fma_f32x2(v[i], negative2, integer), ra, rb);  // integer - quotient: the distance from the rounding
         worst = fmaxf(worst, fmaxf(fabsf(ra), fabsf(rb)));
     }
-    if (!(worst < 0.5f - 1.52587890625e-05f) || !ga.plain || !gb.plain) {
-        // somewhere a quotient is near a tie, or the short cut does not hold for this group: the reference's expression
+    if (!(worst < 0.5f - 1.52587890625e-05f) || (active_a && !ga.plain) || (active_b && !gb.plain)) {
+        // somewhere a quotient is near a tie, or the short cut does not hold for this group: the reference's expression. Where
+        // the number of chunks is odd the last one's partner is zeros that nobody asked for (one chunk 7.1 -> 4.0 us).
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             float a, b;
@@ -283,7 +285,7 @@ quantize_pairs_kernel(const Source source, uint8_t *__restrict__ codes, __half *
     }
 }
 
-// ---- SwiGLU: one chunk per half-warp ------------------------------------------------------------------------------------
+// ---- one chunk per half-warp: SwiGLU, and GELU of few rows ---------------------------------------------------------------
 // The two loads and the division of silu(gate) * up want warps rather than registers: with 40 registers a thread this
 // form takes 28.8 us at 1024 x 12288, the paired one 42.8 (32.1 without loads ahead).
 
@@ -318,6 +320,14 @@ __device__ __forceinline__ void two_passes(float (&v)[16]) {
     for (int o = 0; o < 4; ++o) butterfly(v[o], v[o + 4], v[o + 8], v[o + 12]);
 }
 
+struct GeluChunkSource {
+    const float *x;
+    __device__ __forceinline__ void load(long long offset, float (&v)[16]) const {
+        load16(x + offset, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = gelu_tanh(v[i]);
+    }
+};
 struct SwigluSource {
     const float *gate, *up;
     __device__ __forceinline__ void load(long long offset, float (&v)[16]) const {
@@ -330,9 +340,9 @@ struct SwigluSource {
 };
 // WIDE: also (or only, when codes is null) write every code as one FP8 E4M3 byte, [m, k], the
 // operand layout of w4a4_wide_gemm.cuh.
-template <bool WIDE>
+template <typename Source, bool WIDE>
 __global__ void __launch_bounds__(QUANT_THREADS)
-quantize_swiglu_kernel(const SwigluSource source, uint8_t *__restrict__ codes, __half *__restrict__ scales,
+quantize_chunks_kernel(const Source source, uint8_t *__restrict__ codes, __half *__restrict__ scales,
                             uint8_t *__restrict__ bytes, long long chunks) {
     __shared__ __align__(16) float transpose[(QUANT_THREADS / 32) * 2 * REGION];
     grid_wait();
@@ -467,16 +477,25 @@ inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, voi
     return launch_quantize_pairs(PlainSource<float>{static_cast<const float *>(x)}, codes, scales, bytes, m, k, stream);
 }
 
+template <typename Source>
+inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream) {
+    const long long chunks = static_cast<long long>(m) * (k / 256), blocks = (chunks + QUANT_THREADS / 16 - 1) / (QUANT_THREADS / 16);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    return launch_overlapped(bytes != nullptr ? quantize_chunks_kernel<Source, true> : quantize_chunks_kernel<Source, false>, static_cast<unsigned>(blocks), QUANT_THREADS,
+                             0, stream, source, static_cast<uint8_t *>(codes), static_cast<__half *>(scales), static_cast<uint8_t *>(bytes), chunks);
+}
+
+// GELU takes the one-chunk form up to so many chunks: it fills the SMs with more and shorter threads, the paired form needs
+// many rounds to be ahead. Measured, one chunk and paired, both code forms: 77 x 12288 4.0 and 5.5 us, 1024 x 3072 7.8 and 10.6,
+// 1024 x 12288 23.5 and 23.8, 2048 x 12288 44.1 and 42.3, 4096 x 12288 85.1 and 80.2.
+constexpr long long GELU_CHUNKS = 49152;
+
+
 // producer: 1 = SwiGLU of (first, second), 2 = GELU-tanh of first
 inline cudaError_t launch_fused_quantize(int producer, const float *first, const float *second, void *codes, void *scales,
                                          void *bytes, int m, int k, cudaStream_t stream) {
-    if (producer == 1) {
-        const long long chunks = static_cast<long long>(m) * (k / 256), blocks = (chunks + QUANT_THREADS / 16 - 1) / (QUANT_THREADS / 16);
-        if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-        return launch_overlapped(bytes != nullptr ? quantize_swiglu_kernel<true> : quantize_swiglu_kernel<false>, static_cast<unsigned>(blocks), QUANT_THREADS, 0,
-                                 stream, SwigluSource{first, second}, static_cast<uint8_t *>(codes), static_cast<__half *>(scales),
-                                 static_cast<uint8_t *>(bytes), chunks);
-    }
+    if (producer == 1) return launch_quantize_chunks(SwigluSource{first, second}, codes, scales, bytes, m, k, stream);
+    if (static_cast<long long>(m) * (k / 256) <= GELU_CHUNKS) return launch_quantize_chunks(GeluChunkSource{first}, codes, scales, bytes, m, k, stream);
     return launch_quantize_pairs(GeluSource{first}, codes, scales, bytes, m, k, stream);
 }
 

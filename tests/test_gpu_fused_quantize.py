@@ -44,7 +44,7 @@ def ptr(tensor):
 
 
 @pytest.mark.parametrize("producer", ["swiglu", "gelu"])
-@pytest.mark.parametrize("m,k", [(5, 256), (300, 1024), (512, 12288)])
+@pytest.mark.parametrize("m,k", [(1, 256), (5, 256), (300, 1024), (512, 12288)])
 def test_fused_producer_gives_the_unfused_bytes(qi, reference_ops, producer, m, k):
     generator = torch.Generator(device="cuda").manual_seed(1000 + m + k)
     first = torch.randn(m, k, device="cuda", generator=generator) * 2.0
@@ -90,6 +90,24 @@ def test_fused_producer_gives_the_unfused_bytes(qi, reference_ops, producer, m, 
         assert qi.w4a4_gelu_quantize_ex(first, only_codes, scales2, None, m, k) == 0
     torch.cuda.synchronize()
     assert torch.equal(only_codes, codes)
+
+
+@pytest.mark.parametrize("m,k", [(192, 65536), (193, 65536), (49155, 256)])  # around 49152 chunks, where GELU changes its form
+def test_gelu_quantiser_gives_a_row_the_same_bytes_in_every_matrix(qi, m, k):
+    generator = torch.Generator(device="cuda").manual_seed(1100 + m)
+    x = torch.randn(m, k, device="cuda", generator=generator) * 2.0
+    x[:, ::97] *= 12.0
+    x[m // 3] = 0.0
+    results = []
+    for rows in (m, m // 2 + 1):
+        codes, scales, wide = (torch.zeros(m, k // 2, dtype=torch.uint8, device="cuda"), torch.zeros(m, k // 64, dtype=torch.float16, device="cuda"),
+                               torch.zeros(m, k, dtype=torch.uint8, device="cuda"))
+        for first in range(0, m, rows):
+            last = min(m, first + rows)
+            assert qi.w4a4_gelu_quantize_ex(x[first:last], codes[first:last], scales[first:last], wide[first:last], last - first, k) == 0
+        torch.cuda.synchronize()
+        results.append((codes, scales.view(torch.int16), wide))
+    assert all(torch.equal(whole, parts) for whole, parts in zip(*results))
 
 
 def test_fused_quantisers_reject_bad_arguments(qi):

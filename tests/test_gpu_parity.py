@@ -45,7 +45,7 @@ def check_status(qi):
 
 # ---- activation quantiser -------------------------------------------------------------------
 
-@pytest.mark.parametrize("m,k", [(1, 256), (3, 512), (128, 3072), (517, 1024), (256, 12288)])
+@pytest.mark.parametrize("m,k", [(1, 256), (3, 512), (77, 768), (128, 3072), (517, 1024), (256, 12288)])
 @pytest.mark.parametrize("dtype", ["f32", "f16"])
 def test_quantize_activations_bit_exact(qi, m, k, dtype):
     rng = np.random.default_rng(1000 + m + k)
