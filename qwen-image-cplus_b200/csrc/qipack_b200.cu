@@ -158,23 +158,6 @@ int rows_in_l2(int tiles_m, long long tile_bytes) {
 
 // ---- the exchanged-operand kernel (w4a16_swap_gemm.cuh): its plan for a shape ----------------------------------------
 
-struct SwapSmem {
-    int stages, code_stages, bytes;
-};
-SwapSmem swap_smem(int columns) {
-    namespace ws = w4a16_swap;
-    // At least two chunks of codes; more of them, before more of the activations, as long as four stages of those fit.
-    const int room = 232448 - ws::BARRIER_BYTES - 1024;
-    int code_stages = (room - 4 * ws::stage_bytes(columns)) / ws::CODE_BYTES;
-    code_stages = code_stages < 2 ? 2 : code_stages > ws::MAX_CODE_STAGES ? ws::MAX_CODE_STAGES : code_stages;
-    int stages = (room - code_stages * ws::CODE_BYTES) / ws::stage_bytes(columns);
-    if (stages > ws::MAX_STAGES) stages = ws::MAX_STAGES;
-    // One CTA per SM, always: it takes all of TMEM, and a second would wait for it while its cluster waits for the second.
-    int bytes = ws::smem_bytes(columns, stages, code_stages);
-    if (bytes < 116 * 1024) bytes = 116 * 1024;
-    return {stages, code_stages, bytes};
-}
-
 template <bool PAIRED>
 cudaError_t configure_swap(int device) {
     static std::atomic<bool> configured[MAX_DEVICES];
@@ -259,7 +242,7 @@ int launch_w4a16_swap(const void *x_half, const void *codes, const void *scales,
         return INVALID;
     const bool paired = ((reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(minimums)) & 3) == 0 && shape.k % 128 == 0;
     if (const cudaError_t error = paired ? configure_swap<true>(device) : configure_swap<false>(device)) return static_cast<int>(error);
-    const SwapSmem smem = swap_smem(columns);
+    const ws::SmemPlan smem = ws::smem_plan(columns);
     const ws::Plan plan = {columns, split, smem.stages, smem.code_stages};
     const long long ctas = static_cast<long long>((shape.m + columns - 1) / columns) * ((shape.n + ws::BN - 1) / ws::BN) * split;
     if (ctas > 0x7fffffffLL) return INVALID;

@@ -34,7 +34,8 @@ constexpr int THREADS = 32 * (UNPACK_WARP0 + UNPACK_WARPS);
 constexpr int A_SLOTS = 4, A_COLUMNS = BK / 2, TMEM_COLUMNS = 512;
 static_assert(MAX_COLUMNS + A_SLOTS * A_COLUMNS <= TMEM_COLUMNS && A_SLOTS == UNPACK_GROUPS, "accumulator and unpacked steps");
 constexpr int STAGES = 5, HALF_BYTES = MAX_COLUMNS / 2 * 128, X_BYTES = 2 * HALF_BYTES;  // a stage: two boxes of 64 inputs
-constexpr int CODE_STAGES = 3, CODE_BYTES = BN * 128, CODE_READERS = 8;                  // a chunk of codes: two steps, two groups read it
+constexpr int CODE_STAGES = 4, CODE_BYTES = BN * 128, CODE_READERS = 8;                  // a chunk of codes: two steps, two groups read it
+static_assert(CODE_STAGES == 2 || CODE_STAGES >= 4, "a group reads every second chunk: see w4a16_swap::smem_plan");
 static_assert(STAGES >= A_SLOTS, "a stage's release stands for that of the slot of the step four before");
 constexpr int BARRIER_BYTES = 256;
 constexpr int SMEM_BYTES = STAGES * X_BYTES + CODE_STAGES * CODE_BYTES + BARRIER_BYTES + 1024;

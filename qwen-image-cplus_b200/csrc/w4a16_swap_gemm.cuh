@@ -27,7 +27,6 @@ namespace w4a16_swap {
 
 constexpr int BK = 128, BN = 128;         // inputs per step: two quantisation groups; weight rows of a tile
 constexpr int MAX_COLUMNS = 256, MAX_STAGES = 8, MAX_SPLIT = 8;
-static_assert(MAX_STAGES % 2 == 0, "the longest ring");
 constexpr int PRODUCER_WARP = 0, MMA_WARP = 1, CODE_WARP = 2, SECOND_MMA_WARP = 3, UNPACK_WARP0 = 4;
 constexpr int UNPACK_GROUPS = 4, UNPACK_WARPS = 4 * UNPACK_GROUPS;  // a group: one warp per 32 TMEM lanes; groups take the steps in turn
 constexpr int THREADS = 128 + 32 * UNPACK_WARPS;
@@ -57,6 +56,37 @@ __host__ __device__ constexpr int tile_bytes(int columns, int stages, int code_s
     return loads > partial ? loads : partial;
 }
 __host__ __device__ constexpr int smem_bytes(int columns, int stages, int code_stages) { return tile_bytes(columns, stages, code_stages) + BARRIER_BYTES + 1024; }
+
+// How shared memory is divided for a width: at least two chunks of codes; more of them, before more of the activations, as
+// long as four stages of those fit.
+// Two lengths are left out. A wait asks for the parity of a phase, and passes at once where the phase BEFORE the one in
+// front of it is still open: whoever waits for a stage's next load must know that the last one has landed.
+//   * Codes: a group reads every second chunk. In a ring of two the last load was its own; in a ring of four or more the
+//     slot it filled before was free of the MMAs of eight steps ago, which had read it. In a ring of three nothing says so.
+//   * Activations: of two issuers each takes every second step, and knows that of its own steps only: an even ring.
+struct SmemPlan {
+    int stages, code_stages, bytes;
+};
+__host__ __device__ constexpr SmemPlan smem_plan(int columns) {
+    const int room = 232448 - BARRIER_BYTES - 1024;
+    int code_stages = (room - 4 * stage_bytes(columns)) / CODE_BYTES;
+    code_stages = code_stages < 4 ? 2 : code_stages > MAX_CODE_STAGES ? MAX_CODE_STAGES : code_stages;
+    int stages = (room - code_stages * CODE_BYTES) / stage_bytes(columns);
+    if (stages > MAX_STAGES) stages = MAX_STAGES;
+    if (issuers_of(columns) == 2) stages = stages / 2 * 2;
+    // One CTA per SM, always: it takes all of TMEM, and a second would wait for it while its cluster waits for the second.
+    const int bytes = smem_bytes(columns, stages, code_stages);
+    return {stages, code_stages, bytes < 116 * 1024 ? 116 * 1024 : bytes};
+}
+constexpr bool smem_plans_are_sound() {
+    for (int columns = 16; columns <= MAX_COLUMNS; columns += 16) {
+        const SmemPlan plan = smem_plan(columns);
+        if (plan.bytes > 232448 || plan.stages < 3 || plan.stages > MAX_STAGES || plan.code_stages < 2 || plan.code_stages == 3 || plan.code_stages > MAX_CODE_STAGES) return false;
+        if (issuers_of(columns) == 2 && (plan.stages < A_SLOTS || plan.stages % 2 != 0)) return false;
+    }
+    return true;
+}
+static_assert(smem_plans_are_sound(), "shared memory of every width");
 
 // 32 registers into this thread's TMEM lane, 32 adjacent columns.
 __device__ __forceinline__ void tmem_store_32x32(uint32_t address, const uint4 (&v)[8]) {
@@ -137,10 +167,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     const int rank = static_cast<int>(blockIdx.x) % split, tile = static_cast<int>(blockIdx.x) / split;
     const int tiles_n = (shape.n + BN - 1) / BN, groups = shape.k / 64, k_steps = (groups + 1) / 2;
     const int n0 = (tile % tiles_n) * BN, m0 = (tile / tiles_n) * columns;
-    // The ring is at least as long as the stages of activations and the slots of unpacked weights, and even, so that a barrier
-    // belongs to one issuer: it then completes for a later step only after both that wait on it have passed the earlier one.
-    // (With five barriers the other issuer's next step could complete a slot's barrier before the slot's own step was unpacked.)
-    const int issuers = issuers_of(columns), ring = ((stages >= A_SLOTS ? stages : A_SLOTS) + 1) / 2 * 2;
+    // The ring is as long as the longer of the two that wait on it, the stages of activations and the slots of unpacked
+    // weights, and even where there are two issuers, so that a barrier belongs to one of them: it then completes for a later
+    // step only after both that wait on it have passed the earlier one.
+    const int issuers = issuers_of(columns), ring = stages >= A_SLOTS ? stages : A_SLOTS;
     const int first = k_steps * rank / split, steps = k_steps * (rank + 1) / split - first;  // this CTA's share of K
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) mbarrier_init(&full[s], 1);
