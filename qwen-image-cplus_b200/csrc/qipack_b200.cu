@@ -213,9 +213,14 @@ SwapPlan plan_w4a16_swap(int m, int n, int k, int device, const SwapPlan *like =
     namespace ws = w4a16_swap;
     const int tiles_n = (n + ws::BN - 1) / ws::BN, steps = (k + ws::BK - 1) / ws::BK;
     SwapPlan best = {0, 0, 1e30};
-    for (int tiles_m = (m + ws::MAX_COLUMNS - 1) / ws::MAX_COLUMNS, most = tiles_m + 8; tiles_m < most; ++tiles_m) {
+    // The widest tiles and those a little narrower; narrower ones where all of them run at once (8192 x 32 x 64: 32 tiles of
+    // 256 columns 8.2 us, 128 of 64 5.9).
+    const int widest = (m + ws::MAX_COLUMNS - 1) / ws::MAX_COLUMNS;
+    for (int tiles_m = widest, before = 0; tiles_m < widest + 8 || tiles_m * tiles_n <= sm_count(device); ++tiles_m) {
         const int columns = ((m + tiles_m - 1) / tiles_m + 15) / 16 * 16;
         if (tiles_m > 1 && columns < 64) break;
+        if (columns == before) continue;
+        before = columns;
         if (like != nullptr && ws::issuers_of(columns) != ws::issuers_of(like->columns)) continue;
         const double step = columns * 0.003 > 0.25 ? columns * 0.003 : 0.25;
         for (int split = 1; split <= ws::MAX_SPLIT && split <= steps; ++split) {
@@ -259,7 +264,7 @@ int launch_w4a16_swap(const void *x_half, const void *codes, const void *scales,
 // tile (4096 x {3072, 9216, 12288} x 3072, 4096 x 3072 x 12288, 1024 x 4096 x 4096), and 3 once.
 SwapPlan plan_w4a16_pair_swap(int m, int n, int k, int device) {
     namespace wp = w4a16_pair_swap;
-    const int pairs = sm_count(device) / 2, steps = (k + 255) / 256 * 2;
+    const int pairs = sm_count(device) / 2, steps = (k + 127) / 128;  // what fills up an even number of steps costs next to nothing
     const long long tiles_n = (n + 2 * wp::BN - 1) / (2 * wp::BN);
     SwapPlan best = {0, 2, 1e30};
     for (int columns = wp::MAX_COLUMNS; columns >= 128; columns -= 16) {

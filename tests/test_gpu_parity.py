@@ -227,10 +227,11 @@ def test_w4a16_exchanged_operands_at_the_edges_of_their_tiles(qi, m, n, k):
         assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
 
 
-@pytest.mark.parametrize("m,n,k", [(2048, 2048, 128), (4000, 1504, 192), (3000, 2336, 1216), (9000, 288, 320)])
+@pytest.mark.parametrize("m,n,k", [(2048, 2048, 128), (4000, 1504, 192), (3000, 2336, 1216), (9000, 288, 320),
+                                   (3000, 9216, 64), (3000, 2336, 320), (2000, 4128, 640), (4096, 1504, 1088)])
 def test_w4a16_exchanged_operands_on_pairs_over_several_tiles(qi, m, n, k):
-    # more 256-row tiles than pairs of CTAs, ragged on both sides, an odd number of groups, steps past the end of K;
-    # against the unpacked weights in float32 on the device, every output
+    # more 256-row tiles than pairs of CTAs, ragged on both sides, an odd number of groups or of steps (one step past the
+    # end of K); against the unpacked weights in float64 on the device, every output
     rng = np.random.default_rng(5000 + m + n + k)
     codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
     x, bias = up(qt.make_activations(rng, m, k)), up(qt.make_bias(rng, n))
