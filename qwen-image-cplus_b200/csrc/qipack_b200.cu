@@ -445,8 +445,11 @@ int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_b
     const long long waves_64 = (tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms, waves_32 = (tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms;
     const double us_64 = waves_64 * (waves_64 == 1 ? 0.185 : 0.21), us_32 = waves_32 * (waves_32 == 1 ? 0.12 : 0.135);
     // Weights as the 128 rows of a tile, activation rows as its columns, where that folds less for rows that do not exist:
-    // 0.12, 0.135 (one block of rows: 0.105) and 0.16 for 16, 32 and 48 columns, 15 % more in several waves (16 x 9216 x 3072 11.3 -> 8.7 us, 77 x
-    // 9216 x 3072 11.7 -> 10.4, 77 x 12288 x 3072 18.3 -> 15.4, 256 x 3072 x 3072 11.8 -> 10.0, 16 x 15776 x 768 8.3 -> 6.3).
+    // 0.12, 0.135 and 0.16 for 16, 32 and 48 columns, 15 % more in several waves (77 x 9216 x 3072 11.7 -> 10.4 us, 77 x
+    // 12288 x 3072 18.3 -> 15.4, 256 x 3072 x 3072 11.8 -> 10.0). Where one tile of 32 columns holds all rows it is priced below
+    // two of 16, 0.105, by what long rows measure (with 16 and with 32: 16 x 3072 x 12288 22.4 and 18.9, x 4096 9.2 and 8.2, 16 x
+    // 9216 x 3072 8.2 and 8.4). That line is drawn without K, and at K = 3072 it gives some away (16 x 3072 5.9 and 6.2, 32 x 3072
+    // 6.1 and 7.4, 1 x 12288 9.3 and 10.4; 77 x 3072 6.8 in tiles of 16, 8.0 in 128 x 32).
     const double others_us = us_64 < us_32 ? (us_64 < pair_us ? us_64 : pair_us) : (us_32 < pair_us ? us_32 : pair_us);
     const long long tiles_n = (shape.n + wn::BM - 1) / wn::BM;
     const auto exchanged_us = [&](int columns, double us) {

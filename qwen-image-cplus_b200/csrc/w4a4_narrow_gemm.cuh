@@ -1,4 +1,5 @@
-// W4A4 (H256, g64) GEMM on byte-wide (E4M3) codes for few rows: 128 x 64 or 128 x 32 output tiles, one per CTA. Same
+// W4A4 (H256, g64) GEMM on byte-wide (E4M3) codes for few rows or outputs: one tile per CTA, 128 rows x 64 or 32 outputs,
+// or (EXCHANGED) 128 outputs x 16, 32 or 48 rows. Same
 // operator, arithmetic and bits as w4a4_pair_gemm.cuh (reference: qwen_image_cuda/cuda/gemm.cu:65-189).
 //
 // The groups of an output are added in order, so K cannot be split, and a tile is a chain of k / 64 hand-overs from the
@@ -10,7 +11,7 @@
 //   * a fold warp copies the next group's dots out of TMEM while it folds the current one
 //
 // EXCHANGED, the weights are the 128 rows and 16 to 48 activation rows the columns: nothing is folded for rows that do not
-// exist, and a lane, which owns an output, writes next to its neighbours (77 x 9216 x 3072 11.7 -> 10.4 us, 16 rows 11.3 -> 8.7).
+// exist, and a lane, which owns an output, writes next to its neighbours (77 x 9216 x 3072 11.7 -> 10.4 us, 16 rows 11.3 -> 8.4).
 // What bounds it then: 16 columns still take 0.11 us a group, half of that the 32 KB of weights a stage coming into the SM.
 //
 //   warp 0      TMA: A rows (only those that exist, rounded up to 16) and B rows, 256 inputs a stage

@@ -228,10 +228,12 @@ def test_w4a16_exchanged_operands_at_the_edges_of_their_tiles(qi, m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k", [(2048, 2048, 128), (4000, 1504, 192), (3000, 2336, 1216), (9000, 288, 320),
-                                   (3000, 9216, 64), (3000, 2336, 320), (2000, 4128, 640), (4096, 1504, 1088)])
+                                   (3000, 9216, 64), (3000, 2336, 320), (2000, 4128, 640), (4096, 1504, 1088),
+                                   (4096, 3072, 1024), (3300, 1504, 12288)])
 def test_w4a16_exchanged_operands_on_pairs_over_several_tiles(qi, m, n, k):
     # more 256-row tiles than pairs of CTAs, ragged on both sides, an odd number of groups or of steps (one step past the
-    # end of K); against the unpacked weights in float64 on the device, every output
+    # end of K), scales read in pairs (K a multiple of 128) and one by one, and more activations than stay in L2, walked in
+    # blocks of eight rows of tiles of which the last is shorter; against the unpacked weights in float64, every output
     rng = np.random.default_rng(5000 + m + n + k)
     codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
     x, bias = up(qt.make_activations(rng, m, k)), up(qt.make_bias(rng, n))
@@ -332,6 +334,30 @@ def test_w4a16_gemv_scales_of_one_range(qi, m, n, k, low, high):
     assert qi.w4a16_gemv_ex(up(x16), up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), None, y, qi.DTYPE_F32, n, m, n, k) == 0
     check_status(qi)
     assert qt.max_relative_error(y.cpu().numpy(), expected) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("m", [1, 8])
+@pytest.mark.parametrize("n,k,scale_offset,output_offset", [(48, 4160, 0, 0), (16, 12288, 0, 0), (80, 3072, 1, 0), (96, 4160, 0, 1), (64, 12288, 1, 3), (48, 64, 1, 1)])
+def test_w4a16_gemv_without_what_the_other_kernels_need(qi, m, n, k, scale_offset, output_offset):
+    # long rows of which there is no multiple of 32, or an output that starts or steps off 16 bytes; scales off 16 bytes with
+    # rows the streaming kernel would take: the kernel that reads weights and scales from global memory one by one
+    rng = np.random.default_rng(3170 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x16, bias = qt.make_activations(rng, m, k), qt.make_bias(rng, n)
+    expected = qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)
+    shifted = []
+    for values in (scales, minimums):
+        room = torch.zeros(n * (k // 64) + 8, dtype=torch.float16, device="cuda")
+        shifted.append(room[scale_offset:scale_offset + n * (k // 64)].copy_(up(values.view(np.float16)).flatten()))
+    ldy = n + output_offset
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        room = torch.full((output_offset + (m + 1) * ldy,), -7.0, dtype=dtype, device="cuda")
+        y = room[output_offset:].view(m + 1, ldy)
+        assert qi.w4a16_gemv_ex(up(x16), up(codes), *shifted, up(bias), y, code, ldy, m, n, k) == 0
+        check_status(qi)
+        got = y.float().cpu().numpy()
+        assert np.all(got[m:] == -7.0) and np.all(got[:, n:] == -7.0)
+        assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
 
 
 @pytest.mark.parametrize("m,count,n,k", [(1, 3, 1024, 1216), (1, 70, 256, 512), (2, 5, 18432, 3072)])
@@ -611,7 +637,8 @@ def test_w4a4_packed_few_rows_captured(qi, m, n, k):
     assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 32, 256), (16, 4000, 512), (17, 3072, 1024), (33, 9216, 256), (77, 9216, 512), (96, 9248, 256), (130, 3072, 512), (77, 12288, 256), (256, 3072, 768)])
+@pytest.mark.parametrize("m,n,k", [(1, 32, 256), (16, 4000, 512), (17, 3072, 1024), (33, 9216, 256), (77, 9216, 512), (96, 9248, 256), (130, 3072, 512), (77, 12288, 256), (256, 3072, 768),
+                                   (33, 4768, 768), (40, 5024, 512), (48, 6272, 1024)])  # the last three in tiles of 16 rows
 def test_w4a4_wide_few_rows_as_columns(qi, m, n, k):
     rng = np.random.default_rng(95 + m + n + k)
     w_codes, w_scales = qt.random_w4a4_pack(rng, n, k, 1e-3, 6e-3)
