@@ -250,7 +250,7 @@ def other_kernels(qi, torch, device, stream, peaks, tensor_peaks, m):
         int8_seconds += int8_ms * 1e-3
         packed.append({"linear": name, "ms": ms, "tops": 2.0 * m * n * k / ms / 1e9, "int8_kernel_ms": int8_ms})
         del w_codes, a_codes, w_scales, a_scales, y
-    out["w4a4_packed"] = {"kernel": "qi_w4a4_gemm_ex (the drop-in ABI, nibble-packed operands): two widening kernels into (m + n) k bytes of "
+    out["w4a4_packed"] = {"kernel": "qi_w4a4_gemm_ex (the drop-in ABI, nibble-packed operands): one widening kernel into (m + n) k bytes of "
                                     "pool scratch, then w4a4_pair::gemm_kernel; int8_kernel: w4a4::gemm_kernel on the nibbles",
                           "linears": packed, "tops": ops / seconds / 1e12, "frac_of_e4m3_mma_loop": ops / seconds / 1e12 / tensor_peaks["e4m3"],
                           "int8_kernel_tops": ops / int8_seconds / 1e12,

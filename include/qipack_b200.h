@@ -105,7 +105,7 @@ int qi_w4a4_gemm_noalloc_ex(const void *a_codes, const void *a_scales, const voi
 
 /* As qi_w4a4_gemm_ex with the kernel chosen by the caller instead of by shape (for tests and tuning; every path gives
  * the same bits): 0 = by shape; 1 = the int8 kernel that widens the nibbles in shared memory (any k % 128 == 0);
- * 2 = both operands widened to one byte per code in scratch memory, then the byte-operand kernel on CTA pairs
+ * 2 = both operands widened to one byte per code in scratch memory, then the byte-operand kernels (qi_w4a4_gemm_wide_ex)
  * (k % 256 == 0, scale arrays 8-byte aligned). Path 2, and path 0 where it chooses path 2 (m, n >= 256, or k >= 768
  * and the stream is not being captured, and the conditions of path 2), take (m + n) * k bytes from a memory pool of the library's own (one per device, made at
  * first use, cudaMallocFromPoolAsync) and give them back with cudaFreeAsync, both in stream order; the pool keeps

@@ -101,7 +101,7 @@ bool make_map(CUtensorMap *map, CUtensorMapDataType type, int element_bytes, con
 
 // ---- tile selection -----------------------------------------------------------------------------
 
-// W4A16 tiles: 0 = choose by shape; 1 = 128x128, 2 = 256x128, 3 = 128x256, 4 = 256x256, 5 = 256x256 on a pair of CTAs.
+// W4A16 tiles: 0 = choose by shape (never one of the others, which only qi_w4a16_gemm_tile_ex names); 1 = 128x128, 2 = 256x128, 3 = 128x256, 4 = 256x256, 5 = 256x256 on a pair of CTAs.
 
 template <int NUM_M, int BN, int STAGES>
 int launch_w4a16(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
@@ -635,10 +635,9 @@ int w4a4_gemm_wide(const void *a_bytes, const void *a_scales, const void *w_byte
 }
 
 // The W4A4 GEMM on nibble-packed codes (the reference's operand format). `path`: 1 = the int8 kernel that widens the
-// nibbles in shared memory; 2 = both operands widened to one byte per code in scratch memory of the stream's pool
-// (two small kernels), then the byte-operand kernel on CTA pairs, which is the faster GEMM by more than the
-// widening costs once the matrices are large; 0 = 2 where the pair kernel takes the shape, else 1. Same bits on
-// every path. The scratch is (m + n) * k bytes from the library's own memory pool (cudaMallocFromPoolAsync) and goes
+// nibbles in shared memory; 2 = both operands widened to one byte per code in scratch memory (one small kernel), then
+// the byte-operand kernels, which are faster by more than the widening costs once the matrices are large or the rows
+// long; 0 = by shape, by the rule below. Same bits on every path. The scratch is (m + n) * k bytes from the library's own memory pool (cudaMallocFromPoolAsync) and goes
 // back with cudaFreeAsync, both in stream order; if the pool refuses, path 0 falls back to 1.
 constexpr int W4A4_PATHS = 3;
 

@@ -5,6 +5,9 @@
 // Layout in HBM (row-major, caller-owned): x [m,k] fp16; codes [n,k/2] bytes, even input in
 // the low nibble, values 0..15; scales, minimums [n,k/64] fp16; y [m,ldy] fp32 or fp16.
 //
+// The tiles of this file are chosen by qi_w4a16_gemm_tile_ex only: by shape a call takes the kernels with the operands
+// exchanged (w4a16_swap_gemm.cuh, w4a16_pair_swap_gemm.cuh). The unpacking here is theirs too.
+//
 // One persistent CTA per SM walks output tiles of (NUM_M*128) x BN. Per 64-wide K block
 // (one quantisation group):
 //   warp 0     TMA: the x tile (128-byte swizzled, K-major) and the packed code tile

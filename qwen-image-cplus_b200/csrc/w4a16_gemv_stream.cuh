@@ -87,7 +87,7 @@ struct StreamItems {
     StreamItem item[STREAM_GROUP];
 };
 
-// Dynamic shared memory: `stages` stages of stream_stage_bytes(k), then the activations (m * k * 2 bytes).
+// Dynamic shared memory: `stages` stages of stream_stage_bytes(k), then the activations (stream_x_bytes(m, k)).
 // GROUPED: `count` matrices [n, k] from `group`, tile t of the launch is tile t % (n / 16) of matrix t / (n / 16);
 // otherwise the one matrix given by the pointer arguments.
 template <bool GROUPED>

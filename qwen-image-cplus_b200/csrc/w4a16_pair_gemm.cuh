@@ -2,6 +2,9 @@
 // one 256 x 256 output tile per pair. Same operator and unpacking as w4a16_gemm.cuh
 // (reference: qwen_image_cuda/cuda/gemm.cu:191-268).
 //
+// Chosen by qi_w4a16_gemm_tile_ex only: by shape a call takes the kernels with the operands exchanged (w4a16_swap_gemm.cuh,
+// w4a16_pair_swap_gemm.cuh; 4096 x 9216 x 3072: 180 us here, 165 there), which add up K in the same order.
+//
 // Each CTA loads its own 128 rows of x and the packed codes of HALF of the tile's 256 weight rows,
 // unpacks those 128 rows to fp16 in its own shared memory, and the leader's MMA (M = 256 across the
 // pair, N = 256, K = 16) reads both halves. Compared with a 256 x 256 tile on one CTA this halves
@@ -82,7 +85,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             mbarrier_init(&tmem_full[a], 1);
             mbarrier_init(&tmem_empty[a], 2 * 4);
         }
-                fence_barrier_init();
+        fence_barrier_init();
     }
     if (warp == MMA_WARP) {
         tmem_alloc_pair(tmem_slot, (ACC_STAGES * BN));

@@ -10,9 +10,9 @@
 // Persistent: pair p takes the tiles p, p + pairs, ... Per step of 128 inputs, numbered through over the pair's tiles:
 //   warp 0      TMA: this CTA's half of the activations' tile (completion counted on the LEADER's barrier)
 //   warp 2      TMA: the codes of its 128 weight rows, 128 bytes of a row (two steps) at a time
-//   warps 8-23  four groups of four, steps in turn: unpack 128 codes of one weight row per thread into its TMEM lane
+//   warps 12-27 four groups of four, steps in turn: unpack 128 codes of one weight row per thread into its TMEM lane
 //   warp 1      leader only: tcgen05.mma.cta_group::2 kind::f16 with A in TMEM (M = 256, N = columns, K = 16) x 8
-//   warps 4-7   the finished tile: TMEM -> registers -> y, 32 consecutive outputs of a row per store
+//   warps 4-11  the finished tile: TMEM -> registers -> y, 32 consecutive outputs of a row per store
 // TMEM holds one accumulator (256 columns) and four unpacked steps (4 x 64). A tile's MMAs wait for the accumulator of the
 // tile before to be read; the loads and the unpacking of up to four steps run ahead meanwhile.
 #pragma once

@@ -3,7 +3,7 @@
 // w4a4_wide_gemm.cuh and the reference's w4a4_gemm_kernel (qwen_image_cuda/cuda/gemm.cu:65-189).
 //
 // Per group of 64 inputs the tensor cores leave a tile of EXACT integer dots (as fp32) in TMEM and
-// the fp32 pipe folds them: y += dot * (sa * sw). That fold is two fp32 operations per output and
+// the fp32 pipe folds them: y += (dot * sa) * sw. That fold is two fp32 operations per output and
 // group - at full tensor rate more than the fp32 pipe can do - so the kernel is built around
 // keeping sixteen fold warps busy and everything else out of their way. What was measured on the
 // way, and what the design does about it:
@@ -23,7 +23,7 @@
 //     without a vote around it (-> 823).
 //   * A tcgen05.commit holds up the later tcgen05 instructions of the THREAD that issued it for
 //     some 440 cycles, however deep the pipeline, but not those of other threads. So each team has
-//     two issuing threads (in different warps) that take turns group by group.
+//     two issuing warps (one elected lane each) that take turns slab by slab.
 //   * A fold warp copies its 32 x 32 dots of a group with one tcgen05.ld.32x32b.x32 (about 360
 //     B/clk/SM with eight warps; the 16x256b fragment shape reaches 230), hands the buffer back and
 //     does the arithmetic from registers, as (dot * sa) * sw + acc: dot * sa and sa * sw are both exact
@@ -127,9 +127,9 @@ constexpr int TEAM_COLUMNS = BN / TEAMS;
 constexpr int BUFFERS = 2;     // TMEM buffers per team, each the dots of TWO groups (one 128-byte slab of K): 2 x TEAM_COLUMNS columns
 constexpr int BUFFER_COLUMNS = 2 * TEAM_COLUMNS;
 constexpr int STAGES = 4;
-constexpr int TURNS = 2;       // MMA-issuing threads per team, taking turns group by group
+constexpr int TURNS = 2;       // MMA-issuing warps per team, taking turns slab by slab
 constexpr int PRODUCER_WARP = 0, SW_WARP = 1, SA_WARP = 2, MMA_WARP0 = 4, MMA_WARPS = TURNS * TEAMS, FOLD_WARP0 = 8, FOLD_WARPS = 16;  // warp 3 idle
-static_assert(MMA_WARP0 + MMA_WARPS <= FOLD_WARP0, "the issuing threads sit in control warps");
+static_assert(MMA_WARP0 + MMA_WARPS <= FOLD_WARP0, "the issuing warps are control warps");
 constexpr int COLUMNS = BN / (FOLD_WARPS / 4);  // columns per fold warp: 32
 // Registers live in the four schedulers' own files (16384 each), and warp w runs on scheduler w % 4:
 // six warps per scheduler here, 80 registers per thread at launch. setmaxnreg moves registers
@@ -355,8 +355,8 @@ __device__ __forceinline__ void mma_role(const View &v, uint32_t mine) {
 // of its first HOIST columns meanwhile and does the arithmetic once the copy has landed; the buffer goes back
 // when the copy of the slab's second group has landed. The other three warps of its scheduler fill the waits.
 // All lanes need the same weight scales: one 16-byte broadcast load per four columns.
-// The arithmetic is the packed fp32 pair form of  acc = fma(dot, sa * sw, acc): each half is
-// IEEE-rounded exactly like the scalar instruction, so the result has the reference's bits.
+// The arithmetic is the packed fp32 pair form of  acc = fma(dot * sa, sw, acc): dot * sa is exact and each half is
+// IEEE-rounded exactly like the scalar instruction, so the result has the bits of the reference's fma(dot, sa * sw, acc).
 struct FoldState {
     uint32_t dot_full, leader_dot_empty, sa_base, scale_ready, empty;
     uint32_t s, phase, group_count;
