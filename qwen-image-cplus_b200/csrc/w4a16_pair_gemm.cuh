@@ -3,7 +3,7 @@
 // (reference: qwen_image_cuda/cuda/gemm.cu:191-268).
 //
 // Chosen by qi_w4a16_gemm_tile_ex only: by shape a call takes the kernels with the operands exchanged (w4a16_swap_gemm.cuh,
-// w4a16_pair_swap_gemm.cuh; 4096 x 9216 x 3072: 180 us here, 165 there), which add up K in the same order.
+// w4a16_pair_swap_gemm.cuh; 4096 x 9216 x 3072: 173 us here, 163 there), which add up K in the same order.
 //
 // Each CTA loads its own 128 rows of x and the packed codes of HALF of the tile's 256 weight rows,
 // unpacks those 128 rows to fp16 in its own shared memory, and the leader's MMA (M = 256 across the
