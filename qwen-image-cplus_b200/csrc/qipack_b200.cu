@@ -20,6 +20,7 @@
 #include "w4a4_wide_gemm.cuh"
 #include "w4a4_pair_gemm.cuh"
 #include "w4a4_narrow_gemm.cuh"
+#include "w4a4_tall_gemm.cuh"
 #include "probe.cuh"
 
 namespace qi {
@@ -407,6 +408,41 @@ int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_by
                                               bias, y, dots, shape, outputs, tiling));
 }
 
+// How the tall kernel's tiles cover the output (see w4a4_tall::Tiling).
+w4a4_tall::Tiling w4a4_tall_tiling(const GemmShape &shape, int ctas) {
+    namespace wt = w4a4_tall;
+    const int tiles_m = (shape.m + wt::BM - 1) / wt::BM, tiles_n = (shape.n + wt::BN - 1) / wt::BN, tiles = tiles_m * tiles_n;
+    const int block = rows_in_l2(tiles_m, static_cast<long long>(wt::BM) * shape.k), last = (tiles_m - 1) / block * block, last_rows = tiles_m - last;
+    wt::Tiling tiling = {tiles, tiles, wt::BN, tiles_m, tiles_n, block, last, last_rows, 0, 0, 0, 0};
+    const int wide = tiles / ctas * ctas, before_tail = last_rows * tiles_n - (tiles - wide);  // wide tiles of the last block
+    if (wide == tiles || before_tail < 0) return tiling;
+    const int tail_row = before_tail % last_rows, tail_n = before_tail / last_rows * wt::BN;
+    for (int width = 16; width < wt::BN; width += 16) {
+        const int later = shape.n > tail_n + wt::BN ? (shape.n - tail_n - wt::BN + width - 1) / width : 0, sooner = (shape.n - tail_n + width - 1) / width;
+        const int narrow = tail_row * later + (last_rows - tail_row) * sooner;
+        if (narrow <= ctas) return {wide + narrow, wide, width, tiles_m, tiles_n, block, last, last_rows, tail_row, tail_n, later, sooner};
+    }
+    return tiling;
+}
+
+int launch_w4a4_tall(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
+                     void *y, const GemmShape &shape, cudaStream_t stream, int device) {
+    namespace wt = w4a4_tall;
+    CUtensorMap map_a, map_w;
+    if (!make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_bytes, shape.k, shape.m, static_cast<uint64_t>(shape.k),
+                  wt::SLAB_K, wt::BM, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    if (!make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w_bytes, shape.k, shape.n, static_cast<uint64_t>(shape.k),
+                  wt::SLAB_K, wt::BN, CU_TENSOR_MAP_SWIZZLE_128B))
+        return INVALID;
+    static std::atomic<bool> configured[MAX_DEVICES];
+    if (const cudaError_t error = configure_once(wt::gemm_kernel, wt::SMEM_BYTES, configured[device])) return static_cast<int>(error);
+    const wt::Tiling tiling = w4a4_tall_tiling(shape, sm_count(device));
+    const int grid = tiling.tiles < sm_count(device) ? tiling.tiles : sm_count(device);
+    return static_cast<int>(launch_overlapped(wt::gemm_kernel, grid, wt::THREADS, wt::SMEM_BYTES, stream, map_a, map_w,
+                                              static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales), bias, y, shape, tiling));
+}
+
 template <int BN, bool EXCHANGED>
 int launch_w4a4_narrow(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
                        void *y, const GemmShape &shape, cudaStream_t stream, int device) {
@@ -431,16 +467,22 @@ int launch_w4a4_narrow(const void *a_bytes, const void *a_scales, const void *w_
                                               static_cast<const __half *>(EXCHANGED ? a_scales : w_scales), bias, y, shape, box_rows));
 }
 
-// Byte operands with k a multiple of 256 and 8-byte aligned scales: CTA pairs, or single CTAs with 64 or 32 columns where
-// those are estimated to be faster. Microseconds per group and wave as measured on B200 ({77, 128, 256, 512} rows,
-// outputs 3072 to 12288, K 3072 to 12288): 0.185 and 0.12 for the narrow tiles (0.21 and 0.135 in several waves), 0.35 for a wave of wide pairs, 0.37 and
-// 0.29 for a last wave of 96 or 64 columns.
+// Byte operands with k a multiple of 256 and 8-byte aligned scales: tall tiles (256 x 64), or tiles of 128 rows, or of 16
+// to 48 activation rows, where those are estimated to be faster. Microseconds per group and wave as measured on B200:
+//   narrow tiles ({77, 128, 256, 512} rows, outputs 3072 to 12288, K 3072 to 12288): 0.185 and 0.12 for 64 and 32 columns
+//     (0.21 and 0.135 in several waves)
+//   tall tiles ({256 .. 16384} rows): 0.27 a wave (4096 x 9216 x 3072 198 us, 16 waves of 48 groups; 0.29 where there are
+//     one or two: 512 x 9216 x 3072 27.8), 0.24, 0.20 and 0.14 for a last wave of 48, 32 or 16 columns (1024 x 4096 x 4096
+//     34.0, 1024 x 3072 x 3072 23.4, 1024 x 12288 x 4096 95.0), 0.02 more where it is the only one (256 x 3072 x 3072 10.8,
+//     in 128 x 64 tiles 9.4)
 int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
                       void *y, const GemmShape &shape, cudaStream_t stream, int device) {
     namespace wn = w4a4_narrow;
-    const int sms = sm_count(device), pairs = sms / 2;
-    const w4a4_pair::Tiling tiling = w4a4_tiling(shape.m, shape.n, pairs, true);
-    const double pair_us = (tiling.wide + pairs - 1) / pairs * 0.35 + (tiling.tiles > tiling.wide ? (tiling.width == 64 ? 0.29 : 0.37) : 0.0);
+    const int sms = sm_count(device);
+    const w4a4_tall::Tiling tiling = w4a4_tall_tiling(shape, sms);
+    const int wide_waves = (tiling.wide + sms - 1) / sms;
+    const double last_us = tiling.tiles == tiling.wide ? 0.0 : (tiling.width == 48 ? 0.24 : (tiling.width == 32 ? 0.20 : 0.14)) + (tiling.wide == 0 ? 0.02 : 0.0);
+    const double tall_us = wide_waves * (wide_waves <= 2 ? 0.29 : 0.27) + last_us;
     const long long tiles_m = (shape.m + wn::BM - 1) / wn::BM;
     const long long waves_64 = (tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms, waves_32 = (tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms;
     const double us_64 = waves_64 * (waves_64 == 1 ? 0.185 : 0.21), us_32 = waves_32 * (waves_32 == 1 ? 0.12 : 0.135);
@@ -450,7 +492,7 @@ int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_b
     // two of 16, 0.105, by what long rows measure (with 16 and with 32: 16 x 3072 x 12288 22.4 and 18.9, x 4096 9.2 and 8.2, 16 x
     // 9216 x 3072 8.2 and 8.4). That line is drawn without K, and at K = 3072 it gives some away (16 x 3072 5.9 and 6.2, 32 x 3072
     // 6.1 and 7.4, 1 x 12288 9.3 and 10.4; 77 x 3072 6.8 in tiles of 16, 8.0 in 128 x 32).
-    const double others_us = us_64 < us_32 ? (us_64 < pair_us ? us_64 : pair_us) : (us_32 < pair_us ? us_32 : pair_us);
+    const double others_us = us_64 < us_32 ? (us_64 < tall_us ? us_64 : tall_us) : (us_32 < tall_us ? us_32 : tall_us);
     const long long tiles_n = (shape.n + wn::BM - 1) / wn::BM;
     const auto exchanged_us = [&](int columns, double us) {
         const long long waves = (tiles_n * ((shape.m + columns - 1) / columns) + sms - 1) / sms;
@@ -463,9 +505,9 @@ int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_b
         return launch_w4a4_narrow<32, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
     if (us_48_rows < others_us)
         return launch_w4a4_narrow<48, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    if (us_64 <= us_32 && us_64 < pair_us) return launch_w4a4_narrow<64, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    if (us_32 < pair_us) return launch_w4a4_narrow<32, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    return launch_w4a4_pair(a_bytes, a_scales, w_bytes, w_scales, bias, y, nullptr, shape, stream, device);
+    if (us_64 <= us_32 && us_64 < tall_us) return launch_w4a4_narrow<64, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    if (us_32 < tall_us) return launch_w4a4_narrow<32, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    return launch_w4a4_tall(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
 }
 
 bool output_ok(const void *y, int y_dtype, long long ldy, int n) {

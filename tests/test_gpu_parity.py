@@ -773,6 +773,28 @@ def test_w4a4_wide_gemm_in_narrow_tiles(qi, m, n, k):
         assert torch.equal(got, expected)
 
 
+@pytest.mark.parametrize("m,n,k", [(511, 9248, 256), (600, 2336, 512), (1000, 3104, 512), (1030, 4096, 256), (2049, 6016, 256), (1024, 12288, 256), (9000, 640, 8192)])
+def test_w4a4_wide_gemm_in_tall_tiles(qi, m, n, k):
+    # 256 x 64 tiles on 148 CTAs: a first wave alone, last waves of 16, 32, 48 and 64 columns, rows and columns that end within a
+    # tile, and (9000 rows, 74 MB of activations) blocks of rows of tiles; the bits of the int8 kernel, with whole 32-byte
+    # sectors to store and without
+    generator = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a, w = (torch.randint(-7, 8, (rows, k), dtype=torch.int16, device="cuda", generator=generator) & 0xF for rows in (m, n))
+    a, w = ((v[:, 0::2] | (v[:, 1::2] << 4)).to(torch.uint8).contiguous() for v in (a, w))
+    sa = (torch.rand(m, k // 64, device="cuda", generator=generator) * 0.5 + 0.05).half()
+    sw = (torch.rand(n, k // 64, device="cuda", generator=generator) * 5e-3 + 1e-3).half()
+    bias = torch.randn(n, device="cuda", generator=generator)
+    a_wide, w_wide = (torch.empty(rows, k, dtype=torch.uint8, device="cuda") for rows in (m, n))
+    assert qi.w4a4_widen_codes_ex(a, a_wide, m, k) == 0 and qi.w4a4_widen_codes_ex(w, w_wide, n, k) == 0
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        for ldy in (n, n + 8):
+            got, expected = (torch.full((m, ldy), -7.0, dtype=dtype, device="cuda") for _ in range(2))
+            assert qi.w4a4_gemm_wide_ex(a_wide, sa, w_wide, sw, bias, got, code, ldy, m, n, k) == 0
+            assert qi.w4a4_gemm_path_ex(a, sa, w, sw, bias, expected, code, ldy, m, n, k, qi.W4A4_PATH_INT8) == 0
+            check_status(qi)
+            assert torch.equal(got, expected)
+
+
 def test_w4a4_wide_gemm_extreme_dots(qi, wide_kernel):
     # all codes +-7: every group dot is +-3136, the largest the format allows; fp32 accumulation must stay exact
     m, n, k = 128, 128, 512
