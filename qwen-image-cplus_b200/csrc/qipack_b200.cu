@@ -364,26 +364,10 @@ int launch_w4a4_wide(const void *a_bytes, const void *a_scales, const void *w_by
                                       bias, y, dots, shape));
 }
 
-// How the pair kernel's tiles cover the output (see w4a4_pair::Tiling): the last, partial wave is cut into the narrowest
-// tiles that still fit one wave.
-w4a4_pair::Tiling w4a4_tiling(int m, int n, int pairs, bool may_narrow) {
-    namespace wp = w4a4_pair;
-    const int tiles_m = (m + 2 * wp::BM - 1) / (2 * wp::BM), tiles_n = (n + wp::BN - 1) / wp::BN, tiles = tiles_m * tiles_n;
-    const int wide = tiles / pairs * pairs;
-    if (may_narrow && wide < tiles) {
-        const int tail_n = wide / tiles_m * wp::BN, tail_m0 = wide % tiles_m;
-        for (int width = 64; width < wp::BN; width += 32) {
-            const int later = n > tail_n + wp::BN ? (n - tail_n - wp::BN + width - 1) / width : 0, sooner = (n - tail_n + width - 1) / width;
-            const int narrow = tail_m0 * later + (tiles_m - tail_m0) * sooner;
-            if (narrow <= pairs) return {wide + narrow, wide, width, tail_m0, tail_n, later, sooner};
-        }
-    }
-    return {tiles, tiles, wp::BN, 0, 0, 0, 0};
-}
-
+// `dots` given: the groups' dots are written too. Else `peers`: the tile goes into every GPU's copy of the output.
 int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
                      const float *bias, void *y, int32_t *dots, const GemmShape &shape, cudaStream_t stream, int device,
-                     const w4a4_pair::PeerOutputs *peers = nullptr) {
+                     const w4a4_pair::PeerOutputs *peers) {
     namespace wp = w4a4_pair;
     CUtensorMap map_a, map_w;
     if (!make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_bytes, shape.k, shape.m, static_cast<uint64_t>(shape.k),
@@ -392,20 +376,17 @@ int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_by
     if (!make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w_bytes, shape.k, shape.n, static_cast<uint64_t>(shape.k),
                   128, wp::B_BOX_ROWS, CU_TENSOR_MAP_SWIZZLE_128B))
         return INVALID;
-    if (peers != nullptr && dots != nullptr) return INVALID;
-    const int variant = peers != nullptr ? 2 : (dots != nullptr ? 1 : 0);
-    auto kernel = variant == 2 ? wp::gemm_kernel<false, true>
-                               : (variant == 1 ? wp::gemm_kernel<true, false> : wp::gemm_kernel<false, false>);
-    static std::atomic<bool> configured[MAX_DEVICES][3];
-    if (const cudaError_t error = configure_once(kernel, wp::SMEM_BYTES, configured[device][variant]))
+    if ((peers != nullptr) == (dots != nullptr)) return INVALID;
+    auto kernel = dots != nullptr ? wp::gemm_kernel<true, false> : wp::gemm_kernel<false, true>;
+    static std::atomic<bool> configured[MAX_DEVICES][2];
+    if (const cudaError_t error = configure_once(kernel, wp::SMEM_BYTES, configured[device][dots != nullptr]))
         return static_cast<int>(error);
     const wp::PeerOutputs outputs = peers != nullptr ? *peers : wp::PeerOutputs{};
-    const int pairs = sm_count(device) / 2;
-    const wp::Tiling tiling = w4a4_tiling(shape.m, shape.n, pairs, variant == 0);
-    const int grid = 2 * (tiling.tiles < pairs ? tiling.tiles : pairs);  // the kernel carries __cluster_dims__(2, 1, 1)
+    const int pairs = sm_count(device) / 2, tiles = ((shape.m + 2 * wp::BM - 1) / (2 * wp::BM)) * ((shape.n + wp::BN - 1) / wp::BN);
+    const int grid = 2 * (tiles < pairs ? tiles : pairs);  // the kernel carries __cluster_dims__(2, 1, 1)
     return static_cast<int>(launch_overlapped(kernel, grid, wp::THREADS, wp::SMEM_BYTES, stream, map_a, map_w,
                                               static_cast<const __half *>(a_scales), static_cast<const __half *>(w_scales),
-                                              bias, y, dots, shape, outputs, tiling));
+                                              bias, y, dots, shape, outputs));
 }
 
 // How the tall kernel's tiles cover the output (see w4a4_tall::Tiling).
@@ -673,7 +654,7 @@ int w4a4_gemm_wide(const void *a_bytes, const void *a_scales, const void *w_byte
     if (single_cta || k % w4a4_pair::STAGE_K != 0 || !scales_aligned8)
         return launch_w4a4_wide<6>(a_bytes, a_scales, w_bytes, w_scales, bias, y, dots, shape, stream, device);
     if (dots == nullptr) return launch_w4a4_bytes(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    return launch_w4a4_pair(a_bytes, a_scales, w_bytes, w_scales, bias, y, dots, shape, stream, device);
+    return launch_w4a4_pair(a_bytes, a_scales, w_bytes, w_scales, bias, y, dots, shape, stream, device, nullptr);
 }
 
 // The W4A4 GEMM on nibble-packed codes (the reference's operand format). `path`: 1 = the int8 kernel that widens the

@@ -1,5 +1,6 @@
 // W4A4 (H256, g64) GEMM on byte-wide (E4M3) codes, one 256 x 128 output tile per PAIR of CTAs
-// (thread-block cluster of two, tcgen05 cta_group::2). Same operator, arithmetic and bits as
+// (thread-block cluster of two, tcgen05 cta_group::2): the kernel that writes every GPU's copy of a sharded output, and
+// the one that also writes the groups' dots; plain outputs take w4a4_tall_gemm.cuh. Same operator, arithmetic and bits as
 // w4a4_wide_gemm.cuh and the reference's w4a4_gemm_kernel (qwen_image_cuda/cuda/gemm.cu:65-189).
 //
 // Per group of 64 inputs the tensor cores leave a tile of EXACT integer dots (as fp32) in TMEM and
@@ -178,17 +179,9 @@ struct PeerOutputs {
     int count, first;
 };
 
-// The order of the tiles. Tiles of 256 x 128 walk down the rows first. `wide` of them, a multiple of the pairs that run
-// at once, come first; what would be a last, partly idle wave of them is cut again, into tiles of `width` columns, as many
-// as there are pairs or fewer: 1024 x 4096 outputs are 128 tiles, two waves of 74 pairs, or one wave and 74 tiles of 96
-// columns (K = 4096: 49.9 -> 47.5 us); 4096 x 3072 are 384, five waves and 14, or 28 of 64 (K = 12288: 385 -> 360 us). tail_m0 rows of tiles start their narrow tiles one wide tile later than the others.
-struct Tiling {
-    int tiles, wide, width;
-    int tail_m0, tail_n;       // first column (of the rows of tiles from tail_m0 on) that is left to narrow tiles
-    int tail_later, tail_sooner;  // narrow tiles per row of tiles, for the first tail_m0 rows and for the others
-};
+// Tiles of 256 x 128 walk down the rows first.
 struct TilePlace {
-    int m_index, n0, width;
+    int m_index, n0;
 };
 
 // Everything a role needs to find its way around the CTA's shared memory and the problem.
@@ -199,17 +192,8 @@ struct View {
     uint2 *ring;
     uint64_t *full, *scale_ready, *empty, *dot_full, *dot_empty;
     uint32_t tmem_base, cta;
-    int pair, pairs, tiles_m, k_stages, groups;
-    Tiling tiling;
-    __device__ __forceinline__ TilePlace place(int tile) const {
-        if (tile < tiling.wide) return {tile % tiles_m, tile / tiles_m * BN, BN};
-        int narrow = tile - tiling.wide;
-        const int later = tiling.tail_m0 * tiling.tail_later;
-        if (narrow < later) return {narrow % tiling.tail_m0, tiling.tail_n + BN + narrow / tiling.tail_m0 * tiling.width, tiling.width};
-        narrow -= later;
-        const int rows = tiles_m - tiling.tail_m0;
-        return {tiling.tail_m0 + narrow % rows, tiling.tail_n + narrow / rows * tiling.width, tiling.width};
-    }
+    int pair, pairs, tiles_m, tiles, k_stages, groups;
+    __device__ __forceinline__ TilePlace place(int tile) const { return {tile % tiles_m, tile / tiles_m * BN}; }
 };
 
 // A walk over this pair's (tile, stage) sequence. Integer division costs a warp more than a hundred cycles: it happens
@@ -218,7 +202,7 @@ struct StageWalk {
     int tile, ks;
     TilePlace at;
     __device__ __forceinline__ StageWalk(const View &v) : tile(v.pair), ks(0), at(v.place(v.pair)) {}
-    __device__ __forceinline__ bool done(const View &v) const { return tile >= v.tiling.tiles; }
+    __device__ __forceinline__ bool done(const View &v) const { return tile >= v.tiles; }
     __device__ __forceinline__ void next(const View &v) {
         if (++ks == v.k_stages) {
             ks = 0;
@@ -238,9 +222,9 @@ __device__ __forceinline__ void producer_role(const View &v, const CUtensorMap *
     for (StageWalk walk(v); !walk.done(v); walk.next(v)) {
         if (!mbarrier_wait(&v.empty[s], phase ^ 1, &g_status, STATUS_WAIT_EMPTY | 0x5000 | s, AHEAD_BACKOFF_NS)) break;
         // A tile's columns belong half to one team and half to the other; of a team's columns this CTA holds the first or
-        // the second half (of a narrow tile it loads some rows that nothing reads).
+        // the second half.
         const int m0 = walk.at.m_index * 2 * BM + static_cast<int>(v.cta) * BM;
-        const int n0 = walk.at.n0 + static_cast<int>(v.cta) * (walk.at.width / (2 * TEAMS));
+        const int n0 = walk.at.n0 + static_cast<int>(v.cta) * B_BOX_ROWS;
         // the leader expects the bytes of both CTAs' loads on its barrier
         if (v.cta == 0) mbarrier_arrive_expect_tx(&v.full[s], 2 * (A_BYTES + B_BYTES));
 #pragma unroll
@@ -250,7 +234,7 @@ __device__ __forceinline__ void producer_role(const View &v, const CUtensorMap *
 #pragma unroll
             for (int team = 0; team < TEAMS; ++team)  // this CTA's half of each team's columns
                 tma_load_2d_pair(v.tile_b + s * B_BYTES + half * B_HALF_BYTES + team * (B_BOX_ROWS * 128), map_w, &v.full[s], k0,
-                                 n0 + team * (walk.at.width / TEAMS));
+                                 n0 + team * TEAM_COLUMNS);
         }
         if (++s == STAGES) s = 0, phase ^= 1;
     }
@@ -328,9 +312,9 @@ __device__ __forceinline__ void mma_role(const View &v, uint32_t mine) {
     const uint64_t a_first = umma_desc_k_sw128(smem_u32(v.tile_a) + turn * A_HALF_BYTES);
     const uint64_t b_first = umma_desc_k_sw128(smem_u32(v.tile_b) + turn * B_HALF_BYTES + team * (B_BOX_ROWS * 128));
     const uint32_t accumulator = v.tmem_base + (team * BUFFERS + turn) * BUFFER_COLUMNS;
+    constexpr uint32_t idesc = umma_idesc_e4m3_f32(2 * BM, TEAM_COLUMNS);
     uint32_t s = 0, phase = 0, buffer_phase = 1;
     for (StageWalk walk(v); !walk.done(v); walk.next(v)) {
-        const uint32_t idesc = umma_idesc_e4m3_f32(2 * BM, 0) | (static_cast<uint32_t>(walk.at.width / TEAMS >> 3) << 17);
         if (!mbarrier_wait_uniform2(full + s * 8, phase, dot_empty, buffer_phase, &g_status, STATUS_WAIT_TMEM_EMPTY | 0x5000 | s, MMA_BACKOFF_NS)) break;
         tcgen05_fence_after();
         if (elect_one()) {
@@ -363,14 +347,15 @@ struct FoldState {
     bool failed;
 };
 
-// One tile: WIDTH columns per warp, 32 of a wide tile, 24 or 16 of a narrow one. False when a wait ran out of time.
+// One tile's 32 columns of a warp. False when a wait ran out of time.
 // A look at a barrier is one try_wait by every lane; a lane that finds the phase incomplete polls on its own, with
 // pauses (the fold warps are the pace-setters: that path is for the first groups and for errors). A wait that ran
 // out of time sets `failed` in its lane; the warp looks at the flags once per stage.
-template <int WIDTH, bool DUMP_DOTS, bool SCATTER>
+template <bool DUMP_DOTS, bool SCATTER>
 __device__ __forceinline__ bool fold_tile(FoldState &f, int row, int n0, uint32_t tmem_lane, uint32_t sw_base, int k_stages, int groups,
                                           const float *__restrict__ bias, void *__restrict__ y, const PeerOutputs &peers,
                                           int32_t *__restrict__ dots_out, const GemmShape &shape, int lane) {
+    constexpr int WIDTH = COLUMNS;
     uint32_t dots[COLUMNS];  // dots[j] = dot of this thread's row and column j of the warp's
     uint64_t acc[WIDTH / 2];  // acc[j] = columns 2 j, 2 j + 1
 #pragma unroll
@@ -521,20 +506,11 @@ __device__ __forceinline__ void fold_role(const View &v, const float *__restrict
                    smem_u32(v.sa_tile) + (quadrant * 32 + lane) * 16, smem_u32(v.scale_ready), smem_u32(v.empty), 0, 0, 0, false};
     const uint32_t tmem_lane = v.tmem_base + team * BUFFERS * BUFFER_COLUMNS + (static_cast<uint32_t>(quadrant * 32) << 16);
     const uint32_t sw_tile = smem_u32(v.sw_tile);
-    for (int tile = v.pair; tile < v.tiling.tiles; tile += v.pairs) {
+    const int in_team = slice % (TEAM_COLUMNS / COLUMNS) * COLUMNS, in_tile = slice * COLUMNS;
+    for (int tile = v.pair; tile < v.tiles; tile += v.pairs) {
         const TilePlace at = v.place(tile);
         const int row = at.m_index * 2 * BM + static_cast<int>(v.cta) * BM + quadrant * 32 + lane;
-        const int columns = at.width / (TEAMS * TEAM_COLUMNS / COLUMNS);  // of this warp
-        const int in_team = slice % (TEAM_COLUMNS / COLUMNS) * columns, in_tile = slice * columns;
-        bool alive;
-        if (at.width == BN)
-            alive = fold_tile<32, DUMP_DOTS, SCATTER>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane);
-        else if (DUMP_DOTS || SCATTER) alive = false;  // the launcher cuts no narrow tiles for these
-        else if (at.width == 96)
-            alive = fold_tile<24, false, false>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane);
-        else
-            alive = fold_tile<16, false, false>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane);
-        if (!alive) break;
+        if (!fold_tile<DUMP_DOTS, SCATTER>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane)) break;
     }
     tmem_load_wait();  // nothing of this warp may still be in flight at teardown
 }
@@ -544,7 +520,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
             const __half *__restrict__ a_scales, const __half *__restrict__ w_scales,
             const float *__restrict__ bias, void *__restrict__ y, int32_t *__restrict__ dots_out,
-            const GemmShape shape, const __grid_constant__ PeerOutputs peers, const __grid_constant__ Tiling tiling) {
+            const GemmShape shape, const __grid_constant__ PeerOutputs peers) {
     extern __shared__ uint8_t smem_raw[];
     // the same offsets in both CTAs: the dynamic shared window starts at the same address in each
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -563,7 +539,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t cta = cluster_ctarank();  // 0 = leader
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const int tiles_m = (shape.m + 2 * BM - 1) / (2 * BM), k_stages = shape.k / STAGE_K, groups = shape.k / 64;
+    const int tiles_m = (shape.m + 2 * BM - 1) / (2 * BM), tiles = tiles_m * ((shape.n + BN - 1) / BN), k_stages = shape.k / STAGE_K, groups = shape.k / 64;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -592,7 +568,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 
     const uint32_t tmem_base = *tmem_slot;
     const View view = {tile_a, tile_b, sw_tile, sa_tile, ring, full, scale_ready, empty, dot_full, dot_empty,
-                       tmem_base, cta, pair, pairs, tiles_m, k_stages, groups, tiling};
+                       tmem_base, cta, pair, pairs, tiles_m, tiles, k_stages, groups};
 
     if (warp < FOLD_WARP0) {
         setmaxnreg_dec<CONTROL_REGISTERS>();
