@@ -454,15 +454,16 @@ int launch_w4a4_narrow(const void *a_bytes, const void *a_scales, const void *w_
 //     (0.21 and 0.135 in several waves)
 //   tall tiles ({256 .. 16384} rows): 0.27 a wave (4096 x 9216 x 3072 198 us, 16 waves of 48 groups; 0.29 where there are
 //     one or two: 512 x 9216 x 3072 27.8), 0.24, 0.20 and 0.14 for a last wave of 48, 32 or 16 columns (1024 x 4096 x 4096
-//     34.0, 1024 x 3072 x 3072 23.4, 1024 x 12288 x 4096 95.0), 0.02 more where it is the only one (256 x 3072 x 3072 10.8,
-//     in 128 x 64 tiles 9.4)
+//     34.0, 1024 x 3072 x 3072 23.4, 1024 x 12288 x 4096 95.0), 0.08 more where it is the only one (256 x 3072 x 3072 10.8,
+//     in 128 x 64 tiles 9.4): 0.02 measured, the rest because the others' prices for two waves are as much too high (178 x 5248 x
+//     8960 30.7, in 32 rows 29.6; 401 x 3072 x 12288 43.4 against 62.7 on pairs)
 int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
                       void *y, const GemmShape &shape, cudaStream_t stream, int device) {
     namespace wn = w4a4_narrow;
     const int sms = sm_count(device);
     const w4a4_tall::Tiling tiling = w4a4_tall_tiling(shape, sms);
     const int wide_waves = (tiling.wide + sms - 1) / sms;
-    const double last_us = tiling.tiles == tiling.wide ? 0.0 : (tiling.width == 48 ? 0.24 : (tiling.width == 32 ? 0.20 : 0.14)) + (tiling.wide == 0 ? 0.02 : 0.0);
+    const double last_us = tiling.tiles == tiling.wide ? 0.0 : (tiling.width == 48 ? 0.24 : (tiling.width == 32 ? 0.20 : 0.14)) + (tiling.wide == 0 ? 0.08 : 0.0);
     const double tall_us = wide_waves * (wide_waves <= 2 ? 0.29 : 0.27) + last_us;
     const long long tiles_m = (shape.m + wn::BM - 1) / wn::BM;
     const long long waves_64 = (tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms, waves_32 = (tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms;
@@ -636,7 +637,7 @@ int w4a16_linear(const void *x_half, const void *codes, const void *scales, cons
     return w4a16_gemm(x_half, codes, scales, minimums, bias, y, y_dtype, ldy, m, n, k, whole_n, 0, stream);
 }
 
-// single_cta: always the one-CTA kernel (128 x 128 tiles); otherwise CTA pairs where the shape and pointers allow.
+// single_cta: always 128 x 128 tiles (w4a4_wide); otherwise what launch_w4a4_bytes chooses, where the shape and pointers allow.
 int w4a4_gemm_wide(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
                    const float *bias, void *y, int y_dtype, long long ldy, int32_t *dots, int m, int n, int k,
                    bool single_cta, cudaStream_t stream) {
@@ -648,8 +649,8 @@ int w4a4_gemm_wide(const void *a_bytes, const void *a_scales, const void *w_byte
     const int device = current_device();
     if (device < 0) return INVALID;
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
-    // The pair kernel's stage is four groups, and it stages both scale arrays eight bytes at a time; anything
-    // else goes to the one-CTA kernel, which takes two groups per stage and four-byte-aligned scales.
+    // The other kernels stage both scale arrays four groups, eight bytes, at a time; anything
+    // else goes to the 128 x 128 tiles, which takes two groups per stage and four-byte-aligned scales.
     const bool scales_aligned8 = ((reinterpret_cast<uintptr_t>(a_scales) | reinterpret_cast<uintptr_t>(w_scales)) & 7) == 0;
     if (single_cta || k % w4a4_pair::STAGE_K != 0 || !scales_aligned8)
         return launch_w4a4_wide<6>(a_bytes, a_scales, w_bytes, w_scales, bias, y, dots, shape, stream, device);
