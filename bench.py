@@ -54,10 +54,10 @@ METRIC = "packed W4A4/W4A16 GEMM TOPS at M=4096 block shapes, % of tensor/HBM ro
 UNIT = "TOPS"
 CPU_SAMPLE_ROWS = 256
 CPU_PASSES = 5
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one w4a4_pair::gemm_kernel launch on the qkv
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one w4a4_tall::gemm_kernel launch on the qkv
 # shape at M = 4096, whose 2MNK is the average of the block's four launches: from the ncu capture that the
 # kernel's profile summary records. Scaled by rows and ranks for other workloads; None for other kernels.
-NCU_TRAFFIC_BYTES_QKV_M4096 = 82.7e6
+NCU_TRAFFIC_BYTES_QKV_M4096 = 75.8e6
 
 
 def block_ops(m: int) -> float:
@@ -230,7 +230,7 @@ def other_kernels(qi, torch, device, stream, peaks, tensor_peaks, m):
                                   "peak_source": tensor_peaks["how"]}
 
     # The entry points the reference binds, on its operand format (nibble-packed codes). By shape they widen both operands
-    # into scratch memory of the stream's pool and run the byte-operand kernel on CTA pairs; the int8 kernel that widens
+    # into scratch memory of the stream's pool and run the byte-operand kernels; the int8 kernel that widens
     # the nibbles in shared memory is timed beside it.
     packed, ops, seconds, int8_seconds = [], 0.0, 0.0, 0.0
     for name, n, k, _ in LINEARS:
@@ -251,7 +251,7 @@ def other_kernels(qi, torch, device, stream, peaks, tensor_peaks, m):
         packed.append({"linear": name, "ms": ms, "tops": 2.0 * m * n * k / ms / 1e9, "int8_kernel_ms": int8_ms})
         del w_codes, a_codes, w_scales, a_scales, y
     out["w4a4_packed"] = {"kernel": "qi_w4a4_gemm_ex (the drop-in ABI, nibble-packed operands): one widening kernel into (m + n) k bytes of "
-                                    "pool scratch, then w4a4_pair::gemm_kernel; int8_kernel: w4a4::gemm_kernel on the nibbles",
+                                    "pool scratch, then w4a4_tall::gemm_kernel; int8_kernel: w4a4::gemm_kernel on the nibbles",
                           "linears": packed, "tops": ops / seconds / 1e12, "frac_of_e4m3_mma_loop": ops / seconds / 1e12 / tensor_peaks["e4m3"],
                           "int8_kernel_tops": ops / int8_seconds / 1e12,
                           "int8_kernel_frac_of_int8_mma_loop": ops / int8_seconds / 1e12 / tensor_peaks["s8"]}
@@ -717,7 +717,7 @@ def run_block(args):
             "gpu_launches": timed_launches,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "steps": e2e_steps, "ms_per_step": e2e_ms / e2e_steps},
-            "roofline": {"kernel": "w4a4::gemm_kernel" if args.w4a4_path == "int8" else "w4a4_pair::gemm_kernel", "bound": "tensor",
+            "roofline": {"kernel": "w4a4::gemm_kernel" if args.w4a4_path == "int8" else "w4a4_tall::gemm_kernel", "bound": "tensor",
                          "achieved": achieved, "peak": eight_bit_peak, "unit": "TOP/s", "frac": achieved / eight_bit_peak,
                          "frac_of_2x_bf16_burst": achieved / (2.0 * peaks["bf16_burst"]),
                          "frac_of_2x_bf16_sustained": achieved / (2.0 * peaks["bf16_sustained"]),
@@ -969,7 +969,7 @@ def run_block_pairs(args):
             "gpu_launches": timed_launches,
             "e2e": {"value": ops_per_step * e2e_steps / (e2e_ms * 1e-3) / 1e12, "unit": UNIT, "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "steps": e2e_steps, "ms_per_step": e2e_ms / e2e_steps},
-            "roofline": {"kernel": "w4a4_pair::gemm_kernel", "bound": "tensor", "achieved": achieved, "peak": tensor_peaks["e4m3"],
+            "roofline": {"kernel": "w4a4_tall::gemm_kernel", "bound": "tensor", "achieved": achieved, "peak": tensor_peaks["e4m3"],
                          "unit": "TOP/s", "frac": achieved / tensor_peaks["e4m3"],
                          "frac_of_2x_bf16_burst": achieved / (2.0 * peaks["bf16_burst"]),
                          "frac_of_2x_bf16_sustained": achieved / (2.0 * peaks["bf16_sustained"]),
@@ -1238,7 +1238,7 @@ def main():
                         help="skip the W4A16 GEMM / GEMV / quantiser figures (profiling runs)")
     parser.add_argument("--w4a4-path", default="wide", choices=["packed", "int8", "wide"],
                         help="packed: the drop-in entry points on nibble-packed codes, kernel by shape (both operands widened into "
-                             "pool scratch for the CTA-pair kernel); int8: the same entry points held to the int8 kernel that widens "
+                             "pool scratch for the byte-operand kernels); int8: the same entry points held to the int8 kernel that widens "
                              "the nibbles in shared memory; wide: byte-wide E4M3 codes on CTA pairs (weights widened once at load)")
     parser.add_argument("--gather", default="auto", choices=["auto", "fused", "copy", "slabs", "nccl"],
                         help="N > 1: how the column slices reach every GPU. auto: copy on two GPUs, nccl on more. nccl: an all-gather after each GEMM; fused: the "

@@ -197,8 +197,8 @@ int qi_w4a4_gelu_quantize_ex(const float *x, void *codes, void *scales, void *by
 int qi_w4a4_gemm_wide_ex(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
                          const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, void *stream);
 
-/* The same operator on one CTA per 128x128 tile instead of a CTA pair per 256x128 tile (the kernel
- * qi_w4a4_gemm_wide_ex itself falls back to when k is not a multiple of 256 or a scale array is
+/* The same operator in 128x128 tiles whatever the shape (the kernel qi_w4a4_gemm_wide_ex itself falls back to
+ * when k is not a multiple of 256 or a scale array is
  * not 8-byte aligned). `dots` may be NULL; otherwise [m, n, k/64] as below. Same bits. */
 int qi_w4a4_gemm_wide_single_ex(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
                                 const float *bias, void *y, int y_dtype, long long ldy, int32_t *dots, int m, int n,
