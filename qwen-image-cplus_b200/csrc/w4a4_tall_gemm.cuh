@@ -144,6 +144,7 @@ __device__ __forceinline__ bool fold_tile(FoldState &f, int row, int n0, int slo
             wait_dots<WIDTH>(dots);
             if (g % SLAB_GROUPS == SLAB_GROUPS - 1) {  // the whole warp's dots of both groups are in registers or folded
                 tcgen05_fence_before();
+                __syncwarp();  // every lane's copies are ordered before the one arrival
                 if (lane == 0) arrive_u32(f.dot_empty + buffer * 8);
             }
 #pragma unroll

@@ -1,0 +1,33 @@
+"""Rules of the kernel sources that a run cannot show: a hand-over that is one barrier short gives wrong sums only now and then."""
+import glob
+import os
+import re
+
+import pytest
+
+import __graft_entry__ as entry
+
+KERNELS = sorted(glob.glob(os.path.join(entry.PACKAGE_DIR, "csrc", "*.cuh")))
+
+
+def statements(path):
+    """The file's lines without comments and blank ones, as (number, text)."""
+    lines = (re.sub(r"//.*", "", line).strip() for line in open(path, encoding="utf-8"))
+    return [(number, line) for number, line in enumerate(lines, 1) if line]
+
+
+@pytest.mark.parametrize("path", KERNELS, ids=os.path.basename)
+def test_a_lane_that_arrives_for_its_warp_follows_a_warp_barrier(path):
+    # lane 0's arrival says that ALL lanes have read or written what changes hands; only a __syncwarp() orders theirs before it
+    code = statements(path)
+    for i, (number, line) in enumerate(code):
+        if not line.startswith("if (lane == 0)"):
+            continue
+        first = code[i + 1][1] if line.endswith("{") else line
+        if "arrive" in first and "expect_tx" not in first:
+            assert code[i - 1][1] == "__syncwarp();", f"{os.path.basename(path)}:{number}: arrives for lanes that may not be there yet"
+
+
+def test_the_rule_reaches_the_hand_overs():
+    arrivals = sum(line.startswith("if (lane == 0)") and "arrive" in line for path in KERNELS for _, line in statements(path))
+    assert arrivals >= 15
