@@ -197,6 +197,12 @@ int qi_w4a4_gelu_quantize_ex(const float *x, void *codes, void *scales, void *by
 int qi_w4a4_gemm_wide_ex(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
                          const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, void *stream);
 
+/* Host only: how qi_w4a4_gemm_wide_ex covers an [m, n] output over k inputs (k % 256 == 0, 8-byte-aligned scales) on a
+ * GPU with `sms` multiprocessors. plan[0]: 0 = tiles of 256 rows x 64 outputs, 1 and 2 = 128 x 64 and 128 x 32, 3, 4 and 5 = 128
+ * outputs x 16, 32 and 48 rows. For the first kind, chosen or not: plan[1] whole tiles, then plan[2] tiles of plan[3]
+ * outputs; rows of tiles in a block (plan[4]) and in the last block (plan[5]). For tests and tuning. */
+int qi_w4a4_gemm_plan(int m, int n, int k, int sms, int *plan);
+
 /* The same operator in 128x128 tiles whatever the shape (the kernel qi_w4a4_gemm_wide_ex itself falls back to
  * when k is not a multiple of 256 or a scale array is
  * not 8-byte aligned). `dots` may be NULL; otherwise [m, n, k/64] as below. Same bits. */

@@ -11,6 +11,7 @@ There is no CPU path: loading fails loudly when the library has not been built.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import os
 import subprocess
@@ -145,6 +146,7 @@ SIGNATURES = {
     "qi_probe_wait_timeout": [_ULL, _P],
     "qi_w4a16_gemm_tile_ex": [_P, _P, _P, _P, _P, _P, _I, _LL, _I, _I, _I, _I, _P],
     "qi_w4a4_gemm_wide_single_ex": [_P, _P, _P, _P, _P, _P, _I, _LL, _P, _I, _I, _I, _P],
+    "qi_w4a4_gemm_plan": [_I, _I, _I, _I, ctypes.POINTER(_I)],
 }
 
 _lib = None
@@ -335,6 +337,19 @@ def w4a4_gemm_wide_single_ex(a_bytes, a_scales, w_bytes, w_scales, bias, y, y_dt
     """The byte-operand W4A4 GEMM on single CTAs; `dots` [m, n, k/64] int32 or None."""
     return lib().qi_w4a4_gemm_wide_single_ex(_p(a_bytes), _p(a_scales), _p(w_bytes), _p(w_scales), _p(bias), _p(y),
                                              y_dtype, ldy, _p(dots), m, n, k, _p(stream))
+
+
+# How the byte-operand W4A4 GEMM covers an output; see include/qipack_b200.h.
+W4A4Plan = collections.namedtuple("W4A4Plan", "tiles whole cut width block last_rows")
+W4A4_TILES = ("256x64", "128x64", "128x32", "16 rows", "32 rows", "48 rows")
+
+
+def w4a4_gemm_plan(m: int, n: int, k: int, sms: int = 148) -> W4A4Plan:
+    """Which tiles w4a4_gemm_wide_ex takes for a shape, and how tiles of 256 x 64 would cover it. Needs no GPU."""
+    plan = (ctypes.c_int * 6)()
+    if lib().qi_w4a4_gemm_plan(m, n, k, sms, plan) != 0:
+        raise ValueError(f"no plan for {m} x {n} x {k}")
+    return W4A4Plan(W4A4_TILES[plan[0]], *plan[1:])
 
 
 # ---- transformer::linear (transformer.cplus:673-713) ------------------------------------------

@@ -448,48 +448,62 @@ int launch_w4a4_narrow(const void *a_bytes, const void *a_scales, const void *w_
                                               static_cast<const __half *>(EXCHANGED ? a_scales : w_scales), bias, y, shape, box_rows));
 }
 
-// Byte operands with k a multiple of 256 and 8-byte aligned scales: tall tiles (256 x 64), or tiles of 128 rows, or of 16
-// to 48 activation rows, where those are estimated to be faster. Microseconds per group and wave as measured on B200:
-//   narrow tiles ({77, 128, 256, 512} rows, outputs 3072 to 12288, K 3072 to 12288): 0.185 and 0.12 for 64 and 32 columns
-//     (0.21 and 0.135 in several waves)
-//   tall tiles ({256 .. 16384} rows): 0.27 a wave (4096 x 9216 x 3072 198 us, 16 waves of 48 groups; 0.29 where there are
-//     one or two: 512 x 9216 x 3072 27.8), 0.24, 0.20 and 0.14 for a last wave of 48, 32 or 16 columns (1024 x 4096 x 4096
-//     34.0, 1024 x 3072 x 3072 23.4, 1024 x 12288 x 4096 95.0), 0.08 more where it is the only one (256 x 3072 x 3072 10.8,
-//     in 128 x 64 tiles 9.4): 0.02 measured, the rest because the others' prices for two waves are as much too high (178 x 5248 x
-//     8960 30.7, in 32 rows 29.6; 401 x 3072 x 12288 43.4 against 62.7 on pairs)
+// Byte operands with k a multiple of 256 and 8-byte aligned scales: tall tiles (256 x 64), tiles of 128 rows by 64 or 32
+// outputs, or of 128 outputs by 16, 32 or 48 activation rows; the values are the entry point's (qi_w4a4_gemm_plan).
+enum W4A4Tiles { W4A4_TALL, W4A4_COLUMNS_64, W4A4_COLUMNS_32, W4A4_ROWS_16, W4A4_ROWS_32, W4A4_ROWS_48 };
+
+// The tiles that are estimated to be fastest. A wave costs microseconds of its own and microseconds per group of 64 inputs;
+// what every kernel pays once (2.6) is left out. Fitted to 677 shapes (9 to 16384 rows, 512 to 18432 outputs, 256 to 12288
+// inputs, another matrix of weights every launch): within 2 to 6 % of each kernel's times, and the tiles chosen are
+// 0.3 % slower than the best of the six in the mean. Prices without K, and 15 % more for every wave after the first, were 3.5 % off (264 x
+// 9568 x 3328 37.9 us in tall tiles, 29.5 in 48 rows; 308 x 12288 x 3072 41.5 and 35.1; 708 x 1568 x 4096 19.8 in 128 x 32, 15.5 in tall ones).
+//   far_rows: where rows lie a multiple of 4096 bytes apart their loads are slower, and the kernels that wait for loads lose
+//     by it (593 x 4096 x 4096 34.6 us in 48 rows, 31.4 in tall tiles; 771 x 3072 x 3072 21.9 and 24.5), but for one tile of up to 16 rows
+//   large: every tile of activation rows reads all weights, from DRAM where L2 does not hold them (190 x 8896 x 9728 47.6 us
+//     in 48 rows, 42.0 in tall tiles)
+W4A4Tiles choose_w4a4(const GemmShape &shape, int sms) {
+    namespace wn = w4a4_narrow;
+    const double groups = shape.k / 64;
+    const bool far_rows = shape.k % 4096 == 0, large = static_cast<long long>(shape.n) * shape.k > (64LL << 20);
+    const long long tiles_m = (shape.m + wn::BM - 1) / wn::BM, tiles_n = (shape.n + wn::BM - 1) / wn::BM;
+    const auto columns_us = [&](int columns, double wave, double group) {
+        return ((tiles_m * ((shape.n + columns - 1) / columns) + sms - 1) / sms) * (wave + groups * group);
+    };
+    const auto rows_us = [&](int rows, double wave, double group) {
+        const double again = large && shape.m > rows ? 1.1 : 1.0;
+        return ((tiles_n * ((shape.m + rows - 1) / rows) + sms - 1) / sms) * (wave + groups * group * again);
+    };
+    const w4a4_tall::Tiling tiling = w4a4_tall_tiling(shape, sms);
+    const bool cut = tiling.tiles > tiling.wide;
+    const int wide_waves = (tiling.wide + sms - 1) / sms;
+    const double last = !cut ? 0.0 : tiling.width == 48 ? 0.207 : tiling.width == 32 ? 0.15 : 0.125;
+    const struct {
+        W4A4Tiles tiles;
+        double us;
+    } prices[] = {
+        {W4A4_ROWS_16, rows_us(16, 0.75, far_rows ? 0.110 : 0.073)},
+        {W4A4_ROWS_32, rows_us(32, 0.80, far_rows && shape.m > 16 ? 0.124 : 0.0957)},
+        {W4A4_ROWS_48, rows_us(48, 0.93, far_rows ? 0.150 : 0.1157)},
+        {W4A4_COLUMNS_64, columns_us(64, 1.30, far_rows ? 0.173 : 0.144)},
+        {W4A4_COLUMNS_32, columns_us(32, 0.71, far_rows ? 0.108 : 0.090)},
+        {W4A4_TALL, 0.6 + (wide_waves + cut) * 1.5 + groups * (wide_waves * 0.23 + last)},
+    };
+    int best = 0;
+    for (int i = 1; i < 6; ++i)
+        if (prices[i].us < prices[best].us) best = i;
+    return prices[best].tiles;
+}
+
 int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
                       void *y, const GemmShape &shape, cudaStream_t stream, int device) {
-    namespace wn = w4a4_narrow;
-    const int sms = sm_count(device);
-    const w4a4_tall::Tiling tiling = w4a4_tall_tiling(shape, sms);
-    const int wide_waves = (tiling.wide + sms - 1) / sms;
-    const double last_us = tiling.tiles == tiling.wide ? 0.0 : (tiling.width == 48 ? 0.24 : (tiling.width == 32 ? 0.20 : 0.14)) + (tiling.wide == 0 ? 0.08 : 0.0);
-    const double tall_us = wide_waves * (wide_waves <= 2 ? 0.29 : 0.27) + last_us;
-    const long long tiles_m = (shape.m + wn::BM - 1) / wn::BM;
-    const long long waves_64 = (tiles_m * ((shape.n + 63) / 64) + sms - 1) / sms, waves_32 = (tiles_m * ((shape.n + 31) / 32) + sms - 1) / sms;
-    const double us_64 = waves_64 * (waves_64 == 1 ? 0.185 : 0.21), us_32 = waves_32 * (waves_32 == 1 ? 0.12 : 0.135);
-    // Weights as the 128 rows of a tile, activation rows as its columns, where that folds less for rows that do not exist:
-    // 0.12, 0.135 and 0.16 for 16, 32 and 48 columns, 15 % more in several waves (77 x 9216 x 3072 11.7 -> 10.4 us, 77 x
-    // 12288 x 3072 18.3 -> 15.4, 256 x 3072 x 3072 11.8 -> 10.0). Where one tile of 32 columns holds all rows it is priced below
-    // two of 16, 0.105, by what long rows measure (with 16 and with 32: 16 x 3072 x 12288 22.4 and 18.9, x 4096 9.2 and 8.2, 16 x
-    // 9216 x 3072 8.2 and 8.4). That line is drawn without K, and at K = 3072 it gives some away (16 x 3072 5.9 and 6.2, 32 x 3072
-    // 6.1 and 7.4, 1 x 12288 9.3 and 10.4; 77 x 3072 6.8 in tiles of 16, 8.0 in 128 x 32).
-    const double others_us = us_64 < us_32 ? (us_64 < tall_us ? us_64 : tall_us) : (us_32 < tall_us ? us_32 : tall_us);
-    const long long tiles_n = (shape.n + wn::BM - 1) / wn::BM;
-    const auto exchanged_us = [&](int columns, double us) {
-        const long long waves = (tiles_n * ((shape.m + columns - 1) / columns) + sms - 1) / sms;
-        return waves == 1 ? us : waves * us * 1.15;
-    };
-    const double us_16_rows = exchanged_us(16, 0.12), us_32_rows = exchanged_us(32, shape.m <= 32 ? 0.105 : 0.135), us_48_rows = exchanged_us(48, 0.16);
-    if (us_16_rows <= us_32_rows && us_16_rows <= us_48_rows && us_16_rows < others_us)
-        return launch_w4a4_narrow<16, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    if (us_32_rows <= us_48_rows && us_32_rows < others_us)
-        return launch_w4a4_narrow<32, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    if (us_48_rows < others_us)
-        return launch_w4a4_narrow<48, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    if (us_64 <= us_32 && us_64 < tall_us) return launch_w4a4_narrow<64, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    if (us_32 < tall_us) return launch_w4a4_narrow<32, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
-    return launch_w4a4_tall(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    switch (choose_w4a4(shape, sm_count(device))) {
+        case W4A4_ROWS_16: return launch_w4a4_narrow<16, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+        case W4A4_ROWS_32: return launch_w4a4_narrow<32, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+        case W4A4_ROWS_48: return launch_w4a4_narrow<48, true>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+        case W4A4_COLUMNS_64: return launch_w4a4_narrow<64, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+        case W4A4_COLUMNS_32: return launch_w4a4_narrow<32, false>(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+        default: return launch_w4a4_tall(a_bytes, a_scales, w_bytes, w_scales, bias, y, shape, stream, device);
+    }
 }
 
 bool output_ok(const void *y, int y_dtype, long long ldy, int n) {
@@ -812,6 +826,19 @@ int qi_w4a4_gemm_wide_ex(const void *a_bytes, const void *a_scales, const void *
                          const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, void *stream) {
     return w4a4_gemm_wide(a_bytes, a_scales, w_bytes, w_scales, bias, y, y_dtype, ldy, nullptr, m, n, k, false,
                           static_cast<cudaStream_t>(stream));
+}
+
+int qi_w4a4_gemm_plan(int m, int n, int k, int sms, int *plan) {
+    if (m <= 0 || n <= 0 || k <= 0 || n % 32 != 0 || k % w4a4_pair::STAGE_K != 0 || sms < 2 || plan == nullptr) return INVALID;
+    const GemmShape shape = {m, n, k, n, 0};
+    const w4a4_tall::Tiling tiling = w4a4_tall_tiling(shape, sms);
+    plan[0] = choose_w4a4(shape, sms);
+    plan[1] = tiling.wide;
+    plan[2] = tiling.tiles - tiling.wide;
+    plan[3] = tiling.width;
+    plan[4] = tiling.block;
+    plan[5] = tiling.last_rows;
+    return 0;
 }
 
 int qi_w4a4_gemm_wide_single_ex(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
