@@ -1,6 +1,6 @@
 """Parity at the sizes that are benchmarked, through the C ABI, against the CPU oracle on sampled rows.
 
-The byte-operand W4A4 kernel on CTA pairs (qi_w4a4_gemm_wide_ex, the bench's timed path) on the three
+The byte-operand W4A4 GEMM (qi_w4a4_gemm_wide_ex, the bench's timed path: tiles of 256 x 64) on the three
 wide block linears at M = 4096 and on one M = 16384 shape; the W4A16 kernel on the text stream's
 M = 256 at the four block shapes; both operators on the reference engine's own shapes
 (N, K in {4096, 12288}, qwen_image_cuda/cuda/bench/bench_w4a4.cu:405-410) at M = 1024, there also
@@ -97,7 +97,7 @@ def w4a4_case(qi, rng, m, n, k, kind):
 
 @pytest.mark.parametrize("name,n,k,kind", [("qkv", 9216, 3072, "outliers"), ("fc1", 12288, 3072, "outliers"),
                                            ("fc2", 3072, 12288, "gelu")])
-def test_w4a4_pair_kernel_block_linears_m4096_against_oracle(qi, name, n, k, kind):
+def test_w4a4_wide_gemm_block_linears_m4096_against_oracle(qi, name, n, k, kind):
     m = 4096
     rng = np.random.default_rng(6100 + n + k)
     case = w4a4_case(qi, rng, m, n, k, kind)
@@ -118,8 +118,8 @@ def test_w4a4_pair_kernel_block_linears_m4096_against_oracle(qi, name, n, k, kin
     assert torch.equal(y16, y.half())
 
 
-def test_w4a4_pair_kernel_m16384_against_oracle(qi):
-    # the 2048 x 2048 image: 16384 tokens through the attention-out linear, 64 row tiles per CTA pair column
+def test_w4a4_wide_gemm_m16384_against_oracle(qi):
+    # the 2048 x 2048 image: 16384 tokens through the attention-out linear, 64 rows of tiles
     m, n, k = 16384, 3072, 3072
     rng = np.random.default_rng(6401)
     case = w4a4_case(qi, rng, m, n, k, "outliers")
@@ -129,10 +129,10 @@ def test_w4a4_pair_kernel_m16384_against_oracle(qi):
     check_status(qi)
     distance, checked = qt.fp16_store_error(y16.cpu().numpy()[case["rows"]], case["expected"])
     assert distance <= FP16_STORE_ULPS and checked > 0.25
-    # the drop-in kernel on nibble-packed codes gives the same matrix
+    # the int8 kernel on nibble-packed codes gives the same matrix
     y_packed = torch.zeros(m, n, dtype=torch.float16, device="cuda")
-    assert qi.w4a4_gemm_ex(case["a_codes"], case["a_scales"], case["w_codes"], case["w_scales"], None, y_packed,
-                           qi.DTYPE_F16, n, m, n, k) == 0
+    assert qi.w4a4_gemm_path_ex(case["a_codes"], case["a_scales"], case["w_codes"], case["w_scales"], None, y_packed,
+                                qi.DTYPE_F16, n, m, n, k, qi.W4A4_PATH_INT8) == 0
     check_status(qi)
     assert torch.equal(y_packed, y16)
 

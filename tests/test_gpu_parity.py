@@ -477,7 +477,7 @@ def test_w4a4_gemm_block_shape_sampled(qi):
 @pytest.mark.parametrize("m,n,k", [(256, 384, 512), (512, 256, 3072), (200, 256, 768), (256, 256, 640)])
 def test_w4a4_gemm_paths_give_the_same_bits(qi, m, n, k):
     """The packed-operand entry point on each of its kernels: the int8 kernel on nibbles, and both operands widened
-    into scratch memory for the byte-operand kernel on CTA pairs (twice in a row: the scratch is taken and returned
+    into scratch memory for the byte-operand kernels (twice in a row: the scratch is taken and returned
     in stream order)."""
     rng = np.random.default_rng(4500 + m + n + k)
     if k % 256 == 0:
@@ -502,7 +502,7 @@ def test_w4a4_gemm_paths_give_the_same_bits(qi, m, n, k):
     check_status(qi)
     assert np.array_equal(y.cpu().numpy(), expected)
     assert qi.w4a4_gemm_path_ex(*args, y, qi.DTYPE_F32, n, m, n, k, 3) == qi.CUDA_ERROR_INVALID_VALUE
-    if k % 256 != 0:  # the pair kernel's stage is four groups
+    if k % 256 != 0:  # the byte-operand kernels take groups in fours
         assert qi.w4a4_gemm_path_ex(*args, y, qi.DTYPE_F32, n, m, n, k, qi.W4A4_PATH_WIDENED) == qi.CUDA_ERROR_INVALID_VALUE
 
 
@@ -679,7 +679,7 @@ def test_quantize_wide_writes_the_same_codes_as_bytes(qi, dtype):
 
 
 class WideKernel:
-    """One of the two byte-operand kernels behind the same three calls."""
+    """The byte-operand entry points, by shape or held to 128 x 128 tiles, behind the same two calls."""
 
     def __init__(self, qi, single):
         self.qi, self.single = qi, single
@@ -695,10 +695,10 @@ class WideKernel:
         return self.qi.w4a4_group_dots_wide_ex(a, sa, w, sw, y, dots, m, n, k)
 
 
-@pytest.fixture(params=["pair", "single"])
+@pytest.fixture(params=["by shape", "128x128"])
 def wide_kernel(request, qi):
-    """Both byte-operand kernels: 256x128 tiles on CTA pairs (default) and 128x128 on single CTAs."""
-    return WideKernel(qi, request.param == "single")
+    """The tiles that the shape takes (with the groups' dots: 256 x 128 on CTA pairs), and 128 x 128 tiles."""
+    return WideKernel(qi, request.param == "128x128")
 
 
 @pytest.mark.parametrize("m,n,k", [(128, 128, 128), (256, 384, 512), (128, 256, 3072), (200, 160, 1280),
@@ -729,8 +729,8 @@ def test_w4a4_wide_gemm_bits_and_exact_dots(qi, wide_kernel, m, n, k):
 @pytest.mark.parametrize("m,n,k", [(2304, 2048, 1024), (1000, 1280, 3072), (4096, 3072, 640), (333, 4224, 2048),
                                    (2048, 1152, 12288)])
 def test_w4a4_wide_gemm_equals_packed_kernel_on_many_tiles(qi, wide_kernel, m, n, k):
-    # Shapes with more tiles than CTA pairs, ragged row counts and long K: every CTA walks several tiles and the
-    # pipelines wrap many times. The byte-operand kernels must give the packed kernel's bits, launch after launch.
+    # Shapes with more tiles than CTAs, ragged row counts and long K: CTAs walk several tiles and the
+    # pipelines wrap many times. The byte-operand kernels must give the bits of the int8 kernel, launch after launch.
     generator = torch.Generator(device="cuda").manual_seed(m + n + k)
     def signed_codes(rows):
         v = torch.randint(-7, 8, (rows, k), dtype=torch.int16, device="cuda", generator=generator) & 0xF
@@ -742,7 +742,7 @@ def test_w4a4_wide_gemm_equals_packed_kernel_on_many_tiles(qi, wide_kernel, m, n
     assert qi.w4a4_widen_codes_ex(a_codes, a_wide, m, k) == 0
     assert qi.w4a4_widen_codes_ex(w_codes, w_wide, n, k) == 0
     expected = torch.zeros(m, n, dtype=torch.float32, device="cuda")
-    assert qi.w4a4_gemm_ex(a_codes, a_scales, w_codes, w_scales, None, expected, qi.DTYPE_F32, n, m, n, k) == 0
+    assert qi.w4a4_gemm_path_ex(a_codes, a_scales, w_codes, w_scales, None, expected, qi.DTYPE_F32, n, m, n, k, qi.W4A4_PATH_INT8) == 0
     check_status(qi)
     for _ in range(4):
         y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
@@ -754,8 +754,8 @@ def test_w4a4_wide_gemm_equals_packed_kernel_on_many_tiles(qi, wide_kernel, m, n
 @pytest.mark.parametrize("m,n,k", [(1024, 4096, 256), (4096, 3072, 256), (300, 3072, 512), (1500, 2112, 256), (256, 32, 256), (2048, 9600, 256),
                                    (1, 32, 256), (16, 96, 512), (17, 9216, 256), (77, 3104, 1280), (129, 2048, 768), (300, 480, 2304)])
 def test_w4a4_wide_gemm_in_narrow_tiles(qi, m, n, k):
-    # numbers of 256 x 128 tiles that leave part of a last wave to narrower tiles (74 pairs of CTAs), and few rows, which
-    # take tiles of 64 or 32 columns on single CTAs, against the int8 kernel; float16 into a slice of a wider matrix with a bias, and float32
+    # last waves cut into narrower tiles, and few rows or outputs, against the int8 kernel; float16 into a slice of a wider matrix
+    # with a bias, and float32
     rng = np.random.default_rng(m + n + k)
     a_codes, a_scales = qt.random_w4a4_pack(rng, m, k, 0.02, 0.2)
     w_codes, w_scales = qt.random_w4a4_pack(rng, n, k, 0.002, 0.01)
@@ -773,11 +773,33 @@ def test_w4a4_wide_gemm_in_narrow_tiles(qi, m, n, k):
         assert torch.equal(got, expected)
 
 
-@pytest.mark.parametrize("m,n,k", [(511, 9248, 256), (600, 2336, 512), (1000, 3104, 512), (1030, 4096, 256), (2049, 6016, 256), (1024, 12288, 256), (9000, 640, 8192)])
+# Few rows or outputs, one row past what each kind of tiles covers in a wave of 148 CTAs, several waves, rows and columns that end within a tile.
+NARROW_SHAPES = [("16 rows", 6, 32, 512), ("16 rows", 130, 672, 512), ("32 rows", 19, 9568, 256), ("32 rows", 63, 9568, 256), ("48 rows", 40, 9568, 256),
+                 ("48 rows", 99, 9568, 512), ("48 rows", 600, 2336, 512), ("128x32", 1209, 160, 256), ("128x32", 519, 1888, 256), ("128x64", 97, 6368, 256), ("128x64", 293, 5728, 256)]
+# 256 x 64 tiles: a wave alone, whole or of 16, 32 or 48 columns; last waves of 16, 32, 48 and 64 columns; blocks of rows of tiles (74 MB of
+# activations and more), the last one as high as the others (9000 rows), lower (8900), or shorter than the last wave, which then stays whole (9300).
+TALL_SHAPES = [(200, 7712, 256), (511, 9248, 256), (252, 9600, 256), (385, 6304, 256), (294, 8160, 256), (247, 6304, 256), (1000, 3104, 512), (2049, 6016, 256),
+               (1024, 12288, 256), (1000, 1280, 3072), (9000, 640, 8192), (8900, 640, 8192), (9300, 640, 8192)]
+
+
+def test_the_shapes_of_the_tile_tests_take_the_tiles_that_they_name(qi):
+    for tiles, *shape in NARROW_SHAPES:
+        assert qi.w4a4_gemm_plan(*shape).tiles == tiles, shape
+    plans = [qi.w4a4_gemm_plan(*shape) for shape in TALL_SHAPES]
+    assert {plan.tiles for plan in plans} == {"256x64"}
+    assert {(plan.whole > 0, plan.width) for plan in plans if plan.cut} >= {(False, 48), (True, 16), (True, 32), (True, 48)}
+    assert {plan.whole % 148 > 0 for plan in plans if not plan.cut} == {True}
+    assert [(plan.block, plan.last_rows, plan.cut > 0) for plan in plans[-3:]] == [(12, 12, True), (12, 11, True), (12, 1, False)]
+
+
+@pytest.mark.parametrize("tiles,m,n,k", NARROW_SHAPES)
+def test_w4a4_wide_gemm_in_each_kind_of_narrow_tiles(qi, tiles, m, n, k):
+    test_w4a4_wide_gemm_in_narrow_tiles(qi, m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", TALL_SHAPES)
 def test_w4a4_wide_gemm_in_tall_tiles(qi, m, n, k):
-    # 256 x 64 tiles on 148 CTAs: a first wave alone, last waves of 16, 32, 48 and 64 columns, rows and columns that end within a
-    # tile, and (9000 rows, 74 MB of activations) blocks of rows of tiles; the bits of the int8 kernel, with whole 32-byte
-    # sectors to store and without
+    # the bits of the int8 kernel; rows that start on 32 bytes (whole sectors to store) and rows that start on 16
     generator = torch.Generator(device="cuda").manual_seed(m + n + k)
     a, w = (torch.randint(-7, 8, (rows, k), dtype=torch.int16, device="cuda", generator=generator) & 0xF for rows in (m, n))
     a, w = ((v[:, 0::2] | (v[:, 1::2] << 4)).to(torch.uint8).contiguous() for v in (a, w))
@@ -786,11 +808,11 @@ def test_w4a4_wide_gemm_in_tall_tiles(qi, m, n, k):
     bias = torch.randn(n, device="cuda", generator=generator)
     a_wide, w_wide = (torch.empty(rows, k, dtype=torch.uint8, device="cuda") for rows in (m, n))
     assert qi.w4a4_widen_codes_ex(a, a_wide, m, k) == 0 and qi.w4a4_widen_codes_ex(w, w_wide, n, k) == 0
-    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
-        for ldy in (n, n + 8):
-            got, expected = (torch.full((m, ldy), -7.0, dtype=dtype, device="cuda") for _ in range(2))
-            assert qi.w4a4_gemm_wide_ex(a_wide, sa, w_wide, sw, bias, got, code, ldy, m, n, k) == 0
-            assert qi.w4a4_gemm_path_ex(a, sa, w, sw, bias, expected, code, ldy, m, n, k, qi.W4A4_PATH_INT8) == 0
+    for dtype, code, half_sector in ((torch.float32, qi.DTYPE_F32, 4), (torch.float16, qi.DTYPE_F16, 8)):  # elements of 16 bytes
+        for ldy, start in ((n, 0), (n + half_sector, 0), (n, half_sector)):
+            got, expected = (torch.full((m * ldy + 2 * half_sector,), -7.0, dtype=dtype, device="cuda") for _ in range(2))
+            assert qi.w4a4_gemm_wide_ex(a_wide, sa, w_wide, sw, bias, got[start:], code, ldy, m, n, k) == 0
+            assert qi.w4a4_gemm_path_ex(a, sa, w, sw, bias, expected[start:], code, ldy, m, n, k, qi.W4A4_PATH_INT8) == 0
             check_status(qi)
             assert torch.equal(got, expected)
 
@@ -859,6 +881,48 @@ def test_a_wait_that_runs_out_reports_its_code_and_leaves_the_device_healthy(qi)
     assert qi.w4a4_gemm(up(a_codes), up(a_scales), up(w_codes), up(w_scales), y, m, n, k) == 0
     check_status(qi)
     assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
+
+
+def random_wide_operands(qi, m, n, k):
+    """Packed and byte-wide codes and scales of both operands, made on the device."""
+    generator = torch.Generator(device="cuda").manual_seed(m + n + k)
+    operands = []
+    for rows, low, high in ((m, 0.05, 0.5), (n, 1e-3, 6e-3)):
+        values = torch.randint(-7, 8, (rows, k), dtype=torch.int16, device="cuda", generator=generator) & 0xF
+        codes = (values[:, 0::2] | (values[:, 1::2] << 4)).to(torch.uint8).contiguous()
+        scales = (torch.rand(rows, k // 64, device="cuda", generator=generator) * (high - low) + low).half()
+        wide = torch.empty(rows, k, dtype=torch.uint8, device="cuda")
+        assert qi.w4a4_widen_codes_ex(codes, wide, rows, k) == 0
+        operands.append((codes, wide, scales))
+    return operands
+
+
+# 256 x 128 tiles on 74 pairs of CTAs: two and three tiles a pair, rows and columns that end within a tile, one stage of K and rings that wrap.
+@pytest.mark.parametrize("m,n,k", [(2304, 2048, 1024), (5000, 1056, 768), (700, 4128, 2304), (2048, 1152, 12288), (2300, 2080, 256)])
+def test_w4a4_scatter_over_several_tiles(qi, m, n, k):
+    # into two local buffers as the copies, beside what else stands in their rows: the bits of the int8 kernel
+    (a, a_wide, sa), (w, w_wide, sw) = random_wide_operands(qi, m, n, k)
+    ldy, column = n + 96, 64
+    for bias in (None, torch.randn(n, device="cuda")):
+        for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+            expected = torch.full((m, ldy), -3.0, dtype=dtype, device="cuda")
+            assert qi.w4a4_gemm_path_ex(a, sa, w, sw, bias, expected[:, column:], code, ldy, m, n, k, qi.W4A4_PATH_INT8) == 0
+            outputs = [torch.full((m, ldy), -3.0, dtype=dtype, device="cuda") for _ in range(2)]
+            copies = (ctypes.c_void_p * 2)(*[t.data_ptr() for t in outputs])
+            assert qi.w4a4_gemm_wide_scatter_ex(a_wide, sa, w_wide, sw, bias, copies, 1, code, ldy, column, m, n, k) == 0
+            check_status(qi)
+            assert all(torch.equal(output, expected) for output in outputs)
+
+
+def test_w4a4_group_dots_over_several_tiles(qi):
+    m, n, k = 2100, 2080, 512  # 153 tiles on 74 pairs
+    (a, a_wide, sa), (w, w_wide, sw) = random_wide_operands(qi, m, n, k)
+    y, expected = (torch.full((m, n), float("nan"), device="cuda") for _ in range(2))
+    dots, expected_dots = (torch.full((m, n, k // 64), 12345, dtype=torch.int32, device="cuda") for _ in range(2))
+    assert qi.w4a4_group_dots_wide_ex(a_wide, sa, w_wide, sw, y, dots, m, n, k) == 0
+    assert qi.w4a4_group_dots_ex(a, sa, w, sw, expected, expected_dots, m, n, k) == 0
+    check_status(qi)
+    assert torch.equal(dots, expected_dots) and torch.equal(y, expected)
 
 
 @pytest.mark.parametrize("dtype_name", ["f16", "f32"])

@@ -31,3 +31,8 @@ def test_a_lane_that_arrives_for_its_warp_follows_a_warp_barrier(path):
 def test_the_rule_reaches_the_hand_overs():
     arrivals = sum(line.startswith("if (lane == 0)") and "arrive" in line for path in KERNELS for _, line in statements(path))
     assert arrivals >= 15
+
+
+def test_every_source_makes_the_library_stale():
+    # a kernel file that is not on the list could be edited without the library being built again
+    assert sorted(entry.load_package().SOURCES) == sorted(os.listdir(os.path.join(entry.PACKAGE_DIR, "csrc")))

@@ -57,7 +57,7 @@ def test_too_large_and_unfit_shapes_are_refused_before_anything_runs(qi):
     m = n = k = 8192
     assert (m + n) * k > qi.NOALLOC_SCRATCH_BYTES
     assert qi.w4a4_gemm_noalloc_ex(small, small, small, small, None, y, qi.DTYPE_F32, n, m, n, k) == qi.NOALLOC_TOO_LARGE
-    # k must hold whole pipeline stages of the CTA-pair kernel; the scale arrays must be 8-byte aligned; no null operands
+    # k must hold whole stages of four groups; the scale arrays must be 8-byte aligned; no null operands
     assert qi.w4a4_gemm_noalloc_ex(small, small, small, small, None, y, qi.DTYPE_F32, 128, 128, 128, 128) == qi.CUDA_ERROR_INVALID_VALUE
     assert qi.w4a4_gemm_noalloc_ex(small, small[4:], small, small, None, y, qi.DTYPE_F32, 128, 128, 128, 256) == qi.CUDA_ERROR_INVALID_VALUE
     assert qi.w4a4_gemm_noalloc_ex(None, small, small, small, None, y, qi.DTYPE_F32, 128, 128, 128, 256) == qi.CUDA_ERROR_INVALID_VALUE
