@@ -364,7 +364,7 @@ int launch_w4a4_wide(const void *a_bytes, const void *a_scales, const void *w_by
                                       bias, y, dots, shape));
 }
 
-// `dots` given: the groups' dots are written too. Else `peers`: the tile goes into every GPU's copy of the output.
+// `peers`: the tile goes into every GPU's copy of the output. Else `dots`: y is float32 without bias, and the groups' dots are written too.
 int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,
                      const float *bias, void *y, int32_t *dots, const GemmShape &shape, cudaStream_t stream, int device,
                      const w4a4_pair::PeerOutputs *peers) {
@@ -377,9 +377,9 @@ int launch_w4a4_pair(const void *a_bytes, const void *a_scales, const void *w_by
                   128, wp::B_BOX_ROWS, CU_TENSOR_MAP_SWIZZLE_128B))
         return INVALID;
     if ((peers != nullptr) == (dots != nullptr)) return INVALID;
-    auto kernel = dots != nullptr ? wp::gemm_kernel<true, false> : wp::gemm_kernel<false, true>;
+    auto kernel = peers != nullptr ? wp::gemm_kernel<true> : wp::gemm_kernel<false>;
     static std::atomic<bool> configured[MAX_DEVICES][2];
-    if (const cudaError_t error = configure_once(kernel, wp::SMEM_BYTES, configured[device][dots != nullptr]))
+    if (const cudaError_t error = configure_once(kernel, wp::SMEM_BYTES, configured[device][peers != nullptr]))
         return static_cast<int>(error);
     const wp::PeerOutputs outputs = peers != nullptr ? *peers : wp::PeerOutputs{};
     const int pairs = sm_count(device) / 2, tiles = ((shape.m + 2 * wp::BM - 1) / (2 * wp::BM)) * ((shape.n + wp::BN - 1) / wp::BN);

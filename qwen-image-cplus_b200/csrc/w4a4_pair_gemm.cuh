@@ -82,12 +82,6 @@ __device__ __noinline__ bool wait_slow_u32(uint32_t barrier, uint32_t parity, ui
     atomicCAS(&g_status, 0u, code);
     return false;
 }
-__device__ __forceinline__ bool wait_warp_u32(uint32_t barrier, uint32_t parity, uint32_t code, int lane, uint32_t backoff_ns) {
-    if (__all_sync(0xffffffffu, try_wait_u32(barrier, parity))) return true;
-    uint32_t ok = 1;
-    if (lane == 0) ok = wait_slow_u32(barrier, parity, code, backoff_ns) ? 1u : 0u;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
 __device__ __forceinline__ ulonglong2 lds_pairs(uint32_t address) {
     ulonglong2 value;
     asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(value.x), "=l"(value.y) : "r"(address));
@@ -351,15 +345,16 @@ struct FoldState {
 // A look at a barrier is one try_wait by every lane; a lane that finds the phase incomplete polls on its own, with
 // pauses (the fold warps are the pace-setters: that path is for the first groups and for errors). A wait that ran
 // out of time sets `failed` in its lane; the warp looks at the flags once per stage.
-template <bool DUMP_DOTS, bool SCATTER>
+// SCATTER: the tile goes into every copy of the output. Otherwise y is a float32 matrix without bias, and the groups' dots are
+// written beside it.
+template <bool SCATTER>
 __device__ __forceinline__ bool fold_tile(FoldState &f, int row, int n0, uint32_t tmem_lane, uint32_t sw_base, int k_stages, int groups,
                                           const float *__restrict__ bias, void *__restrict__ y, const PeerOutputs &peers,
                                           int32_t *__restrict__ dots_out, const GemmShape &shape, int lane) {
-    constexpr int WIDTH = COLUMNS;
     uint32_t dots[COLUMNS];  // dots[j] = dot of this thread's row and column j of the warp's
-    uint64_t acc[WIDTH / 2];  // acc[j] = columns 2 j, 2 j + 1
+    uint64_t acc[COLUMNS / 2];  // acc[j] = columns 2 j, 2 j + 1
 #pragma unroll
-    for (int j = 0; j < WIDTH / 2; ++j) acc[j] = 0;
+    for (int j = 0; j < COLUMNS / 2; ++j) acc[j] = 0;
     for (int ks = 0; ks < k_stages; ++ks) {
         if (__any_sync(0xffffffffu, f.failed)) return false;
         f.failed = false;
@@ -394,9 +389,9 @@ __device__ __forceinline__ bool fold_tile(FoldState &f, int row, int n0, uint32_
                 __syncwarp();
                 if (lane == 0) mbarrier_arrive_cluster(f.leader_dot_empty + buffer * 8);
             }
-            if (DUMP_DOTS && row < shape.m) {
+            if (!SCATTER && row < shape.m) {
 #pragma unroll
-                for (int j = 0; j < WIDTH; ++j)
+                for (int j = 0; j < COLUMNS; ++j)
                     if (n0 + j < shape.n)
                         dots_out[(static_cast<size_t>(row) * shape.n + n0 + j) * groups + ks * STAGE_GROUPS + gl] =
                             static_cast<int32_t>(__uint_as_float(dots[j]));
@@ -407,95 +402,63 @@ __device__ __forceinline__ bool fold_tile(FoldState &f, int row, int n0, uint32_
                 acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), p[2 * q + 1], acc[2 * q + 1]);
             }
 #pragma unroll
-            for (int q = HOIST / 4; q < WIDTH / 4; ++q) {
+            for (int q = HOIST / 4; q < COLUMNS / 4; ++q) {
                 sw4 = lds_pairs(sw_group + 16 * q);  // four columns, as two pairs
                 acc[2 * q] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q], dots[4 * q + 1]), sa2), sw4.x, acc[2 * q]);
                 acc[2 * q + 1] = fma_f32x2(mul_f32x2(pack_u32x2(dots[4 * q + 2], dots[4 * q + 3]), sa2), sw4.y, acc[2 * q + 1]);
             }
         }
         __syncwarp();
-        if (lane == 0) arrive_u32(f.empty + f.s * 8);  // done with this stage'f.s scales; its codes were consumed before the dots arrived
+        if (lane == 0) arrive_u32(f.empty + f.s * 8);  // done with this stage's scales; its codes were consumed before the dots arrived
         if (++f.s == STAGES) f.s = 0, f.phase ^= 1;
     }
-    if (row >= shape.m) return true;
-    // y: this thread's row, WIDTH adjacent columns
-    float out[WIDTH];
+    // y: this thread's row, 32 adjacent columns, wholly inside the matrix or wholly outside it (n is a multiple of 32, not of
+    // the tile's 128 columns)
+    if (row >= shape.m || n0 >= shape.n) return true;
+    float out[COLUMNS];
 #pragma unroll
-    for (int j = 0; j < WIDTH / 2; ++j) unpack_f32x2(acc[j], out[2 * j], out[2 * j + 1]);
-    if (bias != nullptr) {
-#pragma unroll
-        for (int j = 0; j < WIDTH; ++j)
-            if (n0 + j < shape.n) out[j] += __ldg(bias + n0 + j);
-    }
+    for (int j = 0; j < COLUMNS / 2; ++j) unpack_f32x2(acc[j], out[2 * j], out[2 * j + 1]);
     const size_t element = static_cast<size_t>(row) * shape.ldy + n0;
-    if constexpr (SCATTER) {
-        // The launcher admits only outputs that take whole 32-byte sectors (32-byte aligned copies,
-        // n a multiple of 32, ldy a multiple of a sector): a warp's 32 columns lie wholly inside the
-        // matrix or wholly outside it (n not a multiple of the tile's 128 columns).
-        if (n0 >= shape.n) return true;
-        if (shape.y_is_half) {
-            uint32_t packed[WIDTH / 2];
+    if constexpr (!SCATTER) {
+        float *target = static_cast<float *>(y) + element;
 #pragma unroll
-            for (int j = 0; j < WIDTH / 2; ++j) {
-                const __half2 h = __floats2half2_rn(out[2 * j], out[2 * j + 1]);
-                packed[j] = *reinterpret_cast<const uint32_t *>(&h);
-            }
-            int index = peers.first;
-            for (int copy = 0; copy < peers.count; ++copy) {
-                __half *target = static_cast<__half *>(peers.y[index]) + element;
-#pragma unroll
-                for (int j = 0; j < WIDTH / 16; ++j)
-                    st_global_v8(target + 16 * j, *reinterpret_cast<const uint32_t(*)[8]>(&packed[8 * j]));
-                if (++index == peers.count) index = 0;
-            }
-        } else {
-            int index = peers.first;
-            for (int copy = 0; copy < peers.count; ++copy) {
-                float *target = static_cast<float *>(peers.y[index]) + element;
-#pragma unroll
-                for (int j = 0; j < WIDTH / 8; ++j)
-                    st_global_v8(target + 8 * j, *reinterpret_cast<const uint32_t(*)[8]>(&out[8 * j]));
-                if (++index == peers.count) index = 0;
-            }
-        }
+        for (int j = 0; j < COLUMNS; j += 4) *reinterpret_cast<float4 *>(target + j) = make_float4(out[j], out[j + 1], out[j + 2], out[j + 3]);
         return true;
     }
-    // whole 32-byte sectors when the row segment is aligned for them, else 16 bytes at a time (n is a multiple of 32)
-    const bool sectors = WIDTH == 32 && (reinterpret_cast<uintptr_t>(y) & 31) == 0 && shape.ldy % (shape.y_is_half ? 16 : 8) == 0;
+    if (bias != nullptr) {
 #pragma unroll
-    for (int j = 0; j < WIDTH; j += 16) {
-        if (n0 + j >= shape.n) break;
-        const bool whole = WIDTH - j >= 16 && n0 + j + 16 <= shape.n;
-        if (shape.y_is_half) {
-            uint32_t packed[8];
+        for (int j = 0; j < COLUMNS; ++j) out[j] += __ldg(bias + n0 + j);
+    }
+    // The launcher admits only outputs that take whole 32-byte sectors (32-byte aligned copies, ldy a multiple of a sector).
+    if (shape.y_is_half) {
+        uint32_t packed[COLUMNS / 2];
 #pragma unroll
-            for (int i = 0; i < 8 && j + 2 * i < WIDTH; ++i) {
-                const __half2 h = __floats2half2_rn(out[j + 2 * i], out[j + 2 * i + 1]);
-                packed[i] = *reinterpret_cast<const uint32_t *>(&h);
-            }
-            __half *target = static_cast<__half *>(y) + element + j;
-            if (sectors) {
-                st_global_v8(target, packed);
-            } else {
-                *reinterpret_cast<uint4 *>(target) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                if (whole) *reinterpret_cast<uint4 *>(target + 8) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-            }
-        } else {
-            float *target = static_cast<float *>(y) + element + j;
-            if (sectors) {
-                st_global_v8(target, reinterpret_cast<const uint32_t(&)[8]>(out[j]));
-                st_global_v8(target + 8, reinterpret_cast<const uint32_t(&)[8]>(out[j + 8]));
-            } else {
+        for (int j = 0; j < COLUMNS / 2; ++j) {
+            const __half2 h = __floats2half2_rn(out[2 * j], out[2 * j + 1]);
+            packed[j] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+        int index = peers.first;
+        for (int copy = 0; copy < peers.count; ++copy) {
+            __half *target = static_cast<__half *>(peers.y[index]) + element;
 #pragma unroll
-                for (int i = 0; i < 16 && j + i < WIDTH; i += 4)
-                    if (i < 8 || whole) *reinterpret_cast<float4 *>(target + i) = make_float4(out[j + i], out[j + i + 1], out[j + i + 2], out[j + i + 3]);
-            }
+            for (int j = 0; j < COLUMNS / 16; ++j)
+                st_global_v8(target + 16 * j, *reinterpret_cast<const uint32_t(*)[8]>(&packed[8 * j]));
+            if (++index == peers.count) index = 0;
+        }
+    } else {
+        int index = peers.first;
+        for (int copy = 0; copy < peers.count; ++copy) {
+            float *target = static_cast<float *>(peers.y[index]) + element;
+#pragma unroll
+            for (int j = 0; j < COLUMNS / 8; ++j)
+                st_global_v8(target + 8 * j, *reinterpret_cast<const uint32_t(*)[8]>(&out[8 * j]));
+            if (++index == peers.count) index = 0;
         }
     }
     return true;
 }
 
-template <bool DUMP_DOTS, bool SCATTER>
+template <bool SCATTER>
 __device__ __forceinline__ void fold_role(const View &v, const float *__restrict__ bias, void *__restrict__ y,
                                           const PeerOutputs &peers,
                                           int32_t *__restrict__ dots_out, const GemmShape &shape, int warp, int lane) {
@@ -510,12 +473,12 @@ __device__ __forceinline__ void fold_role(const View &v, const float *__restrict
     for (int tile = v.pair; tile < v.tiles; tile += v.pairs) {
         const TilePlace at = v.place(tile);
         const int row = at.m_index * 2 * BM + static_cast<int>(v.cta) * BM + quadrant * 32 + lane;
-        if (!fold_tile<DUMP_DOTS, SCATTER>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane)) break;
+        if (!fold_tile<SCATTER>(f, row, at.n0 + in_tile, tmem_lane + in_team, sw_tile + in_tile * 4, v.k_stages, v.groups, bias, y, peers, dots_out, shape, lane)) break;
     }
     tmem_load_wait();  // nothing of this warp may still be in flight at teardown
 }
 
-template <bool DUMP_DOTS, bool SCATTER>
+template <bool SCATTER>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
             const __half *__restrict__ a_scales, const __half *__restrict__ w_scales,
@@ -583,7 +546,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
     } else {
         setmaxnreg_inc<FOLD_REGISTERS>();
-        fold_role<DUMP_DOTS, SCATTER>(view, bias, y, peers, dots_out, shape, warp, lane);
+        fold_role<SCATTER>(view, bias, y, peers, dots_out, shape, warp, lane);
     }
 
     tcgen05_fence_before();
