@@ -4,17 +4,17 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
                     [--workload block|c4|c3|c5] [--m ROWS]
 
-Workloads (zero-indexed as the survey reads them):
-  block  configs[1], the default and the headline: the four linears of one Qwen-Image MMDiT block image
+Workloads:
+  block  the default and the headline: the four linears of one Qwen-Image MMDiT block image
          stream under W4A4 (H256, g64) at M = 4096 tokens, hidden 3072 - fused q/k/v 3072->9216,
          attention out 3072->3072, MLP fc1 3072->12288, fc2 12288->3072 - each with its own activation
          rotation + quantisation (fp16 in) and fp16 outputs: 927.7 G operations per step.
-  c4     configs[3]: the same block at M = 16384 (a 2048 x 2048 image), the shape the sharded scaling
+  c4     the same block at M = 16384 (a 2048 x 2048 image), the shape the sharded scaling
          target is quoted on.
-  c3     configs[2]: one denoising step of the 60-block stack under W4A16 g64: per block the four linears on
+  c3     one denoising step of the 60-block stack under W4A16 g64: per block the four linears on
          the image stream (M = 4096) and on the text stream (M = 256, its own weights) plus the two M = 1
          modulation GEMVs 3072->18432.
-  c5     configs[4]: the image-edit shape, rows 2 x (12288 + 512), 60 blocks, each linear W4A4 with
+  c5     the image-edit shape, rows 2 x (12288 + 512), 60 blocks, each linear W4A4 with
          probability 0.7 and W4A16 otherwise (seeded), through the dispatcher qi_linear.
 
 N > 1 (launched by torch.distributed.run, one rank per GPU): every linear's packed weights are sharded by
@@ -717,11 +717,11 @@ def run_block(args):
             "gpu_launches": timed_launches,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "steps": e2e_steps, "ms_per_step": e2e_ms / e2e_steps},
-            "roofline": {"kernel": "w4a4::gemm_kernel" if args.w4a4_path == "int8" else "w4a4_tall::gemm_kernel", "bound": "tensor",
+            "roofline": {"kernel": "w4a4::gemm_kernel" if args.w4a4_path == "int8" else "w4a4_pair::gemm_kernel" if fused else "w4a4_tall::gemm_kernel", "bound": "tensor",
                          "achieved": achieved, "peak": eight_bit_peak, "unit": "TOP/s", "frac": achieved / eight_bit_peak,
                          "frac_of_2x_bf16_burst": achieved / (2.0 * peaks["bf16_burst"]),
                          "frac_of_2x_bf16_sustained": achieved / (2.0 * peaks["bf16_sustained"]),
-                         "traffic": (NCU_TRAFFIC_BYTES_QKV_M4096 * (m / 4096.0) / world) if wide_path else None,
+                         "traffic": (NCU_TRAFFIC_BYTES_QKV_M4096 * (m / 4096.0) / world) if wide_path and not fused else None,
                          "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the qkv launch at "
                                            "M=4096 (its 2MNK is the average of the four launches), scaled by rows and ranks",
                          "peak_source": tensor_peaks["how"] + f"; bf16 figures of MEASURED_PEAKS.json ({peaks['source']})",
@@ -1230,7 +1230,7 @@ def main():
     parser.add_argument("--warmup", type=int, default=3)
     parser.add_argument("--impl", default="b200", choices=["b200", "reference"])
     parser.add_argument("--workload", default="block", choices=["block", "c4", "c3", "c5"],
-                        help="block: configs[1] (headline); c4: the block at M=16384; c3: the W4A16 stack; c5: the mixed image-edit stack")
+                        help="block: the four linears of a block at M=4096 (headline); c4: the block at M=16384; c3: the W4A16 stack; c5: the mixed image-edit stack")
     parser.add_argument("--m", type=int, default=None, help="rows of the block workloads (default 4096; c4: 16384)")
     parser.add_argument("--blocks", type=int, default=60, help="blocks of the stack workloads")
     parser.add_argument("--no-cpu-baseline", action="store_true", help="skip the CPU and reference-kernel legs (profiling runs)")
@@ -1239,7 +1239,7 @@ def main():
     parser.add_argument("--w4a4-path", default="wide", choices=["packed", "int8", "wide"],
                         help="packed: the drop-in entry points on nibble-packed codes, kernel by shape (both operands widened into "
                              "pool scratch for the byte-operand kernels); int8: the same entry points held to the int8 kernel that widens "
-                             "the nibbles in shared memory; wide: byte-wide E4M3 codes on CTA pairs (weights widened once at load)")
+                             "the nibbles in shared memory; wide: byte-wide E4M3 codes (weights widened once at load)")
     parser.add_argument("--gather", default="auto", choices=["auto", "fused", "copy", "slabs", "nccl"],
                         help="N > 1: how the column slices reach every GPU. auto: copy on two GPUs, nccl on more. nccl: an all-gather after each GEMM; fused: the "
                              "GEMM's epilogue stores its slice into every GPU's output over NVLink, a barrier follows; copy: the copy "

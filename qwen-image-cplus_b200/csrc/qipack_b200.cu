@@ -736,8 +736,8 @@ int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, co
     if (device < 0) return INVALID;
     const GemmShape shape = {m, n, k, ldy, y_dtype == QI_DTYPE_F16};
     const bool scales_aligned8 = ((reinterpret_cast<uintptr_t>(a_scales) | reinterpret_cast<uintptr_t>(w_scales)) & 7) == 0;
-    const bool pair_takes_it = dots == nullptr && k % w4a4_pair::STAGE_K == 0 && scales_aligned8;
-    if (path == 2 && !pair_takes_it) return INVALID;
+    const bool bytes_take_it = dots == nullptr && k % w4a4_pair::STAGE_K == 0 && scales_aligned8;
+    if (path == 2 && !bytes_take_it) return INVALID;
     // Widening first (two launches, ~9 us at the least) against the int8 kernel, whose time is k's: 0.01 us per element
     // and tile, 9 us at k = 768 whatever m and n. Measured, int8 and widened: 1 x 128 x 3072 29.9 and 9.1 us, 77 x 9216 x
     // 3072 32.8 and 17.2, 4096 x 32 x 3072 30.8 and 11.4, 1 x 18432 x 3072 31.5 and 28.2, 1 x 32 x 256 5.9 and 9.4,
@@ -745,7 +745,7 @@ int w4a4_gemm(const void *a_codes, const void *a_scales, const void *w_codes, co
     // Not under stream capture where the int8 kernel will do: scratch makes a graph with allocation nodes, of which CUDA allows
     // one instance and no clone or child, and a caller that captures a prompt's calls may want several.
     const bool large = m >= 256 && n >= 256;
-    if (path == 2 || (path == 0 && pair_takes_it && (large || (k >= 768 && !capturing(stream))))) {
+    if (path == 2 || (path == 0 && bytes_take_it && (large || (k >= 768 && !capturing(stream))))) {
         const size_t a_bytes = (static_cast<size_t>(m) * k + 255) & ~static_cast<size_t>(255);
         const size_t w_bytes = static_cast<size_t>(n) * k;
         uint8_t *scratch = nullptr;

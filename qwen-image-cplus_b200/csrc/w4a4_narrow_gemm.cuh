@@ -3,8 +3,7 @@
 // operator, arithmetic and bits as w4a4_pair_gemm.cuh (reference: qwen_image_cuda/cuda/gemm.cu:65-189).
 //
 // The groups of an output are added in order, so K cannot be split, and a tile is a chain of k / 64 hand-overs from the
-// tensor cores to the fold warps. With few rows the pair kernel's 256 x 128 tiles leave most SMs idle (77 x 9216: 72
-// tiles, the second CTA of each pair folding zeros) and the rest fold more than they must; here the same outputs are
+// tensor cores to the fold warps. With few rows, tiles of 256 leave most SMs idle or folding zeros; here 77 x 9216 outputs are
 // 144 tiles. What counts is the length of the chain's links:
 //   * a TMEM buffer holds four groups, one stage of 256 inputs: one commit, one look and one hand-back per four groups
 //   * two issuing warps take the stages in turn (an issuing warp needs some 500 cycles per turn)
@@ -12,7 +11,8 @@
 //
 // EXCHANGED, the weights are the 128 rows and 16 to 48 activation rows the columns: nothing is folded for rows that do not
 // exist, and a lane, which owns an output, writes next to its neighbours (77 x 9216 x 3072 11.7 -> 10.4 us, 16 rows 11.3 -> 8.4).
-// What bounds it then: 16 columns still take 0.11 us a group, half of that the 32 KB of weights a stage coming into the SM.
+// What bounds it then: 16 columns still take 0.073 us a group (0.11 where rows lie a multiple of 4096 bytes apart), half of that
+// the 32 KB of weights a stage coming into the SM.
 //
 //   warp 0      TMA: A rows (only those that exist, rounded up to 16) and B rows, 256 inputs a stage
 //   warps 1, 3  tcgen05.mma kind::f8f6f4, M = 128, N = the tile's columns

@@ -6,14 +6,14 @@
 // 128 x 128 outputs and a group, and around it the fold warps' other work. The pair kernel's fold threads own 1 row x 32
 // columns: 32 weight scales from shared memory for 32 outputs, and the load/store data path is busy in 457 of the 564
 // cycles of such a step (ncu: l1tex__data_pipe_lsu_wavefronts), the tensor cores' operand reads 157 more. Here
-//   * a fold thread owns 2 rows x 32 columns: a weight scale that it loads serves two rows (457 -> about 280 wavefronts)
+//   * a fold thread owns 2 rows x 32 columns: a weight scale that it loads serves two rows (457 -> 273 wavefronts)
 //   * eight fold warps with up to 208 registers a thread instead of sixteen with 96: half as many looks at barriers, hand-backs
-//     and loop instructions an output (1479 -> about 950 instructions per SM and step), and the dots of a whole group, 64 a
+//     and loop instructions an output (1479 -> 856 instructions per SM and step), and the dots of a whole group, 64 a
 //     thread, in flight at once
 //   * activation scales stand in shared memory as {sa, sa} of both rows, ready for the packed multiplies
 //   * a look at a barrier is one try_wait and one vote: control flow stays uniform (a per-lane branch with the
 //     reconvergence behind it took 17 instructions more), at one look per two groups
-// 4096 x 9216 x 3072: 240.7 -> 209 us. Measured on the way (us): sixteen fold warps of 2 x 16 columns 216; with the next dots
+// 4096 x 9216 x 3072: 240.7 -> 198 us. Measured on the way (us): sixteen fold warps of 2 x 16 columns 216; with the next dots
 // copied while the present ones are folded 232 to 240 there (register moves), 216 to 222 with eight warps; one group per
 // TMEM buffer 217 to 236 (a look costs some 120 cycles of a warp's chain). Taking work away from the sixteen-warp form: no
 // operand loads 211, no MMAs 201, no copies out of TMEM 191, neither of the last two 176, no arithmetic 149.
