@@ -773,6 +773,20 @@ def test_w4a4_wide_gemm_in_narrow_tiles(qi, m, n, k):
         assert torch.equal(got, expected)
 
 
+def random_wide_operands(qi, m, n, k):
+    """Packed and byte-wide codes and scales of both operands, made on the device."""
+    generator = torch.Generator(device="cuda").manual_seed(m + n + k)
+    operands = []
+    for rows, low, high in ((m, 0.05, 0.5), (n, 1e-3, 6e-3)):
+        values = torch.randint(-7, 8, (rows, k), dtype=torch.int16, device="cuda", generator=generator) & 0xF
+        codes = (values[:, 0::2] | (values[:, 1::2] << 4)).to(torch.uint8).contiguous()
+        scales = (torch.rand(rows, k // 64, device="cuda", generator=generator) * (high - low) + low).half()
+        wide = torch.empty(rows, k, dtype=torch.uint8, device="cuda")
+        assert qi.w4a4_widen_codes_ex(codes, wide, rows, k) == 0
+        operands.append((codes, wide, scales))
+    return operands
+
+
 # Few rows or outputs, one row past what each kind of tiles covers in a wave of 148 CTAs, several waves, rows and columns that end within a tile.
 NARROW_SHAPES = [("16 rows", 6, 32, 512), ("16 rows", 130, 672, 512), ("32 rows", 19, 9568, 256), ("32 rows", 63, 9568, 256), ("48 rows", 40, 9568, 256),
                  ("48 rows", 99, 9568, 512), ("48 rows", 600, 2336, 512), ("128x32", 1209, 160, 256), ("128x32", 519, 1888, 256), ("128x64", 97, 6368, 256), ("128x64", 293, 5728, 256)]
@@ -792,22 +806,11 @@ def test_the_shapes_of_the_tile_tests_take_the_tiles_that_they_name(qi):
     assert [(plan.block, plan.last_rows, plan.cut > 0) for plan in plans[-3:]] == [(12, 12, True), (12, 11, True), (12, 1, False)]
 
 
-@pytest.mark.parametrize("tiles,m,n,k", NARROW_SHAPES)
-def test_w4a4_wide_gemm_in_each_kind_of_narrow_tiles(qi, tiles, m, n, k):
-    test_w4a4_wide_gemm_in_narrow_tiles(qi, m, n, k)
-
-
-@pytest.mark.parametrize("m,n,k", TALL_SHAPES)
-def test_w4a4_wide_gemm_in_tall_tiles(qi, m, n, k):
+@pytest.mark.parametrize("m,n,k", [tuple(shape) for _, *shape in NARROW_SHAPES] + TALL_SHAPES)
+def test_w4a4_wide_gemm_in_each_kind_of_tiles(qi, m, n, k):
     # the bits of the int8 kernel; rows that start on 32 bytes (whole sectors to store) and rows that start on 16
-    generator = torch.Generator(device="cuda").manual_seed(m + n + k)
-    a, w = (torch.randint(-7, 8, (rows, k), dtype=torch.int16, device="cuda", generator=generator) & 0xF for rows in (m, n))
-    a, w = ((v[:, 0::2] | (v[:, 1::2] << 4)).to(torch.uint8).contiguous() for v in (a, w))
-    sa = (torch.rand(m, k // 64, device="cuda", generator=generator) * 0.5 + 0.05).half()
-    sw = (torch.rand(n, k // 64, device="cuda", generator=generator) * 5e-3 + 1e-3).half()
-    bias = torch.randn(n, device="cuda", generator=generator)
-    a_wide, w_wide = (torch.empty(rows, k, dtype=torch.uint8, device="cuda") for rows in (m, n))
-    assert qi.w4a4_widen_codes_ex(a, a_wide, m, k) == 0 and qi.w4a4_widen_codes_ex(w, w_wide, n, k) == 0
+    (a, a_wide, sa), (w, w_wide, sw) = random_wide_operands(qi, m, n, k)
+    bias = torch.randn(n, device="cuda")
     for dtype, code, half_sector in ((torch.float32, qi.DTYPE_F32, 4), (torch.float16, qi.DTYPE_F16, 8)):  # elements of 16 bytes
         for ldy, start in ((n, 0), (n + half_sector, 0), (n, half_sector)):
             got, expected = (torch.full((m * ldy + 2 * half_sector,), -7.0, dtype=dtype, device="cuda") for _ in range(2))
@@ -881,20 +884,6 @@ def test_a_wait_that_runs_out_reports_its_code_and_leaves_the_device_healthy(qi)
     assert qi.w4a4_gemm(up(a_codes), up(a_scales), up(w_codes), up(w_scales), y, m, n, k) == 0
     check_status(qi)
     assert np.array_equal(y.cpu().numpy(), qo.w4a4_gemm(a_codes, a_scales, w_codes, w_scales))
-
-
-def random_wide_operands(qi, m, n, k):
-    """Packed and byte-wide codes and scales of both operands, made on the device."""
-    generator = torch.Generator(device="cuda").manual_seed(m + n + k)
-    operands = []
-    for rows, low, high in ((m, 0.05, 0.5), (n, 1e-3, 6e-3)):
-        values = torch.randint(-7, 8, (rows, k), dtype=torch.int16, device="cuda", generator=generator) & 0xF
-        codes = (values[:, 0::2] | (values[:, 1::2] << 4)).to(torch.uint8).contiguous()
-        scales = (torch.rand(rows, k // 64, device="cuda", generator=generator) * (high - low) + low).half()
-        wide = torch.empty(rows, k, dtype=torch.uint8, device="cuda")
-        assert qi.w4a4_widen_codes_ex(codes, wide, rows, k) == 0
-        operands.append((codes, wide, scales))
-    return operands
 
 
 # 256 x 128 tiles on 74 pairs of CTAs: two and three tiles a pair, rows and columns that end within a tile, one stage of K and rings that wrap.
