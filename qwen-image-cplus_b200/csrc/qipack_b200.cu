@@ -532,6 +532,24 @@ __global__ void dequantize_kernel(const uint8_t *__restrict__ codes, const __hal
     for (int j = 0; j < 4; ++j) destination[j] = values[j];
 }
 
+// The streaming GEMV, one CTA per SM: as many stages as fit beside the activations and the partial sums, and teams of as few warps as leave
+// a stage for each team: the fewer they are, the less of a tile's time is a team's own waiting, but the longer
+// the last tile takes. Microseconds with teams of 3, 4 and 6: 60 x 18432 x 3072 308, 318, 319, 100 x 6144 x 2048 123, 135, 143; one
+// 18432 x 3072 8.8, 9.2, 9.0, one 9216 x 3072 5.3, 5.2, 5.1, one 3072 x 3072 4.2, 3.9, 3.7; with fewer stages one 12288 x 4096
+// 10.5, 9.9, 9.5, eight rows of 18432 x 3072 11.7, 11.4, 10.9. Four steps of K are for teams of four (9216 x 1024 3.7, 3.5,
+// 3.7), and up to two for teams of two. By m and k alone: the order of the sums follows from it (w4a16_gemv_stream.cuh).
+constexpr int STREAM_CTA_BYTES = 232448 - 1024;  // the rest is the barriers'
+struct StreamPlan {
+    int stages, team_warps, smem_bytes;
+};
+StreamPlan plan_stream(int m, int k) {
+    const int fixed = w4a16::stream_fixed_bytes(m, k), stage = w4a16::stream_stage_bytes(k), steps = w4a16::stream_steps(k);
+    int stages = (STREAM_CTA_BYTES - fixed) / stage;
+    stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
+    const int team_warps = steps <= 2 ? 2 : steps == 4 ? 4 : stages >= w4a16::STREAM_WARPS / 3 ? 3 : 6;
+    return {stages, team_warps, stages * stage + fixed};
+}
+
 int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
                void *y, int y_dtype, long long ldy, int m, int n, int k, int whole_n, cudaStream_t stream) {
     if (m < 1 || m > 8 || n <= 0 || k <= 0 || n % 16 != 0 || k % 64 != 0) return INVALID;
@@ -542,21 +560,18 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
     if (k <= w4a16::STREAM_MAX_K && aligned16(scales) && aligned16(minimums)) {
         const int device = current_device();
         if (device < 0) return INVALID;
-        // one CTA per SM: as many stages (at most eight) as fit beside the activations and the partial sums
-        constexpr int CTA_BYTES = 200 * 1024;
-        int stages = (CTA_BYTES - 128 - w4a16::stream_x_bytes(m, k)) / w4a16::stream_stage_bytes(k);
-        stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
-        static std::atomic<bool> configured[MAX_DEVICES];
-        if (const cudaError_t error = configure_once(w4a16::gemv_stream_kernel, CTA_BYTES, configured[device]))
-            return static_cast<int>(error);
-        if (stages >= 1) {
-            const int smem_bytes = stages * w4a16::stream_stage_bytes(k) + w4a16::stream_x_bytes(m, k) + 128;
-            const int tiles = n / w4a16::STREAM_ROWS, resident = sm_count(device);
-            return static_cast<int>(launch_overlapped(w4a16::gemv_stream_kernel, tiles < resident ? tiles : resident,
-                                      w4a16::STREAM_THREADS, smem_bytes, stream, static_cast<const __half *>(x_half),
+        const int tiles = n / w4a16::STREAM_ROWS, resident = sm_count(device);
+        const StreamPlan plan = plan_stream(m, k);
+        const bool alternate = m <= w4a16::STREAM_ALTERNATE_M;
+        auto kernel = alternate ? w4a16::gemv_stream_kernel<true> : w4a16::gemv_stream_kernel<false>;
+        static std::atomic<bool> configured[MAX_DEVICES][2];
+        if (const cudaError_t error = configure_once(kernel, STREAM_CTA_BYTES, configured[device][alternate])) return static_cast<int>(error);
+        if (plan.stages >= 1) {
+            return static_cast<int>(launch_overlapped(kernel, tiles < resident ? tiles : resident,
+                                      w4a16::STREAM_THREADS, plan.smem_bytes, stream, static_cast<const __half *>(x_half),
                                       static_cast<const uint8_t *>(codes), static_cast<const __half *>(scales),
                                       static_cast<const __half *>(minimums), bias, y, m, n, k, ldy,
-                                      y_dtype == QI_DTYPE_F16, stages));
+                                      y_dtype == QI_DTYPE_F16, plan.stages, plan.team_warps));
         }
     }
     // Longer rows: the exchanged-operand GEMM kernel, whose clusters split K, where its alignments hold (5 x 4096 x 12288:
@@ -594,15 +609,13 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
     }
     const int device = current_device();
     if (device < 0) return INVALID;
-    constexpr int CTA_BYTES = 200 * 1024;  // one CTA per SM, as for the single matrix
-    int stages = (CTA_BYTES - 128 - w4a16::stream_x_bytes(m, k)) / w4a16::stream_stage_bytes(k);
-    stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
-    if (stages < 1) return INVALID;
-    static std::atomic<bool> configured[MAX_DEVICES];
-    if (const cudaError_t error = configure_once(w4a16::gemv_stream_grouped_kernel, CTA_BYTES, configured[device]))
-        return static_cast<int>(error);
-    const int smem_bytes = stages * w4a16::stream_stage_bytes(k) + w4a16::stream_x_bytes(m, k) + 128;
     const int resident = sm_count(device);
+    const StreamPlan plan = plan_stream(m, k);
+    if (plan.stages < 1) return INVALID;
+    const bool alternate = m <= w4a16::STREAM_ALTERNATE_M;
+    auto kernel = alternate ? w4a16::gemv_stream_grouped_kernel<true> : w4a16::gemv_stream_grouped_kernel<false>;
+    static std::atomic<bool> configured[MAX_DEVICES][2];
+    if (const cudaError_t error = configure_once(kernel, STREAM_CTA_BYTES, configured[device][alternate])) return static_cast<int>(error);
     for (int first = 0; first < count; first += w4a16::STREAM_GROUP) {
         const int now = count - first < w4a16::STREAM_GROUP ? count - first : w4a16::STREAM_GROUP;
         w4a16::StreamItems group;
@@ -613,9 +626,9 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
         }
         for (int i = now; i < w4a16::STREAM_GROUP; ++i) group.item[i] = {nullptr, nullptr, nullptr, nullptr, nullptr};
         const long long tiles = static_cast<long long>(now) * (n / w4a16::STREAM_ROWS);
-        const cudaError_t launched = launch_overlapped(w4a16::gemv_stream_grouped_kernel, tiles < resident ? static_cast<int>(tiles) : resident,
-                                                       w4a16::STREAM_THREADS, smem_bytes, stream, static_cast<const __half *>(x_half), group,
-                                                       now, m, n, k, ldy, y_dtype == QI_DTYPE_F16, stages);
+        const cudaError_t launched = launch_overlapped(kernel, tiles < resident ? static_cast<int>(tiles) : resident,
+                                                       w4a16::STREAM_THREADS, plan.smem_bytes, stream, static_cast<const __half *>(x_half), group,
+                                                       now, m, n, k, ldy, y_dtype == QI_DTYPE_F16, plan.stages, plan.team_warps);
         if (launched != cudaSuccess) return static_cast<int>(launched);
     }
     return 0;

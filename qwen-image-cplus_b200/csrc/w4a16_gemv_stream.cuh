@@ -3,19 +3,28 @@
 // to 128), for matrices whose rows are short enough that 16 of them fit a shared-memory stage (K <= 4096).
 //
 // A CTA per SM walks over tiles of 16 weight rows. A tile's codes, scales and minimums are three contiguous ranges of the
-// pack (16 whole rows each), so one thread fetches them with three bulk asynchronous copies (cp.async.bulk, completion
-// counted on an mbarrier) into a ring of up to eight stages, and the copies of the next tiles are in flight while the
-// warps unpack. The tiles in the ring are dealt out to four teams of six warps; within a tile the team's warps split K:
-// lane (r, q) = (lane / 4, lane % 4) takes 32 codes (half a group) of rows r and r + 8 per step, unpacks them, and
+// pack (16 whole rows each), so one thread, in a warp of its own, fetches them with three bulk asynchronous copies
+// (cp.async.bulk, completion counted on an mbarrier) into a ring of up to sixteen stages, and the copies of the next tiles
+// are in flight while the others unpack. The tiles in the ring are dealt out to teams of warps; within a tile the team's warps split K:
+// lane (r, q) = (lane / 4, lane % 4) takes the 64 codes of one group of rows r and r + 8 per step, unpacks them, and
 // feeds them as the A operand of mma.sync.m16n8k16 (fp32 accumulate) whose B operand carries up to 8 activation rows;
 // the order of k inside an MMA is free as long as both operands agree. The K slices are summed through shared memory in a
-// fixed order. The teams have a barrier each and drift apart: against two CTAs of eight warps with two CTA-wide barriers
-// per tile, 18432 x 3072 went from 14.7 to 11.9 us alone and from 9.1 to 7.5 us in groups of 60 (512 threads: 12.2 and
-// 7.9; 1024: 11.6 and 8.0).
+// fixed order. How many warps a team has, and so that order, is chosen by m and k alone: a slice of a matrix, a matrix alone and
+// in a group give the same bits.
 //
-// Unpacking is what the SMs spend their time on (18432 x 3072 in groups of 60: the copies alone 4.6 us a matrix; before,
-// 62 % of the integer pipe and 205 instructions per 2048 weights, 7.5 us; now 167 and 6.3 us; alone 11.9 -> 10.8), so it is
-// cut to ten instructions per eight weights. A nibble moved to bits 2..5 or 6..9 of a 16-bit lane is the fp16 denormal
+// What bounds it, 18432 x 3072 on cold weights: alone the first load, the copies (31.9 MB, 4.7 us) and the last tiles' steps
+// (10.3 -> 8.9 us); in groups of 60 instructions and copies about alike (6.9 -> 5.2 us a matrix; the copies alone 4.6).
+// What counted, in that order: shared memory by 32-bit addresses instead of generic pointers (76.0 -> 60.0 million
+// warp instructions for sixteen matrices); a step of whole groups, which halves what a step spends on its scales; a warp that does nothing
+// but fetch, since a thread that unpacks held its team up while the copy engine took its requests; and codes read without
+// bank conflicts (5.7 -> 1.0 million). Rows lie a multiple of 128 bytes apart, so the eight lanes that a 16-byte load serves at a time
+// would meet on four banks. So the odd rows read the two halves of their group in the other order, and the columns of B
+// that one or a few activation rows leave idle hold those rows once more with the halves of each group exchanged: column 2a + p
+// serves the weight rows of parity p (up to four activation rows; with more, every row reads in the same order).
+// Measured without gain: two accumulator chains, two steps unrolled, a limit on the copies in flight, a warp that does nothing but the final
+// sums (10.2 us alone), teams of 8 and 12 warps (10.7, 10.5).
+//
+// Unpacking takes ten instructions per eight weights. A nibble moved to bits 2..5 or 6..9 of a 16-bit lane is the fp16 denormal
 // code * 2^-22 or code * 2^-18, so one shift serves two nibbles; one half2 fused multiply-add with the scale times 2^22 or
 // 2^18 and the minimum gives fp16(code * scale + minimum) with a single rounding, which is what the reference's
 // __float2half(fmaf(code, scale, minimum)) gives whenever |w| <= 1 (gemm.cu:229-230; see w4a16_gemm.cuh). A word of eight
@@ -29,20 +38,43 @@
 namespace qi {
 namespace w4a16 {
 
-constexpr int STREAM_THREADS = 768, STREAM_MAX_STAGES = 8, STREAM_ROWS = 16;
-constexpr int STREAM_TEAMS = 4, STREAM_TEAM_WARPS = STREAM_THREADS / 32 / STREAM_TEAMS;
+// 24 warps unpack, one fetches
+constexpr int STREAM_WARPS = 24, STREAM_THREADS = (STREAM_WARPS + 1) * 32, STREAM_MAX_STAGES = 16, STREAM_ROWS = 16;
+constexpr int STREAM_MAX_TEAM_WARPS = 6;
+constexpr int STREAM_STEP_GROUPS = 4;  // a step of a warp: a group for each of a row's four lanes
 constexpr int STREAM_MAX_K = 4096;  // 16 rows of codes, scales and minimums: 36 KB per stage
+constexpr int STREAM_ALTERNATE_M = 4;  // activation rows up to which each has two columns of the MMA
 
 __host__ __device__ constexpr int stream_stage_bytes(int k) { return STREAM_ROWS * (k / 2) + 2 * STREAM_ROWS * (k / 64) * 2; }
-// a row of activations: a step's 16 pieces of 16 bytes, the four lanes' first pieces, their second, ...; 64 bytes more
-// set the next row on the other banks
-__host__ __device__ constexpr int stream_x_pieces(int k) { return (k + 127) / 128 * 16 + 4; }
+// a row of activations in pieces of 16 bytes; 64 bytes more set the next row on the other banks
+__host__ __device__ constexpr int stream_steps(int k) { return (k / 64 + STREAM_STEP_GROUPS - 1) / STREAM_STEP_GROUPS; }
+__host__ __device__ constexpr int stream_x_pieces(int k) { return stream_steps(k) * STREAM_STEP_GROUPS * 8 + 4; }
 __host__ __device__ constexpr int stream_x_bytes(int m, int k) { return m * stream_x_pieces(k) * 16; }
+__host__ __device__ constexpr int stream_partial_bytes(int m) { return 2 * STREAM_WARPS * m * STREAM_ROWS * 4; }  // a warp's, twice
+__host__ __device__ constexpr int stream_fixed_bytes(int m, int k) { return stream_x_bytes(m, k) + stream_partial_bytes(m) + 128; }
 
+__device__ __forceinline__ uint4 lds_16(uint32_t address) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(address));
+    return v;
+}
+__device__ __forceinline__ __half lds_half(uint32_t address) {
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(address));
+    return __ushort_as_half(v);
+}
+__device__ __forceinline__ float lds_float(uint32_t address) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(address));
+    return v;
+}
+__device__ __forceinline__ void sts_float(uint32_t address, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(address), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts_16(uint32_t address, uint4 v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(address), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 // global -> shared, any multiple of 16 bytes, both addresses 16-byte aligned; completion on an mbarrier of this CTA
-__device__ __forceinline__ void bulk_load(void *smem, const void *global, uint32_t bytes, uint64_t *barrier) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem)),
-                 "l"(global), "r"(bytes), "r"(smem_u32(barrier))
+__device__ __forceinline__ void bulk_load(uint32_t smem, const void *global, uint32_t bytes, uint32_t barrier) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem), "l"(global), "r"(bytes), "r"(barrier)
                  : "memory");
 }
 
@@ -87,127 +119,155 @@ struct StreamItems {
     StreamItem item[STREAM_GROUP];
 };
 
-// Dynamic shared memory: `stages` stages of stream_stage_bytes(k), then the activations (stream_x_bytes(m, k)).
+// Dynamic shared memory: `stages` stages of stream_stage_bytes(k), then the activations (stream_x_bytes(m, k)), then the
+// teams' partial sums (stream_partial_bytes(m)).
 // GROUPED: `count` matrices [n, k] from `group`, tile t of the launch is tile t % (n / 16) of matrix t / (n / 16);
 // otherwise the one matrix given by the pointer arguments.
-template <bool GROUPED>
+template <bool GROUPED, bool ALTERNATE>
 __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, const uint8_t *__restrict__ codes, const __half *__restrict__ scales,
                    const __half *__restrict__ minimums, const float *__restrict__ bias, void *__restrict__ y,
-                   int m, int n, int k, long long ldy, int y_is_half, int stages, const StreamItems *group, int count) {
+                   int m, int n, int k, long long ldy, int y_is_half, int stages, int team_warps, const StreamItems *group, int count) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-    __shared__ uint64_t full[STREAM_MAX_STAGES];
+    const uint32_t smem = (smem_u32(smem_raw) + 127) & ~127u;
+    __shared__ uint64_t full[STREAM_MAX_STAGES], empty[STREAM_MAX_STAGES];
     __shared__ volatile int fetched[STREAM_MAX_STAGES];  // the tile that was last sent for into each stage
-    __shared__ alignas(8) float partials[STREAM_TEAMS][2][STREAM_TEAM_WARPS][16][8];
-    const int team = threadIdx.x / (STREAM_TEAM_WARPS * 32), warp = threadIdx.x / 32 % STREAM_TEAM_WARPS, lane = threadIdx.x & 31;
-    const int team_thread = threadIdx.x % (STREAM_TEAM_WARPS * 32);
-    const int r = lane >> 2, q = lane & 3;
-    const int groups = k / 64, steps = (groups + 1) / 2;  // a step: two groups, a quarter of the lanes on each half group
-    const int code_bytes = STREAM_ROWS * (k / 2), scale_bytes = STREAM_ROWS * groups * 2;
-    const int stage_bytes = code_bytes + 2 * scale_bytes;
+    const uint32_t full_u = smem_u32(full), empty_u = smem_u32(empty);
+    const int cta_warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int teams = STREAM_WARPS / team_warps, team = cta_warp / team_warps, warp = cta_warp - team * team_warps;
+    const int team_threads = team_warps * 32, team_thread = warp * 32 + lane;
+    const uint32_t r = lane >> 2, q = lane & 3, odd = ALTERNATE ? r & 1 : 0;
+    const uint32_t groups = k / 64, steps = stream_steps(k), row_bytes = k / 2;
+    const uint32_t code_bytes = STREAM_ROWS * row_bytes, scale_bytes = STREAM_ROWS * groups * 2;
+    const uint32_t stage_bytes = code_bytes + 2 * scale_bytes;
     const int tiles_each = n / STREAM_ROWS, tiles = GROUPED ? tiles_each * count : tiles_each;
+    const int step_tiles = static_cast<int>(gridDim.x);
 
+    // one thread sends for a tile: its place among all and, GROUPED, its matrix and its place in that
+    auto fetch = [&](int tile, int item_index, int local, uint32_t s) {
+        const uint32_t stage = smem + s * stage_bytes, barrier = full_u + s * 8;
+        const uint8_t *from_codes = codes;
+        const __half *from_scales = scales, *from_minimums = minimums;
+        if (GROUPED) {
+            const StreamItem &item = group->item[item_index];
+            from_codes = item.codes, from_scales = item.scales, from_minimums = item.minimums;
+        }
+        mbarrier_arrive_expect_tx_u32(barrier, stage_bytes);
+        bulk_load(stage, from_codes + static_cast<size_t>(local) * code_bytes, code_bytes, barrier);
+        bulk_load(stage + code_bytes, reinterpret_cast<const uint8_t *>(from_scales) + static_cast<size_t>(local) * scale_bytes, scale_bytes, barrier);
+        bulk_load(stage + code_bytes + scale_bytes, reinterpret_cast<const uint8_t *>(from_minimums) + static_cast<size_t>(local) * scale_bytes, scale_bytes, barrier);
+        __threadfence_block();
+        fetched[s] = tile;
+    };
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
             mbarrier_init(&full[s], 1);
+            mbarrier_init(&empty[s], team_warps);
             fetched[s] = -1;
         }
         fence_barrier_init();
     }
     grid_wait();
     grid_release();
-    // the activations, once per CTA, every eight inputs in the order (0,4,1,5,2,6,3,7) the unpacked pairs have
-    uint4 *x_pairs = reinterpret_cast<uint4 *>(smem + static_cast<size_t>(stages) * stage_bytes);
-    const int x_row = stream_x_pieces(k);
-    for (int item = threadIdx.x; item < m * steps * 16; item += STREAM_THREADS) {
-        const int row = item / (steps * 16), piece = item % (steps * 16);  // input / 8; a ragged last step is filled with zeros
+    // The activations, once per CTA, every eight inputs in the order (0,4,1,5,2,6,3,7) the unpacked pairs have. Eight pieces
+    // that lie together: piece j and j + 4 of a step's four groups, which is what the lanes of a warp read at a time.
+    const uint32_t x_pairs = smem + stages * stage_bytes, x_row = stream_x_pieces(k) * 16;
+    const int x_pieces = steps * STREAM_STEP_GROUPS * 8;
+    for (int item = threadIdx.x; item < m * x_pieces; item += STREAM_THREADS) {
+        const int row = item / x_pieces, piece = item - row * x_pieces;  // input / 8; a ragged last step is filled with zeros
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (piece < k / 8) v = __ldg(reinterpret_cast<const uint4 *>(x) + static_cast<size_t>(row) * (k / 8) + piece);
-        x_pairs[row * x_row + piece / 16 * 16 + piece % 4 * 4 + piece / 4 % 4] =
-            make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
+        sts_16(x_pairs + row * x_row + ((piece & ~31) + (piece & 3) * 8 + (piece >> 2 & 1) * 4 + (piece >> 3 & 3)) * 16,
+               make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632)));
     }
     __syncthreads();
-    auto fetch = [&](int tile, int s) {  // one thread
-        uint8_t *stage = smem + static_cast<size_t>(s) * stage_bytes;
-        const int of_launch = tile;
-        const uint8_t *from_codes = codes;
-        const __half *from_scales = scales, *from_minimums = minimums;
-        if (GROUPED) {
-            const StreamItem &item = group->item[tile / tiles_each];
-            from_codes = item.codes, from_scales = item.scales, from_minimums = item.minimums;
-            tile %= tiles_each;
+    if (cta_warp == STREAM_WARPS) {
+        if (lane == 0) {
+            int item_index = 0, local = blockIdx.x;
+            uint32_t s = 0, phase = 1;
+            for (int tile = local; tile < tiles; tile += step_tiles, local += step_tiles) {
+                if (GROUPED)
+                    while (local >= tiles_each) local -= tiles_each, ++item_index;
+                if (!mbarrier_wait(&empty[s], phase, &g_status, STATUS_WAIT_EMPTY | 0xB100 | s, 64)) break;
+                fetch(tile, item_index, local, s);
+                if (++s == static_cast<uint32_t>(stages)) s = 0, phase ^= 1;
+            }
         }
-        const size_t row0 = static_cast<size_t>(tile) * STREAM_ROWS;
-        mbarrier_arrive_expect_tx(&full[s], static_cast<uint32_t>(stage_bytes));
-        bulk_load(stage, from_codes + row0 * (k / 2), code_bytes, &full[s]);
-        bulk_load(stage + code_bytes, from_scales + row0 * groups, scale_bytes, &full[s]);
-        bulk_load(stage + code_bytes + scale_bytes, from_minimums + row0 * groups, scale_bytes, &full[s]);
-        __threadfence_block();
-        fetched[s] = of_launch;
-    };
-    if (threadIdx.x == 0) {
-        int tile = blockIdx.x;
-        for (int s = 0; s < stages && tile < tiles; ++s, tile += gridDim.x) fetch(tile, s);
+        return;
     }
 
-    const __half nothing = __ushort_as_half(0);
     const __half2 sixty_fourth = __float2half2_rn(1.0f / 64.0f), quarter = __float2half2_rn(0.25f), two_to_9 = __float2half2_rn(512.0f), sixteen = __float2half2_rn(16.0f);
-    // Activation row lane / 4 is the B operand's column of that number, and a column only ever meets its own results: a
-    // lane past the last row feeds row 0 again, and what comes of it is not stored.
-    const uint4 *my_x = x_pairs + (r < m ? r : 0) * x_row + q;
-    // Team t takes the CTA's tiles t, t + 4, ...; tile i of the CTA lies in stage i modulo the number of stages.
-    uint32_t s = team, phase = 0;
+    const uint32_t whole = groups / STREAM_STEP_GROUPS, first = steps * warp / team_warps, last = steps * (warp + 1) / team_warps;  // this warp's range
+    // Lane / 4 is the number of the B operand's column. ALTERNATE: columns 2a and 2a + 1 are activation row a for the even and the
+    // odd weight rows. A column only ever meets its own results: a lane past the last row feeds row 0 again, and what comes of it is not stored.
+    const uint32_t x_of = ALTERNATE ? r >> 1 : r;
+    const uint32_t my_x = x_pairs + (x_of < static_cast<uint32_t>(m) ? x_of : 0) * x_row + q * 16 + odd * 64 + first * 512;
+    const uint32_t my_codes = r * row_bytes + q * 32 + odd * 16 + first * 128, my_scales = code_bytes + (r * groups + q + first * STREAM_STEP_GROUPS) * 2;
+    const int other_piece = odd ? -16 : 16, other_x = odd ? -64 : 64;
+    const uint32_t slice_bytes = m * STREAM_ROWS * 4;
+    const uint32_t partials = x_pairs + m * x_row + team * 2 * team_warps * slice_bytes;
+    const uint32_t my_partial = warp * slice_bytes + r * 4 + (ALTERNATE ? q : 2 * q) * (STREAM_ROWS * 4);
+    const bool stores = (ALTERNATE ? q : 2 * q) < static_cast<uint32_t>(m), stores_too = 2 * q + 1 < static_cast<uint32_t>(m);
+    const bool sums = team_thread < m * STREAM_ROWS;
+    // Team t takes the CTA's tiles t, t + teams, ...; tile i of the CTA lies in stage i modulo the number of stages.
+    uint32_t s = team, phase = 0, parity = 0;
     while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
-    int parity = 0;
+    const int team_step = teams * step_tiles;
+    int item_index = 0, local = blockIdx.x + team * step_tiles;
     bool gave_up = false;
-    for (int tile = blockIdx.x + team * gridDim.x; tile < tiles; tile += STREAM_TEAMS * gridDim.x, parity ^= 1) {
-        float (&partial)[STREAM_TEAM_WARPS][16][8] = partials[team][parity];
+    for (int tile = local; tile < tiles; tile += team_step, local += team_step, parity ^= 1) {
+        if (GROUPED)
+            while (local >= tiles_each) local -= tiles_each, ++item_index;
+        const uint32_t partial = partials + parity * team_warps * slice_bytes;
+        const float *to_bias = bias;
+        void *to_y = y;
+        if (GROUPED) to_bias = group->item[item_index].bias, to_y = group->item[item_index].y;
+        const int out_row = local * STREAM_ROWS + (team_thread & 15);
+        float add = 0.0f;
+        if (sums && to_bias != nullptr) add = __ldg(to_bias + out_row);
         // The stage's last user may have been another team. Only once this tile has been sent for is the phase before complete,
         // and the parity of this one's unambiguous.
         const bool arrived = wait_uniform([&]() { return fetched[s] == tile; }, &g_status, STATUS_WAIT_EMPTY | 0xB000 | s, 32) &&
-                             mbarrier_wait_uniform(smem_u32(&full[s]), phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
-        const uint8_t *stage = smem + static_cast<size_t>(s) * stage_bytes;
-        const __half *stage_scales = reinterpret_cast<const __half *>(stage + code_bytes);
-        const __half *stage_minimums = reinterpret_cast<const __half *>(stage + code_bytes + scale_bytes);
+                             mbarrier_wait_uniform(full_u + s * 8, phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
+        const uint32_t stage = smem + s * stage_bytes;
         float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (arrived) {
-            for (int step = warp; step < steps; step += STREAM_TEAM_WARPS) {
-                const int g = 2 * step + (q >> 1);  // this lane's group; q & 1 is the half of it
-                const uint8_t *my_codes = stage + r * (k / 2) + step * 64 + q * 16;
-                const uint4 code_a = *reinterpret_cast<const uint4 *>(my_codes);
-                const uint4 code_b = *reinterpret_cast<const uint4 *>(my_codes + 8 * (k / 2));
-                __half scale_a = stage_scales[r * groups + g], scale_b = stage_scales[(r + 8) * groups + g];
-                __half minimum_a = stage_minimums[r * groups + g], minimum_b = stage_minimums[(r + 8) * groups + g];
-                if (2 * step + 1 >= groups && q >= 2) {  // past a ragged end: what was read lies in the CTA's shared memory; zeros
-                    scale_a = scale_b = minimum_a = minimum_b = nothing;
-                }
-                const uint32_t wa[4] = {code_a.x, code_a.y, code_a.z, code_a.w};
-                const uint32_t wb[4] = {code_b.x, code_b.y, code_b.z, code_b.w};
+            uint32_t at_codes = stage + my_codes, at_codes_b = at_codes + 8 * row_bytes, at_x = my_x;
+            uint32_t at_scales = stage + my_scales, at_scales_b = at_scales + 16 * groups;
+#pragma unroll 1
+            for (uint32_t step = first; step < last; ++step, at_codes += 128, at_codes_b += 128, at_x += 512, at_scales += 8, at_scales_b += 8) {
+                __half scale_a = lds_half(at_scales), scale_b = lds_half(at_scales_b);
+                __half minimum_a = lds_half(at_scales + scale_bytes), minimum_b = lds_half(at_scales_b + scale_bytes);
+                if (step >= whole && step * STREAM_STEP_GROUPS + q >= groups)  // past a ragged end: what was read lies in the CTA's shared memory; zeros
+                    scale_a = scale_b = minimum_a = minimum_b = __ushort_as_half(0);
+                uint4 code_a[2], code_b[2];
+                code_a[0] = lds_16(at_codes), code_b[0] = lds_16(at_codes_b);
+                code_a[1] = lds_16(at_codes + other_piece), code_b[1] = lds_16(at_codes_b + other_piece);
                 const __half2 ma = __half2half2(minimum_a), mb = __half2half2(minimum_b);
-                const uint4 *px = my_x + step * 16;
                 auto multiply = [&](auto unpack) {
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) {  // 8 inputs of each row per word, two MMA steps
-                        const uint4 xv = px[4 * w];
+                    for (int w = 0; w < 8; ++w) {  // 8 inputs of each row per word, two MMA steps
+                        const uint4 xv = lds_16((w >> 2 ? at_x + other_x : at_x) + (w & 3) * 128);
+                        const uint4 from_a = code_a[w >> 2], from_b = code_b[w >> 2];
+                        const uint32_t a = (w & 3) == 0 ? from_a.x : (w & 3) == 1 ? from_a.y : (w & 3) == 2 ? from_a.z : from_a.w;
+                        const uint32_t b = (w & 3) == 0 ? from_b.x : (w & 3) == 1 ? from_b.y : (w & 3) == 2 ? from_b.z : from_b.w;
                         uint32_t pa[4], pb[4];
-                        unpack(wa[w], wb[w], pa, pb);
-                        const uint32_t first[4] = {pa[0], pb[0], pa[1], pb[1]}, second[4] = {pa[2], pb[2], pa[3], pb[3]};
-                        mma_m16n8k16(c, first, xv.x, xv.y);
-                        mma_m16n8k16(c, second, xv.z, xv.w);
+                        unpack(a, b, pa, pb);
+                        const uint32_t one[4] = {pa[0], pb[0], pa[1], pb[1]}, two[4] = {pa[2], pb[2], pa[3], pb[3]};
+                        mma_m16n8k16(c, one, xv.x, xv.y);
+                        mma_m16n8k16(c, two, xv.z, xv.w);
                     }
                 };
                 // scale * 2^22 is an fp16 number below 1/64, scale * 2^18 below 1/4 (a NaN fails both tests)
-                const __half2 magnitudes = __habs2(__halves2half2(scale_a, scale_b));
+                const __half2 both = __halves2half2(scale_a, scale_b), magnitudes = __habs2(both);
                 if (__all_sync(0xffffffffu, __hblt2(magnitudes, sixty_fourth))) {
-                    const __half2 sa = __hmul2(__hmul2(__half2half2(scale_a), two_to_9), two_to_9), sa_22 = __hmul2(sa, sixteen);
-                    const __half2 sb = __hmul2(__hmul2(__half2half2(scale_b), two_to_9), two_to_9), sb_22 = __hmul2(sb, sixteen);
+                    const __half2 up = __hmul2(__hmul2(both, two_to_9), two_to_9), up_22 = __hmul2(up, sixteen);
+                    const __half2 sa = __low2half2(up), sb = __high2half2(up), sa_22 = __low2half2(up_22), sb_22 = __high2half2(up_22);
                     multiply([&](uint32_t a, uint32_t b, uint32_t(&pa)[4], uint32_t(&pb)[4]) {
                         unpack_word<false>(a, sa_22, sa, ma, pa);
                         unpack_word<false>(b, sb_22, sb, mb, pb);
                     });
                 } else if (__all_sync(0xffffffffu, __hblt2(magnitudes, quarter))) {
-                    const __half2 sa = __hmul2(__hmul2(__half2half2(scale_a), two_to_9), two_to_9);
-                    const __half2 sb = __hmul2(__hmul2(__half2half2(scale_b), two_to_9), two_to_9);
+                    const __half2 up = __hmul2(__hmul2(both, two_to_9), two_to_9), sa = __low2half2(up), sb = __high2half2(up);
                     multiply([&](uint32_t a, uint32_t b, uint32_t(&pa)[4], uint32_t(&pb)[4]) {
                         unpack_word<true>(a, sixteen, sa, ma, pa);
                         unpack_word<true>(b, sixteen, sb, mb, pb);
@@ -221,37 +281,38 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
                 }
             }
         }
-        // c[0], c[1]: weight row r, activation rows 2q, 2q+1; c[2], c[3]: weight row r + 8
-        *reinterpret_cast<float2 *>(&partial[warp][r][2 * q]) = make_float2(c[0], c[1]);
-        *reinterpret_cast<float2 *>(&partial[warp][r + 8][2 * q]) = make_float2(c[2], c[3]);
-        // The team is done with the stage, and the partial sums are complete. The sums alternate between two places: those of
-        // this tile are read below and written again two tiles on, with the next tile's barrier in between.
-        named_barrier_sync(1 + team, STREAM_TEAM_WARPS * 32);
+        // c[0], c[1]: weight row r, columns 2q, 2q+1; c[2], c[3]: weight row r + 8
+        if (stores) {
+            sts_float(partial + my_partial, ALTERNATE && odd ? c[1] : c[0]);
+            sts_float(partial + my_partial + 32, ALTERNATE && odd ? c[3] : c[2]);
+        }
+        if (!ALTERNATE && stores_too) {
+            sts_float(partial + my_partial + STREAM_ROWS * 4, c[1]);
+            sts_float(partial + my_partial + STREAM_ROWS * 4 + 32, c[3]);
+        }
+        __syncwarp();
+        if (lane == 0) mbarrier_arrive_u32(empty_u + s * 8);  // this warp is done with the stage
+        // The partial sums are complete. They alternate between two places: those of this tile are read below and
+        // written again two tiles on, with the next tile's barrier in between.
+        named_barrier_sync(1 + team, team_threads);
         gave_up |= !arrived;
-        if (team_thread == 0 && arrived) {
-            const int next = tile + stages * gridDim.x;
-            if (next < tiles) fetch(next, s);
-        }
         // fixed-order sum over the K slices: thread -> (activation row, weight row), so that few rows keep few warps
-        const int b = team_thread >> 4, row = team_thread & 15;
-        if (b < m) {
-            const float *to_bias = bias;
-            void *to_y = y;
-            int local_tile = tile;
-            if (GROUPED) {
-                const StreamItem &item = group->item[tile / tiles_each];
-                to_bias = item.bias, to_y = item.y;
-                local_tile = tile % tiles_each;
-            }
-            const int out_row = local_tile * STREAM_ROWS + row;
-            float total = 0.0f;
+        if (sums) {
+            for (uint32_t item = team_thread; item < slice_bytes / 4; item += team_threads) {
+                float of_warp[STREAM_MAX_TEAM_WARPS], total = 0.0f;
 #pragma unroll
-            for (int slice = 0; slice < STREAM_TEAM_WARPS; ++slice) total += partial[slice][row][b];
-            if (to_bias != nullptr) total += __ldg(to_bias + out_row);
-            if (y_is_half) static_cast<__half *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = __float2half_rn(total);
-            else static_cast<float *>(to_y)[static_cast<size_t>(b) * ldy + out_row] = total;
+                for (int i = 0; i < STREAM_MAX_TEAM_WARPS; ++i)
+                    if (i < team_warps) of_warp[i] = lds_float(partial + i * slice_bytes + item * 4);
+#pragma unroll
+                for (int i = 0; i < STREAM_MAX_TEAM_WARPS; ++i)
+                    if (i < team_warps) total += of_warp[i];
+                total += add;
+                const size_t element = static_cast<size_t>(item >> 4) * ldy + out_row;
+                if (y_is_half) static_cast<__half *>(to_y)[element] = __float2half_rn(total);
+                else static_cast<float *>(to_y)[element] = total;
+            }
         }
-        s += STREAM_TEAMS;
+        s += teams;
         while (s >= static_cast<uint32_t>(stages)) s -= stages, phase ^= 1;
     }
     // Every copy has a team that waits for it. Where a wait gave up, let the copies already issued land. (Asking the status
@@ -261,17 +322,19 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     }
 }
 
+template <bool ALTERNATE>
 __global__ void __launch_bounds__(STREAM_THREADS, 1)
 gemv_stream_kernel(const __half *__restrict__ x, const uint8_t *__restrict__ codes, const __half *__restrict__ scales,
                    const __half *__restrict__ minimums, const float *__restrict__ bias, void *__restrict__ y,
-                   int m, int n, int k, long long ldy, int y_is_half, int stages) {
-    gemv_stream_body<false>(x, codes, scales, minimums, bias, y, m, n, k, ldy, y_is_half, stages, nullptr, 1);
+                   int m, int n, int k, long long ldy, int y_is_half, int stages, int team_warps) {
+    gemv_stream_body<false, ALTERNATE>(x, codes, scales, minimums, bias, y, m, n, k, ldy, y_is_half, stages, team_warps, nullptr, 1);
 }
 
+template <bool ALTERNATE>
 __global__ void __launch_bounds__(STREAM_THREADS, 1)
 gemv_stream_grouped_kernel(const __half *__restrict__ x, const __grid_constant__ StreamItems group, int count,
-                           int m, int n, int k, long long ldy, int y_is_half, int stages) {
-    gemv_stream_body<true>(x, nullptr, nullptr, nullptr, nullptr, nullptr, m, n, k, ldy, y_is_half, stages, &group, count);
+                           int m, int n, int k, long long ldy, int y_is_half, int stages, int team_warps) {
+    gemv_stream_body<true, ALTERNATE>(x, nullptr, nullptr, nullptr, nullptr, nullptr, m, n, k, ldy, y_is_half, stages, team_warps, &group, count);
 }
 
 }  // namespace w4a16

@@ -299,6 +299,19 @@ def test_w4a16_gemv_matches_oracle(qi, m, n, k, kind):
     assert distance <= FP16_STORE_ULPS
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 48, 192), (2, 32, 512), (4, 2400, 1024), (5, 2400, 1088), (1, 21328, 1536), (3, 4784, 2880), (4, 64, 4096)])
+def test_w4a16_gemv_teams_and_steps(qi, m, n, k):
+    # teams of 2, 4, 3 and 6 warps, last steps of one to four groups, as many activation rows as have two columns of the MMA and
+    # one more, and more tiles than a CTA has stages
+    rng = np.random.default_rng(3050 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x16, bias = qt.make_activations(rng, m, k, "silu"), qt.make_bias(rng, n)
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert qt.max_relative_error(y.cpu().numpy(), qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)) <= OUTPUT_TOLERANCE
+
+
 @pytest.mark.parametrize("m", [1, 3])
 def test_w4a16_gemv_scales_of_every_size(qi, m):
     # scales from fp16 denormals up to 4: the GEMV's unpack treats scale >= 1/16 (where scale * 2^20 leaves fp16)
