@@ -61,25 +61,28 @@ struct Tile {
 };
 
 // WORDS x 8 packed nibbles -> WORDS x 8 fp16 values in input order.
-// Byte b of a word holds codes 2b (low nibble) and 2b + 1. The fast path puts each code into mantissa bits 4..7 of
-// an fp16 with a zero exponent field, i.e. the subnormal code * 2^-20, and lets ONE fused multiply-add per pair do
-// the rest: fma(code * 2^-20, scale * 2^20, minimum) = fp16(code * scale + minimum), the product exact and the
-// sum rounded once like the reference's (gemm.cu:223-230). It needs scale * 2^20 to be an fp16 number: |scale| < 1/16.
-// Any other scale (a NaN included) takes the path that first makes each code an fp16 integer.
+// Byte b of a word holds codes 2b (low nibble) and 2b + 1. The fast path leaves the high nibbles where they are and moves
+// the low ones to bits 3..6 of their bytes; a byte alone in an fp16 whose other bits are zero is then the subnormal
+// code * 2^-20 or code * 2^-21, and ONE fused multiply-add per pair does the rest: fma(code * 2^-20, scale * 2^20, minimum) =
+// fp16(code * scale + minimum), the product exact and the sum rounded once like the reference's (gemm.cu:223-230). Bytes with
+// bit 7 clear are also where the byte permutes find their zeros, as copies of that bit: eleven instructions for eight
+// codes, six of them the integer pipe's (thirteen and eight with a mask after each permute). It needs
+// scale * 2^21 to be an fp16 number: |scale| < 1/32. Any other scale (a NaN included) takes the path that first makes each
+// code an fp16 integer.
 template <int WORDS>
 __device__ __forceinline__ void unpack_words(const uint32_t (&words)[WORDS], const __half2 scale2, const __half2 minimum2,
                                              uint32_t (&values)[4 * WORDS]) {
-    const __half sixteenth = __ushort_as_half(0x2C00), two_to_10 = __ushort_as_half(0x6400);
-    if (__hlt(__habs(__low2half(scale2)), sixteenth)) {
-        const __half2 up = __half2half2(two_to_10);
-        const __half2 scale_up = __hmul2(__hmul2(scale2, up), up);
+    const __half limit = __ushort_as_half(0x2800), two_to_10 = __ushort_as_half(0x6400), two_to_11 = __ushort_as_half(0x6800);
+    if (__hlt(__habs(__low2half(scale2)), limit)) {
+        const __half2 scale_up = __hmul2(__hmul2(scale2, __half2half2(two_to_10)), __halves2half2(two_to_11, two_to_10));
 #pragma unroll
         for (int w = 0; w < WORDS; ++w) {
-            const uint32_t low_nibbles_up = words[w] << 4;
+            const uint32_t low = (words[w] << 3) & 0x78787878u, high = words[w] & 0xF0F0F0F0u;
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                // [byte b of the shifted word, -, byte b of the word, -], then the two nibbles in bits 4..7 and 20..23
-                uint32_t pair = __byte_perm(low_nibbles_up, words[w], 0x4400u + 0x1111u * b) & 0x00F000F0u;
+                // [byte b of low, its bit 7, byte b of high, bit 7 of byte b of low]
+                uint32_t pair;
+                asm("prmt.b32 %0, %1, %2, %3;" : "=r"(pair) : "r"(low), "r"(high), "r"(0x8480u + 0x1111u * b));
                 const __half2 weight = __hfma2(*reinterpret_cast<__half2 *>(&pair), scale_up, minimum2);
                 values[4 * w + b] = *reinterpret_cast<const uint32_t *>(&weight);
             }

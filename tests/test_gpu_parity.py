@@ -269,6 +269,23 @@ def test_w4a16_same_bits_on_every_call(qi, m, n, k):
     assert float((results[0] - exact).norm() / exact.norm()) <= 1e-4  # 12288 float32 additions: 12288 ** 0.5 * 2 ** -23 = 1.3e-5
 
 
+def test_w4a16_unpack_scales_about_its_limit(qi):
+    # the unpack's fast path takes |scale| < 1/32: both sides of it, either sign, and the smallest scales there are
+    n, k = 64, 1024
+    rng = np.random.default_rng(3010)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    edge = np.float16(1 / 32)
+    values = np.array([edge, np.nextafter(edge, np.float16(0)), np.nextafter(edge, np.float16(1)), 1 / 16, 3 / 64, 2.0 ** -24, 2.0 ** -14, 0.0065], dtype=np.float16)
+    scales = (values[rng.integers(0, len(values), size=(n, k // 64))] * rng.choice([-1.0, 1.0], size=(n, k // 64))).astype(np.float16)
+    minimums = rng.uniform(-0.06, 0.06, size=scales.shape).astype(np.float16)
+    nibbles = np.stack([codes & 15, codes >> 4], axis=-1).reshape(n, k // 64, 64).astype(np.float64)
+    expected = (nibbles * scales.astype(np.float64)[:, :, None] + minimums.astype(np.float64)[:, :, None]).astype(np.float16).reshape(n, k)  # one rounding
+    weights = torch.zeros(n, k, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_dequantize_ex(up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), weights, n, k) == 0
+    check_status(qi)
+    assert np.array_equal(weights.cpu().numpy().view(np.uint16), expected.view(np.uint16))
+
+
 def test_w4a16_gemm_rejects_what_the_reference_rejects(qi):  # gemm.cu:264
     t = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
     assert qi.w4a16_gemm(t, t, t, t, t, 100, 128, 64) == qi.CUDA_ERROR_INVALID_VALUE
