@@ -17,7 +17,8 @@
 //               never pass through shared memory
 //   warps 1, 3  tcgen05.mma kind::f16 with A in TMEM (M = 128, N = columns, K = 16) x 8; up to 128 columns the two take
 //               the steps in turn, each into an accumulator of its own, above that warp 1 issues all
-// then all warps: accumulator -> shared memory, sum over the cluster, bias, store (rows of y contiguous per warp).
+// then the unpack warps: accumulator -> bias -> y, or where CTAs share the tile accumulator -> shared memory of the CTA that
+// sums the row, and all warps: sum over the cluster, bias, store (rows of y contiguous per warp).
 #pragma once
 #include "ptx.cuh"
 #include "w4a16_gemm.cuh"
@@ -183,14 +184,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         mbarrier_init(done, steps < issuers ? steps : issuers);
         fence_barrier_init();
     }
+    if (warp == PRODUCER_WARP && elect_one()) prefetch_tensormap(&map_x);
+    if (warp == CODE_WARP && elect_one()) prefetch_tensormap(&map_codes);
+    // TMEM too before the wait: whatever holds it on this SM is an earlier kernel's, which waits for nothing here.
+    if (warp == MMA_WARP) {
+        tmem_alloc(tmem_slot, TMEM_COLUMNS);
+        tmem_relinquish();
+        grid_release();  // not before this CTA has its TMEM
+    }
+    tcgen05_fence_before();
     __syncthreads();
+    tcgen05_fence_after();
     grid_wait();
     bool alive = true;
+    float own_bias = 0.0f;  // one CTA to a tile: of this thread's weight row
 
     // The single-threaded roles run as converged warps with one elected lane: their addresses and descriptors live in
     // uniform registers; a diverged thread takes several times as long for the same few instructions.
     if (warp == PRODUCER_WARP) {
-        if (elect_one()) prefetch_tensormap(&map_x);
         const uint32_t full_u = smem_u32(full), done_u = smem_u32(step_done), x_u = smem_u32(smem_x);
         uint32_t s = 0;
         int before = -1, before_phase = 0;  // the step that had the stage before
@@ -208,7 +219,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             if (++s == static_cast<uint32_t>(stages)) s = 0;
         }
     } else if (warp == CODE_WARP) {
-        if (elect_one()) prefetch_tensormap(&map_codes);
         const uint32_t full_u = smem_u32(code_full), empty_u = smem_u32(code_empty), c_u = smem_u32(smem_c);
         uint32_t s = 0, phase = 1;
         for (int step = 0; step < steps; step += CODE_STEPS) {
@@ -221,14 +231,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             if (++s == static_cast<uint32_t>(code_stages)) s = 0, phase ^= 1;
         }
     } else if (warp == MMA_WARP || warp == SECOND_MMA_WARP) {
-        if (warp == MMA_WARP) {
-            tmem_alloc(tmem_slot, TMEM_COLUMNS);
-            tmem_relinquish();
-            grid_release();  // not before this CTA has its TMEM
-            tcgen05_fence_before();
-        }
-        named_barrier_sync(1, 32 * (2 + UNPACK_WARPS));
-        tcgen05_fence_after();
         // A step's waits, eight MMAs and commit take a warp some 600 cycles, the tensor cores four per column: up to 128
         // columns two warps take the steps in turn, each into an accumulator of its own. Only the MMAs of ONE thread are sure
         // to reach an accumulator in the order they were issued in; two warps on one accumulator, with a token that passed
@@ -272,8 +274,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         // A slot is free when the MMAs of the step four before are done.
         const uint32_t free_u = smem_u32(step_done);
         int before = group - A_SLOTS, before_phase = 0;
-        named_barrier_sync(1, 32 * (2 + UNPACK_WARPS));
-        tcgen05_fence_after();
         const uint32_t tmem_base = *tmem_slot, tmem_lane = tmem_base + (TMEM_COLUMNS - A_SLOTS * A_COLUMNS) + (static_cast<uint32_t>(quadrant * 32) << 16);
 #pragma unroll 1
         for (; local < steps; local += UNPACK_GROUPS) {
@@ -299,12 +299,51 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             s += UNPACK_GROUPS / CODE_STEPS;
             if (s >= static_cast<uint32_t>(code_stages)) s -= code_stages, phase ^= 1;
         }
+        if (split == 1 && bias != nullptr && inside) own_bias = __ldg(bias + row);  // on its way during the last MMAs
         // Every MMA is done, so nothing of this CTA reads or writes the stages any more.
         alive = mbarrier_wait_uniform(smem_u32(done), 0, &g_status, STATUS_WAIT_TMEM_FULL | 0x8000) && alive;
         tcgen05_fence_after();
     }
-    if (split > 1) cluster_sync();  // every CTA of the cluster is done with its stages
-    if (warp >= UNPACK_WARP0) {
+    float4 add = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // a tile that is shared: of the four outputs this thread stores
+    if (split > 1) {
+        const float *from = bias + n0 + lane * 4;
+        if (bias != nullptr && n0 + lane * 4 < shape.n) add = make_float4(__ldg(from), __ldg(from + 1), __ldg(from + 2), __ldg(from + 3));
+        cluster_sync();  // every CTA of the cluster is done with its stages
+    }
+    if (warp >= UNPACK_WARP0 && split == 1) {
+        // The accumulator, or the sum of the two, goes from registers to y: lane = weight row, so that a warp stores 32 adjacent outputs of one
+        // activation row at a time. Through shared memory, in whole rows of the tile: 1024 x 3072 x 3072 19.9 us.
+        const int quadrant = warp & 3, group = (warp - UNPACK_WARP0) >> 2, n = n0 + quadrant * 32 + lane;
+        const uint32_t tmem_lane = *tmem_slot + (static_cast<uint32_t>(quadrant * 32) << 16);
+        const int rows = shape.m - m0 < columns ? shape.m - m0 : columns;
+        for (int c = group * 16; c < columns; c += 16 * UNPACK_GROUPS) {
+            uint32_t r[16];
+            tmem_load_32x16(tmem_lane + c, r);
+            if (issuers == 2 && steps > 1) {
+                uint32_t second[16];
+                tmem_load_32x16(tmem_lane + TWO_ISSUERS_COLUMNS + c, second);
+                tmem_load_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(second[j]));
+            } else {
+                tmem_load_wait();
+            }
+            if (n >= shape.n) continue;
+            const size_t element = static_cast<size_t>(m0 + c) * shape.ldy + n;
+            if (shape.y_is_half) {
+                __half *out = static_cast<__half *>(y) + element;
+#pragma unroll
+                for (int j = 0; j < 16; ++j, out += shape.ldy)
+                    if (c + j < rows) *out = __float2half_rn(__uint_as_float(r[j]) + own_bias);
+            } else {
+                float *out = static_cast<float *>(y) + element;
+#pragma unroll
+                for (int j = 0; j < 16; ++j, out += shape.ldy)
+                    if (c + j < rows) *out = __uint_as_float(r[j]) + own_bias;
+            }
+        }
+        tcgen05_fence_before();
+    } else if (warp >= UNPACK_WARP0) {
         // The accumulator, or the sum of the two (lane = weight row, column = activation row) goes to the CTA that sums that activation row, in
         // shared memory as [source CTA][row of the share][weight row]: pushed, because a load from another CTA's shared
         // memory is a round trip of a thousand cycles and a store is not.
@@ -324,12 +363,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             } else {
                 tmem_load_wait();
             }
-            if (split == 1) {
-                float *partial = reinterpret_cast<float *>(smem) + c * BN + quadrant * 32 + lane;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) partial[j * BN] = __uint_as_float(r[j]);
-                continue;
-            }
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 st_cluster_f32(map_to_cta(mine + row * (BN * 4), owner), __uint_as_float(r[j]));
@@ -348,9 +381,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     const int n = n0 + lane * 4, first_row = m0 + rank * share;
     int rows = shape.m - first_row < share ? shape.m - first_row : share;
     if (rows > columns - rank * share) rows = columns - rank * share;
-    if (n < shape.n) {
-        float4 add = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (bias != nullptr) add = make_float4(__ldg(bias + n), __ldg(bias + n + 1), __ldg(bias + n + 2), __ldg(bias + n + 3));
+    if (split > 1 && n < shape.n) {
         const float4 *sums = reinterpret_cast<const float4 *>(smem) + lane;
 #pragma unroll 2
         for (int row = warp; row < rows; row += THREADS / 32) {
