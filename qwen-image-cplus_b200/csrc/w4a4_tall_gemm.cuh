@@ -51,7 +51,7 @@ static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA");
 static_assert(BARRIERS * 8 + 4 <= BARRIER_BYTES && BUFFERS * BUFFER_COLUMNS == 512, "barrier block; the whole of TMEM");
 static_assert(STAGES % BUFFERS == 0 && SLOT_SLABS == BUFFERS, "a slab's place in its slot is its TMEM buffer");
 // setmaxnreg: what the two kinds of warps hold afterwards has to be there at launch, or the kernel waits for ever.
-constexpr int LAUNCH_REGISTERS = 168, CONTROL_REGISTERS = 64, FOLD_REGISTERS = 208;
+constexpr int LAUNCH_REGISTERS = 168, CONTROL_REGISTERS = 88, FOLD_REGISTERS = 208;
 static_assert(THREADS * LAUNCH_REGISTERS <= 65536 && 65536 / THREADS / 8 * 8 == LAUNCH_REGISTERS, "what __launch_bounds__ gives a thread");
 static_assert(FOLD_WARP0 * CONTROL_REGISTERS + FOLD_WARPS * FOLD_REGISTERS <= THREADS / 32 * LAUNCH_REGISTERS, "setmaxnreg.inc would wait for registers that do not exist");
 constexpr uint32_t AHEAD_BACKOFF_NS = 100, FOLD_BACKOFF_NS = 100, MMA_BACKOFF_NS = 32;
@@ -292,49 +292,63 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 }
             }
         } else if (warp == SCALE_WARP) {
-            // A lane's columns and rows, four groups (eight bytes) each, fetched while the slot before is folded. Rows and
-            // columns that do not exist take the last one's: nothing reads what becomes of them.
+            // A lane's columns and rows, eight groups (sixteen bytes) each: two slots. They are asked for once the two before are
+            // written, which the fold warps still need for two slots' time. Four groups at a time, a row's 32-byte sector was
+            // asked for four times, and where the rows of a tile are more than L1 keeps beside 190 KB of shared memory, from L2 each
+            // time (without any of these loads 4096 x 3072 x 12288 took 288 us instead of 303): 4096 x 3072 x 12288 305 -> 297 us,
+            // 1024 x 12288 x 4096 108 -> 105, 4096 x 9216 x 3072 the same. Rows and columns that do not exist take the last one's:
+            // nothing reads what becomes of them.
             constexpr int SW_ITEMS = BN / 32, SA_ITEMS = BM / 32, ITEMS = SW_ITEMS + SA_ITEMS, LOWER = SA_ITEMS / HALVES;
-            const uint2 *const sw_values = reinterpret_cast<const uint2 *>(w_scales), *const sa_values = reinterpret_cast<const uint2 *>(a_scales);
+            const bool whole = slots % 2 == 0 && ((reinterpret_cast<uintptr_t>(w_scales) | reinterpret_cast<uintptr_t>(a_scales)) & 15) == 0;
             uint32_t slot = 0, phase = 1;
             bool alive = true;
             for (int tile = blockIdx.x; tile < tiling.tiles && alive; tile += step) {
                 const TilePlace at = place(tiling, tile);
-                const uint2 *from[ITEMS];
-                uint2 next[ITEMS];
+                uint32_t from[ITEMS];  // in slots
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i) {
                     const int index = i < SW_ITEMS ? min(at.n0 + i * 32 + lane, shape.n - 1) : min(at.m0 + (i - SW_ITEMS) * 32 + lane, shape.m - 1);
-                    from[i] = (i < SW_ITEMS ? sw_values : sa_values) + static_cast<size_t>(index) * slots;
-                    next[i] = __ldg(from[i]);
+                    from[i] = static_cast<uint32_t>(index) * slots;
                 }
-                for (int ks = 0; ks < slots; ++ks) {
-                    if (!mbarrier_wait_uniform(scale_empty + slot * 8, phase, &g_status, STATUS_WAIT_EMPTY | 0xA100 | slot, AHEAD_BACKOFF_NS)) { alive = false; break; }
+                for (int ks = 0; ks < slots && alive; ks += 2) {
+                    uint4 next[ITEMS];
 #pragma unroll
-                    for (int i = 0; i < SW_ITEMS; ++i) {
-                        const float2 low = __half22float2(*reinterpret_cast<const __half2 *>(&next[i].x)), high = __half22float2(*reinterpret_cast<const __half2 *>(&next[i].y));
-                        float *to = sw_slots + slot * (SW_BYTES / 4) + i * 32 + lane;
-                        to[0] = low.x, to[BN] = low.y, to[2 * BN] = high.x, to[3 * BN] = high.y;
-                    }
-#pragma unroll
-                    for (int i = 0; i < LOWER; ++i) {
-                        const uint2 upper = next[SW_ITEMS + i], lower = next[SW_ITEMS + LOWER + i];
-                        float4 *to = reinterpret_cast<float4 *>(sa_slots + slot * (SA_BYTES / 4)) + i * 32 + lane;
-#pragma unroll
-                        for (int pair = 0; pair < 2; ++pair) {
-                            const uint32_t raw_upper = pair ? upper.y : upper.x, raw_lower = pair ? lower.y : lower.x;
-                            const float2 u = __half22float2(*reinterpret_cast<const __half2 *>(&raw_upper)), l = __half22float2(*reinterpret_cast<const __half2 *>(&raw_lower));
-                            to[2 * pair * HALF_ROWS] = make_float4(u.x, u.x, l.x, l.x);
-                            to[(2 * pair + 1) * HALF_ROWS] = make_float4(u.y, u.y, l.y, l.y);
+                    for (int i = 0; i < ITEMS; ++i) {
+                        const uint2 *source = reinterpret_cast<const uint2 *>(i < SW_ITEMS ? w_scales : a_scales) + from[i] + ks;
+                        if (whole) {
+                            next[i] = __ldg(reinterpret_cast<const uint4 *>(source));
+                        } else {
+                            const uint2 first = __ldg(source), second = ks + 1 < slots ? __ldg(source + 1) : make_uint2(0u, 0u);
+                            next[i] = make_uint4(first.x, first.y, second.x, second.y);
                         }
                     }
-                    __syncwarp();
-                    if (lane == 0) mbarrier_arrive_u32(scale_full + slot * 8);
-                    if (ks + 1 < slots) {
 #pragma unroll
-                        for (int i = 0; i < ITEMS; ++i) next[i] = __ldg(from[i] + ks + 1);
+                    for (int sub = 0; sub < 2; ++sub) {
+                        if (ks + sub >= slots) break;
+                        if (!mbarrier_wait_uniform(scale_empty + slot * 8, phase, &g_status, STATUS_WAIT_EMPTY | 0xA100 | slot, AHEAD_BACKOFF_NS)) { alive = false; break; }
+#pragma unroll
+                        for (int i = 0; i < SW_ITEMS; ++i) {
+                            const uint32_t raw_low = sub ? next[i].z : next[i].x, raw_high = sub ? next[i].w : next[i].y;
+                            const float2 low = __half22float2(*reinterpret_cast<const __half2 *>(&raw_low)), high = __half22float2(*reinterpret_cast<const __half2 *>(&raw_high));
+                            float *to = sw_slots + slot * (SW_BYTES / 4) + i * 32 + lane;
+                            to[0] = low.x, to[BN] = low.y, to[2 * BN] = high.x, to[3 * BN] = high.y;
+                        }
+#pragma unroll
+                        for (int i = 0; i < LOWER; ++i) {
+                            const uint4 upper = next[SW_ITEMS + i], lower = next[SW_ITEMS + LOWER + i];
+                            float4 *to = reinterpret_cast<float4 *>(sa_slots + slot * (SA_BYTES / 4)) + i * 32 + lane;
+#pragma unroll
+                            for (int pair = 0; pair < 2; ++pair) {
+                                const uint32_t raw_upper = sub ? (pair ? upper.w : upper.z) : pair ? upper.y : upper.x, raw_lower = sub ? (pair ? lower.w : lower.z) : pair ? lower.y : lower.x;
+                                const float2 u = __half22float2(*reinterpret_cast<const __half2 *>(&raw_upper)), l = __half22float2(*reinterpret_cast<const __half2 *>(&raw_lower));
+                                to[2 * pair * HALF_ROWS] = make_float4(u.x, u.x, l.x, l.x);
+                                to[(2 * pair + 1) * HALF_ROWS] = make_float4(u.y, u.y, l.y, l.y);
+                            }
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbarrier_arrive_u32(scale_full + slot * 8);
+                        if (++slot == SLOTS) slot = 0, phase ^= 1;
                     }
-                    if (++slot == SLOTS) slot = 0, phase ^= 1;
                 }
             }
         }
@@ -350,10 +364,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             f.tmem = tmem_lane + first;
             f.sw = sw_first + first * 4;
             bool alive;
-            if (columns == 32) alive = fold_tile<32>(f, row, n0, slots, bias, y, shape, lane);
-            else if (columns == 24) alive = fold_tile<24>(f, row, n0, slots, bias, y, shape, lane);
+            // the wide tiles' loop last: first, the same instructions took up to a percent longer
+            if (columns == 8) alive = fold_tile<8>(f, row, n0, slots, bias, y, shape, lane);
             else if (columns == 16) alive = fold_tile<16>(f, row, n0, slots, bias, y, shape, lane);
-            else alive = fold_tile<8>(f, row, n0, slots, bias, y, shape, lane);
+            else if (columns == 24) alive = fold_tile<24>(f, row, n0, slots, bias, y, shape, lane);
+            else alive = fold_tile<32>(f, row, n0, slots, bias, y, shape, lane);
             if (!alive) break;
             __syncwarp();  // rows that do not exist left the stores early
         }

@@ -850,6 +850,23 @@ def test_w4a4_wide_gemm_in_each_kind_of_tiles(qi, m, n, k):
             assert torch.equal(got, expected)
 
 
+@pytest.mark.parametrize("k", [512, 768])
+def test_w4a4_tall_tiles_scales_from_eight_bytes(qi, k):
+    # scales are read sixteen bytes at a time where rows begin on sixteen (an even number of four groups) and the arrays do, else eight
+    m, n = 1000, 3104
+    assert qi.w4a4_gemm_plan(m, n, k).tiles == "256x64"
+    (a, a_wide, sa), (w, w_wide, sw) = random_wide_operands(qi, m, n, k)
+    later_sa, later_sw = (torch.cat([t.flatten()[:4], t.flatten()])[4:] for t in (sa, sw))
+    assert later_sa.data_ptr() % 16 == later_sw.data_ptr() % 16 == 8
+    expected = torch.full((m, n), -7.0, device="cuda")
+    assert qi.w4a4_gemm_path_ex(a, sa, w, sw, None, expected, qi.DTYPE_F32, n, m, n, k, qi.W4A4_PATH_INT8) == 0
+    for row_scales, column_scales in ((sa, sw), (later_sa, sw), (sa, later_sw)):
+        got = torch.full((m, n), -7.0, device="cuda")
+        assert qi.w4a4_gemm_wide_ex(a_wide, row_scales, w_wide, column_scales, None, got, qi.DTYPE_F32, n, m, n, k) == 0
+        check_status(qi)
+        assert torch.equal(got, expected)
+
+
 def test_w4a4_wide_gemm_extreme_dots(qi, wide_kernel):
     # all codes +-7: every group dot is +-3136, the largest the format allows; fp32 accumulation must stay exact
     m, n, k = 128, 128, 512
