@@ -135,6 +135,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
         fence_barrier_init();
     }
+    if (warp == PRODUCER_WARP && elect_one()) {
+        prefetch_tensormap(&map_a);
+        prefetch_tensormap(&map_w);
+    }
     if (warp == MMA_WARP) {
         tmem_alloc(tmem_slot, T::TMEM_COLUMNS);
         tmem_relinquish();
@@ -147,10 +151,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == PRODUCER_WARP) {
-        if (elect_one()) {
-            prefetch_tensormap(&map_a);
-            prefetch_tensormap(&map_w);
-        }
         uint32_t s = 0, phase = 1;
         bool alive = true;
         for (int tile = blockIdx.x; tile < tiles && alive; tile += gridDim.x) {
@@ -241,6 +241,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             const bool busy = first_row < rows_of_a && n0 < rows_of_w;  // a warp without outputs only hands the buffers back
             const uint2 *row_scales = reinterpret_cast<const uint2 *>(a_scales + static_cast<size_t>(row < rows_of_a ? row : rows_of_a - 1) * groups);
             uint2 sa_next = busy ? __ldg(row_scales) : make_uint2(0u, 0u);
+            const float add = EXCHANGED && bias != nullptr && busy && row < rows_of_a ? __ldg(bias + row) : 0.0f;  // long there when it is asked for
             uint64_t acc[COLUMNS / 2];
 #pragma unroll
             for (int j = 0; j < COLUMNS / 2; ++j) acc[j] = 0;
@@ -291,7 +292,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
             for (int j = 0; j < COLUMNS / 2; ++j) unpack_f32x2(acc[j], out[2 * j], out[2 * j + 1]);
             if constexpr (EXCHANGED) {  // a lane owns an output: a warp writes 32 of an activation row at a time
-                const float add = bias != nullptr ? __ldg(bias + row) : 0.0f;
 #pragma unroll
                 for (int j = 0; j < COLUMNS; ++j) {
                     if (n0 + j >= shape.m) break;
