@@ -285,7 +285,7 @@ quantize_pairs_kernel(const Source source, uint8_t *__restrict__ codes, __half *
     }
 }
 
-// ---- one chunk per half-warp: SwiGLU, and GELU of few rows ---------------------------------------------------------------
+// ---- one chunk per half-warp: SwiGLU, and GELU and plain activations of fewer rows ---------------------------------------------------------------
 // The two loads and the division of silu(gate) * up want warps rather than registers: with 40 registers a thread this
 // form takes 28.8 us at 1024 x 12288, the paired one 42.8 (32.1 without loads ahead).
 
@@ -320,6 +320,15 @@ __device__ __forceinline__ void two_passes(float (&v)[16]) {
     for (int o = 0; o < 4; ++o) butterfly(v[o], v[o + 4], v[o + 8], v[o + 12]);
 }
 
+template <typename T>
+struct PlainChunkSource {
+    const T *x;
+    __device__ __forceinline__ void load(long long offset, float (&v)[16]) const {
+        Raw16<T> raw;
+        raw.load(x + offset, true);
+        raw.convert(v);
+    }
+};
 struct GeluChunkSource {
     const float *x;
     __device__ __forceinline__ void load(long long offset, float (&v)[16]) const {
@@ -350,7 +359,7 @@ quantize_chunks_kernel(const Source source, uint8_t *__restrict__ codes, __half 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int half_warp = lane >> 4, l = lane & 15;
     float *region = transpose + (warp * 2 + half_warp) * REGION;
-    const long long chunk = (static_cast<long long>(blockIdx.x) * (QUANT_THREADS / 32) + warp) * 2 + half_warp;
+    const long long chunk = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + warp) * 2 + half_warp;
     const bool active = chunk < chunks;
 
     float v[16];
@@ -458,7 +467,7 @@ inline cudaError_t launch_quantize_pairs(const Source &source, void *codes, void
     int device = 0, sms = 148;
     if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     // Two CTAs of 256 threads stay resident per SM and walk over the pairs of chunks, a half-warp at a time. Fewer pairs than
-    // that are spread over more and smaller CTAs: 77 x 3072 are 462 pairs, 29 CTAs of 256 threads or 116 of 64.
+    // that are spread over more and smaller CTAs: 300 x 4096 are 2400 pairs, 150 CTAs of 256 threads or 592 of 64.
     const int threads = pairs >= static_cast<long long>(sms) * (QUANT_THREADS / 16) ? QUANT_THREADS : 64;
     long long blocks = (pairs + threads / 16 - 1) / (threads / 16);
     const long long resident = static_cast<long long>(sms) * (threads == QUANT_THREADS ? 2 : 4);
@@ -471,18 +480,32 @@ inline cudaError_t launch_quantize_pairs(const Source &source, void *codes, void
     return launch_overlapped(quantize_pairs_kernel<Source, true, false>, grid, threads, 0, stream, source, c, s, b, chunks);
 }
 
-inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, void *codes, void *scales, void *bytes,
-                                               int m, int k, cudaStream_t stream) {
-    if (x_is_half) return launch_quantize_pairs(PlainSource<__half>{static_cast<const __half *>(x)}, codes, scales, bytes, m, k, stream);
-    return launch_quantize_pairs(PlainSource<float>{static_cast<const float *>(x)}, codes, scales, bytes, m, k, stream);
+template <typename Source>
+inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream, int threads = QUANT_THREADS) {
+    const long long chunks = static_cast<long long>(m) * (k / 256), blocks = (chunks + threads / 16 - 1) / (threads / 16);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    return launch_overlapped(bytes != nullptr ? quantize_chunks_kernel<Source, true> : quantize_chunks_kernel<Source, false>, static_cast<unsigned>(blocks), threads,
+                             0, stream, source, static_cast<uint8_t *>(codes), static_cast<__half *>(scales), static_cast<uint8_t *>(bytes), chunks);
 }
 
-template <typename Source>
-inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream) {
-    const long long chunks = static_cast<long long>(m) * (k / 256), blocks = (chunks + QUANT_THREADS / 16 - 1) / (QUANT_THREADS / 16);
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    return launch_overlapped(bytes != nullptr ? quantize_chunks_kernel<Source, true> : quantize_chunks_kernel<Source, false>, static_cast<unsigned>(blocks), QUANT_THREADS,
-                             0, stream, source, static_cast<uint8_t *>(codes), static_cast<__half *>(scales), static_cast<uint8_t *>(bytes), chunks);
+// Plain activations take the one-chunk form where it is the faster one, alone and in front of a GEMM. Its CTAs of one or two warps of 40 to 48 registers leave room on an SM for the
+// CTA of the narrow GEMM behind it (640 threads of 96), which is then set up when the last of them ends; the paired form's (64
+// threads of 128) did not. Microseconds of the linear, paired and so: 77 x 9216 x 3072 (924 chunks) 14.7 and 13.0, 50 x 12288 x 4096 (800)
+// 24.8 and 22.7, 170 x 3072 x 3072 (2040, two warps) 12.6 and 11.6; two warps at 300 x 4096 x 4096 (4800) lose, 23.8 and 25.7, and CTAs of eight at 384 x 3072 x
+// 3072 (4608), 16.6 and 17.6, while others gain: such calls keep the paired form (as do 520 x 3072 x 3072, 21.9 and 22.6 with eight). From 7168 chunks on eight warps are best: 600 x 2336 x 3072
+// 20.4 and 19.4, 1024 x 9216 x 3072 62.7 and 61.7, the quantiser alone 1024 x 4096 7.4 and 6.2, 2048 x 3072 10.1 and 8.7, 3000 x 3072 (36000) 12.5 and 12.0, 4096 x 3072 15.9 and 16.0.
+constexpr long long ONE_WARP_CHUNKS = 1184, TWO_WARP_CHUNKS = 3072, CHUNKS_FROM = 7168, CHUNKS_TO = 32768;
+
+inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, void *codes, void *scales, void *bytes,
+                                               int m, int k, cudaStream_t stream) {
+    const long long chunks = static_cast<long long>(m) * (k / 256);
+    if (chunks > 0 && (chunks <= TWO_WARP_CHUNKS || (chunks >= CHUNKS_FROM && chunks <= CHUNKS_TO))) {
+        const int threads = chunks <= ONE_WARP_CHUNKS ? 32 : chunks <= TWO_WARP_CHUNKS ? 64 : QUANT_THREADS;
+        if (x_is_half) return launch_quantize_chunks(PlainChunkSource<__half>{static_cast<const __half *>(x)}, codes, scales, bytes, m, k, stream, threads);
+        return launch_quantize_chunks(PlainChunkSource<float>{static_cast<const float *>(x)}, codes, scales, bytes, m, k, stream, threads);
+    }
+    if (x_is_half) return launch_quantize_pairs(PlainSource<__half>{static_cast<const __half *>(x)}, codes, scales, bytes, m, k, stream);
+    return launch_quantize_pairs(PlainSource<float>{static_cast<const float *>(x)}, codes, scales, bytes, m, k, stream);
 }
 
 // GELU takes the one-chunk form up to so many chunks: it fills the SMs with more and shorter threads, the paired form needs

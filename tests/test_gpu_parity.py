@@ -111,6 +111,44 @@ def test_quantize_activations_zero_and_tiny_rows(qi):
     assert np.all(expected_scales[0] == 1)  # the 2^-24 floor (gemm.cu:45)
 
 
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+def test_quantize_activations_in_each_form(qi, dtype):
+    # one chunk or two a half-warp, CTAs of one, two and eight warps, by the number of chunks: the bytes of the oracle, and of rows
+    # with ties, infinities, NaNs, denormals and the largest values those that any other form gives
+    k = 1024
+    rng = np.random.default_rng(41)
+    most = 8300  # chunks: 33200, past the last that one chunk a half-warp takes
+    x = qt.make_activations(rng, most, k)
+    x = x if dtype == "f16" else x.astype(np.float32) + rng.standard_normal((most, k), dtype=np.float32) * 1e-3
+    expected_codes, expected_scales = qo.quantize_activations(x)
+    special = [(0, 5, np.inf), (1, 300, -np.inf), (2, 700, np.nan), (3, slice(None), 6.1e-5), (4, slice(0, 256), 65504.0), (5, slice(None), 0.0), (6, slice(0, None, 64), 3.5), (7, 1000, np.inf), (7, 1001, -np.inf)]
+    strange = x.copy()
+    for row, columns, value in special:
+        strange[row, columns] = value
+    if dtype == "f32":
+        strange[8, ::3] = 1e-40
+        strange[9, ::5] = 1e30
+    first = None
+    for m in (10, 295, 296, 297, 767, 768, 769, 1791, 1792, 8192, 8193, most):
+        for source, plain in ((x, True), (strange, False)):
+            codes = torch.zeros(m, k // 2, dtype=torch.uint8, device="cuda")
+            scales = torch.zeros(m, k // 64, dtype=torch.float16, device="cuda")
+            wide = torch.zeros(m, k, dtype=torch.uint8, device="cuda")
+            code = qi.DTYPE_F32 if dtype == "f32" else qi.DTYPE_F16
+            assert qi.w4a4_quantize_activations_wide_ex(up(source[:m]), code, codes, scales, wide, m, k) == 0
+            check_status(qi)
+            if plain:
+                assert np.array_equal(half_bits(scales), expected_scales[:m])
+                assert np.array_equal(codes.cpu().numpy(), expected_codes[:m])
+                nibbles = torch.zeros_like(wide)
+                assert qi.w4a4_widen_codes_ex(codes, nibbles, m, k) == 0
+                assert torch.equal(wide, nibbles)
+            else:
+                now = [t[:10].cpu().numpy().copy() for t in (codes, scales.view(torch.int16), wide)]
+                first = now if first is None else first
+                assert all(np.array_equal(a, b) for a, b in zip(first, now)), m
+
+
 def test_quantize_rejects_bad_shapes(qi):
     x = torch.zeros(4, 320, device="cuda")
     out = torch.zeros(4096, dtype=torch.uint8, device="cuda")
