@@ -205,10 +205,13 @@ struct SwapPlan {
     double us;  // estimated
 };
 
-// Microseconds as measured on B200 with the weights in L2 or streaming from HBM (77 x {12288, 9216} x 3072, 16 x 18432 x
-// 3072, {77, 256} x 3072 x 12288, {256, 1024} rows): a step of 128 inputs costs a CTA 0.25 (its unpack warps) or 0.003
-// per column (its tensor cores and their operand), a tile 4 + 0.006 per column for its start, its first loads and
-// its results, and sharing a tile over a cluster another 0.8 + 0.016 per column.
+// Microseconds, fitted to 450 shapes of 9 to 1300 rows (every width and split, and the pairs, three sets of operands in turn):
+// a step of 128 inputs costs a CTA 0.395 (its unpack warps, and waits) or 0.003 per column (its tensor cores and their operand), a
+// tile 1.5 + 0.0265 per column for its start, its first loads and its results, and sharing a tile over a cluster another
+// 1.27 + 0.025 per column. What these choose is 0.3 % slower than the best of all in the mean, 12 % at worst; the prices before,
+// from when a tile of one CTA ended in shared memory (0.25, 0.003, 4 + 0.006, 0.8 + 0.016), 1.0 and 25 %: 411 x 3072 x 12288
+// 37.3 us where two CTAs to a tile of 144 columns take 29.9, 783 x 4096 x 12288 77.7 against 62.1. No shape of the 450 is slower for the change; of 160 more, of 900 to 16384 rows,
+// seven take other tiles, four of them faster (0.97) and three slower (966 x 9216 x 3072 1.03, 1431 x 608 x 9856 1.09).
 // `like`: only plans that add up K in that plan's order.
 SwapPlan plan_w4a16_swap(int m, int n, int k, int device, const SwapPlan *like = nullptr) {
     namespace ws = w4a16_swap;
@@ -223,13 +226,13 @@ SwapPlan plan_w4a16_swap(int m, int n, int k, int device, const SwapPlan *like =
         if (columns == before) continue;
         before = columns;
         if (like != nullptr && ws::issuers_of(columns) != ws::issuers_of(like->columns)) continue;
-        const double step = columns * 0.003 > 0.25 ? columns * 0.003 : 0.25;
+        const double step = columns * 0.003 > 0.395 ? columns * 0.003 : 0.395;
         for (int split = 1; split <= ws::MAX_SPLIT && split <= steps; ++split) {
             const long long tiles = static_cast<long long>(tiles_n) * ((m + columns - 1) / columns);
             const int resident = resident_clusters(device, split);
             const long long waves = (tiles + resident - 1) / resident;
             if (like != nullptr ? split != like->split : split > 1 && waves > 1) continue;
-            const double us = waves * (4.0 + columns * 0.006 + (steps + split - 1) / split * step + (split > 1 ? 0.8 + 0.016 * columns : 0.0));
+            const double us = waves * (1.5 + columns * 0.0265 + (steps + split - 1) / split * step + (split > 1 ? 1.27 + 0.025 * columns : 0.0));
             if (us < best.us) best = {columns, split, us};
         }
     }
@@ -262,7 +265,7 @@ int launch_w4a16_swap(const void *x_half, const void *codes, const void *scales,
 
 // The widest tile is not always the best: 4096 x 3072 outputs are 192 tiles of 256 x 256, three waves of 74 pairs, or 288 of
 // 256 x 176, four waves (73.4 against 68.4 us at K = 3072). Microseconds: per column 0.0031 a step of 128 inputs and 0.0137 a
-// tile (4096 x {3072, 9216, 12288} x 3072, 4096 x 3072 x 12288, 1024 x 4096 x 4096), and 3 once.
+// tile (4096 x {3072, 9216, 12288} x 3072, 4096 x 3072 x 12288, 1024 x 4096 x 4096), and 5.2 once (fitted with the prices above).
 SwapPlan plan_w4a16_pair_swap(int m, int n, int k, int device) {
     namespace wp = w4a16_pair_swap;
     const int pairs = sm_count(device) / 2, steps = (k + 127) / 128;  // what fills up an even number of steps costs next to nothing
@@ -270,7 +273,7 @@ SwapPlan plan_w4a16_pair_swap(int m, int n, int k, int device) {
     SwapPlan best = {0, 2, 1e30};
     for (int columns = wp::MAX_COLUMNS; columns >= 128; columns -= 16) {
         const long long waves = (tiles_n * ((m + columns - 1) / columns) + pairs - 1) / pairs;
-        const double us = 3.0 + waves * columns * (steps * 0.0031 + 0.0137);
+        const double us = 5.2 + waves * columns * (steps * 0.0031 + 0.0137);
         if (us < best.us) best = {columns, 2, us};
     }
     return best;
