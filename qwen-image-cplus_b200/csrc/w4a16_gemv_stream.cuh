@@ -21,7 +21,10 @@
 // would meet on four banks. So the odd rows read the two halves of their group in the other order, and the columns of B
 // that one or a few activation rows leave idle hold those rows once more with the halves of each group exchanged: column 2a + p
 // serves the weight rows of parity p (up to four activation rows; with more, every row reads in the same order).
-// Measured without gain: two accumulator chains, two steps unrolled, a limit on the copies in flight, a warp that does nothing but the final
+// The halves of the groups are added up apart: an MMA cuts its sum to 24 bits, always towards zero, so that the error grows with
+// the number of MMAs in a chain. With one chain of 64 in a team of three, 18432 x 3072 was 1.25e-6 off (2-norm, against 64
+// bits), with two of 32 it is 6.4e-7 off, as it was with chains of 32 in teams of six.
+// Measured without gain: two steps unrolled, a limit on the copies in flight, a warp that does nothing but the final
 // sums (10.2 us alone), teams of 8 and 12 warps (10.7, 10.5).
 //
 // Unpacking takes ten instructions per eight weights. A nibble moved to bits 2..5 or 6..9 of a 16-bit lane is the fp16 denormal
@@ -229,7 +232,7 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         const bool arrived = wait_uniform([&]() { return fetched[s] == tile; }, &g_status, STATUS_WAIT_EMPTY | 0xB000 | s, 32) &&
                              mbarrier_wait_uniform(full_u + s * 8, phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
         const uint32_t stage = smem + s * stage_bytes;
-        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // of the groups' halves read first, and second
         if (arrived) {
             uint32_t at_codes = stage + my_codes, at_codes_b = at_codes + 8 * row_bytes, at_x = my_x;
             uint32_t at_scales = stage + my_scales, at_scales_b = at_scales + 16 * groups;
@@ -253,8 +256,8 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
                         uint32_t pa[4], pb[4];
                         unpack(a, b, pa, pb);
                         const uint32_t one[4] = {pa[0], pb[0], pa[1], pb[1]}, two[4] = {pa[2], pb[2], pa[3], pb[3]};
-                        mma_m16n8k16(c, one, xv.x, xv.y);
-                        mma_m16n8k16(c, two, xv.z, xv.w);
+                        mma_m16n8k16(w >> 2 ? d : c, one, xv.x, xv.y);
+                        mma_m16n8k16(w >> 2 ? d : c, two, xv.z, xv.w);
                     }
                 };
                 // scale * 2^22 is an fp16 number below 1/64, scale * 2^18 below 1/4 (a NaN fails both tests)
@@ -281,6 +284,8 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
                 }
             }
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) c[i] += d[i];
         // c[0], c[1]: weight row r, columns 2q, 2q+1; c[2], c[3]: weight row r + 8
         if (stores) {
             sts_float(partial + my_partial, ALTERNATE && odd ? c[1] : c[0]);

@@ -367,6 +367,25 @@ def test_w4a16_gemv_teams_and_steps(qi, m, n, k):
     assert qt.max_relative_error(y.cpu().numpy(), qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)) <= OUTPUT_TOLERANCE
 
 
+@pytest.mark.parametrize("m", [1, 2, 8])
+@pytest.mark.parametrize("n,k,chain", [(576, 256, 8), (2400, 512, 8), (9216, 1024, 8), (18432, 1536, 16), (6144, 2048, 24), (3072, 3072, 32), (4096, 4096, 32)])
+def test_w4a16_gemv_sums_are_as_exact_as_short_chains(qi, m, n, k, chain):
+    # An MMA cuts its float32 sum towards zero, on the mean by half a unit of 2^-24 to 2^-23 of it: 2^-25 for each of a chain of
+    # them that only grows, plus what rounding the chains' sums to nearest adds (2^-23)
+    rng = np.random.default_rng(3060 + m + n + k)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    scales = (rng.uniform(0.9, 1.1, size=(n, k // 64)) * 0.0065).astype(np.float16)
+    minimums = (-7.5 * scales.astype(np.float32)).astype(np.float16)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(1)).half().cuda()
+    nibbles = torch.stack([up(codes) & 15, up(codes) >> 4], -1).reshape(n, k // 64, 64).double()
+    weights = (nibbles * up(scales).double()[..., None] + up(minimums).double()[..., None]).half().double().reshape(n, k)
+    exact = x.double() @ weights.T
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(x, up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert float((y.double() - exact).norm() / exact.norm()) <= chain * 2.0 ** -25 + 2.0 ** -23
+
+
 @pytest.mark.parametrize("m", [1, 3])
 def test_w4a16_gemv_scales_of_every_size(qi, m):
     # scales from fp16 denormals up to 4: the GEMV's unpack treats scale >= 1/16 (where scale * 2^20 leaves fp16)
