@@ -129,7 +129,8 @@ int qi_w4a16_gemm_ex(const void *x_half, const void *codes, const void *scales, 
 
 /* 1 <= m <= 8 activation rows (the per-block adaLN modulation linears are m = 1); n % 16 == 0,
  * k % 64 == 0. Same operator as qi_w4a16_gemm without padding m to 128. The reference has no
- * packed m = 1 path (its modulation linear is a BF16 cuBLAS call, transformer.cplus:716-730). */
+ * packed m = 1 path (its modulation linear is a BF16 cuBLAS call, transformer.cplus:716-730).
+ * With k <= 4096 and scales and minimums 16-byte aligned, the bits of a row of y depend neither on m nor on n. */
 int qi_w4a16_gemv_ex(const void *x_half, const void *codes, const void *scales, const void *minimums,
                      const float *bias, void *y, int y_dtype, long long ldy, int m, int n, int k, void *stream);
 

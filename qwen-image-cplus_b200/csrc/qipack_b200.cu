@@ -535,22 +535,27 @@ __global__ void dequantize_kernel(const uint8_t *__restrict__ codes, const __hal
     for (int j = 0; j < 4; ++j) destination[j] = values[j];
 }
 
-// The streaming GEMV, one CTA per SM: as many stages as fit beside the activations and the partial sums, and teams of as few warps as leave
-// a stage for each team: the fewer they are, the less of a tile's time is a team's own waiting, but the longer
-// the last tile takes. Microseconds with teams of 3, 4 and 6: 60 x 18432 x 3072 308, 318, 319, 100 x 6144 x 2048 123, 135, 143; one
-// 18432 x 3072 8.8, 9.2, 9.0, one 9216 x 3072 5.3, 5.2, 5.1, one 3072 x 3072 4.2, 3.9, 3.7; with fewer stages one 12288 x 4096
-// 10.5, 9.9, 9.5, eight rows of 18432 x 3072 11.7, 11.4, 10.9. Four steps of K are for teams of four (9216 x 1024 3.7, 3.5,
-// 3.7), and up to two for teams of two. By m and k alone: the order of the sums follows from it (w4a16_gemv_stream.cuh).
+// The streaming GEMV, one CTA per SM: as many stages as fit beside the activations and the partial sums. The slices of K follow
+// from k alone, since the order of the sums follows from them (w4a16_gemv_stream.cuh): a row's bits must not depend on how
+// many rows, or which part of a matrix, a call has. Microseconds with 3, 4 and 6 slices, one row: 18432 x 3072 9.5, 9.3, 9.5 (60 of
+// them 304, 314, 322), 12288 x 4096 10.4, 10.1, 9.9 (330, 306, 281), 9216 x 2560 6.0, 5.95, 5.8 (137, 144, 148), 18432 x 1536 6.0, 6.5,
+// 6.3 (194, 199, 210), 9216 x 1024 3.9, 3.7, 3.9. Two steps of K occupy half a team of four, but fewer teams disturb the copies
+// less: 60 x 18432 x 512 with teams of 2, 3 and 4 139, 137, 113.
+// Where a CTA has few tiles, or the stages are few, three slices are for teams of six with half of every group a warp: one and
+// eight rows of 18432 x 3072 9.25 and 11.7 with teams of three, 9.3 and 11.1 with six, of 9216 x 3072 7.0 and 8.2, 6.7 and 7.8,
+// of 3072 x 3072 4.7 and 6.15, 4.35 and 5.7, 60 x 18432 x 3072 297 and 332.
 constexpr int STREAM_CTA_BYTES = 232448 - 1024;  // the rest is the barriers'
 struct StreamPlan {
     int stages, team_warps, smem_bytes;
+    bool halves;
 };
-StreamPlan plan_stream(int m, int k) {
+StreamPlan plan_stream(int m, int k, long long tiles, int ctas) {
     const int fixed = w4a16::stream_fixed_bytes(m, k), stage = w4a16::stream_stage_bytes(k), steps = w4a16::stream_steps(k);
     int stages = (STREAM_CTA_BYTES - fixed) / stage;
     stages = stages > w4a16::STREAM_MAX_STAGES ? w4a16::STREAM_MAX_STAGES : stages;
-    const int team_warps = steps <= 2 ? 2 : steps == 4 ? 4 : stages >= w4a16::STREAM_WARPS / 3 ? 3 : 6;
-    return {stages, team_warps, stages * stage + fixed};
+    const int slices = steps == 1 ? 2 : steps <= 4 ? 4 : steps <= 12 ? 3 : 6;
+    const bool halves = slices == 3 && (tiles < 6LL * ctas || stages < 7);
+    return {stages, halves ? 2 * slices : slices, stages * stage + fixed, halves};
 }
 
 int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,
@@ -564,11 +569,10 @@ int w4a16_gemv(const void *x_half, const void *codes, const void *scales, const 
         const int device = current_device();
         if (device < 0) return INVALID;
         const int tiles = n / w4a16::STREAM_ROWS, resident = sm_count(device);
-        const StreamPlan plan = plan_stream(m, k);
-        const bool alternate = m <= w4a16::STREAM_ALTERNATE_M;
-        auto kernel = alternate ? w4a16::gemv_stream_kernel<true> : w4a16::gemv_stream_kernel<false>;
+        const StreamPlan plan = plan_stream(m, k, tiles, resident);
+        auto kernel = plan.halves ? w4a16::gemv_stream_kernel<true> : w4a16::gemv_stream_kernel<false>;
         static std::atomic<bool> configured[MAX_DEVICES][2];
-        if (const cudaError_t error = configure_once(kernel, STREAM_CTA_BYTES, configured[device][alternate])) return static_cast<int>(error);
+        if (const cudaError_t error = configure_once(kernel, STREAM_CTA_BYTES, configured[device][plan.halves])) return static_cast<int>(error);
         if (plan.stages >= 1) {
             return static_cast<int>(launch_overlapped(kernel, tiles < resident ? tiles : resident,
                                       w4a16::STREAM_THREADS, plan.smem_bytes, stream, static_cast<const __half *>(x_half),
@@ -613,12 +617,12 @@ int w4a16_gemv_grouped(const void *x_half, const qi_gemv_item *items, int count,
     const int device = current_device();
     if (device < 0) return INVALID;
     const int resident = sm_count(device);
-    const StreamPlan plan = plan_stream(m, k);
+    const long long most_tiles = static_cast<long long>(count < w4a16::STREAM_GROUP ? count : w4a16::STREAM_GROUP) * (n / w4a16::STREAM_ROWS);
+    const StreamPlan plan = plan_stream(m, k, most_tiles, resident);
     if (plan.stages < 1) return INVALID;
-    const bool alternate = m <= w4a16::STREAM_ALTERNATE_M;
-    auto kernel = alternate ? w4a16::gemv_stream_grouped_kernel<true> : w4a16::gemv_stream_grouped_kernel<false>;
+    auto kernel = plan.halves ? w4a16::gemv_stream_grouped_kernel<true> : w4a16::gemv_stream_grouped_kernel<false>;
     static std::atomic<bool> configured[MAX_DEVICES][2];
-    if (const cudaError_t error = configure_once(kernel, STREAM_CTA_BYTES, configured[device][alternate])) return static_cast<int>(error);
+    if (const cudaError_t error = configure_once(kernel, STREAM_CTA_BYTES, configured[device][plan.halves])) return static_cast<int>(error);
     for (int first = 0; first < count; first += w4a16::STREAM_GROUP) {
         const int now = count - first < w4a16::STREAM_GROUP ? count - first : w4a16::STREAM_GROUP;
         w4a16::StreamItems group;

@@ -3,29 +3,36 @@
 // to 128), for matrices whose rows are short enough that 16 of them fit a shared-memory stage (K <= 4096).
 //
 // A CTA per SM walks over tiles of 16 weight rows. A tile's codes, scales and minimums are three contiguous ranges of the
-// pack (16 whole rows each), so one thread, in a warp of its own, fetches them with three bulk asynchronous copies
+// pack (16 whole rows each), so one thread, in a warp of its own, fetches them with three or four bulk asynchronous copies
 // (cp.async.bulk, completion counted on an mbarrier) into a ring of up to sixteen stages, and the copies of the next tiles
-// are in flight while the others unpack. The tiles in the ring are dealt out to teams of warps; within a tile the team's warps split K:
-// lane (r, q) = (lane / 4, lane % 4) takes the 64 codes of one group of rows r and r + 8 per step, unpacks them, and
-// feeds them as the A operand of mma.sync.m16n8k16 (fp32 accumulate) whose B operand carries up to 8 activation rows;
-// the order of k inside an MMA is free as long as both operands agree. The K slices are summed through shared memory in a
-// fixed order. How many warps a team has, and so that order, is chosen by m and k alone: a slice of a matrix, a matrix alone and
-// in a group give the same bits.
+// are in flight while the others unpack. The tiles in the ring are dealt out to teams of warps; within a tile the team's
+// warps split K: lane (r, q) = (lane / 4, lane % 4) takes the 64 codes of one group of two weight rows per step, unpacks
+// them, and feeds them as rows r and r + 8 of the A operand of mma.sync.m16n8k16 (fp32 accumulate) whose B operand carries up
+// to 8 activation rows; the order of k inside an MMA is free as long as both operands agree. K is cut into slices, by k alone,
+// and in each the first and the second halves of the groups are added up apart: an MMA cuts its sum to 24 bits, always towards
+// zero, so that the error grows with the number of MMAs in a chain (18432 x 3072 against 64 bits, 2-norm: 1.25e-6 with
+// chains of 64, 6.4e-7 with chains of 32). The sums of the halves, then of the slices, are added through shared memory in a
+// fixed order. A team has a warp for each slice, which keeps both halves' sums, or (HALVES) two, a half each: a tile is done sooner
+// but takes more instructions, and the bits are the same. So a row of activations alone, among others, against a slice of a
+// matrix, a whole one or one in a group gives the same bits.
 //
-// What bounds it, 18432 x 3072 on cold weights: alone the first load, the copies (31.9 MB, 4.7 us) and the last tiles' steps
-// (10.3 -> 8.9 us); in groups of 60 instructions and copies about alike (6.9 -> 5.2 us a matrix; the copies alone 4.6).
+// What bounds it, 18432 x 3072 on cold weights: alone the first load, the copies (31.9 MB, 4.7 us) and the last tiles' steps;
+// in groups of 60 instructions and copies about alike (5.2 us a matrix; the copies alone 4.6).
 // What counted, in that order: shared memory by 32-bit addresses instead of generic pointers (76.0 -> 60.0 million
-// warp instructions for sixteen matrices); a step of whole groups, which halves what a step spends on its scales; a warp that does nothing
-// but fetch, since a thread that unpacks held its team up while the copy engine took its requests; and codes read without
-// bank conflicts (5.7 -> 1.0 million). Rows lie a multiple of 128 bytes apart, so the eight lanes that a 16-byte load serves at a time
-// would meet on four banks. So the odd rows read the two halves of their group in the other order, and the columns of B
-// that one or a few activation rows leave idle hold those rows once more with the halves of each group exchanged: column 2a + p
-// serves the weight rows of parity p (up to four activation rows; with more, every row reads in the same order).
-// The halves of the groups are added up apart: an MMA cuts its sum to 24 bits, always towards zero, so that the error grows with
-// the number of MMAs in a chain. With one chain of 64 in a team of three, 18432 x 3072 was 1.25e-6 off (2-norm, against 64
-// bits), with two of 32 it is 6.4e-7 off, as it was with chains of 32 in teams of six.
-// Measured without gain: two steps unrolled, a limit on the copies in flight, a warp that does nothing but the final
-// sums (10.2 us alone), teams of 8 and 12 warps (10.7, 10.5).
+// warp instructions for sixteen matrices); a step of whole groups, which halves what a step spends on its scales; a warp
+// that does nothing but fetch, since a thread that unpacks held its team up while the copy engine took its requests; and
+// codes read without bank conflicts. Rows lie a multiple of 32 bytes apart, most often of 128, so the eight lanes that a
+// 16-byte load serves at a time, four of each of two MMA rows, would meet on four banks. So the lower eight weight rows lie
+// 16 bytes further on in the stage, by a copy of their own, and MMA rows of either parity are weight rows of either half. From
+// K = 2048 on; below, the fourth copy of a tile costs more than the conflicts (18432 x 512 4.45 us without, 4.75 with it;
+// 60 x 9216 x 1024 88 and 92; 18432 x 2048 7.4 without, 7.1 with it, 3072 x 2048 4.25 and 4.17).
+// Before, odd weight rows read the two halves of their group in the other order, against columns of B that held the activations
+// so. That order of sums is not there for more than four activation rows, whose bits differed from those of one row; it was
+// also slower (m = 8: 18432 x 3072 11.4 -> 11.1 us, 12288 x 4096 13.4 -> 12.7).
+// Measured without gain: two steps unrolled, a limit on the copies in flight, a warp that does nothing but the final sums
+// (10.2 us alone), teams of 8 and 12 warps (10.7, 10.5), lanes that send for one range each (60 x 18432 x 512 150 us -> 217),
+// two slices a warp one after the other, so that teams of three and of six had the same slices (60 x 18432 x 3072 300 ->
+// 334), a second MMA for the rows past the fourth (8 x 18432 x 3072 11.3 -> 13.1).
 //
 // Unpacking takes ten instructions per eight weights. A nibble moved to bits 2..5 or 6..9 of a 16-bit lane is the fp16 denormal
 // code * 2^-22 or code * 2^-18, so one shift serves two nibbles; one half2 fused multiply-add with the scale times 2^22 or
@@ -43,12 +50,14 @@ namespace w4a16 {
 
 // 24 warps unpack, one fetches
 constexpr int STREAM_WARPS = 24, STREAM_THREADS = (STREAM_WARPS + 1) * 32, STREAM_MAX_STAGES = 16, STREAM_ROWS = 16;
-constexpr int STREAM_MAX_TEAM_WARPS = 6;
+constexpr uint32_t STREAM_MAX_SLICES = 6;
 constexpr int STREAM_STEP_GROUPS = 4;  // a step of a warp: a group for each of a row's four lanes
 constexpr int STREAM_MAX_K = 4096;  // 16 rows of codes, scales and minimums: 36 KB per stage
-constexpr int STREAM_ALTERNATE_M = 4;  // activation rows up to which each has two columns of the MMA
+constexpr int STREAM_SHIFT_FROM = 2048;  // see above
+// Bytes that the lower eight rows' codes lie further on in a stage.
+__host__ __device__ constexpr int stream_shift(int k) { return k >= STREAM_SHIFT_FROM ? 16 : 0; }
 
-__host__ __device__ constexpr int stream_stage_bytes(int k) { return STREAM_ROWS * (k / 2) + 2 * STREAM_ROWS * (k / 64) * 2; }
+__host__ __device__ constexpr int stream_stage_bytes(int k) { return STREAM_ROWS * (k / 2) + stream_shift(k) + 2 * STREAM_ROWS * (k / 64) * 2; }
 // a row of activations in pieces of 16 bytes; 64 bytes more set the next row on the other banks
 __host__ __device__ constexpr int stream_steps(int k) { return (k / 64 + STREAM_STEP_GROUPS - 1) / STREAM_STEP_GROUPS; }
 __host__ __device__ constexpr int stream_x_pieces(int k) { return stream_steps(k) * STREAM_STEP_GROUPS * 8 + 4; }
@@ -126,7 +135,7 @@ struct StreamItems {
 // teams' partial sums (stream_partial_bytes(m)).
 // GROUPED: `count` matrices [n, k] from `group`, tile t of the launch is tile t % (n / 16) of matrix t / (n / 16);
 // otherwise the one matrix given by the pointer arguments.
-template <bool GROUPED, bool ALTERNATE>
+template <bool GROUPED, bool HALVES>
 __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, const uint8_t *__restrict__ codes, const __half *__restrict__ scales,
                    const __half *__restrict__ minimums, const float *__restrict__ bias, void *__restrict__ y,
                    int m, int n, int k, long long ldy, int y_is_half, int stages, int team_warps, const StreamItems *group, int count) {
@@ -138,10 +147,10 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     const int cta_warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int teams = STREAM_WARPS / team_warps, team = cta_warp / team_warps, warp = cta_warp - team * team_warps;
     const int team_threads = team_warps * 32, team_thread = warp * 32 + lane;
-    const uint32_t r = lane >> 2, q = lane & 3, odd = ALTERNATE ? r & 1 : 0;
+    const uint32_t r = lane >> 2, q = lane & 3;
     const uint32_t groups = k / 64, steps = stream_steps(k), row_bytes = k / 2;
     const uint32_t code_bytes = STREAM_ROWS * row_bytes, scale_bytes = STREAM_ROWS * groups * 2;
-    const uint32_t stage_bytes = code_bytes + 2 * scale_bytes;
+    const uint32_t shift = stream_shift(k), scales_at = code_bytes + shift, stage_bytes = scales_at + 2 * scale_bytes;
     const int tiles_each = n / STREAM_ROWS, tiles = GROUPED ? tiles_each * count : tiles_each;
     const int step_tiles = static_cast<int>(gridDim.x);
 
@@ -154,19 +163,20 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
             const StreamItem &item = group->item[item_index];
             from_codes = item.codes, from_scales = item.scales, from_minimums = item.minimums;
         }
-        mbarrier_arrive_expect_tx_u32(barrier, stage_bytes);
-        bulk_load(stage, from_codes + static_cast<size_t>(local) * code_bytes, code_bytes, barrier);
-        bulk_load(stage + code_bytes, reinterpret_cast<const uint8_t *>(from_scales) + static_cast<size_t>(local) * scale_bytes, scale_bytes, barrier);
-        bulk_load(stage + code_bytes + scale_bytes, reinterpret_cast<const uint8_t *>(from_minimums) + static_cast<size_t>(local) * scale_bytes, scale_bytes, barrier);
+        from_codes += static_cast<size_t>(local) * code_bytes;
+        mbarrier_arrive_expect_tx_u32(barrier, code_bytes + 2 * scale_bytes);
+        const uint32_t upper = shift != 0 ? code_bytes / 2 : code_bytes;
+        bulk_load(stage, from_codes, upper, barrier);
+        if (shift != 0) bulk_load(stage + upper + shift, from_codes + upper, upper, barrier);
+        bulk_load(stage + scales_at, reinterpret_cast<const uint8_t *>(from_scales) + static_cast<size_t>(local) * scale_bytes, scale_bytes, barrier);
+        bulk_load(stage + scales_at + scale_bytes, reinterpret_cast<const uint8_t *>(from_minimums) + static_cast<size_t>(local) * scale_bytes, scale_bytes, barrier);
         __threadfence_block();
         fetched[s] = tile;
     };
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) {
-            mbarrier_init(&full[s], 1);
-            mbarrier_init(&empty[s], team_warps);
-            fetched[s] = -1;
-        }
+    if (threadIdx.x < stages) {
+        mbarrier_init(&full[threadIdx.x], 1);
+        mbarrier_init(&empty[threadIdx.x], team_warps);
+        fetched[threadIdx.x] = -1;
         fence_barrier_init();
     }
     grid_wait();
@@ -199,17 +209,20 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     }
 
     const __half2 sixty_fourth = __float2half2_rn(1.0f / 64.0f), quarter = __float2half2_rn(0.25f), two_to_9 = __float2half2_rn(512.0f), sixteen = __float2half2_rn(16.0f);
-    const uint32_t whole = groups / STREAM_STEP_GROUPS, first = steps * warp / team_warps, last = steps * (warp + 1) / team_warps;  // this warp's range
-    // Lane / 4 is the number of the B operand's column. ALTERNATE: columns 2a and 2a + 1 are activation row a for the even and the
-    // odd weight rows. A column only ever meets its own results: a lane past the last row feeds row 0 again, and what comes of it is not stored.
-    const uint32_t x_of = ALTERNATE ? r >> 1 : r;
-    const uint32_t my_x = x_pairs + (x_of < static_cast<uint32_t>(m) ? x_of : 0) * x_row + q * 16 + odd * 64 + first * 512;
-    const uint32_t my_codes = r * row_bytes + q * 32 + odd * 16 + first * 128, my_scales = code_bytes + (r * groups + q + first * STREAM_STEP_GROUPS) * 2;
-    const int other_piece = odd ? -16 : 16, other_x = odd ? -64 : 64;
+    // This warp's slice of K; HALVES: of two warps with one slice each takes one half of every group.
+    const uint32_t slices = HALVES ? team_warps / 2 : team_warps, slice = HALVES ? warp >> 1 : warp, half = HALVES ? warp & 1 : 0;
+    const uint32_t whole = groups / STREAM_STEP_GROUPS, first = steps * slice / slices, last = steps * (slice + 1) / slices;
+    // Row r of the MMA is weight row r / 2 where r is even, 8 + r / 2 where it is odd; row r + 8 the fourth after that.
+    const uint32_t weight_row = (r >> 1) + (r & 1) * 8;
+    // Lane / 4 is the number of the B operand's column, an activation row. A column only ever meets its own results: a lane past
+    // the last row feeds row 0 again, and what comes of it is not stored.
+    const uint32_t my_x = x_pairs + (r < static_cast<uint32_t>(m) ? r : 0) * x_row + q * 16 + half * 64 + first * 512;
+    const uint32_t my_codes = weight_row * row_bytes + (r & 1) * shift + q * 32 + half * 16 + first * 128;
+    const uint32_t my_scales = scales_at + (weight_row * groups + q + first * STREAM_STEP_GROUPS) * 2;
     const uint32_t slice_bytes = m * STREAM_ROWS * 4;
     const uint32_t partials = x_pairs + m * x_row + team * 2 * team_warps * slice_bytes;
-    const uint32_t my_partial = warp * slice_bytes + r * 4 + (ALTERNATE ? q : 2 * q) * (STREAM_ROWS * 4);
-    const bool stores = (ALTERNATE ? q : 2 * q) < static_cast<uint32_t>(m), stores_too = 2 * q + 1 < static_cast<uint32_t>(m);
+    const uint32_t my_partial = warp * slice_bytes + weight_row * 4 + 2 * q * (STREAM_ROWS * 4);
+    const bool stores = 2 * q < static_cast<uint32_t>(m), stores_too = 2 * q + 1 < static_cast<uint32_t>(m);
     const bool sums = team_thread < m * STREAM_ROWS;
     // Team t takes the CTA's tiles t, t + teams, ...; tile i of the CTA lies in stage i modulo the number of stages.
     uint32_t s = team, phase = 0, parity = 0;
@@ -232,10 +245,10 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         const bool arrived = wait_uniform([&]() { return fetched[s] == tile; }, &g_status, STATUS_WAIT_EMPTY | 0xB000 | s, 32) &&
                              mbarrier_wait_uniform(full_u + s * 8, phase, &g_status, STATUS_WAIT_FULL | 0xB000 | s);
         const uint32_t stage = smem + s * stage_bytes;
-        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // of the groups' halves read first, and second
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // of a group's first half, of its second
         if (arrived) {
-            uint32_t at_codes = stage + my_codes, at_codes_b = at_codes + 8 * row_bytes, at_x = my_x;
-            uint32_t at_scales = stage + my_scales, at_scales_b = at_scales + 16 * groups;
+            uint32_t at_codes = stage + my_codes, at_codes_b = at_codes + 4 * row_bytes, at_x = my_x;
+            uint32_t at_scales = stage + my_scales, at_scales_b = at_scales + 8 * groups;
 #pragma unroll 1
             for (uint32_t step = first; step < last; ++step, at_codes += 128, at_codes_b += 128, at_x += 512, at_scales += 8, at_scales_b += 8) {
                 __half scale_a = lds_half(at_scales), scale_b = lds_half(at_scales_b);
@@ -244,12 +257,12 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
                     scale_a = scale_b = minimum_a = minimum_b = __ushort_as_half(0);
                 uint4 code_a[2], code_b[2];
                 code_a[0] = lds_16(at_codes), code_b[0] = lds_16(at_codes_b);
-                code_a[1] = lds_16(at_codes + other_piece), code_b[1] = lds_16(at_codes_b + other_piece);
+                if constexpr (!HALVES) code_a[1] = lds_16(at_codes + 16), code_b[1] = lds_16(at_codes_b + 16);
                 const __half2 ma = __half2half2(minimum_a), mb = __half2half2(minimum_b);
                 auto multiply = [&](auto unpack) {
 #pragma unroll
-                    for (int w = 0; w < 8; ++w) {  // 8 inputs of each row per word, two MMA steps
-                        const uint4 xv = lds_16((w >> 2 ? at_x + other_x : at_x) + (w & 3) * 128);
+                    for (int w = 0; w < (HALVES ? 4 : 8); ++w) {  // 8 inputs of each row per word, two MMA steps
+                        const uint4 xv = lds_16(at_x + (w >> 2) * 64 + (w & 3) * 128);
                         const uint4 from_a = code_a[w >> 2], from_b = code_b[w >> 2];
                         const uint32_t a = (w & 3) == 0 ? from_a.x : (w & 3) == 1 ? from_a.y : (w & 3) == 2 ? from_a.z : from_a.w;
                         const uint32_t b = (w & 3) == 0 ? from_b.x : (w & 3) == 1 ? from_b.y : (w & 3) == 2 ? from_b.z : from_b.w;
@@ -284,16 +297,18 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
                 }
             }
         }
+        if constexpr (!HALVES) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) c[i] += d[i];
-        // c[0], c[1]: weight row r, columns 2q, 2q+1; c[2], c[3]: weight row r + 8
-        if (stores) {
-            sts_float(partial + my_partial, ALTERNATE && odd ? c[1] : c[0]);
-            sts_float(partial + my_partial + 32, ALTERNATE && odd ? c[3] : c[2]);
+            for (int i = 0; i < 4; ++i) c[i] += d[i];
         }
-        if (!ALTERNATE && stores_too) {
+        // c[0], c[1]: MMA row r, columns 2q, 2q+1; c[2], c[3]: MMA row r + 8
+        if (stores) {
+            sts_float(partial + my_partial, c[0]);
+            sts_float(partial + my_partial + 16, c[2]);
+        }
+        if (stores_too) {
             sts_float(partial + my_partial + STREAM_ROWS * 4, c[1]);
-            sts_float(partial + my_partial + STREAM_ROWS * 4 + 32, c[3]);
+            sts_float(partial + my_partial + STREAM_ROWS * 4 + 16, c[3]);
         }
         __syncwarp();
         if (lane == 0) mbarrier_arrive_u32(empty_u + s * 8);  // this warp is done with the stage
@@ -304,13 +319,16 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
         // fixed-order sum over the K slices: thread -> (activation row, weight row), so that few rows keep few warps
         if (sums) {
             for (uint32_t item = team_thread; item < slice_bytes / 4; item += team_threads) {
-                float of_warp[STREAM_MAX_TEAM_WARPS], total = 0.0f;
+                float of_slice[STREAM_MAX_SLICES], of_half[STREAM_MAX_SLICES], total = 0.0f;
 #pragma unroll
-                for (int i = 0; i < STREAM_MAX_TEAM_WARPS; ++i)
-                    if (i < team_warps) of_warp[i] = lds_float(partial + i * slice_bytes + item * 4);
+                for (uint32_t i = 0; i < (HALVES ? STREAM_MAX_SLICES / 2 : STREAM_MAX_SLICES); ++i)
+                    if (i < slices) {
+                        of_slice[i] = lds_float(partial + (HALVES ? 2 * i : i) * slice_bytes + item * 4);
+                        if constexpr (HALVES) of_half[i] = lds_float(partial + (2 * i + 1) * slice_bytes + item * 4);
+                    }
 #pragma unroll
-                for (int i = 0; i < STREAM_MAX_TEAM_WARPS; ++i)
-                    if (i < team_warps) total += of_warp[i];
+                for (uint32_t i = 0; i < (HALVES ? STREAM_MAX_SLICES / 2 : STREAM_MAX_SLICES); ++i)
+                    if (i < slices) total += HALVES ? of_slice[i] + of_half[i] : of_slice[i];
                 total += add;
                 const size_t element = static_cast<size_t>(item >> 4) * ldy + out_row;
                 if (y_is_half) static_cast<__half *>(to_y)[element] = __float2half_rn(total);
@@ -327,19 +345,19 @@ __device__ __forceinline__ void gemv_stream_body(const __half *__restrict__ x, c
     }
 }
 
-template <bool ALTERNATE>
+template <bool HALVES>
 __global__ void __launch_bounds__(STREAM_THREADS, 1)
 gemv_stream_kernel(const __half *__restrict__ x, const uint8_t *__restrict__ codes, const __half *__restrict__ scales,
                    const __half *__restrict__ minimums, const float *__restrict__ bias, void *__restrict__ y,
                    int m, int n, int k, long long ldy, int y_is_half, int stages, int team_warps) {
-    gemv_stream_body<false, ALTERNATE>(x, codes, scales, minimums, bias, y, m, n, k, ldy, y_is_half, stages, team_warps, nullptr, 1);
+    gemv_stream_body<false, HALVES>(x, codes, scales, minimums, bias, y, m, n, k, ldy, y_is_half, stages, team_warps, nullptr, 1);
 }
 
-template <bool ALTERNATE>
+template <bool HALVES>
 __global__ void __launch_bounds__(STREAM_THREADS, 1)
 gemv_stream_grouped_kernel(const __half *__restrict__ x, const __grid_constant__ StreamItems group, int count,
                            int m, int n, int k, long long ldy, int y_is_half, int stages, int team_warps) {
-    gemv_stream_body<true, ALTERNATE>(x, nullptr, nullptr, nullptr, nullptr, nullptr, m, n, k, ldy, y_is_half, stages, team_warps, &group, count);
+    gemv_stream_body<true, HALVES>(x, nullptr, nullptr, nullptr, nullptr, nullptr, m, n, k, ldy, y_is_half, stages, team_warps, &group, count);
 }
 
 }  // namespace w4a16

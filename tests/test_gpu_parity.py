@@ -386,6 +386,33 @@ def test_w4a16_gemv_sums_are_as_exact_as_short_chains(qi, m, n, k, chain):
     assert float((y.double() - exact).norm() / exact.norm()) <= chain * 2.0 ** -25 + 2.0 ** -23
 
 
+@pytest.mark.parametrize("n,k", [(48, 64), (576, 256), (4784, 512), (2400, 704), (4784, 1024), (2400, 1088), (14224, 1536), (4784, 1984), (2400, 2048),
+                                 (4784, 2560), (14224, 3072), (2400, 3136), (4784, 4096)])
+def test_w4a16_gemv_rows_do_not_depend_on_their_number(qi, n, k):
+    # every kind of teams, with the lower rows' codes where the others end and further on: the bits of a row of activations alone
+    # are those it has among others, and against a few weight rows those against all (many are for teams of three warps, few
+    # for teams of six with the same slices of K)
+    rng = np.random.default_rng(3070 + n + k)
+    codes, scales, minimums = (up(a) for a in qt.random_w4a16_pack(rng, n, k))
+    x, bias = up(qt.make_activations(rng, 8, k, "silu")), up(qt.make_bias(rng, n))
+    results = []
+    for m in range(1, 9):
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        assert qi.w4a16_gemv_ex(x, codes, scales, minimums, bias, y, qi.DTYPE_F32, n, m, n, k) == 0
+        results.append(y)
+    check_status(qi)
+    for m, y in enumerate(results, 1):
+        assert torch.equal(y, results[-1][:m]), m
+    alone = torch.full((1, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(x[5:], codes, scales, minimums, bias, alone, qi.DTYPE_F32, n, 1, n, k) == 0
+    check_status(qi)
+    assert torch.equal(alone[0], results[-1][5])
+    few = torch.full((8, 48), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(x, codes[:48], scales[:48], minimums[:48], bias[:48], few, qi.DTYPE_F32, 48, 8, 48, k) == 0
+    check_status(qi)
+    assert torch.equal(few, results[-1][:, :48])
+
+
 @pytest.mark.parametrize("m", [1, 3])
 def test_w4a16_gemv_scales_of_every_size(qi, m):
     # scales from fp16 denormals up to 4: the GEMV's unpack treats scale >= 1/16 (where scale * 2^20 leaves fp16)
