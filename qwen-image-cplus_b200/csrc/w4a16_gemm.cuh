@@ -66,14 +66,19 @@ struct Tile {
 // code * 2^-20 or code * 2^-21, and ONE fused multiply-add per pair does the rest: fma(code * 2^-20, scale * 2^20, minimum) =
 // fp16(code * scale + minimum), the product exact and the sum rounded once like the reference's (gemm.cu:223-230). Bytes with
 // bit 7 clear are also where the byte permutes find their zeros, as copies of that bit: eleven instructions for eight
-// codes, six of them the integer pipe's (thirteen and eight with a mask after each permute). It needs
-// scale * 2^21 to be an fp16 number: |scale| < 1/32. Any other scale (a NaN included) takes the path that first makes each
-// code an fp16 integer.
+// codes, six of them the integer pipe's. That needs scale * 2^21 to be an fp16 number, |scale| < 1/32, and a lane is a weight
+// row with scales of its own: where one of a warp's is larger, all with |scale| < 1/16 take thirteen instructions, eight of
+// them the integer pipe's, with both nibbles at bits 4..7 and a mask after each permute, so that a warp does not walk through
+// both (77 x 12288 x 3072 with a tenth of the groups at 0.046: 17.1 us with the path for any scale beside the first, 12.6
+// so; without such groups 12.1 -> 11.95, as the branch is the whole warp's). Any other scale (a NaN included) takes the path that
+// first makes each code an fp16 integer. All lanes of a warp that have not returned call together.
 template <int WORDS>
 __device__ __forceinline__ void unpack_words(const uint32_t (&words)[WORDS], const __half2 scale2, const __half2 minimum2,
                                              uint32_t (&values)[4 * WORDS]) {
-    const __half limit = __ushort_as_half(0x2800), two_to_10 = __ushort_as_half(0x6400), two_to_11 = __ushort_as_half(0x6800);
-    if (__hlt(__habs(__low2half(scale2)), limit)) {
+    const __half limit = __ushort_as_half(0x2800), twice_limit = __ushort_as_half(0x2C00);
+    const __half two_to_10 = __ushort_as_half(0x6400), two_to_11 = __ushort_as_half(0x6800);
+    const __half magnitude = __habs(__low2half(scale2));
+    if (__all_sync(0xffffffffu, __hlt(magnitude, limit))) {
         const __half2 scale_up = __hmul2(__hmul2(scale2, __half2half2(two_to_10)), __halves2half2(two_to_11, two_to_10));
 #pragma unroll
         for (int w = 0; w < WORDS; ++w) {
@@ -83,6 +88,19 @@ __device__ __forceinline__ void unpack_words(const uint32_t (&words)[WORDS], con
                 // [byte b of low, its bit 7, byte b of high, bit 7 of byte b of low]
                 uint32_t pair;
                 asm("prmt.b32 %0, %1, %2, %3;" : "=r"(pair) : "r"(low), "r"(high), "r"(0x8480u + 0x1111u * b));
+                const __half2 weight = __hfma2(*reinterpret_cast<__half2 *>(&pair), scale_up, minimum2);
+                values[4 * w + b] = *reinterpret_cast<const uint32_t *>(&weight);
+            }
+        }
+    } else if (__hlt(magnitude, twice_limit)) {
+        const __half2 up = __half2half2(two_to_10), scale_up = __hmul2(__hmul2(scale2, up), up);
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w) {
+            const uint32_t low_nibbles_up = words[w] << 4;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                // [byte b of the shifted word, -, byte b of the word, -], then the two nibbles in bits 4..7 and 20..23
+                uint32_t pair = __byte_perm(low_nibbles_up, words[w], 0x4400u + 0x1111u * b) & 0x00F000F0u;
                 const __half2 weight = __hfma2(*reinterpret_cast<__half2 *>(&pair), scale_up, minimum2);
                 values[4 * w + b] = *reinterpret_cast<const uint32_t *>(&weight);
             }
