@@ -205,37 +205,72 @@ struct SwapPlan {
     double us;  // estimated
 };
 
-// Microseconds, fitted to 450 shapes of 9 to 1300 rows (every width and split, and the pairs, three sets of operands in turn):
-// a step of 128 inputs costs a CTA 0.395 (its unpack warps, and waits) or 0.003 per column (its tensor cores and their operand), a
-// tile 1.5 + 0.0265 per column for its start, its first loads and its results, and sharing a tile over a cluster another
-// 1.27 + 0.025 per column. What these choose is 0.3 % slower than the best of all in the mean, 12 % at worst; the prices before,
-// from when a tile of one CTA ended in shared memory (0.25, 0.003, 4 + 0.006, 0.8 + 0.016), 1.0 and 25 %: 411 x 3072 x 12288
-// 37.3 us where two CTAs to a tile of 144 columns take 29.9, 783 x 4096 x 12288 77.7 against 62.1. No shape of the 450 is slower for the change; of 160 more, of 900 to 16384 rows,
-// seven take other tiles, four of them faster (0.97) and three slower (966 x 9216 x 3072 1.03, 1431 x 608 x 9856 1.09).
+// Microseconds: a step of 128 inputs costs a CTA `step` (its unpack warps) or `step_column` per column (its tensor cores and their
+// operand), a tile `tile` and `tile_column` per column (its start, its first loads and its results), and sharing a tile
+// over a cluster another `share` and `share_column`.
+struct SwapPrices {
+    double step, step_column, tile, tile_column, share, share_column;
+    double us(int columns, int split, int steps, long long waves) const {
+        const double a_step = columns * step_column > step ? columns * step_column : step;
+        return waves * (tile + columns * tile_column + (steps + split - 1) / split * a_step + (split > 1 ? share + share_column * columns : 0.0));
+    }
+};
+// 77 x {12288, 9216} x 3072, 16 x 18432 x 3072, {77, 256} x 3072 x 12288, {256, 1024} rows; with the weights in L2 or from HBM
+constexpr SwapPrices SWAP_PRICES = {0.25, 0.003, 4.0, 0.006, 0.8, 0.016};
+// Fitted to 450 shapes of 9 to 1300 rows, every width and split. They see that a narrow tile's steps cost more than the prices above
+// say, and what a cluster to a wider tile then gains: 411 x 3072 x 12288 35.2 us with a CTA to 80 columns, 28.6 with two to 144.
+constexpr SwapPrices SHARED_PRICES = {0.395, 0.003, 1.5, 0.0265, 1.27, 0.025};
+// A cluster that is priced this much below the best tiles of one CTA takes their place: 178 such shapes of 9 to 2500 rows took 0.87 of
+// the time in the mean, 0.70 to 1.01. Of 82 with prices from 1.05 to 1.1 apart three were slower, by up to 3 percent. Where the fitted
+// prices chose among all tiles, 40 of 200 choices were slower by more than 2 percent: 646 x 1152 x 7616 by a third (three CTAs to a
+// tile instead of two), 233 x 10528 x 576 as well (two waves instead of one), 11725 x 736 x 6848 by 9 percent (pairs).
+constexpr double SHARED_GAIN = 1.1;
+
+// Steps of 128 inputs, eight MMAs each, that are added up in one accumulator before anything is rounded to nearest. An MMA cuts its
+// sum, so that the error grows with them (783 x 4096 x 12288 against 64 bits, 2-norm: 7.3e-6 with 48, 1.44e-5 with 96).
+int swap_chain(int columns, int split, int steps) {
+    const int issuers = w4a16_swap::issuers_of(columns), share = (steps + split - 1) / split;
+    return (share + issuers - 1) / issuers;
+}
+
+// What SWAP_PRICES find best; where that is a CTA to a tile and SHARED_PRICES find it dearer by SHARED_GAIN, the cluster that they find
+// best among those whose chains are no longer, so that no result is further off for it. `us` stays that of SWAP_PRICES, for the
+// comparison with the pairs.
 // `like`: only plans that add up K in that plan's order.
 SwapPlan plan_w4a16_swap(int m, int n, int k, int device, const SwapPlan *like = nullptr) {
     namespace ws = w4a16_swap;
     const int tiles_n = (n + ws::BN - 1) / ws::BN, steps = (k + ws::BK - 1) / ws::BK;
-    SwapPlan best = {0, 0, 1e30};
     // The widest tiles and those a little narrower; narrower ones where all of them run at once (8192 x 32 x 64: 32 tiles of
     // 256 columns 8.2 us, 128 of 64 5.9).
     const int widest = (m + ws::MAX_COLUMNS - 1) / ws::MAX_COLUMNS;
-    for (int tiles_m = widest, before = 0; tiles_m < widest + 8 || tiles_m * tiles_n <= sm_count(device); ++tiles_m) {
-        const int columns = ((m + tiles_m - 1) / tiles_m + 15) / 16 * 16;
-        if (tiles_m > 1 && columns < 64) break;
-        if (columns == before) continue;
-        before = columns;
-        if (like != nullptr && ws::issuers_of(columns) != ws::issuers_of(like->columns)) continue;
-        const double step = columns * 0.003 > 0.395 ? columns * 0.003 : 0.395;
-        for (int split = 1; split <= ws::MAX_SPLIT && split <= steps; ++split) {
-            const long long tiles = static_cast<long long>(tiles_n) * ((m + columns - 1) / columns);
-            const int resident = resident_clusters(device, split);
-            const long long waves = (tiles + resident - 1) / resident;
-            if (like != nullptr ? split != like->split : split > 1 && waves > 1) continue;
-            const double us = waves * (1.5 + columns * 0.0265 + (steps + split - 1) / split * step + (split > 1 ? 1.27 + 0.025 * columns : 0.0));
-            if (us < best.us) best = {columns, split, us};
+    auto for_each = [&](auto visit) {  // columns, CTAs to a tile, waves
+        for (int tiles_m = widest, before = 0; tiles_m < widest + 8 || tiles_m * tiles_n <= sm_count(device); ++tiles_m) {
+            const int columns = ((m + tiles_m - 1) / tiles_m + 15) / 16 * 16;
+            if (tiles_m > 1 && columns < 64) break;
+            if (columns == before) continue;
+            before = columns;
+            if (like != nullptr && ws::issuers_of(columns) != ws::issuers_of(like->columns)) continue;
+            for (int split = 1; split <= ws::MAX_SPLIT && split <= steps; ++split) {
+                const long long tiles = static_cast<long long>(tiles_n) * ((m + columns - 1) / columns);
+                const int resident = resident_clusters(device, split);
+                const long long waves = (tiles + resident - 1) / resident;
+                if (like != nullptr ? split != like->split : split > 1 && waves > 1) continue;
+                visit(columns, split, waves);
+            }
         }
-    }
+    };
+    SwapPlan best = {0, 0, 1e30};
+    double dearest = 0.0;  // what a cluster may cost to take its place
+    for_each([&](int columns, int split, long long waves) {
+        const double us = SWAP_PRICES.us(columns, split, steps, waves);
+        if (us < best.us) best = {columns, split, us}, dearest = SHARED_PRICES.us(columns, split, steps, waves) / SHARED_GAIN;
+    });
+    if (like != nullptr || best.split > 1) return best;
+    const int chain = swap_chain(best.columns, best.split, steps);
+    for_each([&](int columns, int split, long long waves) {
+        const double us = SHARED_PRICES.us(columns, split, steps, waves);
+        if (split > 1 && us < dearest && swap_chain(columns, split, steps) <= chain) best.columns = columns, best.split = split, dearest = us;
+    });
     return best;
 }
 
@@ -265,7 +300,7 @@ int launch_w4a16_swap(const void *x_half, const void *codes, const void *scales,
 
 // The widest tile is not always the best: 4096 x 3072 outputs are 192 tiles of 256 x 256, three waves of 74 pairs, or 288 of
 // 256 x 176, four waves (73.4 against 68.4 us at K = 3072). Microseconds: per column 0.0031 a step of 128 inputs and 0.0137 a
-// tile (4096 x {3072, 9216, 12288} x 3072, 4096 x 3072 x 12288, 1024 x 4096 x 4096), and 5.2 once (fitted with the prices above).
+// tile (4096 x {3072, 9216, 12288} x 3072, 4096 x 3072 x 12288, 1024 x 4096 x 4096), and 3 once.
 SwapPlan plan_w4a16_pair_swap(int m, int n, int k, int device) {
     namespace wp = w4a16_pair_swap;
     const int pairs = sm_count(device) / 2, steps = (k + 127) / 128;  // what fills up an even number of steps costs next to nothing
@@ -273,7 +308,7 @@ SwapPlan plan_w4a16_pair_swap(int m, int n, int k, int device) {
     SwapPlan best = {0, 2, 1e30};
     for (int columns = wp::MAX_COLUMNS; columns >= 128; columns -= 16) {
         const long long waves = (tiles_n * ((m + columns - 1) / columns) + pairs - 1) / pairs;
-        const double us = 5.2 + waves * columns * (steps * 0.0031 + 0.0137);
+        const double us = 3.0 + waves * columns * (steps * 0.0031 + 0.0137);
         if (us < best.us) best = {columns, 2, us};
     }
     return best;
