@@ -4,6 +4,8 @@ Bars (from the operator's definition): activation codes and scales, unpacked wei
 per-group integer dots bit-exact; fp32 outputs within 1e-3 of max|y|; fp16 stores within
 2 fp16 ulp of the fp32 oracle rounded to fp16."""
 import ctypes
+import pathlib
+import re
 
 import numpy as np
 import pytest
@@ -18,6 +20,7 @@ torch = pytest.importorskip("torch")
 
 OUTPUT_TOLERANCE = 1e-3  # max |y - oracle| / max |oracle|, fp32 accumulate
 FP16_STORE_ULPS = 2
+CSRC = pathlib.Path(entry.__file__).parent / "qwen-image-cplus_b200" / "csrc"
 
 
 @pytest.fixture(scope="module")
@@ -44,6 +47,538 @@ def check_status(qi):
 
 
 # ---- activation quantiser -------------------------------------------------------------------
+
+@pytest.mark.parametrize("m,k", [(1, 256), (3, 512), (77, 768), (128, 3072), (517, 1024), (256, 12288)])
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+def test_quantize_activations_bit_exact(qi, m, k, dtype):
+    rng = np.random.default_rng(1000 + m + k)
+    x16 = qt.make_activations(rng, m, k)
+    x = x16 if dtype == "f16" else (x16.astype(np.float32) + rng.standard_normal((m, k), dtype=np.float32) * 1e-3)
+    codes = torch.zeros(m, k // 2, dtype=torch.uint8, device="cuda")
+    scales = torch.zeros(m, k // 64, dtype=torch.float16, device="cuda")
+    xd = up(x)
+    if dtype == "f32":
+        assert qi.w4a4_quantize_activations(xd, codes, scales, m, k) == 0
+    else:
+        assert qi.w4a4_quantize_activations_ex(xd, qi.DTYPE_F16, codes, scales, m, k) == 0
+    check_status(qi)
+    expected_codes, expected_scales = qo.quantize_activations(x)
+    assert np.array_equal(half_bits(scales), expected_scales)
+    assert np.array_equal(codes.cpu().numpy(), expected_codes)
+
+
+def test_quantize_activations_rounding_ties(qi):
+    # values that sit exactly on, and one fp32 step either side of, every rounding tie
+    # (n + 0.5) * scale, so that the reciprocal shortcut must defer to the exact division
+    rng = np.random.default_rng(77)
+    m, k = 64, 1024
+    # rotating H256(v) gives v back: build the wanted post-rotation values and rotate them
+    target = np.zeros((m, k), dtype=np.float32)
+    for row in range(m):
+        for g in range(k // 64):
+            scale = np.float16(rng.uniform(0.01, 2.0))
+            peak = np.float32(scale) * np.float32(7.0)
+            ties = (rng.integers(-7, 7, size=64).astype(np.float32) + np.float32(0.5)) * np.float32(scale)
+            nudge = rng.integers(-2, 3, size=64)
+            values = ties.copy()
+            for _ in range(2):
+                values = np.where(nudge > 0, np.nextafter(values, np.float32(np.inf)), values)
+                values = np.where(nudge < 0, np.nextafter(values, np.float32(-np.inf)), values)
+                nudge = nudge - np.sign(nudge)
+            values[0] = peak
+            target[row, g * 64:(g + 1) * 64] = values
+    x = qo.hadamard_256(target)
+    codes = torch.zeros(m, k // 2, dtype=torch.uint8, device="cuda")
+    scales = torch.zeros(m, k // 64, dtype=torch.float16, device="cuda")
+    assert qi.w4a4_quantize_activations(up(x), codes, scales, m, k) == 0
+    check_status(qi)
+    expected_codes, expected_scales = qo.quantize_activations(x)
+    assert np.array_equal(half_bits(scales), expected_scales)
+    assert np.array_equal(codes.cpu().numpy(), expected_codes)
+
+
+def test_quantize_activations_zero_and_tiny_rows(qi):
+    m, k = 8, 512
+    x = np.zeros((m, k), dtype=np.float32)
+    x[1, :] = 1e-9
+    x[2, 5] = 1e-7
+    x[3, :] = -3e-8
+    x[4, 0::2] = 65504.0
+    codes = torch.full((m, k // 2), 0xAB, dtype=torch.uint8, device="cuda")
+    scales = torch.zeros(m, k // 64, dtype=torch.float16, device="cuda")
+    assert qi.w4a4_quantize_activations(up(x), codes, scales, m, k) == 0
+    check_status(qi)
+    expected_codes, expected_scales = qo.quantize_activations(x)
+    assert np.array_equal(half_bits(scales), expected_scales)
+    assert np.array_equal(codes.cpu().numpy(), expected_codes)
+    assert np.all(expected_scales[0] == 1)  # the 2^-24 floor (gemm.cu:45)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+def test_quantize_activations_in_each_form(qi, dtype):
+    # one chunk or two a half-warp, CTAs of one, two and eight warps, by the number of chunks: the bytes of the oracle, and of rows
+    # with ties, infinities, NaNs, denormals and the largest values those that any other form gives
+    k = 1024
+    rng = np.random.default_rng(41)
+    most = 8300  # chunks: 33200, past the last that one chunk a half-warp takes
+    x = qt.make_activations(rng, most, k)
+    x = x if dtype == "f16" else x.astype(np.float32) + rng.standard_normal((most, k), dtype=np.float32) * 1e-3
+    expected_codes, expected_scales = qo.quantize_activations(x)
+    special = [(0, 5, np.inf), (1, 300, -np.inf), (2, 700, np.nan), (3, slice(None), 6.1e-5), (4, slice(0, 256), 65504.0), (5, slice(None), 0.0), (6, slice(0, None, 64), 3.5), (7, 1000, np.inf), (7, 1001, -np.inf)]
+    strange = x.copy()
+    for row, columns, value in special:
+        strange[row, columns] = value
+    if dtype == "f32":
+        strange[8, ::3] = 1e-40
+        strange[9, ::5] = 1e30
+    first = None
+    for m in (10, 295, 296, 297, 767, 768, 769, 1791, 1792, 8192, 8193, most):
+        for source, plain in ((x, True), (strange, False)):
+            codes = torch.zeros(m, k // 2, dtype=torch.uint8, device="cuda")
+            scales = torch.zeros(m, k // 64, dtype=torch.float16, device="cuda")
+            wide = torch.zeros(m, k, dtype=torch.uint8, device="cuda")
+            code = qi.DTYPE_F32 if dtype == "f32" else qi.DTYPE_F16
+            assert qi.w4a4_quantize_activations_wide_ex(up(source[:m]), code, codes, scales, wide, m, k) == 0
+            check_status(qi)
+            if plain:
+                assert np.array_equal(half_bits(scales), expected_scales[:m])
+                assert np.array_equal(codes.cpu().numpy(), expected_codes[:m])
+                nibbles = torch.zeros_like(wide)
+                assert qi.w4a4_widen_codes_ex(codes, nibbles, m, k) == 0
+                assert torch.equal(wide, nibbles)
+            else:
+                now = [t[:10].cpu().numpy().copy() for t in (codes, scales.view(torch.int16), wide)]
+                first = now if first is None else first
+                assert all(np.array_equal(a, b) for a, b in zip(first, now)), m
+
+
+def test_quantize_rejects_bad_shapes(qi):
+    x = torch.zeros(4, 320, device="cuda")
+    out = torch.zeros(4096, dtype=torch.uint8, device="cuda")
+    assert qi.w4a4_quantize_activations(x, out, out, 4, 320) == qi.CUDA_ERROR_INVALID_VALUE
+    assert qi.w4a4_quantize_activations(x, out, out, 0, 256) == 0  # empty input: nothing to do
+    assert qi.w4a4_quantize_activations(None, out, out, 4, 256) == qi.CUDA_ERROR_INVALID_VALUE
+
+
+def test_f32_to_f16_bit_exact(qi):
+    rng = np.random.default_rng(3)
+    for count in (1, 7, 8, 4099, 1 << 20):
+        x = np.concatenate([rng.standard_normal(count).astype(np.float32) * np.float32(10.0 ** rng.integers(-8, 5)),
+                            ])[:count]
+        out = torch.zeros(count, dtype=torch.float16, device="cuda")
+        assert qi.f32_to_f16(up(x), out, count) == 0
+        torch.cuda.synchronize()
+        assert np.array_equal(half_bits(out), qo.f32_to_f16(x))
+        on_stream = torch.zeros(count, dtype=torch.float16, device="cuda")
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        assert qi.f32_to_f16_ex(up(x), on_stream, count, stream.cuda_stream) == 0
+        stream.synchronize()
+        assert np.array_equal(half_bits(on_stream), qo.f32_to_f16(x))
+
+
+# ---- W4A16 ---------------------------------------------------------------------------------------
+
+def test_w4a16_dequantize_bit_exact(qi):
+    rng = np.random.default_rng(11)
+    n, k = 384, 1024
+    for source in ("packer", "packer_clip", "random", "wide"):
+        if source.startswith("packer"):
+            codes, scales, minimums = qt.pack_w4a16(qt.make_weights(rng, n, k), clip=source.endswith("clip"))
+        elif source == "random":
+            codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+        else:  # |w| up to 1: the edge of the range where a single rounding equals the reference's two
+            codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+            scales = rng.uniform(0.01, 0.12, size=(n, k // 64)).astype(np.float16).view(np.uint16)
+            minimums = rng.uniform(-0.95, -0.85, size=(n, k // 64)).astype(np.float16).view(np.uint16)
+        out = torch.zeros(n, k, dtype=torch.float16, device="cuda")
+        assert qi.w4a16_dequantize_ex(up(codes), up(scales), up(minimums), out, n, k) == 0
+        torch.cuda.synchronize()
+        expected = qo.w4a16_dequantize(codes, scales, minimums)
+        assert np.abs(expected.astype(np.float32)).max() <= 1.0
+        assert np.array_equal(half_bits(out), expected.view(np.uint16)), source
+
+
+@pytest.mark.parametrize("tile", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("m,n,k", [(128, 128, 64), (256, 256, 512), (384, 640, 1024), (128, 384, 3072)])
+def test_w4a16_gemm_matches_oracle(qi, tile, m, n, k):
+    rng = np.random.default_rng(2000 + m + n + k)
+    codes, scales, minimums = qt.pack_w4a16(qt.make_weights(rng, n, k))
+    x16 = qt.make_activations(rng, m, k)
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemm_tile_ex(up(x16), up(codes), up(scales), up(minimums), None, y, qi.DTYPE_F32, n, m, n, k,
+                                 tile) == 0
+    check_status(qi)
+    expected = qo.w4a16_gemm(x16, codes, scales, minimums)
+    assert qt.max_relative_error(y.cpu().numpy(), expected) <= OUTPUT_TOLERANCE
+
+
+def test_w4a16_gemm_default_tiles_large(qi):
+    # the block shapes' to_q linear at 512x512 image size: m=1024, n=k=3072, checked on sampled rows
+    rng = np.random.default_rng(31)
+    m, n, k = 1024, 3072, 3072
+    codes, scales, minimums = qt.pack_w4a16(qt.make_weights(rng, n, k))
+    x16 = qt.make_activations(rng, m, k)
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemm(up(x16), up(codes), up(scales), up(minimums), y, m, n, k) == 0
+    check_status(qi)
+    got = y.cpu().numpy()
+    assert np.isfinite(got).all()
+    rows = np.sort(rng.choice(m, size=48, replace=False))
+    expected = qo.w4a16_gemm(x16[rows], codes, scales, minimums)
+    assert qt.max_relative_error(got[rows], expected) <= OUTPUT_TOLERANCE
+
+
+def test_w4a16_gemm_ex_bias_fp16_and_leading_dimension(qi):
+    rng = np.random.default_rng(41)
+    m, n, k, ldy = 200, 256, 512, 512  # m is not a multiple of 128: the _ex form takes any m > 8
+    codes, scales, minimums = qt.pack_w4a16(qt.make_weights(rng, n, k))
+    x16, bias = qt.make_activations(rng, m, k), qt.make_bias(rng, n)
+    expected = qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)
+    wide = torch.full((m, ldy), -7.0, dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemm_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), wide[:, 128:], qi.DTYPE_F32, ldy,
+                            m, n, k) == 0
+    check_status(qi)
+    got = wide.cpu().numpy()
+    assert qt.max_relative_error(got[:, 128:128 + n], expected) <= OUTPUT_TOLERANCE
+    assert np.all(got[:, :128] == -7.0) and np.all(got[:, 128 + n:] == -7.0)  # nothing outside the slice
+    y16 = torch.zeros(m, n, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_gemm_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), y16, qi.DTYPE_F16, n, m, n, k) == 0
+    check_status(qi)
+    distance, checked = qt.fp16_store_error(y16.cpu().numpy(), expected)
+    assert distance <= FP16_STORE_ULPS and checked > 0.5
+    assert qt.max_relative_error(y16.cpu().numpy().astype(np.float32), expected) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 32, 64), (16, 160, 192), (17, 4096, 64), (77, 288, 1216), (100, 1024, 3072), (255, 416, 448),
+                                   (257, 96, 1024), (130, 3072, 128), (1, 256, 12288), (8, 480, 4160), (520, 64, 640)])
+def test_w4a16_exchanged_operands_at_the_edges_of_their_tiles(qi, m, n, k):
+    # rows and columns that end inside a tile, an odd number of groups, K split over a cluster and not; few enough rows
+    # (or long enough ones) that the kernel with the weights as first operand takes the shape
+    rng = np.random.default_rng(4000 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x16, bias = qt.make_activations(rng, m, k), qt.make_bias(rng, n)
+    expected = qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        wide = torch.full((m + 1, n + 32), -7.0, dtype=dtype, device="cuda")
+        assert qi.w4a16_gemm_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), wide, code, n + 32, m, n, k) == 0
+        check_status(qi)
+        got = wide.float().cpu().numpy()
+        assert np.all(got[m:] == -7.0) and np.all(got[:, n:] == -7.0)  # nothing outside the matrix
+        assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("m,n,k", [(2048, 2048, 128), (4000, 1504, 192), (3000, 2336, 1216), (9000, 288, 320),
+                                   (3000, 9216, 64), (3000, 2336, 320), (2000, 4128, 640), (4096, 1504, 1088),
+                                   (4096, 3072, 1024), (3300, 1504, 12288)])
+def test_w4a16_exchanged_operands_on_pairs_over_several_tiles(qi, m, n, k):
+    # more 256-row tiles than pairs of CTAs, ragged on both sides, an odd number of groups or of steps (one step past the
+    # end of K), scales read in pairs (K a multiple of 128) and one by one, and more activations than stay in L2, walked in
+    # blocks of eight rows of tiles of which the last is shorter; against the unpacked weights in float64, every output
+    rng = np.random.default_rng(5000 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x, bias = up(qt.make_activations(rng, m, k)), up(qt.make_bias(rng, n))
+    c, s, z = up(codes), up(scales.view(np.float16)), up(minimums.view(np.float16))
+    weights = torch.empty(n, k, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_dequantize_ex(c, s, z, weights, n, k) == 0
+    expected = (x.double() @ weights.double().T + bias.double()).cpu().numpy()
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        wide = torch.full((m + 1, n + 32), -7.0, dtype=dtype, device="cuda")
+        assert qi.w4a16_gemm_ex(x, c, s, z, bias, wide, code, n + 32, m, n, k) == 0
+        check_status(qi)
+        got = wide.float().cpu().numpy()
+        assert np.all(got[m:] == -7.0) and np.all(got[:, n:] == -7.0)  # nothing outside the matrix
+        assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 96, 3072), (77, 12288, 3072), (96, 1024, 6144), (100, 3072, 3072), (200, 9216, 3072), (256, 3072, 12288),
+                                   (384, 1024, 6144), (512, 1536, 12288), (1024, 384, 3072), (1500, 1152, 3072), (300, 1024, 192)])
+def test_w4a16_same_bits_on_every_call(qi, m, n, k):
+    # one accumulator and two, from eight stages of activations down to three, K split over a cluster and not: the order of
+    # the sums is fixed, whatever else runs at the time; and each result is the product of the unpacked weights
+    rng = np.random.default_rng(5500 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x, c, s, z = up(qt.make_activations(rng, m, k)), up(codes), up(scales.view(np.float16)), up(minimums.view(np.float16))
+    weights = torch.empty(n, k, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_dequantize_ex(c, s, z, weights, n, k) == 0
+    results = [torch.full((m, n), float("nan"), device="cuda") for _ in range(8)]
+    for y in results:
+        assert qi.w4a16_gemm_ex(x, c, s, z, None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert all(torch.equal(results[0], y) for y in results[1:])
+    exact = x.double() @ weights.double().T
+    assert float((results[0] - exact).norm() / exact.norm()) <= 1e-4  # 12288 float32 additions: 12288 ** 0.5 * 2 ** -23 = 1.3e-5
+
+
+@pytest.mark.parametrize("m,n,k,steps", [(495, 7456, 5568, 22), (201, 10304, 9920, 39), (783, 4096, 12288, 48)])
+def test_w4a16_gemm_sums_are_as_exact_as_short_chains(qi, m, n, k, steps):
+    # as for the GEMV below: 2^-25 for each MMA of a chain, eight a step of 128 inputs, and 2^-23 for the sums of the chains. These
+    # shapes have tiles of 80 to 112 columns, whose two accumulators take the steps in turn; wider ones have one and all steps in it
+    rng = np.random.default_rng(3015 + m + n + k)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    scales = (rng.uniform(0.9, 1.1, size=(n, k // 64)) * 0.0065).astype(np.float16)
+    minimums = (-7.5 * scales.astype(np.float32)).astype(np.float16)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(1)).half().cuda()
+    nibbles = torch.stack([up(codes) & 15, up(codes) >> 4], -1).reshape(n, k // 64, 64).half().double()
+    weights = (nibbles * up(scales).double()[..., None] + up(minimums).double()[..., None]).half().double().reshape(n, k)
+    exact = x.double() @ weights.T
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemm_ex(x, up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert float((y.double() - exact).norm() / exact.norm()) <= steps * 8 * 2.0 ** -25 + 2.0 ** -23
+
+
+def test_w4a16_unpack_scales_about_its_limit(qi):
+    # the unpack's fast path takes |scale| < 1/32: both sides of it, either sign, and the smallest scales there are
+    n, k = 64, 1024
+    rng = np.random.default_rng(3010)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    edge = np.float16(1 / 32)
+    values = np.array([edge, np.nextafter(edge, np.float16(0)), np.nextafter(edge, np.float16(1)), 1 / 16, 3 / 64, 2.0 ** -24, 2.0 ** -14, 0.0065], dtype=np.float16)
+    scales = (values[rng.integers(0, len(values), size=(n, k // 64))] * rng.choice([-1.0, 1.0], size=(n, k // 64))).astype(np.float16)
+    minimums = rng.uniform(-0.06, 0.06, size=scales.shape).astype(np.float16)
+    nibbles = np.stack([codes & 15, codes >> 4], axis=-1).reshape(n, k // 64, 64).astype(np.float64)
+    expected = (nibbles * scales.astype(np.float64)[:, :, None] + minimums.astype(np.float64)[:, :, None]).astype(np.float16).reshape(n, k)  # one rounding
+    weights = torch.zeros(n, k, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_dequantize_ex(up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), weights, n, k) == 0
+    check_status(qi)
+    assert np.array_equal(weights.cpu().numpy().view(np.uint16), expected.view(np.uint16))
+
+
+def test_w4a16_unpack_of_a_few_larger_scales_costs_little(qi):
+    # a warp that has one scale of 1/32 or more among its 32 rows takes the longer unpack once, not both one after the other:
+    # 13 instructions for 11, with both it would be 24 (5 % and 41 % of this call)
+    m, n, k = 77, 12288, 3072
+    rng = np.random.default_rng(3020)
+    x, y = up(qt.make_activations(rng, m, k)), torch.zeros(m, n, dtype=torch.float16, device="cuda")
+    codes = up(rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8))
+    small = rng.uniform(0.006, 0.007, size=(n, k // 64)).astype(np.float16)
+    mixed = np.where(rng.random(small.shape) < 0.1, np.float16(0.046), small)
+    best = []
+    for scales in (small, mixed):
+        minimums = up((-7.5 * scales.astype(np.float32)).astype(np.float16).view(np.uint16))
+        device = up(scales.view(np.uint16))
+        times = []
+        for _ in range(9):  # the best of them: others may use the machine
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(100):
+                assert qi.w4a16_gemm_ex(x, codes, device, minimums, None, y, qi.DTYPE_F16, n, m, n, k) == 0
+            end.record()
+            check_status(qi)
+            times.append(begin.elapsed_time(end))
+        best.append(min(times))
+    assert best[1] <= 1.2 * best[0], best
+
+
+def test_w4a16_gemm_rejects_what_the_reference_rejects(qi):  # gemm.cu:264
+    t = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
+    assert qi.w4a16_gemm(t, t, t, t, t, 100, 128, 64) == qi.CUDA_ERROR_INVALID_VALUE
+    assert qi.w4a16_gemm(t, t, t, t, t, 128, 120, 64) == qi.CUDA_ERROR_INVALID_VALUE
+    assert qi.w4a16_gemm(t, t, t, t, t, 128, 128, 96) == qi.CUDA_ERROR_INVALID_VALUE
+    assert qi.w4a16_gemm(None, t, t, t, t, 128, 128, 64) == qi.CUDA_ERROR_INVALID_VALUE
+
+
+@pytest.mark.parametrize("m", [1, 2, 8])
+@pytest.mark.parametrize("n,k,kind", [(256, 64, "silu"), (1024, 1216, "silu"), (18432, 3072, "silu"),
+                                      (3072, 12288, "outliers")])
+def test_w4a16_gemv_matches_oracle(qi, m, n, k, kind):
+    rng = np.random.default_rng(3000 + m + n + k)
+    if n * k > (1 << 22):
+        codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    else:
+        codes, scales, minimums = qt.pack_w4a16(qt.make_weights(rng, n, k))
+    x16, bias = qt.make_activations(rng, m, k, kind), qt.make_bias(rng, n)
+    expected = qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), y, qi.DTYPE_F32, n, m, n, k) == 0
+    torch.cuda.synchronize()
+    assert qt.max_relative_error(y.cpu().numpy(), expected) <= OUTPUT_TOLERANCE
+    y16 = torch.zeros(m, n, dtype=torch.float16, device="cuda")
+    assert qi.w4a16_gemm_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), y16, qi.DTYPE_F16, n, m, n, k) == 0
+    torch.cuda.synchronize()
+    distance, _ = qt.fp16_store_error(y16.cpu().numpy(), expected)
+    assert distance <= FP16_STORE_ULPS
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 48, 192), (2, 32, 512), (4, 2400, 1024), (5, 2400, 1088), (1, 21328, 1536), (3, 4784, 2880), (4, 64, 4096)])
+def test_w4a16_gemv_teams_and_steps(qi, m, n, k):
+    # 2, 4, 3 and 6 slices of K, last steps of one to four groups, activation rows that fill the MMA's columns to half and one more
+    rng = np.random.default_rng(3050 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x16, bias = qt.make_activations(rng, m, k, "silu"), qt.make_bias(rng, n)
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(up(x16), up(codes), up(scales), up(minimums), up(bias), y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert qt.max_relative_error(y.cpu().numpy(), qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("m", [1, 2, 8])
+@pytest.mark.parametrize("n,k,chain", [(576, 256, 8), (2400, 512, 8), (9216, 1024, 8), (18432, 1536, 16), (6144, 2048, 24), (3072, 3072, 32), (4096, 4096, 32)])
+def test_w4a16_gemv_sums_are_as_exact_as_short_chains(qi, m, n, k, chain):
+    # An MMA cuts its float32 sum towards zero, on the mean by half a unit of 2^-24 to 2^-23 of it: 2^-25 for each of a chain of
+    # them that only grows, plus what rounding the chains' sums to nearest adds (2^-23)
+    rng = np.random.default_rng(3060 + m + n + k)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    scales = (rng.uniform(0.9, 1.1, size=(n, k // 64)) * 0.0065).astype(np.float16)
+    minimums = (-7.5 * scales.astype(np.float32)).astype(np.float16)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(1)).half().cuda()
+    nibbles = torch.stack([up(codes) & 15, up(codes) >> 4], -1).reshape(n, k // 64, 64).double()
+    weights = (nibbles * up(scales).double()[..., None] + up(minimums).double()[..., None]).half().double().reshape(n, k)
+    exact = x.double() @ weights.T
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(x, up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert float((y.double() - exact).norm() / exact.norm()) <= chain * 2.0 ** -25 + 2.0 ** -23
+
+
+@pytest.mark.parametrize("n,k", [(48, 64), (576, 256), (4784, 512), (2400, 704), (4784, 1024), (2400, 1088), (14224, 1536), (4784, 1984), (2400, 2048),
+                                 (4784, 2560), (14224, 3072), (2400, 3136), (4784, 4096)])
+def test_w4a16_gemv_rows_do_not_depend_on_their_number(qi, n, k):
+    # every kind of teams, with the lower rows' codes where the others end and further on: the bits of a row of activations alone
+    # are those it has among others, and against a few weight rows those against all (many are for teams of three warps, few
+    # for teams of six with the same slices of K)
+    rng = np.random.default_rng(3070 + n + k)
+    codes, scales, minimums = (up(a) for a in qt.random_w4a16_pack(rng, n, k))
+    x, bias = up(qt.make_activations(rng, 8, k, "silu")), up(qt.make_bias(rng, n))
+    results = []
+    for m in range(1, 9):
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        assert qi.w4a16_gemv_ex(x, codes, scales, minimums, bias, y, qi.DTYPE_F32, n, m, n, k) == 0
+        results.append(y)
+    check_status(qi)
+    for m, y in enumerate(results, 1):
+        assert torch.equal(y, results[-1][:m]), m
+    alone = torch.full((1, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(x[5:], codes, scales, minimums, bias, alone, qi.DTYPE_F32, n, 1, n, k) == 0
+    check_status(qi)
+    assert torch.equal(alone[0], results[-1][5])
+    few = torch.full((8, 48), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(x, codes[:48], scales[:48], minimums[:48], bias[:48], few, qi.DTYPE_F32, 48, 8, 48, k) == 0
+    check_status(qi)
+    assert torch.equal(few, results[-1][:, :48])
+
+
+@pytest.mark.parametrize("m", [1, 3])
+def test_w4a16_gemv_scales_of_every_size(qi, m):
+    # scales from fp16 denormals up to 4: the GEMV's unpack treats scale >= 1/16 (where scale * 2^20 leaves fp16)
+    # and denormal scales on paths of their own; every one must give the reference's weights
+    n, k = 512, 1024
+    rng = np.random.default_rng(3100 + m)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    exponents = rng.integers(-20, 3, size=(n, k // 64)).astype(np.float32)
+    scales = (np.exp2(exponents) * rng.uniform(1.0, 2.0, size=exponents.shape)).astype(np.float16)
+    scales[::7, ::3] = np.float16(0.0)
+    minimums = (-7.5 * scales.astype(np.float32)).astype(np.float16)
+    x16 = qt.make_activations(rng, m, k, "silu")
+    expected = qo.w4a16_gemm(x16, codes, scales.view(np.uint16), minimums.view(np.uint16))
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(up(x16), up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), None, y,
+                            qi.DTYPE_F32, n, m, n, k) == 0
+    torch.cuda.synchronize()
+    assert qt.max_relative_error(y.cpu().numpy(), expected) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("low,high", [(2.0 ** -9, 1 / 64 - 2.0 ** -16), (1 / 64, 1 / 4 - 2.0 ** -12), (1 / 4, 1.0)])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 64), (8, 48, 4096), (5, 2384, 1216)])
+def test_w4a16_gemv_scales_of_one_range(qi, m, n, k, low, high):
+    # all scales of a matrix in one of the three ranges that the unpack tells apart, both ends of each included
+    rng = np.random.default_rng(3150 + m + n + k)
+    codes = rng.integers(0, 256, size=(n, k // 2), dtype=np.uint8)
+    scales = rng.uniform(low, high, size=(n, k // 64)).astype(np.float16)
+    scales[0, 0], scales[-1, -1] = np.float16(low), np.float16(-high)
+    minimums = (-7.5 * scales.astype(np.float32)).astype(np.float16)
+    x16 = qt.make_activations(rng, m, k)
+    expected = qo.w4a16_gemm(x16, codes, scales.view(np.uint16), minimums.view(np.uint16))
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    assert qi.w4a16_gemv_ex(up(x16), up(codes), up(scales.view(np.uint16)), up(minimums.view(np.uint16)), None, y, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    assert qt.max_relative_error(y.cpu().numpy(), expected) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("m", [1, 8])
+@pytest.mark.parametrize("n,k,scale_offset,output_offset", [(48, 4160, 0, 0), (16, 12288, 0, 0), (80, 3072, 1, 0), (96, 4160, 0, 1), (64, 12288, 1, 3), (48, 64, 1, 1)])
+def test_w4a16_gemv_without_what_the_other_kernels_need(qi, m, n, k, scale_offset, output_offset):
+    # long rows of which there is no multiple of 32, or an output that starts or steps off 16 bytes; scales off 16 bytes with
+    # rows the streaming kernel would take: the kernel that reads weights and scales from global memory one by one
+    rng = np.random.default_rng(3170 + m + n + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+    x16, bias = qt.make_activations(rng, m, k), qt.make_bias(rng, n)
+    expected = qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)
+    shifted = []
+    for values in (scales, minimums):
+        room = torch.zeros(n * (k // 64) + 8, dtype=torch.float16, device="cuda")
+        shifted.append(room[scale_offset:scale_offset + n * (k // 64)].copy_(up(values.view(np.float16)).flatten()))
+    ldy = n + output_offset
+    for dtype, code in ((torch.float32, qi.DTYPE_F32), (torch.float16, qi.DTYPE_F16)):
+        room = torch.full((output_offset + (m + 1) * ldy,), -7.0, dtype=dtype, device="cuda")
+        y = room[output_offset:].view(m + 1, ldy)
+        assert qi.w4a16_gemv_ex(up(x16), up(codes), *shifted, up(bias), y, code, ldy, m, n, k) == 0
+        check_status(qi)
+        got = y.float().cpu().numpy()
+        assert np.all(got[m:] == -7.0) and np.all(got[:, n:] == -7.0)
+        assert qt.max_relative_error(got[:m, :n], expected) <= OUTPUT_TOLERANCE
+
+
+@pytest.mark.parametrize("m,count,n,k", [(1, 3, 1024, 1216), (1, 70, 256, 512), (2, 5, 18432, 3072)])
+def test_w4a16_gemv_grouped_matches_oracle_and_the_single_launches(qi, m, count, n, k):
+    """Several matrices of one shape against the same activations in one launch (two for more than 64 matrices): every
+    output equals the oracle's within the tolerance and the single-matrix GEMV's bit for bit."""
+    rng = np.random.default_rng(3200 + m + count + n + k)
+    x16 = qt.make_activations(rng, m, k, "silu")
+    x = up(x16)
+    entries, singles, expected = [], [], []
+    for index in range(count):
+        codes, scales, minimums = qt.random_w4a16_pack(rng, n, k)
+        bias = qt.make_bias(rng, n) if index % 2 == 0 else None
+        device = (up(codes), up(scales), up(minimums), up(bias) if bias is not None else None,
+                  torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda"))
+        entries.append(device)
+        single = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        assert qi.w4a16_gemv_ex(x, device[0], device[1], device[2], device[3], single, qi.DTYPE_F32, n, m, n, k) == 0
+        singles.append(single)
+        if index < 4 or index == count - 1:  # the oracle on a few of them; the single launches cover the rest
+            expected.append((index, qo.w4a16_gemm(x16, codes, scales, minimums, bias=bias)))
+    table, keep = qi.gemv_items(entries)
+    assert qi.w4a16_gemv_grouped_ex(x, table, qi.DTYPE_F32, n, m, n, k) == 0
+    torch.cuda.synchronize()
+    check_status(qi)
+    for index, (entry, single) in enumerate(zip(entries, singles)):
+        assert torch.equal(entry[4], single), index
+    for index, want in expected:
+        assert qt.max_relative_error(entries[index][4].cpu().numpy(), want) <= OUTPUT_TOLERANCE
+    # refused: no items, a misaligned region, rows too long for the streaming kernel
+    assert qi.lib().qi_w4a16_gemv_grouped_ex(qi._p(x), table, 0, qi.DTYPE_F32, n, m, n, k, None) == qi.CUDA_ERROR_INVALID_VALUE
+    bad, _ = qi.gemv_items([(entries[0][0].view(-1)[1:], entries[0][1], entries[0][2], None, entries[0][4])])
+    assert qi.w4a16_gemv_grouped_ex(x, bad, qi.DTYPE_F32, n, m, n, k) == qi.CUDA_ERROR_INVALID_VALUE
+    assert qi.w4a16_gemv_grouped_ex(x, table, qi.DTYPE_F32, n, m, n, 8192) == qi.CUDA_ERROR_INVALID_VALUE
+
+
+@pytest.mark.parametrize("m,k", [(1, 256), (3, 512), (1, 1024), (1, 1088), (1, 3072), (2, 3072), (8, 3072), (1, 4096), (8, 4096)])
+def test_w4a16_gemv_rings_go_round(qi, m, k):
+    # each kind of teams with tiles for every stage of a CTA's ring twice and more, where the number of stages is a multiple of
+    # the teams' number and where it is not: stages are handed back, fetched into again and waited for in either phase
+    n, count = 1200, 64
+    most_stages = int(re.search(r"STREAM_MAX_STAGES = (\d+)", (CSRC / "w4a16_gemv_stream.cuh").read_text()).group(1))
+    assert count * (n // 16) > 2 * most_stages * torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(3250 + m + k)
+    codes, scales, minimums = qt.random_w4a16_pack(rng, count * n, k)
+    x16, bias = qt.make_activations(rng, m, k, "silu"), qt.make_bias(rng, count * n)
+    x, device = up(x16), [up(a) for a in (codes, scales, minimums, bias)]
+    y = torch.full((count, m, n), float("nan"), dtype=torch.float32, device="cuda")
+    items = [tuple(a[i * n:(i + 1) * n] for a in device) + (y[i],) for i in range(count)]
+    table, keep = qi.gemv_items(items)
+    assert qi.w4a16_gemv_grouped_ex(x, table, qi.DTYPE_F32, n, m, n, k) == 0
+    check_status(qi)
+    for i, item in enumerate(items):  # 75 tiles alone: no stage is used twice
+        single = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        assert qi.w4a16_gemv_ex(x, *item[:4], single, qi.DTYPE_F32, n, m, n, k) == 0
+        assert torch.equal(y[i], single), i
+    check_status(qi)
+    for i in (0, count // 2, count - 1):
+        of = slice(i * n, (i + 1) * n)
+        assert qt.max_relative_error(y[i].cpu().numpy(), qo.w4a16_gemm(x16, codes[of], scales[of], minimums[of], bias=bias[of])) <= OUTPUT_TOLERANCE
+
 
 # ---- W4A4 ----------------------------------------------------------------------------------------
 
