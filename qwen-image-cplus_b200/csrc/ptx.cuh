@@ -192,6 +192,15 @@ inline cudaError_t launch_overlapped(void (*kernel)(Parameters...), unsigned gri
     config.numAttrs = 1;
     return launched(cudaLaunchKernelEx(&config, kernel, static_cast<Parameters>(arguments)...));
 }
+// Kernels that take TMEM do so before grid_wait(), and a tcgen05.alloc waits for whatever holds it on that SM, also a kernel of
+// another stream that is in grid_wait() itself. Two things keep such waits from going round in a ring:
+//   * A kernel with TMEM calls grid_release() only once its CTA has that, or not at all. So when a later kernel of its stream
+//     starts, all its CTAs have theirs, and what waits for it in grid_wait() waits for something that can end.
+//   * No two CTAs that wait for others of their clusters share an SM: each takes at least ONE_CTA_SMEM of shared memory (two, with
+//     the system's 1 KB each, are more than the 228 KB of an SM). Else one that holds TMEM could wait for a CTA that waits for
+//     TMEM beside a CTA of another cluster, and that one for a CTA behind the first.
+constexpr int ONE_CTA_SMEM = 116 * 1024;
+static_assert(2 * (ONE_CTA_SMEM + 1024) > 228 * 1024, "at most one such CTA on an SM");
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- TMA ---------------------------------------------------------------------------------

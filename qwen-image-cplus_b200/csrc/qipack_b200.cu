@@ -189,7 +189,7 @@ int resident_clusters(int device, int split) {
     if (count == 0) {
         cudaLaunchConfig_t config;
         cudaLaunchAttribute attributes[2];
-        swap_config(config, attributes, split, split, 116 * 1024, nullptr);
+        swap_config(config, attributes, split, split, ONE_CTA_SMEM, nullptr);
         config.attrs = attributes + 1, config.numAttrs = 1;
         if (configure_swap<true>(device) != cudaSuccess || cudaOccupancyMaxActiveClusters(&count, ws::gemm_kernel<true>, &config) != cudaSuccess || count <= 0) {
             (void)cudaGetLastError();

@@ -41,7 +41,7 @@ constexpr int BARRIER_BYTES = 512;
 template <int STAGES>
 struct Tile {
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CODE_STAGES * C_BYTES + BARRIER_BYTES + 1024;
-    static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA");
+    static_assert(SMEM_BYTES <= 232448 && SMEM_BYTES >= ONE_CTA_SMEM, "shared memory budget of one CTA; one per SM: see grid_release()");
     static_assert(STAGES >= CODE_BLOCKS, "a chunk's K blocks wrap around the stages at most once");
     static_assert((3 * STAGES + 2 * CODE_STAGES + 2 * ACC_STAGES) * 8 + 8 <= BARRIER_BYTES, "barrier block");
 };

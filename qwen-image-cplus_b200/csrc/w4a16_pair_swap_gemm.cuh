@@ -39,7 +39,7 @@ static_assert(CODE_STAGES == 2 || CODE_STAGES >= 4, "a group reads every second 
 static_assert(STAGES >= A_SLOTS, "a stage's release stands for that of the slot of the step four before");
 constexpr int BARRIER_BYTES = 256;
 constexpr int SMEM_BYTES = STAGES * X_BYTES + CODE_STAGES * CODE_BYTES + BARRIER_BYTES + 1024;
-static_assert(SMEM_BYTES <= 232448 && SMEM_BYTES > 116 * 1024, "one CTA per SM");
+static_assert(SMEM_BYTES <= 232448 && SMEM_BYTES >= ONE_CTA_SMEM, "one CTA per SM: see grid_release()");
 static_assert((2 * STAGES + 2 * CODE_STAGES + A_SLOTS + 2) * 8 + 4 <= BARRIER_BYTES, "barrier block");
 constexpr uint32_t AHEAD_BACKOFF_NS = 100, UNPACK_BACKOFF_NS = 20;
 

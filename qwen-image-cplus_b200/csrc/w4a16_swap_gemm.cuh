@@ -75,9 +75,9 @@ __host__ __device__ constexpr SmemPlan smem_plan(int columns) {
     int stages = (room - code_stages * CODE_BYTES) / stage_bytes(columns);
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     if (issuers_of(columns) == 2) stages = stages / 2 * 2;
-    // One CTA per SM, always: it takes all of TMEM, and a second would wait for it while its cluster waits for the second.
+    // One CTA per SM, always: it takes all of TMEM, and a second would wait for it while its cluster waits for the second (grid_release()).
     const int bytes = smem_bytes(columns, stages, code_stages);
-    return {stages, code_stages, bytes < 116 * 1024 ? 116 * 1024 : bytes};
+    return {stages, code_stages, bytes < ONE_CTA_SMEM ? ONE_CTA_SMEM : bytes};
 }
 constexpr bool smem_plans_are_sound() {
     for (int columns = 16; columns <= MAX_COLUMNS; columns += 16) {
@@ -186,7 +186,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     }
     if (warp == PRODUCER_WARP && elect_one()) prefetch_tensormap(&map_x);
     if (warp == CODE_WARP && elect_one()) prefetch_tensormap(&map_codes);
-    // TMEM too before the wait: whatever holds it on this SM is an earlier kernel's, which waits for nothing here.
+    // TMEM too before the wait. Whatever holds it on this SM can end without this kernel: see grid_release().
     if (warp == MMA_WARP) {
         tmem_alloc(tmem_slot, TMEM_COLUMNS);
         tmem_relinquish();

@@ -44,7 +44,7 @@ struct Tile {
     static constexpr int BUFFER_COLUMNS = STAGE_GROUPS * BN, TMEM_COLUMNS = BUFFERS * BUFFER_COLUMNS > 256 ? 512 : 256;
     static constexpr int BARRIER_BYTES = 256;
     static constexpr int SMEM_BYTES = STAGES * (A_BYTES + B_BYTES) + SLOTS * SW_BYTES + BARRIER_BYTES + 1024;
-    static_assert(SMEM_BYTES <= 232448 && SMEM_BYTES > 116 * 1024, "one CTA per SM: a second would wait for TMEM");
+    static_assert(SMEM_BYTES <= 232448 && SMEM_BYTES >= ONE_CTA_SMEM, "one CTA per SM: a second would wait for TMEM");
     static_assert(BUFFERS * BUFFER_COLUMNS <= TMEM_COLUMNS, "TMEM allocation size");
     static_assert((2 * STAGES + 2 * SLOTS + 2 * BUFFERS) * 8 + 4 <= BARRIER_BYTES, "barrier block");
 };

@@ -157,7 +157,7 @@ constexpr int SA_BYTES = BM * 16;                 // float4 [row] = the stage's 
 constexpr int RING_BYTES = SCALE_RING * (BN + BM) * 8;  // four fp16 per column / row and slot
 constexpr int BARRIER_BYTES = 512;
 constexpr int SMEM_BYTES = STAGES * (A_BYTES + B_BYTES + SW_BYTES + SA_BYTES) + RING_BYTES + BARRIER_BYTES + 1024;
-static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA");
+static_assert(SMEM_BYTES <= 232448 && SMEM_BYTES >= ONE_CTA_SMEM, "shared memory budget of one CTA; one per SM: see grid_release()");
 static_assert((3 * STAGES + 2 * TEAMS * BUFFERS) * 8 + 8 <= BARRIER_BYTES, "barrier block");
 constexpr int B_BOX_ROWS = TEAM_COLUMNS / 2;  // rows of B per TMA load: one CTA's half of one team's columns
 static_assert(BN == 128 && BM == 128, "the staging warp handles four columns and four rows per lane");

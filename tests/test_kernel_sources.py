@@ -33,6 +33,24 @@ def test_the_rule_reaches_the_hand_overs():
     assert arrivals >= 15
 
 
+def test_tmem_is_taken_before_the_next_kernel_may_start():
+    # else a CTA could wait for TMEM that a later kernel's CTA holds, which waits for this one's kernel to end; and no two CTAs
+    # that wait for others of their clusters may share an SM (both conditions: beside grid_release)
+    kernels = clusters = 0
+    for path in KERNELS:
+        source = "\n".join(line for _, line in statements(path))
+        for kernel in re.split(r"__global__", source)[1:]:
+            taken = kernel.find("tmem_alloc")
+            if taken < 0 or "grid_wait()" not in kernel:
+                continue
+            kernels += 1
+            assert "grid_release()" not in kernel[:taken], os.path.basename(path)
+            if "cluster_sync()" in kernel:
+                clusters += 1
+                assert "ONE_CTA_SMEM" in source, os.path.basename(path)
+    assert kernels >= 9 and clusters == 4
+
+
 def test_every_source_makes_the_library_stale():
     # a kernel file that is not on the list could be edited without the library being built again
     assert sorted(entry.load_package().SOURCES) == sorted(os.listdir(os.path.join(entry.PACKAGE_DIR, "csrc")))
