@@ -850,6 +850,14 @@ int qi_w4a4_quantize_activations_wide_ex(const void *x, int x_dtype, void *codes
                                                         static_cast<cudaStream_t>(stream)));
 }
 
+int qi_w4a4_quantize_plan(int m, int k, int sms, int *plan) {
+    if (m <= 0 || k <= 0 || k % 256 != 0 || sms < 2 || plan == nullptr) return INVALID;
+    const QuantizePlan chosen = plan_quantize(m, k, sms);
+    plan[0] = chosen.threads;
+    plan[1] = chosen.smem_bytes;
+    return 0;
+}
+
 static int fused_quantize(int producer, const float *first, const float *second, void *codes, void *scales, void *bytes,
                           int m, int k, void *stream) {
     if (m < 0 || k <= 0 || k % 256 != 0) return INVALID;

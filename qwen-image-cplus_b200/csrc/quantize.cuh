@@ -20,11 +20,12 @@
 // rounding; a lane whose quotient lies within 2^-16 of a rounding tie redoes it with the
 // IEEE division the reference uses, so the codes are identical.
 //
-// A half-warp takes TWO chunks and keeps value i of both in one 64-bit register, so that the butterflies, the rounding
-// and its check are packed fp32 pair instructions (add / sub / fma .f32x2: the same IEEE results, half the issue
-// slots), moves the pairs through the transposes with 8- and 16-byte accesses, checks for rounding ties once per
-// thread instead of once per value, and emits only the code formats asked for. One chunk per half-warp and scalar
-// arithmetic took 34 instructions per value instead of 19 and was bound by that.
+// Two forms, by the number of chunks (plan_quantize, GELU_CHUNKS). In the paired one a half-warp takes TWO chunks and keeps value i
+// of both in one 64-bit register, so that the butterflies, the rounding and its check are packed fp32 pair instructions
+// (add / sub / fma .f32x2: the same IEEE results, half the issue slots), moves the pairs through the transposes with 8- and
+// 16-byte accesses, checks for rounding ties once per thread instead of once per value, and emits only the code formats asked
+// for: 19 instructions per value, where one chunk a half-warp with scalar arithmetic takes 34. That other form is done sooner
+// where the chunks fill no more than a few rounds of the SMs, so that a chunk's own chain of steps counts and not the instructions.
 #pragma once
 #include <cuda_fp8.h>
 
@@ -285,12 +286,13 @@ quantize_pairs_kernel(const Source source, uint8_t *__restrict__ codes, __half *
     }
 }
 
-// ---- one chunk per half-warp: SwiGLU, and GELU and plain activations of fewer rows ---------------------------------------------------------------
+// ---- one chunk per half-warp: SwiGLU, and GELU and plain activations of fewer rows -------------------------------------
 // The two loads and the division of silu(gate) * up want warps rather than registers: with 40 registers a thread this
 // form takes 28.8 us at 1024 x 12288, the paired one 42.8 (32.1 without loads ahead).
 
 constexpr int PITCH = 20;                  // floats per transposed row: 128-bit reads stay conflict-free
 constexpr int REGION = 16 * PITCH + 16;    // second half-warp lands 16 banks away from the first
+constexpr int CHUNK_WARP_BYTES = 2 * REGION * 4, CHUNK_CTA_BYTES = QUANT_THREADS / 32 * CHUNK_WARP_BYTES;
 constexpr int MAGIC_BITS = 0x4B400000;
 
 __device__ __forceinline__ void load16(const float *source, float (&v)[16]) {
@@ -353,7 +355,7 @@ template <typename Source, bool WIDE>
 __global__ void __launch_bounds__(QUANT_THREADS)
 quantize_chunks_kernel(const Source source, uint8_t *__restrict__ codes, __half *__restrict__ scales,
                             uint8_t *__restrict__ bytes, long long chunks) {
-    __shared__ __align__(16) float transpose[(QUANT_THREADS / 32) * 2 * REGION];
+    extern __shared__ __align__(16) float transpose[];  // CHUNK_WARP_BYTES a warp; a CTA may be given more (plan_quantize)
     grid_wait();
     grid_release();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -460,12 +462,17 @@ __global__ void f32_to_f16_kernel(const float *__restrict__ source, __half *__re
 
 }  // namespace
 
+inline int quantize_sms() {
+    int device = 0, sms = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return sms;
+}
+
 template <typename Source>
 inline cudaError_t launch_quantize_pairs(const Source &source, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream) {
     const long long chunks = static_cast<long long>(m) * (k / 256), pairs = (chunks + 1) / 2;
     if (chunks == 0) return cudaSuccess;
-    int device = 0, sms = 148;
-    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int sms = quantize_sms();
     // Two CTAs of 256 threads stay resident per SM and walk over the pairs of chunks, a half-warp at a time. Fewer pairs than
     // that are spread over more and smaller CTAs: 300 x 4096 are 2400 pairs, 150 CTAs of 256 threads or 592 of 64.
     const int threads = pairs >= static_cast<long long>(sms) * (QUANT_THREADS / 16) ? QUANT_THREADS : 64;
@@ -481,38 +488,60 @@ inline cudaError_t launch_quantize_pairs(const Source &source, void *codes, void
 }
 
 template <typename Source>
-inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream, int threads = QUANT_THREADS) {
+inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream,
+                                          int threads = QUANT_THREADS, int smem_bytes = CHUNK_CTA_BYTES) {
     const long long chunks = static_cast<long long>(m) * (k / 256), blocks = (chunks + threads / 16 - 1) / (threads / 16);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
     return launch_overlapped(bytes != nullptr ? quantize_chunks_kernel<Source, true> : quantize_chunks_kernel<Source, false>, static_cast<unsigned>(blocks), threads,
-                             0, stream, source, static_cast<uint8_t *>(codes), static_cast<__half *>(scales), static_cast<uint8_t *>(bytes), chunks);
+                             smem_bytes, stream, source, static_cast<uint8_t *>(codes), static_cast<__half *>(scales), static_cast<uint8_t *>(bytes), chunks);
 }
 
-// Plain activations take the one-chunk form where it is the faster one, alone and in front of a GEMM. Its CTAs of one or two warps of 40 to 48 registers leave room on an SM for the
-// CTA of the narrow GEMM behind it (640 threads of 96), which is then set up when the last of them ends; the paired form's (64
-// threads of 128) did not. Microseconds of the linear, paired and so: 77 x 9216 x 3072 (924 chunks) 14.7 and 13.0, 50 x 12288 x 4096 (800)
-// 24.8 and 22.7, 170 x 3072 x 3072 (2040, two warps) 12.6 and 11.6; two warps at 300 x 4096 x 4096 (4800) lose, 23.8 and 25.7, and CTAs of eight at 384 x 3072 x
-// 3072 (4608), 16.6 and 17.6, while others gain: such calls keep the paired form (as do 520 x 3072 x 3072, 21.9 and 22.6 with eight). From 7168 chunks on eight warps are best: 600 x 2336 x 3072
-// 20.4 and 19.4, 1024 x 9216 x 3072 62.7 and 61.7, the quantiser alone 1024 x 4096 7.4 and 6.2, 2048 x 3072 10.1 and 8.7, 3000 x 3072 (36000) 12.5 and 12.0, 4096 x 3072 15.9 and 16.0.
-constexpr long long ONE_WARP_CHUNKS = 1184, TWO_WARP_CHUNKS = 3072, CHUNKS_FROM = 7168, CHUNKS_TO = 32768;
+// Plain activations: CTAs of one, two or eight warps with a chunk a half-warp (threads), or the paired form (0).
+// The limits are chunks per SM. Microseconds of a linear on 148 SMs, the paired form first:
+//   to 8, one warp: 77 x 9216 x 3072 (924 chunks) 13.7 and 12.4, 50 x 12288 x 4096 (800) 23.5 and 22.4. 130 shapes: 0.90 of the
+//     time in the mean, one more than 1.01
+//   to 21, two warps: 170 x 3072 x 3072 (2040) 12.3 and 11.4; 130 shapes to 14: 0.93, one more than 1.01
+//   from 48 to 222, eight warps: 600 x 3072 x 3072 (7200) 21.1 and 19.8, 1024 x 3072 x 3072 (12288) 29.8 and 28.6, 2048 x 9216 x 3072
+//     (24576) 120 and 118. From 222 on the two differ by less than they vary (3072 x 3072 x 3072 (36864) 65.2 and 64.5, 4096 x
+//     9216 x 3072 (49152) 226.9 and 228.6), although alone the one-chunk form is ahead up to 330 (36864: 12.1 and 11.5)
+// Between 21 and 48, and above, the paired form stays: 300 x 12288 x 4096 (4800) 54.8, in two warps 60.9.
+// A CTA of one or two warps is given as much shared memory as one of eight. With what it uses (2.7 KB a warp) it is slower in front of
+// a GEMM whose CTAs take up most SMs: 50 x 9216 x 3072 11.3 us and then 12.6, 77 x 9216 x 3072 12.4 and 14.1, 170 x 3072 x 3072 11.4 and
+// 13.4; alone and in front of fewer CTAs it is the same. It isn't the split of an SM's memory into L1 and shared memory (asking the
+// launch for the most shared memory changed nothing); presumably it is where they stand: two of them fit beside a CTA of the GEMM
+// before, for whose end they wait, and else fifteen, so that some SMs have many to do.
+struct QuantizePlan {
+    int threads, smem_bytes;
+};
+constexpr int ONE_WARP_TO = 8, TWO_WARPS_TO = 21, EIGHT_WARPS_FROM = 48, EIGHT_WARPS_TO = 222;
+
+inline QuantizePlan plan_quantize(int m, int k, int sms) {
+    const long long chunks = static_cast<long long>(m) * (k / 256), per_sm = (chunks + sms - 1) / sms;
+    if (per_sm <= ONE_WARP_TO) return {32, CHUNK_CTA_BYTES};
+    if (per_sm <= TWO_WARPS_TO) return {64, CHUNK_CTA_BYTES};
+    if (per_sm <= EIGHT_WARPS_FROM || per_sm > EIGHT_WARPS_TO) return {0, 0};
+    return {QUANT_THREADS, CHUNK_CTA_BYTES};
+}
+
+template <typename T>
+inline cudaError_t launch_quantize_plain(const QuantizePlan &plan, const void *x, void *codes, void *scales, void *bytes, int m, int k, cudaStream_t stream) {
+    const T *source = static_cast<const T *>(x);
+    if (plan.threads == 0) return launch_quantize_pairs(PlainSource<T>{source}, codes, scales, bytes, m, k, stream);
+    return launch_quantize_chunks(PlainChunkSource<T>{source}, codes, scales, bytes, m, k, stream, plan.threads, plan.smem_bytes);
+}
 
 inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, void *codes, void *scales, void *bytes,
                                                int m, int k, cudaStream_t stream) {
-    const long long chunks = static_cast<long long>(m) * (k / 256);
-    if (chunks > 0 && (chunks <= TWO_WARP_CHUNKS || (chunks >= CHUNKS_FROM && chunks <= CHUNKS_TO))) {
-        const int threads = chunks <= ONE_WARP_CHUNKS ? 32 : chunks <= TWO_WARP_CHUNKS ? 64 : QUANT_THREADS;
-        if (x_is_half) return launch_quantize_chunks(PlainChunkSource<__half>{static_cast<const __half *>(x)}, codes, scales, bytes, m, k, stream, threads);
-        return launch_quantize_chunks(PlainChunkSource<float>{static_cast<const float *>(x)}, codes, scales, bytes, m, k, stream, threads);
-    }
-    if (x_is_half) return launch_quantize_pairs(PlainSource<__half>{static_cast<const __half *>(x)}, codes, scales, bytes, m, k, stream);
-    return launch_quantize_pairs(PlainSource<float>{static_cast<const float *>(x)}, codes, scales, bytes, m, k, stream);
+    if (m == 0) return cudaSuccess;
+    const QuantizePlan plan = plan_quantize(m, k, quantize_sms());
+    if (x_is_half) return launch_quantize_plain<__half>(plan, x, codes, scales, bytes, m, k, stream);
+    return launch_quantize_plain<float>(plan, x, codes, scales, bytes, m, k, stream);
 }
 
 // GELU takes the one-chunk form up to so many chunks: it fills the SMs with more and shorter threads, the paired form needs
 // many rounds to be ahead. Measured, one chunk and paired, both code forms: 77 x 12288 4.0 and 5.5 us, 1024 x 3072 7.8 and 10.6,
 // 1024 x 12288 23.5 and 23.8, 2048 x 12288 44.1 and 42.3, 4096 x 12288 85.1 and 80.2.
 constexpr long long GELU_CHUNKS = 49152;
-
 
 // producer: 1 = SwiGLU of (first, second), 2 = GELU-tanh of first
 inline cudaError_t launch_fused_quantize(int producer, const float *first, const float *second, void *codes, void *scales,

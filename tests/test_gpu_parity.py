@@ -152,6 +152,23 @@ def test_quantize_activations_in_each_form(qi, dtype):
                 assert all(np.array_equal(a, b) for a, b in zip(first, now)), m
 
 
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+def test_quantize_activations_at_the_limits_of_its_forms(qi, dtype):
+    # the last chunk count of a form and the first of the next (148 SMs), in rows of one chunk
+    rng = np.random.default_rng(43)
+    limits = [limit * 148 for limit in (8, 21, 48, 222)]
+    x = qt.make_activations(rng, limits[-1] + 1, 256)
+    x = x if dtype == "f16" else x.astype(np.float32)
+    expected_codes, expected_scales = qo.quantize_activations(x)
+    source = up(x)
+    for m in (edge for limit in limits for edge in (limit, limit + 1)):
+        codes, scales = torch.zeros(m, 128, dtype=torch.uint8, device="cuda"), torch.zeros(m, 4, dtype=torch.float16, device="cuda")
+        assert qi.w4a4_quantize_activations_ex(source, qi.DTYPE_F32 if dtype == "f32" else qi.DTYPE_F16, codes, scales, m, 256) == 0
+        check_status(qi)
+        assert np.array_equal(half_bits(scales), expected_scales[:m])
+        assert np.array_equal(codes.cpu().numpy(), expected_codes[:m])
+
+
 def test_quantize_rejects_bad_shapes(qi):
     x = torch.zeros(4, 320, device="cuda")
     out = torch.zeros(4096, dtype=torch.uint8, device="cuda")
