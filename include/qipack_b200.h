@@ -194,9 +194,10 @@ int qi_w4a4_swiglu_quantize_ex(const float *gate, const float *up, void *codes, 
                                void *stream);
 int qi_w4a4_gelu_quantize_ex(const float *x, void *codes, void *scales, void *bytes, int m, int k, void *stream);
 
-/* Host only: how the plain quantisers take an [m, k] matrix on a GPU with `sms` multiprocessors. plan[0]: threads of a CTA whose
- * half-warps take a 256-chunk each, 0 = the form that takes two; plan[1]: bytes of shared memory it is given. For tests and tuning. */
-int qi_w4a4_quantize_plan(int m, int k, int sms, int *plan);
+/* Host only: how the plain quantisers take an [m, k] matrix on a GPU with `sms` multiprocessors, in qi_linear in front of a byte-operand
+ * GEMM of n outputs (n = 0: called by themselves). plan[0]: threads of a CTA whose half-warps take a 256-chunk each, 0 = the form
+ * that takes two; plan[1]: bytes of shared memory it is given. For tests and tuning. */
+int qi_w4a4_quantize_plan(int m, int k, int n, int sms, int *plan);
 
 /* As qi_w4a4_gemm_ex on byte operands a_bytes [m, k], w_bytes [n, k]; k % 128 == 0. */
 int qi_w4a4_gemm_wide_ex(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales,

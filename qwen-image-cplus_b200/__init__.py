@@ -147,7 +147,7 @@ SIGNATURES = {
     "qi_w4a16_gemm_tile_ex": [_P, _P, _P, _P, _P, _P, _I, _LL, _I, _I, _I, _I, _P],
     "qi_w4a4_gemm_wide_single_ex": [_P, _P, _P, _P, _P, _P, _I, _LL, _P, _I, _I, _I, _P],
     "qi_w4a4_gemm_plan": [_I, _I, _I, _I, ctypes.POINTER(_I)],
-    "qi_w4a4_quantize_plan": [_I, _I, _I, ctypes.POINTER(_I)],
+    "qi_w4a4_quantize_plan": [_I, _I, _I, _I, ctypes.POINTER(_I)],
 }
 
 _lib = None
@@ -356,10 +356,10 @@ def w4a4_gemm_plan(m: int, n: int, k: int, sms: int = 148) -> W4A4Plan:
 QuantizePlan = collections.namedtuple("QuantizePlan", "threads smem_bytes")  # of a CTA with a chunk a half-warp; threads 0: the paired form
 
 
-def w4a4_quantize_plan(m: int, k: int, sms: int = 148) -> QuantizePlan:
-    """Which form the plain activation quantisers take. Needs no GPU."""
+def w4a4_quantize_plan(m: int, k: int, sms: int = 148, n: int = 0) -> QuantizePlan:
+    """Which form the plain activation quantisers take, in front of a byte-operand GEMM of n outputs or by themselves. Needs no GPU."""
     plan = (ctypes.c_int * 2)()
-    if lib().qi_w4a4_quantize_plan(m, k, sms, plan) != 0:
+    if lib().qi_w4a4_quantize_plan(m, k, n, sms, plan) != 0:
         raise ValueError(f"no plan for {m} x {k}")
     return QuantizePlan(*plan)
 

@@ -532,6 +532,9 @@ W4A4Tiles choose_w4a4(const GemmShape &shape, int sms) {
     return prices[best].tiles;
 }
 
+// Whether the byte-operand GEMM of n outputs that comes next (n = 0: not known) takes any but tall tiles.
+bool narrow_w4a4(int m, int n, int k, int sms) { return m > 0 && n > 0 && k > 0 && choose_w4a4({m, n, k, n, 0}, sms) != W4A4_TALL; }
+
 int launch_w4a4_bytes(const void *a_bytes, const void *a_scales, const void *w_bytes, const void *w_scales, const float *bias,
                       void *y, const GemmShape &shape, cudaStream_t stream, int device) {
     switch (choose_w4a4(shape, sm_count(device))) {
@@ -838,8 +841,8 @@ int qi_w4a4_quantize_activations_ex(const void *x, int x_dtype, void *codes, voi
                                                         static_cast<cudaStream_t>(stream)));
 }
 
-int qi_w4a4_quantize_activations_wide_ex(const void *x, int x_dtype, void *codes, void *scales, void *bytes, int m,
-                                         int k, void *stream) {
+// next_n: outputs of the byte-operand GEMM behind it, 0 = not known.
+static int quantize_wide(const void *x, int x_dtype, void *codes, void *scales, void *bytes, int m, int k, int next_n, void *stream) {
     if (m < 0 || k <= 0 || k % 256 != 0) return INVALID;
     if (x_dtype != QI_DTYPE_F32 && x_dtype != QI_DTYPE_F16) return INVALID;
     if (m == 0) return 0;
@@ -847,12 +850,17 @@ int qi_w4a4_quantize_activations_wide_ex(const void *x, int x_dtype, void *codes
         (reinterpret_cast<uintptr_t>(scales) & 1))
         return INVALID;
     return static_cast<int>(launch_quantize_activations(x, x_dtype == QI_DTYPE_F16, codes, scales, bytes, m, k,
-                                                        static_cast<cudaStream_t>(stream)));
+                                                        static_cast<cudaStream_t>(stream), narrow_w4a4(m, next_n, k, quantize_sms())));
 }
 
-int qi_w4a4_quantize_plan(int m, int k, int sms, int *plan) {
-    if (m <= 0 || k <= 0 || k % 256 != 0 || sms < 2 || plan == nullptr) return INVALID;
-    const QuantizePlan chosen = plan_quantize(m, k, sms);
+int qi_w4a4_quantize_activations_wide_ex(const void *x, int x_dtype, void *codes, void *scales, void *bytes, int m,
+                                         int k, void *stream) {
+    return quantize_wide(x, x_dtype, codes, scales, bytes, m, k, 0, stream);
+}
+
+int qi_w4a4_quantize_plan(int m, int k, int n, int sms, int *plan) {
+    if (m <= 0 || k <= 0 || k % 256 != 0 || n < 0 || sms < 2 || plan == nullptr) return INVALID;
+    const QuantizePlan chosen = plan_quantize(m, k, sms, narrow_w4a4(m, n, k, sms));
     plan[0] = chosen.threads;
     plan[1] = chosen.smem_bytes;
     return 0;
@@ -1092,8 +1100,7 @@ static int linear_slice(const qi_packed_linear *record, int whole_n, const qi_li
         if (record->weights_wide != nullptr && work->wide != nullptr) {
             // one byte per code on both sides: no unpacking inside the GEMM
             if (!reuse_input) {
-                const int status = qi_w4a4_quantize_activations_wide_ex(input, input_dtype, work->codes, work->code_scales,
-                                                                        work->wide, rows, k, stream);
+                const int status = quantize_wide(input, input_dtype, work->codes, work->code_scales, work->wide, rows, k, n, stream);
                 if (status != 0) return status;
             }
             return qi_w4a4_gemm_wide_ex(work->wide, work->code_scales, record->weights_wide, record->scales, record->bias,

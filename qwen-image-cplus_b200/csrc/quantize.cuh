@@ -504,7 +504,10 @@ inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, voi
 //   from 48 to 222, eight warps: 600 x 3072 x 3072 (7200) 21.1 and 19.8, 1024 x 3072 x 3072 (12288) 29.8 and 28.6, 2048 x 9216 x 3072
 //     (24576) 120 and 118. From 222 on the two differ by less than they vary (3072 x 3072 x 3072 (36864) 65.2 and 64.5, 4096 x
 //     9216 x 3072 (49152) 226.9 and 228.6), although alone the one-chunk form is ahead up to 330 (36864: 12.1 and 11.5)
-// Between 21 and 48, and above, the paired form stays: 300 x 12288 x 4096 (4800) 54.8, in two warps 60.9.
+// Between 21 and 48, and above, the paired form stays: 300 x 12288 x 4096 (4800) 54.8, in two warps 60.9. It also stays up to 64, where its CTAs have
+// one round to do, in front of a byte-operand GEMM in narrow tiles: of 61 shapes eight warps made 54 slower, by 3 percent in the mean
+// (501 x 1248 x 4608 18.1 and 18.9, 600 x 1024 x 3072 14.2 and 15.0); in front of tall tiles all of 69 were faster (0.966), and in front
+// of a GEMM that widens its operands first 33 of 36, the others within 0.4 percent. A quantiser that is called by itself doesn't know what comes after it.
 // A CTA of one or two warps is given as much shared memory as one of eight. With what it uses (2.7 KB a warp) it is slower in front of
 // a GEMM whose CTAs take up most SMs: 50 x 9216 x 3072 11.3 us and then 12.6, 77 x 9216 x 3072 12.4 and 14.1, 170 x 3072 x 3072 11.4 and
 // 13.4; alone and in front of fewer CTAs it is the same. It isn't the split of an SM's memory into L1 and shared memory (asking the
@@ -513,13 +516,13 @@ inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, voi
 struct QuantizePlan {
     int threads, smem_bytes;
 };
-constexpr int ONE_WARP_TO = 8, TWO_WARPS_TO = 21, EIGHT_WARPS_FROM = 48, EIGHT_WARPS_TO = 222;
+constexpr int ONE_WARP_TO = 8, TWO_WARPS_TO = 21, EIGHT_WARPS_FROM = 48, EIGHT_WARPS_FROM_NARROW = 64, EIGHT_WARPS_TO = 222;
 
-inline QuantizePlan plan_quantize(int m, int k, int sms) {
+inline QuantizePlan plan_quantize(int m, int k, int sms, bool narrow_next) {
     const long long chunks = static_cast<long long>(m) * (k / 256), per_sm = (chunks + sms - 1) / sms;
     if (per_sm <= ONE_WARP_TO) return {32, CHUNK_CTA_BYTES};
     if (per_sm <= TWO_WARPS_TO) return {64, CHUNK_CTA_BYTES};
-    if (per_sm <= EIGHT_WARPS_FROM || per_sm > EIGHT_WARPS_TO) return {0, 0};
+    if (per_sm <= (narrow_next ? EIGHT_WARPS_FROM_NARROW : EIGHT_WARPS_FROM) || per_sm > EIGHT_WARPS_TO) return {0, 0};
     return {QUANT_THREADS, CHUNK_CTA_BYTES};
 }
 
@@ -531,9 +534,9 @@ inline cudaError_t launch_quantize_plain(const QuantizePlan &plan, const void *x
 }
 
 inline cudaError_t launch_quantize_activations(const void *x, int x_is_half, void *codes, void *scales, void *bytes,
-                                               int m, int k, cudaStream_t stream) {
+                                               int m, int k, cudaStream_t stream, bool narrow_next = false) {
     if (m == 0) return cudaSuccess;
-    const QuantizePlan plan = plan_quantize(m, k, quantize_sms());
+    const QuantizePlan plan = plan_quantize(m, k, quantize_sms(), narrow_next);
     if (x_is_half) return launch_quantize_plain<__half>(plan, x, codes, scales, bytes, m, k, stream);
     return launch_quantize_plain<float>(plan, x, codes, scales, bytes, m, k, stream);
 }
