@@ -500,7 +500,10 @@ inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, voi
 // The limits are chunks per SM. Microseconds of a linear on 148 SMs, the paired form first:
 //   to 8, one warp: 77 x 9216 x 3072 (924 chunks) 13.7 and 12.4, 50 x 12288 x 4096 (800) 23.5 and 22.4. 130 shapes: 0.90 of the
 //     time in the mean, one more than 1.01
-//   to 21, two warps: 170 x 3072 x 3072 (2040) 12.3 and 11.4; 130 shapes to 14: 0.93, one more than 1.01
+//   to 21, two warps: 170 x 3072 x 3072 (2040) 12.3 and 11.4; 130 shapes to 14: 0.93, one more than 1.01. From 14 on that holds for rows of up
+//     to 16 chunks (k = 4096; 94 shapes, none more than 1.005). Of 197 with longer rows 22 were slower by up to 12 percent (94 x 1504 x 6144
+//     13.7 and 15.2, 50 x 3072 x 12288 25.3 and 26.7): such calls take four warps with half as much memory again (12.7 and 25.4; 0.95 in
+//     the mean, one more than 1.01), which loses 1 to 4 percent where rows are shorter (300 x 3072 x 2048 12.6 and 13.0)
 //   from 48 to 222, eight warps: 600 x 3072 x 3072 (7200) 21.1 and 19.8, 1024 x 3072 x 3072 (12288) 29.8 and 28.6, 2048 x 9216 x 3072
 //     (24576) 120 and 118. From 222 on the two differ by less than they vary (3072 x 3072 x 3072 (36864) 65.2 and 64.5, 4096 x
 //     9216 x 3072 (49152) 226.9 and 228.6), although alone the one-chunk form is ahead up to 330 (36864: 12.1 and 11.5)
@@ -516,12 +519,13 @@ inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, voi
 struct QuantizePlan {
     int threads, smem_bytes;
 };
-constexpr int ONE_WARP_TO = 8, TWO_WARPS_TO = 21, EIGHT_WARPS_FROM = 48, EIGHT_WARPS_FROM_NARROW = 64, EIGHT_WARPS_TO = 222;
+constexpr int ONE_WARP_TO = 8, TWO_WARPS_TO = 21, TWO_WARPS_LONG_TO = 14, LONG_ROW = 4096, FOUR_WARPS_BYTES = 32768, EIGHT_WARPS_FROM = 48, EIGHT_WARPS_FROM_NARROW = 64, EIGHT_WARPS_TO = 222;
 
 inline QuantizePlan plan_quantize(int m, int k, int sms, bool narrow_next) {
     const long long chunks = static_cast<long long>(m) * (k / 256), per_sm = (chunks + sms - 1) / sms;
     if (per_sm <= ONE_WARP_TO) return {32, CHUNK_CTA_BYTES};
-    if (per_sm <= TWO_WARPS_TO) return {64, CHUNK_CTA_BYTES};
+    if (per_sm <= (k > LONG_ROW ? TWO_WARPS_LONG_TO : TWO_WARPS_TO)) return {64, CHUNK_CTA_BYTES};
+    if (per_sm <= TWO_WARPS_TO) return {128, FOUR_WARPS_BYTES};
     if (per_sm <= (narrow_next ? EIGHT_WARPS_FROM_NARROW : EIGHT_WARPS_FROM) || per_sm > EIGHT_WARPS_TO) return {0, 0};
     return {QUANT_THREADS, CHUNK_CTA_BYTES};
 }

@@ -169,6 +169,27 @@ def test_quantize_activations_at_the_limits_of_its_forms(qi, dtype):
         assert np.array_equal(codes.cpu().numpy(), expected_codes[:m])
 
 
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+def test_quantize_activations_in_ctas_of_four_warps(qi, dtype):
+    # the first and the last row count that long rows have it for (148 SMs), one beyond either, and CTAs whose last warps have no chunk
+    rng = np.random.default_rng(47)
+    for k, rows in ((4352, (121, 122, 182, 183)), (12288, (44, 47, 64))):
+        assert {qi.w4a4_quantize_plan(m, k).threads for m in rows[1:3]} == {128}
+        x = qt.make_activations(rng, rows[-1], k)
+        x = x if dtype == "f16" else x.astype(np.float32)
+        expected_codes, expected_scales = qo.quantize_activations(x)
+        source = up(x)
+        for m in rows:
+            codes, scales = torch.zeros(m, k // 2, dtype=torch.uint8, device="cuda"), torch.zeros(m, k // 64, dtype=torch.float16, device="cuda")
+            wide, nibbles = torch.zeros(m, k, dtype=torch.uint8, device="cuda"), torch.zeros(m, k, dtype=torch.uint8, device="cuda")
+            assert qi.w4a4_quantize_activations_wide_ex(source, qi.DTYPE_F32 if dtype == "f32" else qi.DTYPE_F16, codes, scales, wide, m, k) == 0
+            check_status(qi)
+            assert np.array_equal(half_bits(scales), expected_scales[:m])
+            assert np.array_equal(codes.cpu().numpy(), expected_codes[:m])
+            assert qi.w4a4_widen_codes_ex(codes, nibbles, m, k) == 0
+            assert torch.equal(wide, nibbles)
+
+
 def test_quantize_rejects_bad_shapes(qi):
     x = torch.zeros(4, 320, device="cuda")
     out = torch.zeros(4096, dtype=torch.uint8, device="cuda")

@@ -39,6 +39,24 @@ def test_one_round_of_the_paired_form_is_for_narrow_tiles_alone(qi):
         assert [qi.w4a4_quantize_plan(m, 4096, n=n).threads for n in (896, 3072, 0)] == [narrow, 256, 256]
 
 
+# Microseconds likewise with the paired form and with two and four warps a CTA.
+@pytest.mark.parametrize("shape,paired,two,four", [
+    ((94, 1504, 6144), 13.69, 15.16, 12.73), ((50, 3072, 12288), 25.3, 26.7, 25.4), ((116, 1024, 6144), 13.3, 14.8, 12.5), ((100, 6144, 6144), 20.9, 21.6, 20.1),
+    ((75, 6144, 8192), 24.2, 25.5, 23.5), ((68, 5216, 11264), 24.5, 26.7, 23.9), ((132, 1024, 5120), 12.05, 12.44, 11.05), ((86, 1120, 8704), 15.2, 16.6, 14.6),
+    ((300, 3072, 2048), 13.75, 12.6, 13.03), ((256, 1024, 3072), 10.89, 9.96, 10.36), ((200, 3072, 3072), 13.75, 12.93, 13.12), ((170, 3072, 3072), 12.3, 11.4, 11.9),
+], ids=str)
+def test_long_rows_take_more_warps(qi, shape, paired, two, four):
+    m, n, k = shape
+    chosen = {0: paired, 64: two, 128: four}[qi.w4a4_quantize_plan(m, k, n=n).threads]
+    assert chosen <= min(paired, two, four) * 1.015
+
+
+def test_the_limits_of_four_warps(qi):
+    # 14 and 21 chunks on each of 148 multiprocessors, in rows of 16 and of 17 chunks and of 256 inputs
+    for m, k, threads in ((129, 4096, 64), (194, 4096, 64), (195, 4096, 0), (121, 4352, 64), (122, 4352, 128), (182, 4352, 128), (183, 4352, 0)):
+        assert qi.w4a4_quantize_plan(m, k).threads == threads, (m, k)
+
+
 @pytest.mark.parametrize("m,k", [(0, 256), (1, 0), (1, 128), (-1, 256)])
 def test_no_plan_for_what_the_quantiser_refuses(qi, m, k):
     with pytest.raises(ValueError):
