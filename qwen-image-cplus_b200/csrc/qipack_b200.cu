@@ -102,7 +102,8 @@ bool make_map(CUtensorMap *map, CUtensorMapDataType type, int element_bytes, con
 
 // ---- tile selection -----------------------------------------------------------------------------
 
-// W4A16 tiles: 0 = choose by shape (never one of the others, which only qi_w4a16_gemm_tile_ex names); 1 = 128x128, 2 = 256x128, 3 = 128x256, 4 = 256x256, 5 = 256x256 on a pair of CTAs.
+// W4A16 tiles: 0 = choose by shape (never one of the others, which only qi_w4a16_gemm_tile_ex names); 1 = 128x128, 2 = 256x128,
+// 3 = 128x256, 4 = 256x256, 5 = 256x256 on a pair of CTAs.
 
 template <int NUM_M, int BN, int STAGES>
 int launch_w4a16(const void *x_half, const void *codes, const void *scales, const void *minimums, const float *bias,

@@ -17,8 +17,8 @@
 // matrix, a whole one or one in a group gives the same bits.
 //
 // What bounds it, 18432 x 3072 on cold weights: alone the first load, the copies (31.9 MB, 4.7 us) and the last tiles' steps;
-// in groups of 60 instructions and copies about alike (5.2 us a matrix; the copies alone 4.6).
-// What counted, in that order: shared memory by 32-bit addresses instead of generic pointers (76.0 -> 60.0 million
+// in groups of 60 instructions and copies about alike (5.0 us a matrix; the copies alone 4.6).
+// What counted, in that order: shared memory by 32-bit addresses instead of generic pointers (76.0 -> 61.2 million
 // warp instructions for sixteen matrices); a step of whole groups, which halves what a step spends on its scales; a warp
 // that does nothing but fetch, since a thread that unpacks held its team up while the copy engine took its requests; and
 // codes read without bank conflicts. Rows lie a multiple of 32 bytes apart, most often of 128, so the eight lanes that a

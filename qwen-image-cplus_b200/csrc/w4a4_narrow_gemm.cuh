@@ -2,8 +2,8 @@
 // or (EXCHANGED) 128 outputs x 16, 32 or 48 rows. Same
 // operator, arithmetic and bits as w4a4_pair_gemm.cuh (reference: qwen_image_cuda/cuda/gemm.cu:65-189).
 //
-// The groups of an output are added in order, so K cannot be split, and a tile is a chain of k / 64 hand-overs from the
-// tensor cores to the fold warps. With few rows, tiles of 256 leave most SMs idle or folding zeros; here 77 x 9216 outputs are
+// The groups of an output are added in order, so K cannot be split, and a tile is a chain of k / 256 hand-overs from the
+// tensor cores to the fold warps, of four groups each. With few rows, tiles of 256 leave most SMs idle or folding zeros; here 77 x 9216 outputs are
 // 144 tiles. What counts is the length of the chain's links:
 //   * a TMEM buffer holds four groups, one stage of 256 inputs: one commit, one look and one hand-back per four groups
 //   * two issuing warps take the stages in turn (an issuing warp needs some 500 cycles per turn)

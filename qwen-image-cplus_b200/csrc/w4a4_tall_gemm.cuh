@@ -296,8 +296,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             // written, which the fold warps still need for two slots' time. Four groups at a time, a row's 32-byte sector was
             // asked for four times, and where the rows of a tile are more than L1 keeps beside 190 KB of shared memory, from L2 each
             // time (without any of these loads 4096 x 3072 x 12288 took 288 us instead of 303): 4096 x 3072 x 12288 305 -> 297 us,
-            // 1024 x 12288 x 4096 108 -> 105, 4096 x 9216 x 3072 the same. Rows and columns that do not exist take the last one's:
-            // nothing reads what becomes of them.
+            // 1024 x 12288 x 4096 108 -> 105, 4096 x 9216 x 3072 the same. Where rows do not begin on sixteen bytes (an odd number of slots)
+            // each half is a load of its own, and 62 such GEMMs take 0.7 percent longer than with four groups at a time, up to 1.6 (1995 x 2976 x 3328
+            // 42.3 -> 42.9; one, 970 x 1504 x 5376, 3). A loop of its own for them made all shapes 1 to 2 percent slower, one loop of single slots
+            // for both 1 to 5: the fold warps feel every instruction here. Rows and columns that do not exist take the last one's: nothing
+            // reads what becomes of them.
             constexpr int SW_ITEMS = BN / 32, SA_ITEMS = BM / 32, ITEMS = SW_ITEMS + SA_ITEMS, LOWER = SA_ITEMS / HALVES;
             const bool whole = slots % 2 == 0 && ((reinterpret_cast<uintptr_t>(w_scales) | reinterpret_cast<uintptr_t>(a_scales)) & 15) == 0;
             uint32_t slot = 0, phase = 1;
