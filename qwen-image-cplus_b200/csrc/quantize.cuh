@@ -496,12 +496,12 @@ inline cudaError_t launch_quantize_chunks(const Source &source, void *codes, voi
                              smem_bytes, stream, source, static_cast<uint8_t *>(codes), static_cast<__half *>(scales), static_cast<uint8_t *>(bytes), chunks);
 }
 
-// Plain activations: CTAs of one, two or eight warps with a chunk a half-warp (threads), or the paired form (0).
+// Plain activations: CTAs of one, two, four or eight warps with a chunk a half-warp (threads), or the paired form (0).
 // The limits are chunks per SM. Microseconds of a linear on 148 SMs, the paired form first:
 //   to 8, one warp: 77 x 9216 x 3072 (924 chunks) 13.7 and 12.4, 50 x 12288 x 4096 (800) 23.5 and 22.4. 130 shapes: 0.90 of the
 //     time in the mean, one more than 1.01
 //   to 21, two warps: 170 x 3072 x 3072 (2040) 12.3 and 11.4; 130 shapes to 14: 0.93, one more than 1.01. From 14 on that holds for rows of up
-//     to 16 chunks (k = 4096; 94 shapes, none more than 1.005). Of 197 with longer rows 22 were slower by up to 12 percent (94 x 1504 x 6144
+//     to 16 chunks (k = 4096; 93 drawn shapes, none slower; 150 x 12288 x 4096 1.005). Of 197 with longer rows 22 were slower by up to 12 percent (94 x 1504 x 6144
 //     13.7 and 15.2, 50 x 3072 x 12288 25.3 and 26.7): such calls take four warps with half as much memory again (12.7 and 25.4; 0.95 in
 //     the mean, one more than 1.01), which loses 1 to 4 percent where rows are shorter (300 x 3072 x 2048 12.6 and 13.0)
 //   from 48 to 222, eight warps: 600 x 3072 x 3072 (7200) 21.1 and 19.8, 1024 x 3072 x 3072 (12288) 29.8 and 28.6, 2048 x 9216 x 3072
